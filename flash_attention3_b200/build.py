@@ -1,4 +1,5 @@
-"""Build recipe of the shared library (nvcc, sm_100a only, in-tree output).
+"""Build recipe of the shared library (nvcc, sm_100a only) and of the torch front end over it (host C++),
+both in-tree.
 
     python -m flash_attention3_b200.build            # build if sources are newer
     python -m flash_attention3_b200.build --force
@@ -14,6 +15,8 @@ PKG = pathlib.Path(__file__).resolve().parent
 ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libfa3bwd_b200.so"
+NATIVE = PKG / "_native.so"
+NATIVE_SOURCE = CSRC / "torch_native.cpp"
 SOURCES = [CSRC / "fa3_api.cpp", CSRC / "fa3_launch.cu"]
 HEADERS = sorted(CSRC.glob("*.h")) + sorted(CSRC.glob("*.cuh")) + sorted((ROOT / "include").glob("*.h"))
 
@@ -49,6 +52,44 @@ def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
     return LIB
 
 
+def build_native(force: bool = False) -> pathlib.Path:
+    """Compile the torch front end when missing or older than its sources; it is linked against the
+    library, which is built first."""
+    build()
+    newest = max(p.stat().st_mtime for p in [NATIVE_SOURCE, *(ROOT / "include").glob("*.h")])
+    if not force and NATIVE.exists() and NATIVE.stat().st_mtime >= newest:
+        return NATIVE
+    import sysconfig
+    from torch.utils import cpp_extension
+    cuda = pathlib.Path(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc").resolve().parent.parent
+    includes = [ROOT / "include", *cpp_extension.include_paths(), sysconfig.get_paths()["include"], cuda / "include"]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", *(f"-I{p}" for p in includes), str(NATIVE_SOURCE),
+           "-o", str(NATIVE), f"-L{PKG}", f"-l:{LIB.name}", *(f"-L{p}" for p in cpp_extension.library_paths()), "-ltorch_python", "-ltorch", "-ltorch_cpu",
+           "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
+    proc = subprocess.run(cmd, capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + (proc.stdout + proc.stderr)[-4000:])
+    return NATIVE
+
+
+_native = None
+
+
+def load_native():
+    """The compiled torch front end (built when missing; there is no Python fallback)."""
+    global _native
+    if _native is None:
+        import importlib.util
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        if not NATIVE.exists() or not LIB.exists():
+            build_native()
+        spec = importlib.util.spec_from_file_location(__package__ + "._native", NATIVE)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _native = module
+    return _native
+
+
 def ptxas_report() -> list[dict]:
     """Per-kernel registers / spills from the last build log (no-spill gate)."""
     import re
@@ -68,5 +109,6 @@ def ptxas_report() -> list[dict]:
 
 
 if __name__ == "__main__":
-    path = build(force="--force" in sys.argv, verbose="-v" in sys.argv)
-    print(path)
+    force = "--force" in sys.argv
+    print(build(force=force, verbose="-v" in sys.argv))
+    print(build_native(force=force))

@@ -1,4 +1,5 @@
-"""Tensor-level wrapper over the C ABI (torch provides device memory only)."""
+"""Tensor-level wrapper over the C ABI (torch provides device memory only).  The checks of a call, its
+allocations and its parameter block are native (csrc/torch_native.cpp)."""
 from __future__ import annotations
 
 import ctypes
@@ -6,7 +7,9 @@ import math
 
 import torch
 
-from . import capi
+from . import build, capi
+
+_native = build.load_native()
 
 _DTYPES = {torch.float16: capi.DTYPE_FP16, torch.bfloat16: capi.DTYPE_BF16}
 
@@ -64,39 +67,11 @@ def make_params(q: torch.Tensor, k: torch.Tensor, causal: bool, softmax_scale=No
     return p
 
 
-def _require_cuda(*tensors):
-    for t in tensors:
-        if t is not None and not t.is_cuda:
-            raise RuntimeError("flash_attention3_b200 has no CPU path: tensors must live on a CUDA device")
-        if t is not None and not t.is_contiguous():
-            raise RuntimeError("contiguous tensors are required ([B,H,S,D] or [B,S,H,D])")
-
-
-def _check_problem(q, k, v, layout, out=None, dout=None, softmax_lse=None):
-    """Shapes, dtypes and devices of one fixed-length problem: the C ABI takes raw pointers, so a
-    tensor of the wrong size would be read or written out of bounds."""
-    if q.dim() != 4 or k.dim() != 4:
-        raise ValueError("q and k must be 4-D ([B,H,S,D] or [B,S,H,D])")
-    if q.dtype not in _DTYPES:
-        raise TypeError(f"unsupported dtype {q.dtype}: fp16 or bf16")
-    if v.shape != k.shape:
-        raise ValueError(f"v {tuple(v.shape)} must have the shape of k {tuple(k.shape)}")
-    hq, hkv = (q.shape[2], k.shape[2]) if layout == "bshd" else (q.shape[1], k.shape[1])
-    sq = q.shape[1] if layout == "bshd" else q.shape[2]
-    if q.shape[0] != k.shape[0] or q.shape[3] != k.shape[3] or hkv == 0 or hq % hkv != 0:
-        raise ValueError(f"q {tuple(q.shape)} and k {tuple(k.shape)} do not describe one problem")
-    for name, t in (("k", k), ("v", v), ("out", out), ("dout", dout)):
-        if t is None:
-            continue
-        if t.dtype != q.dtype or t.device != q.device:
-            raise TypeError(f"{name} must have the dtype and device of q")
-        if name in ("out", "dout") and t.shape != q.shape:
-            raise ValueError(f"{name} {tuple(t.shape)} must have the shape of q {tuple(q.shape)}")
-    if softmax_lse is not None:
-        if softmax_lse.dtype != torch.float32 or softmax_lse.device != q.device:
-            raise TypeError("softmax_lse must be fp32 on the device of q")
-        if tuple(softmax_lse.shape) != (q.shape[0], hq, sq):
-            raise ValueError(f"softmax_lse {tuple(softmax_lse.shape)} must be [B,Hq,Sq] = {(q.shape[0], hq, sq)}")
+def _result(r):
+    """What a native call returned: its tensors, or (entry, status) when the C ABI refused the call."""
+    if type(r[0]) is str:
+        raise Fa3Error(*r)
+    return r
 
 
 def fa3_bwd(dout, q, k, v, out, softmax_lse, causal: bool, softmax_scale=None, deterministic=False,
@@ -112,95 +87,26 @@ def fa3_bwd(dout, q, k, v, out, softmax_lse, causal: bool, softmax_scale=None, d
     gradient rows behind them are zero.  outputs = (dq, dk, dv): write into these tensors instead of
     allocating.  Calls shaobo_fa3_bwd_v2.
     """
-    _require_cuda(dout, q, k, v, out, softmax_lse)
-    _check_problem(q, k, v, layout, out, dout, softmax_lse)
-    lib = capi.load()
-    p = make_params(q, k, causal, softmax_scale, layout=layout, seqused_q=seqused_q, seqused_k=seqused_k,
-                    softcap=float(softcap), deterministic=int(deterministic),
-                    sync_after_launch=int(sync), window_left=int(window[0]), window_right=int(window[1]))
-    need = lib.shaobo_fa3_bwd_v2_workspace_bytes(ctypes.byref(p))
-    if need == 0:
-        raise Fa3Error("shaobo_fa3_bwd_v2_validate", lib.shaobo_fa3_bwd_v2_validate(ctypes.byref(p)))
-    if workspace is None or workspace.numel() * workspace.element_size() < need:
-        workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
-    p.workspace = workspace.data_ptr()
-    p.workspace_bytes = workspace.numel() * workspace.element_size()
-    if outputs is None:
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    else:
-        dq, dk, dv = outputs
-        _require_cuda(dq, dk, dv)
-        for t, like in ((dq, q), (dk, k), (dv, v)):
-            if t.shape != like.shape or t.dtype != like.dtype or t.device != like.device:
-                raise ValueError("outputs must match q, k, v in shape, dtype and device")
-    delta = (torch.empty((p.batch, p.num_heads_q, p.seqlen_q), dtype=torch.float32, device=q.device)
-             if return_delta else None)
-    with torch.cuda.device(q.device):
-        p.reserved_ptr[capi.RESERVED_PTR_STREAM] = torch.cuda.current_stream().cuda_stream or None
-        code = lib.shaobo_fa3_bwd_v2(_ptr(dout), _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(softmax_lse),
-                                     _ptr(dq), _ptr(dk), _ptr(dv), _ptr(delta), ctypes.byref(p))
-    if code != capi.STATUS_SUCCESS:
-        raise Fa3Error("shaobo_fa3_bwd_v2", code)
+    r = _result(_native.bwd(dout, q, k, v, out, softmax_lse, causal, softmax_scale, deterministic, workspace, return_delta,
+                            sync, layout, window, seqused_q, seqused_k, outputs, softcap))
     if sync:
-        _raise_on_device_error(lib, "shaobo_fa3_bwd_v2")
-    return (dq, dk, dv, delta) if return_delta else (dq, dk, dv)
+        _raise_on_device_error(capi.load(), "shaobo_fa3_bwd_v2")
+    return r
 
 
 def fa3_fwd(q, k, v, causal: bool, softmax_scale=None, layout: str = "bhsd", window=(-1, -1), sync=False,
             seqused_q=None, seqused_k=None, softcap: float = 0.0):
     """out, softmax_lse = forward of softmax(q k^T * scale) v (shaobo_fa3_b200_fwd).  Shapes, layouts,
     masks as in fa3_bwd; softmax_lse is fp32 [B,Hq,Sq] natural log."""
-    _require_cuda(q, k, v)
-    _check_problem(q, k, v, layout)
-    lib = capi.load()
-    p = make_params(q, k, causal, softmax_scale, layout=layout, seqused_q=seqused_q, seqused_k=seqused_k,
-                    softcap=float(softcap), sync_after_launch=int(sync),
-                    window_left=int(window[0]), window_right=int(window[1]))
-    out = torch.empty_like(q)
-    lse = torch.empty((p.batch, p.num_heads_q, p.seqlen_q), dtype=torch.float32, device=q.device)
-    with torch.cuda.device(q.device):
-        p.reserved_ptr[capi.RESERVED_PTR_STREAM] = torch.cuda.current_stream().cuda_stream or None
-        code = lib.shaobo_fa3_b200_fwd(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), ctypes.byref(p))
-    if code != capi.STATUS_SUCCESS:
-        raise Fa3Error("shaobo_fa3_b200_fwd", code)
-    return out, lse
-
-
-def _varlen_params(q, k, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, causal, softmax_scale, window,
-                   **extra) -> capi.Params:
-    if cu_seqlens_q.dtype != torch.int32 or cu_seqlens_k.dtype != torch.int32:
-        raise TypeError("cu_seqlens must be int32")
-    total_q, hq, d = q.shape
-    total_k, hkv, _ = k.shape
-    p = capi.new_params(batch=cu_seqlens_q.numel() - 1, seqlen_q=int(max_seqlen_q), seqlen_k=int(max_seqlen_k),
-                        num_heads_q=hq, num_heads_kv=hkv, head_dim_qk=d, head_dim_v=d, causal=int(causal),
-                        dtype=_DTYPES[q.dtype], layout=capi.LAYOUT_BSHD,
-                        window_left=int(window[0]), window_right=int(window[1]),
-                        cu_seqlens_q=cu_seqlens_q.data_ptr(), cu_seqlens_k=cu_seqlens_k.data_ptr(),
-                        max_seqlen_q=int(max_seqlen_q), max_seqlen_k=int(max_seqlen_k),
-                        total_q=int(total_q), total_k=int(total_k), **extra)
-    if softmax_scale is not None:
-        p.softmax_scale = float(softmax_scale)
-        p.softmax_scale_is_set = 1
-    return p
+    return _result(_native.fwd(q, k, v, causal, softmax_scale, layout, window, sync, seqused_q, seqused_k, softcap))
 
 
 def fa3_fwd_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q: int, max_seqlen_k: int, causal: bool,
                    softmax_scale=None, window=(-1, -1), sync=False):
     """Forward over packed sequences: q [total_q,Hq,D], k/v [total_k,Hkv,D] -> out [total_q,Hq,D],
     softmax_lse fp32 [Hq,total_q]."""
-    _require_cuda(q, k, v, cu_seqlens_q, cu_seqlens_k)
-    lib = capi.load()
-    p = _varlen_params(q, k, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, causal, softmax_scale,
-                       window, sync_after_launch=int(sync))
-    out = torch.empty_like(q)
-    lse = torch.empty((q.shape[1], q.shape[0]), dtype=torch.float32, device=q.device)
-    with torch.cuda.device(q.device):
-        p.reserved_ptr[capi.RESERVED_PTR_STREAM] = torch.cuda.current_stream().cuda_stream or None
-        code = lib.shaobo_fa3_b200_fwd(_ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(lse), ctypes.byref(p))
-    if code != capi.STATUS_SUCCESS:
-        raise Fa3Error("shaobo_fa3_b200_fwd", code)
-    return out, lse
+    return _result(_native.fwd_packed(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, causal,
+                                      softmax_scale, window, sync))
 
 
 def fa3_bwd_varlen(dout, q, k, v, out, softmax_lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q: int,
@@ -209,27 +115,11 @@ def fa3_bwd_varlen(dout, q, k, v, out, softmax_lse, cu_seqlens_q, cu_seqlens_k, 
     """Backward over packed sequences.  q, out, dout: [total_q, Hq, D]; k, v: [total_k, Hkv, D];
     softmax_lse: fp32 [Hq, total_q]; cu_seqlens_*: int32 device tensors of batch+1 row offsets.
     Returns dq, dk, dv in the shapes of q, k, v (and delta [Hq, total_q]).  Calls shaobo_fa3_bwd_v2."""
-    _require_cuda(dout, q, k, v, out, softmax_lse, cu_seqlens_q, cu_seqlens_k)
-    lib = capi.load()
-    total_q, hq = q.shape[0], q.shape[1]
-    p = _varlen_params(q, k, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, causal, softmax_scale,
-                       window, deterministic=int(deterministic), sync_after_launch=int(sync))
-    need = lib.shaobo_fa3_bwd_v2_workspace_bytes(ctypes.byref(p))
-    if need == 0:
-        raise Fa3Error("shaobo_fa3_bwd_v2_validate", lib.shaobo_fa3_bwd_v2_validate(ctypes.byref(p)))
-    workspace = torch.empty(need, dtype=torch.uint8, device=q.device)
-    p.workspace, p.workspace_bytes = workspace.data_ptr(), need
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    delta = torch.empty((hq, total_q), dtype=torch.float32, device=q.device) if return_delta else None
-    with torch.cuda.device(q.device):
-        p.reserved_ptr[capi.RESERVED_PTR_STREAM] = torch.cuda.current_stream().cuda_stream or None
-        code = lib.shaobo_fa3_bwd_v2(_ptr(dout), _ptr(q), _ptr(k), _ptr(v), _ptr(out), _ptr(softmax_lse),
-                                     _ptr(dq), _ptr(dk), _ptr(dv), _ptr(delta), ctypes.byref(p))
-    if code != capi.STATUS_SUCCESS:
-        raise Fa3Error("shaobo_fa3_bwd_v2", code)
+    r = _result(_native.bwd_packed(dout, q, k, v, out, softmax_lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
+                                   causal, softmax_scale, deterministic, window, return_delta, sync))
     if sync:
-        _raise_on_device_error(lib, "shaobo_fa3_bwd_v2")
-    return (dq, dk, dv, delta) if return_delta else (dq, dk, dv)
+        _raise_on_device_error(capi.load(), "shaobo_fa3_bwd_v2")
+    return r
 
 
 class HostBackward:

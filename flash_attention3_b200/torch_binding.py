@@ -15,44 +15,30 @@ from __future__ import annotations
 
 import torch
 
-from . import ops
+from . import build, ops
+
+_native = build.load_native()  # registers the two ops (csrc/torch_native.cpp): schema, CUDA kernels
+
+attention_bwd = torch.ops.fa3b200.attention_bwd.default
+attention_fwd = torch.ops.fa3b200.attention_fwd.default
 
 
-@torch.library.custom_op("fa3b200::attention_bwd", mutates_args=(), device_types="cuda")
-def attention_bwd(dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor,
-                  softmax_lse: torch.Tensor, causal: bool, softmax_scale: float,
-                  deterministic: bool, window_left: int = -1, window_right: int = -1, softcap: float = 0.0,
-                  layout: str = "bhsd") -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-    # (the kernels read dense tensors: strided views are copied, as in the forward op)
-    dq, dk, dv = ops.fa3_bwd(dout.contiguous(), q.contiguous(), k.contiguous(), v.contiguous(), out.contiguous(),
-                             softmax_lse.contiguous(), causal, softmax_scale, deterministic=deterministic,
-                             window=(window_left, window_right), softcap=softcap, layout=layout)
-    return dq, dk, dv
-
-
-@attention_bwd.register_fake
+@torch.library.register_fake("fa3b200::attention_bwd")
 def _(dout, q, k, v, out, softmax_lse, causal, softmax_scale, deterministic, window_left=-1, window_right=-1,
       softcap=0.0, layout="bhsd"):
     # dense outputs whatever the strides of the inputs, like the real op
     return q.new_empty(q.shape), k.new_empty(k.shape), v.new_empty(v.shape)
 
 
-@torch.library.custom_op("fa3b200::attention_fwd", mutates_args=(), device_types="cuda")
-def attention_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool, softmax_scale: float,
-                  window_left: int = -1, window_right: int = -1, softcap: float = 0.0,
-                  layout: str = "bhsd") -> tuple[torch.Tensor, torch.Tensor]:
-    out, lse = ops.fa3_fwd(q.contiguous(), k.contiguous(), v.contiguous(), causal, softmax_scale,
-                           window=(window_left, window_right), softcap=softcap, layout=layout)
-    return out, lse
-
-
-@attention_fwd.register_fake
+@torch.library.register_fake("fa3b200::attention_fwd")
 def _(q, k, v, causal, softmax_scale, window_left=-1, window_right=-1, softcap=0.0, layout="bhsd"):
     b, h, s = (q.shape[0], q.shape[2], q.shape[1]) if layout == "bshd" else q.shape[:3]
     return q.new_empty(q.shape), q.new_empty((b, h, s), dtype=torch.float32)
 
 
 class _Attention(torch.autograd.Function):
+    """The autograd function as a tracer sees it; eager calls go through its C++ twin."""
+
     @staticmethod
     def forward(ctx, q, k, v, causal, softmax_scale, deterministic, window, softcap, layout):
         scale = softmax_scale if softmax_scale is not None else ops.default_scale(q.shape[-1])
@@ -77,4 +63,6 @@ class _Attention(torch.autograd.Function):
 def attention(q, k, v, causal: bool = False, softmax_scale: float | None = None, deterministic: bool = False,
               window=(-1, -1), softcap: float = 0.0, layout: str = "bhsd"):
     """softmax(q k^T * scale) v with this library's forward and backward behind autograd."""
+    if not torch.compiler.is_compiling():
+        return _native.attention(q, k, v, causal, softmax_scale, deterministic, window, softcap, layout)
     return _Attention.apply(q, k, v, causal, softmax_scale, deterministic, tuple(window), float(softcap), layout)

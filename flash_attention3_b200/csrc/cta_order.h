@@ -148,4 +148,44 @@ inline CtaOrderPlan plan_cta_order(int n_tiles, int bh_count, int group, bool ca
     return plan_cta_order(TileWork::square(n_tiles, causal), bh_count, group, sms, dq_bytes_per_head);
 }
 
+// How many CTAs (a cluster of 1, 2, 4 or 8) share the key tiles of a pair of query tiles in the forward.
+// Pairs are launched heaviest first when the mask makes them unequal; a cluster needs its SMs at the same
+// time, so the model hands the pairs to sms / splits gangs as these free up.  A CTA costs its key tiles plus
+// what corresponds to 3 of them (set-up, first loads, pipeline fill, output), and a split one 3 more (partial
+// outputs exchanged through distributed shared memory).  The fewest CTAs within 3 % of the best are taken.
+// us per call, one against the planned number: S=2048, 4 heads, D=128 causal 33.1 and 18.0; S=1024, 1 head 19.2
+// and 13.2; 300 queries x 8000 keys, 2 heads 156 and 24; S=512, 1 head 12.5 and 13.4 (not split).
+inline int plan_fwd_splits(const Band& band, long long bh_count, int sms) {
+    const int pairs = (tiles_of(band.seqlen_q) + 1) / 2;
+    if (pairs * bh_count > 8LL * sms) return 1;  // many waves: nothing stands idle for long
+    int best = 1;
+    long long best_cost = -1;
+    for (int splits = 1; splits <= 8; splits *= 2) {
+        std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free_at;
+        for (int i = 0; i < sms / splits; ++i) free_at.push(0);
+        long long makespan = 0;
+        for (int pair = pairs - 1; pair >= 0; --pair) {
+            int first = kUnbounded, last = -1;
+            for (int qt = 2 * pair; qt < 2 * pair + 2 && qt < tiles_of(band.seqlen_q); ++qt) {
+                if (k_tiles_of_q_tile(qt, band) == 0) continue;
+                first = std::min(first, first_k_tile(qt, band));
+                last = std::max(last, last_k_tile(qt, band));
+            }
+            const int tiles = last >= first ? last - first + 1 : 0;
+            const long long cost = 3 + (splits > 1 ? 3 : 0) + (tiles + splits - 1) / splits;
+            for (long long i = 0; i < bh_count; ++i) {
+                const long long end = free_at.top() + cost;
+                free_at.pop();
+                free_at.push(end);
+                makespan = std::max(makespan, end);
+            }
+        }
+        if (best_cost < 0 || makespan * 103 < best_cost * 100) {
+            best_cost = makespan;
+            best = splits;
+        }
+    }
+    return best;
+}
+
 }  // namespace fa3b200

@@ -98,8 +98,8 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     auto bar = [&](int i) -> uint32_t { return sbase + C::kOffBar + 8 * i; };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::kOffBar + 8 * kDqbNum);
-    volatile uint32_t* abort_flag = tmem_slot + 1;
+    const uint32_t tmem_slot = sbase + C::kOffBar + 8 * kDqbNum;
+    const uint32_t abort_flag = tmem_slot + 4;
 
     const int n_q_tiles = tiles_of(a.band.seqlen_q);  // of the longest sequence
     const int bh_count = a.batch * a.heads_q;
@@ -144,17 +144,17 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         ptx::mbar_init(bar(kDqbSFree), 128);
         ptx::mbar_init(bar(kDqbDsReady), 128);
         ptx::mbar_init(bar(kDqbDone), 1);
-        *abort_flag = 0;
+        flag_set(abort_flag, 0);
         ptx::fence_mbar_init();
     }
     if (warp == 1) {
-        ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), C::kTmemCols);
+        ptx::tmem_alloc(tmem_slot, C::kTmemCols);
         ptx::tmem_relinquish();
     }
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = flag_value(tmem_slot);
     const int q_row = qt * C::kTile;  // row inside the head
 
     if (!misaligned) {
@@ -186,33 +186,23 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                 }
             }
         } else if (warp == 1) {
-            // MMA issuer: the whole warp runs the role converged; the lean issue forms and the commits
+            // MMA issuer: the whole warp runs the role converged; the issue forms and the commits
             // elect their lane inside the asm (a lone divergent lane is starved by the math warps).
             {
                 constexpr uint32_t kIdSdP = ptx::instr_desc_f16(kBf16, 128, 128, false, false);
                 constexpr uint32_t kIdDq = ptx::instr_desc_f16(kBf16, 128, D, false, true);
-                constexpr uint32_t kHi = ptx::kDescHiSw128;
-                constexpr uint32_t kBoxStep = C::kBoxBytes >> 4;
-                auto k_step = [](int kk) -> uint32_t { return uint32_t(kk >> 2) * kBoxStep + uint32_t(kk & 3) * 2u; };
-                auto mn_step = [](int kk) -> uint32_t { return uint32_t(kk) * 128u; };
                 const uint32_t loQ = ptx::desc_lo_k_major(sbase + C::kOffQ);
                 const uint32_t loDO = ptx::desc_lo_k_major(sbase + C::kOffDO);
                 auto sK = [&](int t) { return sbase + C::kOffK + (t & 1) * C::kOperandBytes; };
                 auto sV = [&](int t) { return sbase + C::kOffV + (t & 1) * C::kOperandBytes; };
                 auto issue_s = [&](int t) {
                     const uint32_t loK = ptx::desc_lo_k_major(sK(t));
-                    ptx::mma_ss_lean<false>(tmem + C::kColS, loQ, loK, kHi, kIdSdP);
-#pragma unroll
-                    for (int kk = 1; kk < D / 16; ++kk)
-                        ptx::mma_ss_lean<true>(tmem + C::kColS, loQ + k_step(kk), loK + k_step(kk), kHi, kIdSdP);
+                    ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(tmem + C::kColS, loQ, loK, kIdSdP, 0);
                     ptx::tc_commit_elect(bar(kDqbSFull));
                 };
                 auto issue_dp = [&](int t) {
                     const uint32_t loV = ptx::desc_lo_k_major(sV(t));
-                    ptx::mma_ss_lean<false>(tmem + C::kColDP, loDO, loV, kHi, kIdSdP);
-#pragma unroll
-                    for (int kk = 1; kk < D / 16; ++kk)
-                        ptx::mma_ss_lean<true>(tmem + C::kColDP, loDO + k_step(kk), loV + k_step(kk), kHi, kIdSdP);
+                    ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(tmem + C::kColDP, loDO, loV, kIdSdP, 0);
                     ptx::tc_commit_elect(bar(kDqbDpFull));
                 };
                 bool ok = n_steps > 0 && warp_wait<false>(bar(kDqbQFull), 0, abort_flag) &&
@@ -236,10 +226,7 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     ptx::tc_fence_after();
                     {
                         const uint32_t loK = ptx::desc_lo_mn_major(sK(t), C::kBoxBytes);
-                        ptx::mma_ts_lean_rt(tmem + C::kColDQ, tmem + C::kColDP, loK, kHi, kIdDq, t > 0 ? 1u : 0u);
-#pragma unroll
-                        for (int kk = 1; kk < 8; ++kk)
-                            ptx::mma_ts_lean<true>(tmem + C::kColDQ, tmem + C::kColDP + kk * 8, loK + mn_step(kk), kHi, kIdDq);
+                        ptx::mma_ts_8<ptx::TmemPacked, ptx::MnMajor>(tmem + C::kColDQ, tmem + C::kColDP, loK, kIdDq, t > 0 ? 1u : 0u);
                     }
                     if (more) issue_dp(t + 1);  // after dQ(t) in issue order: dS(t) is consumed first
                     ptx::tc_commit_elect(bar(kDqbKvEmpty + (t & 1)));

@@ -138,6 +138,17 @@ CtaOrderPlan cached_plan(const TileWork& work, int bh, int group, int sms, long 
     return plan;
 }
 
+int cached_fwd_splits(const Band& band, int64_t bh, int sms) {
+    static std::mutex mu;
+    static std::map<std::tuple<int, int, int, int, int64_t, int>, int> cache;
+    const auto key = std::make_tuple(band.seqlen_q, band.seqlen_k, band.left, band.right, bh, sms);
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = cache.find(key);
+    if (it != cache.end()) return it->second;
+    if (cache.size() > 4096) cache.clear();
+    return cache[key] = plan_fwd_splits(band, bh, sms);
+}
+
 // Remembers, per CUDA device, that a one-time set-up step has been done
 // (function attributes are per device).
 struct DeviceOnce {
@@ -607,9 +618,14 @@ int launch_dq(const ShaoboFa3Params* p, const void* dout, const void* q, const v
 }
 
 // ---------------------------------------------------------- forward kernel
+struct FwdLaunch {
+    CUtensorMap mq, mk, mv, mo;
+    FwdArgs args;
+    int blocks;
+};
+
 template <typename T, int D, bool kMasked, bool kSoftcap = false>
-int launch_fwd_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                 const FwdArgs& args, int blocks, cudaStream_t st) {
+int launch_fwd_t(const FwdLaunch& L, cudaStream_t st) {
     auto kernel = fwd_kernel<T, D, kMasked, kSoftcap>;
     static DeviceOnce configured;
     if (!configured.done()) {
@@ -619,25 +635,35 @@ int launch_fwd_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap
         }
         configured.mark();
     }
-    kernel<<<blocks, FwdCfg<D>::kThreads, FwdCfg<D>::kSmemBytes, st>>>(mq, mk, mv, args);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(L.blocks));
+    cfg.blockDim = dim3(FwdCfg<D>::kThreads);
+    cfg.dynamicSmemBytes = FwdCfg<D>::kSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // set-up overlaps the kernel in front
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = unsigned(L.args.splits);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = L.args.splits > 1 ? 2 : 1;
+    if (cudaLaunchKernelEx(&cfg, kernel, L.mq, L.mk, L.mv, L.mo, L.args) != cudaSuccess) return SHAOBO_FA3_STATUS_HIP_ERROR;
     return SHAOBO_FA3_STATUS_SUCCESS;
 }
 
 template <typename T>
-int launch_fwd_d(const ShaoboFa3Params* p, const CUtensorMap& mq, const CUtensorMap& mk,
-                 const CUtensorMap& mv, const FwdArgs& args, int blocks) {
+int launch_fwd_d(const ShaoboFa3Params* p, const FwdLaunch& L) {
     cudaStream_t st = stream_of(p);
     const bool masked = needs_general_form(p);
     if (p->softcap > 0.0f) {
-        return p->head_dim_qk == 128 ? launch_fwd_t<T, 128, true, true>(mq, mk, mv, args, blocks, st)
-                                     : launch_fwd_t<T, 64, true, true>(mq, mk, mv, args, blocks, st);
+        return p->head_dim_qk == 128 ? launch_fwd_t<T, 128, true, true>(L, st) : launch_fwd_t<T, 64, true, true>(L, st);
     }
     if (p->head_dim_qk == 128) {
-        return masked ? launch_fwd_t<T, 128, true>(mq, mk, mv, args, blocks, st)
-                      : launch_fwd_t<T, 128, false>(mq, mk, mv, args, blocks, st);
+        return masked ? launch_fwd_t<T, 128, true>(L, st) : launch_fwd_t<T, 128, false>(L, st);
     }
-    return masked ? launch_fwd_t<T, 64, true>(mq, mk, mv, args, blocks, st)
-                  : launch_fwd_t<T, 64, false>(mq, mk, mv, args, blocks, st);
+    return masked ? launch_fwd_t<T, 64, true>(L, st) : launch_fwd_t<T, 64, false>(L, st);
 }
 
 int launch_fwd(const ShaoboFa3Params* p, const void* q, const void* k, const void* v, void* out,
@@ -646,13 +672,14 @@ int launch_fwd(const ShaoboFa3Params* p, const void* q, const void* k, const voi
     const CUtensorMapDataType type = bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const int d = p->head_dim_qk;
     const TensorShape shape = shape_of(p);
-    CUtensorMap mq, mk, mv;
-    if (!make_map_16(&mq, type, q, shape.batch, p->num_heads_q, shape.rows_q, d, shape.bshd) ||
-        !make_map_16(&mk, type, k, shape.batch, p->num_heads_kv, shape.rows_k, d, shape.bshd) ||
-        !make_map_16(&mv, type, v, shape.batch, p->num_heads_kv, shape.rows_k, d, shape.bshd)) {
+    FwdLaunch L;
+    if (!make_map_16(&L.mq, type, q, shape.batch, p->num_heads_q, shape.rows_q, d, shape.bshd) ||
+        !make_map_16(&L.mk, type, k, shape.batch, p->num_heads_kv, shape.rows_k, d, shape.bshd) ||
+        !make_map_16(&L.mv, type, v, shape.batch, p->num_heads_kv, shape.rows_k, d, shape.bshd) ||
+        !make_map_16(&L.mo, type, out, shape.batch, p->num_heads_q, shape.rows_q, d, shape.bshd, 32)) {
         return SHAOBO_FA3_STATUS_HIP_ERROR;
     }
-    FwdArgs args;
+    FwdArgs& args = L.args;
     args.out = out;
     args.lse = lse;
     args.o_strides = strides_of(shape.bshd, p->num_heads_q, shape.rows_q, d);
@@ -665,14 +692,17 @@ int launch_fwd(const ShaoboFa3Params* p, const void* q, const void* k, const voi
     args.seqused_q = p->seqused_q;
     args.seqused_k = p->seqused_k;
     args.lse_rows = shape.rows_q;
-    args.scale_log2 = p->softmax_scale * kLog2E;
+    args.scale_log2 = std::max(p->softmax_scale * kLog2E, 1e-30f);  // (a scale of 0 would turn a masked -inf into NaN)
     args.softcap_pre = p->softcap > 0.0f ? p->softmax_scale / p->softcap : 0.0f;
     args.softcap_post = p->softcap * kLog2E;
-    // one CTA per pair of query tiles
-    const int64_t blocks64 = int64_t((tiles_of(plan_seqlen_q(p)) + 1) / 2) * p->batch * p->num_heads_q;
+    args.staged_store = is_varlen(p) ? 0 : 1;
+    // one CTA per pair of query tiles, or a cluster of `splits` of them
+    const int64_t units = int64_t((tiles_of(plan_seqlen_q(p)) + 1) / 2) * p->batch * p->num_heads_q;
+    args.splits = cached_fwd_splits(args.band, int64_t(p->batch) * p->num_heads_q, sm_count());
+    const int64_t blocks64 = units * args.splits;
     if (blocks64 > 0x7fffffffLL) return SHAOBO_FA3_STATUS_UNSUPPORTED;
-    return bf ? launch_fwd_d<__nv_bfloat16>(p, mq, mk, mv, args, int(blocks64))
-              : launch_fwd_d<__half>(p, mq, mk, mv, args, int(blocks64));
+    L.blocks = int(blocks64);
+    return bf ? launch_fwd_d<__nv_bfloat16>(p, L) : launch_fwd_d<__half>(p, L);
 }
 
 bool stage_params_ok(const ShaoboFa3Params* p) {

@@ -199,18 +199,27 @@ enum Bar : int {
     kNumBars = 18,
 };
 
-constexpr long long kWaitTimeoutCycles = 2000000000LL;  // about one second
+constexpr uint32_t kWaitTimeoutCycles = 2000000000u;  // about one second, of a 32-bit cycle counter
 
-// Bounded mbarrier wait.  Returns false when the wait timed out here or was
-// abandoned because another thread of the CTA timed out.
+// Bounded mbarrier wait of a single thread (the TMA producer).  Returns false when the wait timed out
+// here or was abandoned because another thread of the CTA timed out (abort_flag: its shared-memory address).
+__device__ __forceinline__ uint32_t flag_value(uint32_t flag) {
+    uint32_t v;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(v) : "r"(flag) : "memory");
+    return v;
+}
+__device__ __forceinline__ void flag_set(uint32_t flag, uint32_t v) {
+    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(flag), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t clock_lo() {
+    uint32_t c;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
+    return c;
+}
 template <bool kBackoff = false>
-__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity,
-                                             volatile uint32_t* abort_flag) {
-#pragma unroll 1
-    for (int i = 0; i < 4; ++i) {
-        if (ptx::mbar_try_wait(bar, parity)) return true;
-    }
-    const long long start = clock64();
+__device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity, uint32_t abort_flag) {
+    if (ptx::mbar_try_wait(bar, parity)) return true;
+    const uint32_t start = clock_lo();
 #pragma unroll 1
     while (true) {
 #pragma unroll 1
@@ -218,20 +227,37 @@ __device__ __forceinline__ bool bounded_wait(uint32_t bar, uint32_t parity,
             if (ptx::mbar_try_wait(bar, parity)) return true;
             if (kBackoff) __nanosleep(32);  // keep a waiting warp off the issue ports
         }
-        if (*abort_flag != 0) return false;
-        if (clock64() - start > kWaitTimeoutCycles) {
-            *abort_flag = 1;
+        if (flag_value(abort_flag) != 0) return false;
+        if (clock_lo() - start > kWaitTimeoutCycles) {
+            flag_set(abort_flag, 1);
             atomicCAS(&g_device_error, kDevOk, kDevWaitTimeout);
             return false;
         }
     }
 }
 
+// The same for a converged warp.  The votes make every branch uniform: a wait for a barrier that has
+// completed costs one round trip to the barrier (97 clk; 107-153 beside busy math warps), where per-lane
+// polling with a vote behind it costs the reconvergence of a divergent loop on top (174 clk, 189-262).
 template <bool kBackoff = true>
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity,
-                                          volatile uint32_t* abort_flag) {
-    const bool ok = bounded_wait<kBackoff>(bar, parity, abort_flag);
-    return __all_sync(0xffffffffu, ok);
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, uint32_t abort_flag) {
+    constexpr uint32_t kAll = 0xffffffffu;
+    if (__all_sync(kAll, ptx::mbar_try_wait(bar, parity))) return true;
+    const uint32_t start = clock_lo();
+#pragma unroll 1
+    while (true) {
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i) {
+            if (__all_sync(kAll, ptx::mbar_try_wait(bar, parity))) return true;
+            if (kBackoff) __nanosleep(32);
+        }
+        if (__any_sync(kAll, flag_value(abort_flag) != 0)) return false;
+        if (__any_sync(kAll, clock_lo() - start > kWaitTimeoutCycles)) {
+            flag_set(abort_flag, 1);
+            atomicCAS(&g_device_error, kDevOk, kDevWaitTimeout);
+            return false;
+        }
+    }
 }
 
 // kCausal: general form -- the visible band may be bounded (causal mask, sliding window) and the
@@ -259,8 +285,8 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int lane = threadIdx.x & 31;
     const int wg = warp >> 2;
     auto bar = [&](int i) -> uint32_t { return sbase + C::kOffBar + 8 * i; };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::kOffBar + 8 * kNumBars);
-    volatile uint32_t* abort_flag = tmem_slot + 1;
+    const uint32_t tmem_slot = sbase + C::kOffBar + 8 * kNumBars;
+    const uint32_t abort_flag = tmem_slot + 4;
 
     if (threadIdx.x == 0) {
         TRACE(0, 0);
@@ -342,18 +368,18 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         ptx::mbar_init(bar(kDqFull), 1);
         ptx::mbar_init(bar(kDqEmpty), 128);
         ptx::mbar_init(bar(kDkvFull), 1);
-        *abort_flag = 0;
+        flag_set(abort_flag, 0);
         ptx::fence_mbar_init();
         TRACE(0, 2);
     }
     if (warp == 1) {
-        ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), C::kTmemCols);
+        ptx::tmem_alloc(tmem_slot, C::kTmemCols);
         ptx::tmem_relinquish();
     }
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = flag_value(tmem_slot);
     // The kernel behind this one (dQ convert) may begin to launch; it waits for our completion itself.
     ptx::launch_dependents();
 
@@ -424,13 +450,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 constexpr uint32_t kIdSdP = ptx::instr_desc_f16(kBf16, 128, 128, false, false);
                 constexpr uint32_t kIdDkv = ptx::instr_desc_f16(kBf16, 128, D, false, true);
                 constexpr uint32_t kIdDq = ptx::instr_desc_f16(kBf16, 128, D, true, true);
-                // Descriptor low words (address >> 4 | LBO) of every operand tile; a K step advances them
-                // by a compile-time constant: K-major +2 per 16 elements inside a box and +box/16 per box,
-                // MN-major +128 per 16 rows.  One constant high word serves every descriptor.
-                constexpr uint32_t kHi = ptx::kDescHiSw128;
-                constexpr uint32_t kBoxStep = C::kBoxBytes >> 4;
-                auto k_step = [](int kk) -> uint32_t { return uint32_t(kk >> 2) * kBoxStep + uint32_t(kk & 3) * 2u; };
-                auto mn_step = [](int kk) -> uint32_t { return uint32_t(kk) * 128u; };
+                // Descriptor low words (address >> 4 | LBO) of every operand tile.
                 const uint32_t loK_k = ptx::desc_lo_k_major(sbase + C::kOffK);
                 const uint32_t loV_k = ptx::desc_lo_k_major(sbase + C::kOffV);
                 const uint32_t loDS_k = ptx::desc_lo_k_major(sbase + C::kOffDS);
@@ -440,18 +460,12 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 auto sDO = [&](int t) { return sbase + C::kOffDO + (t % C::kDoStages) * C::kOperandBytes; };
                 auto issue_s = [&](int t) {
                     const uint32_t loQ = ptx::desc_lo_k_major(sQ(t));
-                    ptx::mma_ss_lean<false>(tmem + C::kColS, loK_k, loQ, kHi, kIdSdP);
-#pragma unroll
-                    for (int kk = 1; kk < D / 16; ++kk)
-                        ptx::mma_ss_lean<true>(tmem + C::kColS, loK_k + k_step(kk), loQ + k_step(kk), kHi, kIdSdP);
+                    ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(tmem + C::kColS, loK_k, loQ, kIdSdP, 0);
                     ptx::tc_commit_elect(bar(kSFull));
                 };
                 auto issue_dp = [&](int t) {
                     const uint32_t loDO = ptx::desc_lo_k_major(sDO(t));
-                    ptx::mma_ss_lean<false>(tmem + C::kColDP, loV_k, loDO, kHi, kIdSdP);
-#pragma unroll
-                    for (int kk = 1; kk < D / 16; ++kk)
-                        ptx::mma_ss_lean<true>(tmem + C::kColDP, loV_k + k_step(kk), loDO + k_step(kk), kHi, kIdSdP);
+                    ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(tmem + C::kColDP, loV_k, loDO, kIdSdP, 0);
                     ptx::tc_commit_elect(bar(kDpFull));
                 };
                 bool ok = warp_wait<false>(bar(kKvFull), 0, abort_flag) &&
@@ -478,11 +492,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     ptx::tc_fence_after();
                     {
                         const uint32_t loDO = ptx::desc_lo_mn_major(sDO(t), C::kBoxBytes);
-                        ptx::mma_ts_lean_rt(tmem + C::kColDV, tmem + C::kColS, loDO, kHi, kIdDkv, t > 0 ? 1u : 0u);
-#pragma unroll
-                        for (int kk = 1; kk < 8; ++kk)
-                            ptx::mma_ts_lean<true>(tmem + C::kColDV, tmem + C::kColS + (kk >> 2) * 64 + (kk & 3) * 8,
-                                                   loDO + mn_step(kk), kHi, kIdDkv);
+                        ptx::mma_ts_8<ptx::TmemHalves, ptx::MnMajor>(tmem + C::kColDV, tmem + C::kColS, loDO, kIdDkv, t > 0 ? 1u : 0u);
                     }
                     ptx::tc_commit_elect(bar(kDoEmpty + t % C::kDoStages));
                     if (t < 6) TRACE(1, 8 + 8 * t + 1);
@@ -500,10 +510,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     ptx::tc_fence_after();
                     {
                         const uint32_t loQ = ptx::desc_lo_mn_major(sQ(t), C::kBoxBytes);
-                        ptx::mma_ss_lean_rt(tmem + C::kColDK, loDS_k, loQ, kHi, kIdDkv, t > 0 ? 1u : 0u);
-#pragma unroll
-                        for (int kk = 1; kk < 8; ++kk)
-                            ptx::mma_ss_lean<true>(tmem + C::kColDK, loDS_k + k_step(kk), loQ + mn_step(kk), kHi, kIdDkv);
+                        ptx::mma_ss_8<ptx::KMajor, ptx::MnMajor>(tmem + C::kColDK, loDS_k, loQ, kIdDkv, t > 0 ? 1u : 0u);
                     }
                     ptx::tc_commit_elect(bar(kQEmpty + t % C::kQStages));
                     if (kWithDq) {
@@ -512,10 +519,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                             ptx::tc_fence_after();
                         }
                         // dQ = dS K  (overwrites dP(t) when D = 128: dP(t) was consumed before kDsReady)
-                        ptx::mma_ss_lean<false>(tmem + C::kColDQ, loDS_mn, loK_mn, kHi, kIdDq);
-#pragma unroll
-                        for (int kk = 1; kk < 8; ++kk)
-                            ptx::mma_ss_lean<true>(tmem + C::kColDQ, loDS_mn + mn_step(kk), loK_mn + mn_step(kk), kHi, kIdDq);
+                        ptx::mma_ss_8<ptx::MnMajor, ptx::MnMajor>(tmem + C::kColDQ, loDS_mn, loK_mn, kIdDq, 0);
                         ptx::tc_commit_elect(bar(kDqFull));
                     }
                     if (t < 6) TRACE(1, 8 + 8 * t + 4);

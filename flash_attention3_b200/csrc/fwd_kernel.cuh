@@ -3,25 +3,40 @@
 // sequences as the backward kernels (geometry.h).
 //
 // One CTA owns one (batch, query head) and TWO neighbouring 128-row query tiles, A and B.  Both Q tiles
-// stay in shared memory, K and V tiles stream through two-stage rings and are used by both query
-// tiles, and each query tile has its own softmax warpgroup, score buffer and output accumulator in
-// tensor memory.  Per key tile and query tile:
+// stay in shared memory, K and V tiles stream through rings and are used by both query tiles, and each
+// query tile has its own softmax warpgroup, score buffer and output accumulator in tensor memory.  Per
+// key tile and query tile:
 //
 //     S  = Q K^T          [query i on TMEM lanes, key j on columns]           SS MMA
 //     m  = max(m, rowmax S),  P = exp2((S - m) * scale*log2e),  l = l*alpha + rowsum P
-//          (thread i owns query row i: no shuffles; P is written over S as 16-bit pairs)
+//          (thread i owns query row i: no shuffles; P goes back to tensor memory as 16-bit pairs)
 //     O += P V            A = P from TMEM, B = V (MN-major)                   TS MMA
 //
 // The two query tiles alternate on the tensor pipe: while the softmax warpgroup of tile A works on
-// S_A(t), the pipe computes S_B(t) and P_B V, and the other way round.
+// S_A(t), the pipe computes S_B(t) and P_B V, and the other way round.  At D=128 P is written over S, so
+// S(t+1) follows P(t) V; at D=64 P has columns of its own and S(t+1) is computed while the softmax of
+// step t runs.  P V starts on the first 64 keys while the exponentials of the others are computed.
 // The running maximum is updated lazily: a row keeps its reference maximum until the new maximum
 // exceeds it by more than 2^8, so P stays below 256 and the accumulator only has to be rescaled
 // (tensor memory -> registers -> tensor memory) on the rare steps where some row of a warp moves
 // its reference.  The result is exact: O and l carry the same factor, which cancels in O / l.
 //
-// Tensor-memory ledger: S_A [0,128)  S_B [128,256)  O_A [256,256+D)  O_B [256+D,256+2D).
-// Shared-memory ledger: Q_A, Q_B resident (2 x D*256), K and V two stages each (4 x D*256),
-// mbarriers 256: 196,864 bytes at D=128, 98,560 at D=64.
+// What bounds it: the chain S -> softmax -> P V of a tile.  An iteration (both tiles, one key tile) takes 3030
+// clk at D=128 (2048 of MMA) and 2500 at D=64 (1280 of MMA, 2048 of exponentials at 16 per clk).  A lone
+// busy warp of a scheduler issues an instruction every 1.9 clk, so the softmax is written for few
+// instructions: packed two-value arithmetic, three-input maxima, at D=64 every eighth exponential on the FMA
+// pipe (more of them cost more issue slots than they free), votes instead of divergent polling at the
+// barriers (see warp_wait), P's barrier asked for ahead of its use.  TFLOP/s, before and after: B=4, H=16,
+// S=4096 full, D=64 560 and 811, D=128 1050 and 1130-1180 (there the power limit holds the clock near
+// 1.6 GHz); B=2, Hq=32, Hkv=8, S=8192 causal, D=128 905 and 1150.
+//
+// When the pairs are too few to fill the GPU a cluster of 2, 4 or 8 CTAs shares the key tiles of a pair
+// (plan_fwd_splits) and merges the partial outputs through distributed shared memory.
+//
+// Tensor-memory ledger: S_A [0,128)  S_B [128,256)  O_A [256,256+D)  O_B [256+D,256+2D); at D=64 also
+// P_A [384,448)  P_B [448,512).
+// Shared-memory ledger: Q_A, Q_B resident (2 x D*256), K and V rings of two stages (D=128) or three (D=64),
+// partial row statistics 2 KiB, mbarriers 256: 198,912 bytes at D=128, 133,376 at D=64.
 #pragma once
 
 #include <cuda.h>
@@ -50,6 +65,8 @@ struct FwdArgs {
     float scale_log2;         // softmax scale * log2(e)
     float softcap_pre;        // softcap variant: scores become softcap_post * tanh(score * softcap_pre),
     float softcap_post;       // with softcap_pre = scale / softcap and softcap_post = softcap * log2(e)
+    int splits;               // CTAs per pair of query tiles: a cluster of so many shares its key tiles
+    int staged_store;         // out goes through tm_o (not packed: the copy engine cannot clip at a sequence's end)
 };
 
 template <int D>
@@ -59,86 +76,106 @@ struct FwdCfg {
     static constexpr int kBoxBytes = 128 * 128;
     static constexpr int kBoxes = D / 64;
     static constexpr int kOperandBytes = kBoxes * kBoxBytes;
-    static constexpr int kStages = 2;
+    static constexpr int kStages = D == 64 ? 3 : 2;
     static constexpr int kOffQ = 0;                                  // two query tiles
     static constexpr int kOffK = 2 * kOperandBytes;
     static constexpr int kOffV = kOffK + kStages * kOperandBytes;
-    static constexpr int kOffBar = kOffV + kStages * kOperandBytes;
+    static constexpr int kOffMerge = kOffK;                          // split: [2 tiles][128 rows][D] fp32 over the dead rings
+    static constexpr int kOffStats = kOffV + kStages * kOperandBytes;  // split: [2 tiles][128 rows] {m, l}
+    static constexpr int kOffBar = kOffStats + 2 * 128 * 8;
     static constexpr int kSmemBytes = kOffBar + 256;
     static_assert(kSmemBytes <= 232448, "shared-memory ledger exceeds 227 KiB");
+    static_assert(2 * 128 * D * 4 <= kOffStats - kOffMerge, "partial outputs do not fit over the rings");
+    // P in columns of its own where they are free (D=64): the scores of the next key tile are then computed
+    // while the exponentials of this one are, because the score columns are free once they are in registers
+    static constexpr bool kOwnP = D == 64;
     static constexpr int kTmemCols = 512;
-    static constexpr int kColS = 0;     // + 128 per query tile
-    static constexpr int kColO = 256;   // + D per query tile
-    static_assert(kColO + 2 * D <= kTmemCols, "tensor-memory ledger exceeds 512 columns");
+    static constexpr int kColS = 0;                     // + 128 per query tile
+    static constexpr int kColO = 256;                   // + D per query tile
+    static constexpr int kColP = kOwnP ? 384 : kColS;   // + kPStride per query tile
+    static constexpr int kPStride = kOwnP ? 64 : 128;
+    static_assert(kColO + 2 * D <= (kOwnP ? kColP : kTmemCols) && kColP + 2 * 64 <= kTmemCols, "tensor-memory ledger exceeds 512 columns");
     static constexpr float kRescaleThreshold = 8.0f;  // log2 units
+    // Of every 8 pairs of exponentials, how many go to the FMA pipe (exp2_poly) instead of the special-function unit.
+    // us per call of B=4, H=16, S=4096 full for 0, 1, 2, 3 of 8: D=64 348, 338, 355, 371; D=128 486, 492, 490, 500.
+    static constexpr int kPolyPairs = D == 64 ? 1 : 0;
     // setmaxnreg split: the kernel starts with 168 registers per thread (384 threads); the producer /
     // MMA warpgroup gives most of its share to the two softmax warpgroups, which hold a whole score
     // row (128 values) in registers
-    static constexpr int kRegsControl = 64;
+    static constexpr int kRegsControl = 72;
     static constexpr int kRegsSoftmax = 216;
     static_assert(kRegsControl + 2 * kRegsSoftmax <= 504, "more registers than the CTA was launched with (168 x 384)");
 };
 
 enum FwdBar : int {
     kFwdQFull = 0,    // per query tile
-    kFwdKFull = 2,    // 2 stages
-    kFwdKEmpty = 4,   // 2 stages
-    kFwdVFull = 6,    // 2 stages
-    kFwdVEmpty = 8,   // 2 stages
-    kFwdSFull = 10,   // per query tile
-    kFwdPReady = 12,  // per query tile
-    kFwdPvDone = 14,  // per query tile
-    kFwdNum = 16,
+    kFwdKFull = 2,    // up to 3 stages
+    kFwdKEmpty = 5,   // up to 3 stages
+    kFwdVFull = 8,    // up to 3 stages
+    kFwdVEmpty = 11,  // up to 3 stages
+    kFwdSFull = 14,   // per query tile
+    kFwdSFree = 16,   // per query tile: the scores are in registers (kOwnP)
+    kFwdPFirst = 18,  // per query tile: the first half of P is written
+    kFwdPReady = 20,  // per query tile: all of P is written
+    kFwdPvDone = 22,  // per query tile
+    kFwdAllDone = 24, // every MMA of the CTA has completed
+    kFwdNum = 25,
 };
 
-// kSoftcap: the scaled scores go through softcap * tanh(x / softcap) before the softmax.
-template <typename T, int D, bool kMasked, bool kSoftcap = false>
-__global__ void __launch_bounds__(384, 1)
-fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-           const __grid_constant__ CUtensorMap tm_v, const FwdArgs a) {
-    using C = FwdCfg<D>;
-    constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
-    extern __shared__ __align__(1024) uint8_t smem[];
-    const uint32_t sbase = ptx::smem_u32(smem);
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    auto bar = [&](int i) -> uint32_t { return sbase + C::kOffBar + 8 * i; };
-    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + C::kOffBar + 8 * kFwdNum);
-    volatile uint32_t* abort_flag = tmem_slot + 1;
+// Which query tiles and keys a CTA works on.
+struct FwdWork {
+    int pair, rank, hq, kvh, b, b_coord, q_base, k_base;
+    int slot_q;          // rows of out this batch entry owns
+    int t_begin, n_iter; // the CTA walks key tiles t_begin .. t_begin + n_iter - 1;
+    int lo[2], hi[2];    // query tile x takes part in iterations lo[x] .. hi[x] - 1 (none when it sees no key or
+                         // lies past the end of its sequence)
+    Band band;
+    __device__ __forceinline__ bool active(int x, int it) const { return it >= lo[x] && it < hi[x]; }
+};
 
+// (Each role works this out for itself behind its setmaxnreg: values carried across a change of the register
+// budget were spilled.)
+template <bool kMasked>
+__device__ __forceinline__ FwdWork fwd_work(const FwdArgs& a) {
+    FwdWork w;
     const int n_pairs = (tiles_of(a.band.seqlen_q) + 1) / 2;  // of the longest sequence
     const int bh_count = a.batch * a.heads_q;
+    const int unit = int(blockIdx.x) / a.splits;
+    w.rank = int(blockIdx.x) - unit * a.splits;       // == rank in the cluster
     // heaviest query tiles (most visible keys) are launched first
-    const int pair = kMasked ? n_pairs - 1 - int(blockIdx.x) / bh_count : int(blockIdx.x) / bh_count;
-    const int bhi = int(blockIdx.x) % bh_count;
-    const int b = bhi / a.heads_q;
-    const int hq = bhi % a.heads_q;
-    const int kvh = hq / (a.heads_q / a.heads_kv);
+    w.pair = kMasked ? n_pairs - 1 - unit / bh_count : unit / bh_count;
+    const int bhi = unit % bh_count;
+    w.b = bhi / a.heads_q;
+    w.hq = bhi % a.heads_q;
+    w.kvh = w.hq / (a.heads_q / a.heads_kv);
+    ptx::grid_dependency_wait();
     // packed sequences: this batch entry's own lengths and first rows
     Band band = a.band;
-    int q_base = 0, k_base = 0, b_coord = b;
+    w.q_base = w.k_base = 0;
+    w.b_coord = w.b;
     if (a.cu_seqlens_q != nullptr) {
-        q_base = a.cu_seqlens_q[b];
-        k_base = a.cu_seqlens_k[b];
-        band.seqlen_q = a.cu_seqlens_q[b + 1] - q_base;
-        band.seqlen_k = a.cu_seqlens_k[b + 1] - k_base;
+        w.q_base = a.cu_seqlens_q[w.b];
+        w.k_base = a.cu_seqlens_k[w.b];
+        band.seqlen_q = a.cu_seqlens_q[w.b + 1] - w.q_base;
+        band.seqlen_k = a.cu_seqlens_k[w.b + 1] - w.k_base;
         band.off = band.seqlen_k - band.seqlen_q;
-        b_coord = 0;
+        w.b_coord = 0;
     }
-    const int slot_q = band.seqlen_q;  // rows of out this batch entry owns
+    w.slot_q = band.seqlen_q;
     if (a.seqused_q != nullptr || a.seqused_k != nullptr) {
-        if (a.seqused_q != nullptr) band.seqlen_q = max(0, min(band.seqlen_q, a.seqused_q[b]));
-        if (a.seqused_k != nullptr) band.seqlen_k = max(0, min(band.seqlen_k, a.seqused_k[b]));
+        if (a.seqused_q != nullptr) band.seqlen_q = max(0, min(band.seqlen_q, a.seqused_q[w.b]));
+        if (a.seqused_k != nullptr) band.seqlen_k = max(0, min(band.seqlen_k, a.seqused_k[w.b]));
         band.off = band.seqlen_k - band.seqlen_q;
     }
     // Query tile x (0 = A, 1 = B) visits key tiles first[x] .. first[x] + count[x] - 1; count is 0 when
-    // no key is visible or the tile lies past the end of this sequence.  The CTA walks the union.
+    // no key is visible or the tile lies past the end of this sequence.  The CTA walks the union, or its
+    // share of it when a cluster splits the keys.
     int first[2], count[2];
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
-        const int qt = 2 * pair + x;
+        const int qt = 2 * w.pair + x;
         first[x] = first_k_tile(qt, band);
-        count[x] = qt * C::kTile < band.seqlen_q ? k_tiles_of_q_tile(qt, band) : 0;
+        count[x] = qt * kTileRows < band.seqlen_q ? k_tiles_of_q_tile(qt, band) : 0;
     }
     int t_begin = 0, t_end = -1;  // inclusive range of key tiles
     if (count[0] > 0 && count[1] > 0) {
@@ -151,183 +188,328 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         t_begin = first[1];
         t_end = first[1] + count[1] - 1;
     }
-    const int n_iter = t_end - t_begin + 1;
-    auto active = [&](int x, int t) { return t >= first[x] && t < first[x] + count[x]; };
-    const bool misaligned = (sbase & 1023u) != 0;
+    if (a.splits > 1) {
+        const int share = (t_end - t_begin + a.splits) / a.splits;  // ceil(tiles / splits)
+        t_begin += w.rank * share;
+        t_end = min(t_end, t_begin + share - 1);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+            const int lo = max(first[x], t_begin), hi = min(first[x] + count[x] - 1, t_end);
+            first[x] = lo;
+            count[x] = max(0, hi - lo + 1);
+        }
+    }
+    w.t_begin = t_begin;
+    w.n_iter = max(0, t_end - t_begin + 1);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+        w.lo[x] = first[x] - t_begin;
+        w.hi[x] = w.lo[x] + count[x];
+    }
+    w.band = band;
+    return w;
+}
 
+// The 256 softmax threads finish 256 / kSplits rows of the pair of query tiles from the cluster's kSplits partial
+// outputs, which they read through distributed shared memory.  All reads of a row are requested before the first
+// is used: one after the other, they cost 10 us per call at four CTAs per pair.
+template <typename T, int D, int kSplits>
+__device__ __forceinline__ void fwd_merge(const FwdArgs& a, const FwdWork& w, uint32_t sbase) {
+    using C = FwdCfg<D>;
+    constexpr int kLanes = D / 8;  // threads per row: columns 4*col .. 4*col+3 of either half (a warp reads whole lines)
+    constexpr int kRows = 256 / kSplits;
+    const int tid = threadIdx.x - 128;
+    const int col = tid % kLanes;
+    uint32_t peer[kSplits];
+#pragma unroll
+    for (int s = 0; s < kSplits; ++s) peer[s] = ptx::map_to_cta(sbase, s);
+#pragma unroll 1
+    for (int rr = tid / kLanes; rr < kRows; rr += 256 / kLanes) {
+        const int row = w.rank * kRows + rr;  // row of the pair
+        const int qi = 2 * w.pair * kTileRows + row;
+        if (qi >= w.slot_q) break;
+        float2 ml[kSplits];
+        float4 part[kSplits][2];
+#pragma unroll
+        for (int s = 0; s < kSplits; ++s) {
+            const uint32_t base = peer[s] + C::kOffMerge + row * (D * 4);
+            ml[s] = ptx::ld_cluster_f2(peer[s] + C::kOffStats + row * 8);
+            part[s][0] = ptx::ld_cluster_f4(base + ((col ^ (row & 7)) << 4));
+            part[s][1] = ptx::ld_cluster_f4(base + (((kLanes + col) ^ (row & 7)) << 4));
+        }
+        float m = ml[0].x;
+#pragma unroll
+        for (int s = 1; s < kSplits; ++s) m = fmaxf(m, ml[s].x);
+        float l = 0.0f, acc[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] = 0.0f;
+#pragma unroll
+        for (int s = 0; s < kSplits; ++s) {
+            const float f = m == -INFINITY ? 0.0f : ptx::ex2_approx(ml[s].x - m);
+            l = fmaf(f, ml[s].y, l);
+            acc[0] = fmaf(f, part[s][0].x, acc[0]); acc[1] = fmaf(f, part[s][0].y, acc[1]);
+            acc[2] = fmaf(f, part[s][0].z, acc[2]); acc[3] = fmaf(f, part[s][0].w, acc[3]);
+            acc[4] = fmaf(f, part[s][1].x, acc[4]); acc[5] = fmaf(f, part[s][1].y, acc[5]);
+            acc[6] = fmaf(f, part[s][1].z, acc[6]); acc[7] = fmaf(f, part[s][1].w, acc[7]);
+        }
+        const float inv = l > 0.0f ? 1.0f / l : 0.0f;  // (l = 0: no visible key, or behind the used length)
+        uint4 o;
+        o.x = ptx::Pack2<T>::pack(acc[0] * inv, acc[1] * inv);
+        o.y = ptx::Pack2<T>::pack(acc[2] * inv, acc[3] * inv);
+        o.z = ptx::Pack2<T>::pack(acc[4] * inv, acc[5] * inv);
+        o.w = ptx::Pack2<T>::pack(acc[6] * inv, acc[7] * inv);
+        T* dst = reinterpret_cast<T*>(a.out) + w.b_coord * a.o_strides.batch + w.hq * a.o_strides.head +
+                 int64_t(w.q_base + qi) * a.o_strides.row + col * 4;
+        *reinterpret_cast<uint2*>(dst) = make_uint2(o.x, o.y);
+        *reinterpret_cast<uint2*>(dst + D / 2) = make_uint2(o.z, o.w);
+        if (col == 0)
+            a.lse[int64_t(w.b_coord * a.heads_q + w.hq) * a.lse_rows + w.q_base + qi] =
+                l > 0.0f ? (m + __log2f(l)) * 0.69314718055994531f : -INFINITY;
+    }
+}
+
+// kSoftcap: the scaled scores go through softcap * tanh(x / softcap) before the softmax.
+template <typename T, int D, bool kMasked, bool kSoftcap = false>
+__global__ void __launch_bounds__(384, 1)
+fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+           const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
+           const __grid_constant__ FwdArgs a) {
+    using C = FwdCfg<D>;
+    constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
+    extern __shared__ __align__(1024) uint8_t smem[];
+    const uint32_t sbase = ptx::smem_u32(smem);
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    auto bar = [&](int i) -> uint32_t { return sbase + C::kOffBar + 8 * i; };
+    const uint32_t tmem_slot = sbase + C::kOffBar + 8 * kFwdNum;
+    const uint32_t abort_flag = tmem_slot + 4;
+
+    // Set-up first: launched programmatically, it overlaps the end of the kernel in front, which
+    // grid_dependency_wait() below waits for before any of its outputs is read.
+    const bool misaligned = (sbase & 1023u) != 0;
     if (threadIdx.x == 0) {
         if (misaligned) atomicCAS(&g_device_error, kDevOk, kDevSmemMisaligned);
-        for (int s = 0; s < 2; ++s) {
-            ptx::mbar_init(bar(kFwdQFull + s), 1);
+        for (int x = 0; x < 2; ++x) {
+            ptx::mbar_init(bar(kFwdQFull + x), 1);
+            ptx::mbar_init(bar(kFwdSFull + x), 1);
+            ptx::mbar_init(bar(kFwdSFree + x), 4);
+            ptx::mbar_init(bar(kFwdPFirst + x), 4);
+            ptx::mbar_init(bar(kFwdPReady + x), 4);
+            ptx::mbar_init(bar(kFwdPvDone + x), 1);
+        }
+        for (int s = 0; s < C::kStages; ++s) {
             ptx::mbar_init(bar(kFwdKFull + s), 1);
             ptx::mbar_init(bar(kFwdKEmpty + s), 1);
             ptx::mbar_init(bar(kFwdVFull + s), 1);
             ptx::mbar_init(bar(kFwdVEmpty + s), 1);
-            ptx::mbar_init(bar(kFwdSFull + s), 1);
-            ptx::mbar_init(bar(kFwdPReady + s), 128);
-            ptx::mbar_init(bar(kFwdPvDone + s), 1);
         }
-        *abort_flag = 0;
+        ptx::mbar_init(bar(kFwdAllDone), 1);
+        flag_set(abort_flag, 0);
         ptx::fence_mbar_init();
     }
+    if (warp == 0 && lane == 0) {
+        ptx::prefetch_tensormap(&tm_q);
+        ptx::prefetch_tensormap(&tm_k);
+        ptx::prefetch_tensormap(&tm_v);
+    }
     if (warp == 1) {
-        ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), C::kTmemCols);
+        ptx::tmem_alloc(tmem_slot, C::kTmemCols);
         ptx::tmem_relinquish();
     }
-    ptx::tc_fence_before();
-    __syncthreads();
-    ptx::tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    ptx::launch_dependents();
+
+    // (all threads: barriers initialised, tensor memory allocated)
+    auto set_up_done = [&] {
+        ptx::tc_fence_before();
+        asm volatile("bar.sync 0;" ::: "memory");
+        ptx::tc_fence_after();
+        return flag_value(tmem_slot);
+    };
 
     // (each role changes its register budget at the top of its own branch, where the compiler can see
     // which code runs under which budget)
     if (warp < 4) {
         ptx::setmaxnreg_dec<C::kRegsControl>();
+        const FwdWork w = fwd_work<kMasked>(a);
+        const uint32_t tmem = set_up_done();
+        const int n_iter = w.n_iter;
         if (misaligned) {
             // nothing to do
         } else if (warp == 0) {
-            if (lane == 0 && n_iter > 0) {
-                ptx::prefetch_tensormap(&tm_q);
-                ptx::prefetch_tensormap(&tm_k);
-                ptx::prefetch_tensormap(&tm_v);
+            // TMA producer, converged like the MMA issuer
+            if (n_iter > 0) {
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    if (count[x] == 0) continue;  // nothing is loaded for a tile that sees no key
-                    ptx::mbar_arrive_expect_tx(bar(kFwdQFull + x), C::kOperandBytes);
-#pragma unroll
-                    for (int bx = 0; bx < C::kBoxes; ++bx) {
-                        ptx::tma_load_4d(sbase + C::kOffQ + x * C::kOperandBytes + bx * C::kBoxBytes, &tm_q,
-                                         bar(kFwdQFull + x), bx * 64, q_base + (2 * pair + x) * C::kTile, hq, b_coord);
-                    }
+                    if (w.lo[x] >= w.hi[x]) continue;  // nothing is loaded for a tile that sees no key
+                    ptx::tma_load_tile_elect<C::kBoxes>(sbase + C::kOffQ + x * C::kOperandBytes, &tm_q, bar(kFwdQFull + x),
+                                                        w.q_base + (2 * w.pair + x) * C::kTile, w.hq, w.b_coord);
                 }
 #pragma unroll 1
                 for (int it = 0; it < n_iter; ++it) {
-                    const int s = it & 1;
-                    const uint32_t wait_parity = ((it >> 1) & 1) ^ 1;
-                    const int kv_row = k_base + (t_begin + it) * C::kTile;
-                    if (!bounded_wait(bar(kFwdKEmpty + s), wait_parity, abort_flag)) break;
-                    ptx::mbar_arrive_expect_tx(bar(kFwdKFull + s), C::kOperandBytes);
-#pragma unroll
-                    for (int bx = 0; bx < C::kBoxes; ++bx) {
-                        ptx::tma_load_4d(sbase + C::kOffK + s * C::kOperandBytes + bx * C::kBoxBytes, &tm_k,
-                                         bar(kFwdKFull + s), bx * 64, kv_row, kvh, b_coord);
-                    }
-                    if (!bounded_wait(bar(kFwdVEmpty + s), wait_parity, abort_flag)) break;
-                    ptx::mbar_arrive_expect_tx(bar(kFwdVFull + s), C::kOperandBytes);
-#pragma unroll
-                    for (int bx = 0; bx < C::kBoxes; ++bx) {
-                        ptx::tma_load_4d(sbase + C::kOffV + s * C::kOperandBytes + bx * C::kBoxBytes, &tm_v,
-                                         bar(kFwdVFull + s), bx * 64, kv_row, kvh, b_coord);
-                    }
+                    const int s = it % C::kStages;
+                    const uint32_t wait_parity = ((it / C::kStages) & 1) ^ 1;
+                    const int kv_row = w.k_base + (w.t_begin + it) * C::kTile;
+                    if (!warp_wait(bar(kFwdKEmpty + s), wait_parity, abort_flag)) break;
+                    ptx::tma_load_tile_elect<C::kBoxes>(sbase + C::kOffK + s * C::kOperandBytes, &tm_k, bar(kFwdKFull + s), kv_row, w.kvh, w.b_coord);
+                    if (!warp_wait(bar(kFwdVEmpty + s), wait_parity, abort_flag)) break;
+                    ptx::tma_load_tile_elect<C::kBoxes>(sbase + C::kOffV + s * C::kOperandBytes, &tm_v, bar(kFwdVFull + s), kv_row, w.kvh, w.b_coord);
                 }
             }
         } else if (warp == 1) {
-            // MMA issuer: the whole warp runs the role converged; the lean issue forms and the commits
-            // elect their lane inside the asm.
+            // MMA issuer: the whole warp runs the role converged; the issue forms and the commits elect their
+            // lane inside the asm.
             constexpr uint32_t kIdS = ptx::instr_desc_f16(kBf16, 128, 128, false, false);
             constexpr uint32_t kIdO = ptx::instr_desc_f16(kBf16, 128, D, false, true);
-            constexpr uint32_t kHi = ptx::kDescHiSw128;
-            constexpr uint32_t kBoxStep = C::kBoxBytes >> 4;
-            auto k_step = [](int kk) -> uint32_t { return uint32_t(kk >> 2) * kBoxStep + uint32_t(kk & 3) * 2u; };
-            auto mn_step = [](int kk) -> uint32_t { return uint32_t(kk) * 128u; };
-            // S of query tile x against the key tile in ring slot `it`
+            // S of query tile x against the key tile of iteration `it`
             auto issue_s = [&](int x, int it) {
                 const uint32_t loQ = ptx::desc_lo_k_major(sbase + C::kOffQ + x * C::kOperandBytes);
-                const uint32_t loK = ptx::desc_lo_k_major(sbase + C::kOffK + (it & 1) * C::kOperandBytes);
+                const uint32_t loK = ptx::desc_lo_k_major(sbase + C::kOffK + (it % C::kStages) * C::kOperandBytes);
                 const uint32_t dst = tmem + C::kColS + x * 128;
-                ptx::mma_ss_lean<false>(dst, loQ, loK, kHi, kIdS);
-#pragma unroll
-                for (int kk = 1; kk < D / 16; ++kk)
-                    ptx::mma_ss_lean<true>(dst, loQ + k_step(kk), loK + k_step(kk), kHi, kIdS);
+                ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(dst, loQ, loK, kIdS, 0);
                 ptx::tc_commit_elect(bar(kFwdSFull + x));
             };
-            auto issue_pv = [&](int x, int it, bool accumulate) {
-                const uint32_t loV = ptx::desc_lo_mn_major(sbase + C::kOffV + (it & 1) * C::kOperandBytes, C::kBoxBytes);
-                const uint32_t p_cols = tmem + C::kColS + x * 128;
+            auto wait_k = [&](int it) { return warp_wait<false>(bar(kFwdKFull + it % C::kStages), (it / C::kStages) & 1, abort_flag); };
+            auto wait_v = [&](int it) { return warp_wait<false>(bar(kFwdVFull + it % C::kStages), (it / C::kStages) & 1, abort_flag); };
+            // O of query tile x += P V of iteration `it`: on the first part of P as soon as it is there, then on the rest
+            auto issue_pv = [&](int x, int it) {
+                const uint32_t loV = ptx::desc_lo_mn_major(sbase + C::kOffV + (it % C::kStages) * C::kOperandBytes, C::kBoxBytes);
+                const uint32_t p_cols = tmem + C::kColP + x * C::kPStride;
                 const uint32_t o_cols = tmem + C::kColO + x * D;
-                ptx::mma_ts_lean_rt(o_cols, p_cols, loV, kHi, kIdO, accumulate ? 1u : 0u);
-#pragma unroll
-                for (int kk = 1; kk < 8; ++kk)
-                    ptx::mma_ts_lean<true>(o_cols, p_cols + kk * 8, loV + mn_step(kk), kHi, kIdO);
+                const uint32_t parity = (it - w.lo[x]) & 1;
+                const uint32_t accumulate = it > w.lo[x] ? 1u : 0u;
+                if (!warp_wait<false>(bar(kFwdPFirst + x), parity, abort_flag)) return false;
+                ptx::tc_fence_after();
+                ptx::mma_ts_4<0, ptx::TmemPacked, ptx::MnMajor>(o_cols, p_cols, loV, kIdO, accumulate);
+                if (!warp_wait<false>(bar(kFwdPReady + x), parity, abort_flag)) return false;
+                ptx::tc_fence_after();
+                ptx::mma_ts_4<4, ptx::TmemPacked, ptx::MnMajor>(o_cols, p_cols, loV, kIdO, 1);
                 ptx::tc_commit_elect(bar(kFwdPvDone + x));
+                return true;
             };
             bool ok = n_iter > 0;
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                if (ok && count[x] > 0) ok = warp_wait<false>(bar(kFwdQFull + x), 0, abort_flag);
+                if (ok && w.lo[x] < w.hi[x]) ok = warp_wait<false>(bar(kFwdQFull + x), 0, abort_flag);
             }
-            if (ok) ok = warp_wait<false>(bar(kFwdKFull + 0), 0, abort_flag);
+            if (ok) ok = wait_k(0);
             if (ok) {
                 ptx::tc_fence_after();
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    if (active(x, t_begin)) issue_s(x, 0);
+                    if (w.active(x, 0)) issue_s(x, 0);
                 }
                 ptx::tc_commit_elect(bar(kFwdKEmpty + 0));
             }
-            int done[2] = {0, 0};  // local step counters of the two query tiles
+            if constexpr (!C::kOwnP) {
 #pragma unroll 1
-            for (int it = 0; ok && it < n_iter; ++it) {
-                const int t = t_begin + it;
-                const bool more = it + 1 < n_iter;
-                bool v_ready = false, k_ready = false;
+                for (int it = 0; ok && it < n_iter; ++it) {
+                    const bool more = it + 1 < n_iter;
+                    bool v_ready = false, k_ready = false;
 #pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    if (active(x, t)) {
-                        if (!(ok = warp_wait<false>(bar(kFwdPReady + x), done[x] & 1, abort_flag))) break;
-                        if (!v_ready) {
-                            if (!(ok = warp_wait<false>(bar(kFwdVFull + (it & 1)), (it >> 1) & 1, abort_flag))) break;
-                            v_ready = true;
+                    for (int x = 0; x < 2; ++x) {
+                        if (w.active(x, it)) {
+                            if (!v_ready) {
+                                if (!(ok = wait_v(it))) break;
+                                v_ready = true;
+                            }
+                            if (!(ok = issue_pv(x, it))) break;
                         }
-                        ptx::tc_fence_after();
-                        issue_pv(x, it, done[x] > 0);
-                        ++done[x];
-                    }
-                    // S of the next key tile goes over P of this one: it follows P V in the pipe
-                    if (more && active(x, t + 1)) {
-                        if (!k_ready) {
-                            if (!(ok = warp_wait<false>(bar(kFwdKFull + ((it + 1) & 1)), ((it + 1) >> 1) & 1, abort_flag))) break;
-                            k_ready = true;
+                        // S of the next key tile goes over P of this one: it follows P V in the pipe
+                        if (more && w.active(x, it + 1)) {
+                            if (!k_ready) {
+                                if (!(ok = wait_k(it + 1))) break;
+                                k_ready = true;
+                                ptx::tc_fence_after();
+                            }
+                            issue_s(x, it + 1);
                         }
-                        ptx::tc_fence_after();
-                        issue_s(x, it + 1);
                     }
+                    if (!ok) break;
+                    if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + (it + 1) % C::kStages));
+                    ptx::tc_commit_elect(bar(kFwdVEmpty + it % C::kStages));
                 }
-                if (!ok) break;
-                if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + ((it + 1) & 1)));
-                ptx::tc_commit_elect(bar(kFwdVEmpty + (it & 1)));
+            } else {
+                // S(x, it+1) needs only "scores (x, it) in registers"; P V of tile B is issued one half
+                // iteration late, because the two softmax warpgroups settle half an iteration apart
+#pragma unroll 1
+                for (int it = 0; ok && it <= n_iter; ++it) {
+                    const bool more = it + 1 < n_iter;
+#pragma unroll
+                    for (int x = 0; x < 2; ++x) {
+                        if (more && w.active(x, it + 1)) {
+                            // (its first key tile has no scores in front of it)
+                            if (w.active(x, it)) ok = warp_wait<false>(bar(kFwdSFree + x), (it - w.lo[x]) & 1, abort_flag);
+                            if (!(ok = ok && wait_k(it + 1))) break;
+                            ptx::tc_fence_after();
+                            issue_s(x, it + 1);
+                        }
+                        // x = 0: P V of tile B, previous iteration; x = 1: P V of tile A, this iteration
+                        const int pv = it - (x == 0 ? 1 : 0);
+                        const int y = x ^ 1;
+                        if (pv < n_iter && w.active(y, pv)) {
+                            if (!(ok = wait_v(pv) && issue_pv(y, pv))) break;
+                        }
+                        if (x == 0 && it > 0) ptx::tc_commit_elect(bar(kFwdVEmpty + (it - 1) % C::kStages));
+                    }
+                    if (!ok) break;
+                    if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + (it + 1) % C::kStages));
+                }
             }
+            if (ok) ptx::tc_commit_elect(bar(kFwdAllDone));
+        }
+        if (a.splits > 1) {  // (the softmax warps meet their peers around the merge)
+            __syncwarp();
+            ptx::cluster_sync();
+            ptx::cluster_sync();
         }
     } else {
         ptx::setmaxnreg_inc<C::kRegsSoftmax>();
-        if (!misaligned) {
+        const FwdWork w = fwd_work<kMasked>(a);
+        const uint32_t tmem = set_up_done();
+        if (misaligned) {
+            if (a.splits > 1) {
+                ptx::cluster_sync();
+                ptx::cluster_sync();
+            }
+        } else {
             const int x = (warp - 4) >> 2;      // which query tile
             const int i = threadIdx.x & 127;    // query row inside the tile == TMEM lane
-            const int qt = 2 * pair + x;
-            const int n_steps = x == 0 ? count[0] : count[1];  // (selects, not indexing: no local array)
-            const int k_begin = x == 0 ? first[0] : first[1];
+            const int qt = 2 * w.pair + x;
+            const int n_steps = x == 0 ? w.hi[0] - w.lo[0] : w.hi[1] - w.lo[1];  // (selects, not indexing: no local array)
+            const int k_begin = w.t_begin + (x == 0 ? w.lo[0] : w.lo[1]);
             const uint32_t tl = tmem + (uint32_t((warp & 3) * 32) << 16);
             const uint32_t s_cols = tl + C::kColS + x * 128;
+            const uint32_t p_cols = tl + C::kColP + x * C::kPStride;
             const uint32_t o_cols = tl + C::kColO + x * D;
             const int qi = qt * C::kTile + i;  // query row inside the head
-            const bool q_valid = qi < band.seqlen_q;
+            const bool q_valid = qi < w.band.seqlen_q;
             float m_ref = -INFINITY;  // reference maximum (raw scores) the exponentials are taken against
             float l = 0.0f;           // sum of the exponentials, in units of exp2(m_ref * scale_log2)
             const float sl = kSoftcap ? 1.0f : a.scale_log2;  // log2 units per unit of (transformed) score
+            const uint64_t sl2 = ptx::f2_pack(sl, sl);
+            // one arrival per warp: every lane's accesses are ordered before it by the fence and the warp barrier
+            auto arrive = [&](int which) {
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar(which + x));
+            };
+            // key j of key tile k_begin + u survives for query i iff mask_from <= j <= mask_to
+            int mask_from = 0, mask_to = 0;
+            if (kMasked) key_range_of_query(qi, k_begin * C::kTile, w.band, &mask_from, &mask_to);
             bool ok = true;
 #pragma unroll 1
             for (int u = 0; u < n_steps; ++u) {
-                if (!(ok = warp_wait(bar(kFwdSFull + x), u & 1, abort_flag))) break;
+                if (!(ok = warp_wait<false>(bar(kFwdSFull + x), u & 1, abort_flag))) break;
                 ptx::tc_fence_after();
-                // key j of this tile survives for query i iff mask_from <= j <= mask_to
-                const bool diagonal = kMasked && tile_needs_mask(k_begin + u, qt, band);
-                int mask_from = 0, mask_to = 0;
-                if (diagonal) key_range_of_query(qi, (k_begin + u) * C::kTile, band, &mask_from, &mask_to);
+                const bool diagonal = kMasked && __any_sync(0xffffffffu, mask_from > 0 || mask_to < C::kTile - 1);
                 // ---- the whole score row of this tile goes to registers in one round trip
                 uint32_t r[4][32];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) ptx::tmem_ld32(s_cols + c * 32, r[c]);
+                // (asked ahead of its use: has P V of the previous key tile completed?)
+                const bool p_free = !C::kOwnP || u == 0 || ptx::mbar_test_wait(bar(kFwdPvDone + x), (u - 1) & 1);
                 ptx::tmem_ld_wait();
+                if (C::kOwnP) arrive(kFwdSFree);
                 if (kSoftcap) {
                     // capped scores, already in log2 units: from here on they are used with a scale of 1
 #pragma unroll
@@ -339,78 +521,125 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                         }
                     }
                 }
-                float mt = -INFINITY;
                 if (diagonal) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
 #pragma unroll
                         for (int e = 0; e < 32; ++e) {
                             const int j = c * 32 + e;
-                            if (j >= mask_from && j <= mask_to) mt = fmaxf(mt, __uint_as_float(r[c][e]));
+                            if (j < mask_from || j > mask_to) r[c][e] = 0xff800000u;  // -inf
                         }
                     }
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) mt = fmaxf(mt, __uint_as_float(r[c][e]));
-                    }
                 }
+                // four chains of three-input maxima
+                float mx[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) mx[c] = fmaxf(__uint_as_float(r[c][0]), __uint_as_float(r[c][1]));
+#pragma unroll
+                for (int e = 2; e < 32; e += 2) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) mx[c] = ptx::max3(mx[c], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
+                }
+                const float mt = fmaxf(ptx::max3(mx[0], mx[1], mx[2]), mx[3]);
                 // ---- move the reference maximum only when it is more than 2^8 too small
-                float alpha = 1.0f;
-                const bool move = (mt - m_ref) * sl > C::kRescaleThreshold;  // also -inf -> finite
-                if (move) {
-                    alpha = ptx::ex2_approx((m_ref - mt) * sl);  // exp2(-inf) = 0 on the first move
-                    m_ref = mt;
+                const bool move = m_ref == -INFINITY ? mt != -INFINITY : (mt - m_ref) * sl > C::kRescaleThreshold;
+                if (__any_sync(0xffffffffu, move)) {
+                    // exp2(-inf) = 0 on the first move
+                    const float alpha = move ? ptx::ex2_approx((m_ref - mt) * sl) : 1.0f;
+                    if (move) m_ref = mt;
                     l *= alpha;
-                }
-                if (u > 0 && __any_sync(0xffffffffu, move)) {
-                    // O carries the old reference: wait for P V of step u-1, then rescale these 32 rows
-                    if (!(ok = warp_wait(bar(kFwdPvDone + x), (u - 1) & 1, abort_flag))) break;
-                    ptx::tc_fence_after();
-                    // (16 columns at a time: the score row is still held in registers)
+                    if (u > 0) {
+                        // O carries the old reference: wait for P V of step u-1, then rescale these 32 rows (16
+                        // columns at a time: the score row is still held in registers)
+                        if (!(ok = warp_wait<false>(bar(kFwdPvDone + x), (u - 1) & 1, abort_flag))) break;
+                        ptx::tc_fence_after();
 #pragma unroll 1
-                    for (int c = 0; c < D / 16; ++c) {
-                        uint32_t acc[16];
-                        ptx::tmem_ld16(o_cols + c * 16, acc);
-                        ptx::tmem_ld_wait();
+                        for (int c = 0; c < D / 16; ++c) {
+                            uint32_t acc[16];
+                            ptx::tmem_ld16(o_cols + c * 16, acc);
+                            ptx::tmem_ld_wait();
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
-                        ptx::tmem_st16(o_cols + c * 16, acc);
+                            for (int e = 0; e < 16; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
+                            ptx::tmem_st16(o_cols + c * 16, acc);
+                        }
+                        ptx::tmem_st_wait();
                     }
-                    ptx::tmem_st_wait();
                 }
-                // ---- P = exp2((S - m_ref) * scale_log2), written over S as 16-bit pairs (every column of
-                // S has been read by now)
+                // ---- P = exp2((S - m_ref) * scale_log2), written as 16-bit pairs (over S, every column of which
+                // has been read by now, where P has no columns of its own)
+                if (C::kOwnP) {
+                    // P of the previous key tile must have been used before it is overwritten
+                    if (!__all_sync(0xffffffffu, p_free) && !(ok = warp_wait<false>(bar(kFwdPvDone + x), (u - 1) & 1, abort_flag))) break;
+                    ptx::tc_fence_after();
+                }
                 const float neg = m_ref == -INFINITY ? 0.0f : -m_ref * sl;
-                float sum = 0.0f;
+                const uint64_t neg2 = ptx::f2_pack(neg, neg);
+                uint64_t sum2[2] = {0, 0};
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     uint32_t o[16];
 #pragma unroll
                     for (int e = 0; e < 32; e += 2) {
-                        float p0 = ptx::ex2_approx(fmaf(__uint_as_float(r[c][e + 0]), sl, neg));
-                        float p1 = ptx::ex2_approx(fmaf(__uint_as_float(r[c][e + 1]), sl, neg));
-                        if (diagonal) {
-                            const int j = c * 32 + e;
-                            p0 = (j + 0 >= mask_from && j + 0 <= mask_to) ? p0 : 0.0f;
-                            p1 = (j + 1 >= mask_from && j + 1 <= mask_to) ? p1 : 0.0f;
+                        const uint64_t x2 = ptx::f2_fma(ptx::f2_pack(__uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1])), sl2, neg2);
+                        float2 pr;
+                        // (the pairs that take the polynomial are spread evenly over the row)
+                        if (((e / 2) * C::kPolyPairs) % 8 + C::kPolyPairs >= 8 && C::kPolyPairs > 0) {
+                            pr = ptx::exp2_poly(x2);
+                        } else {
+                            pr = ptx::f2_unpack(x2);
+                            pr.x = ptx::ex2_approx(pr.x);
+                            pr.y = ptx::ex2_approx(pr.y);
                         }
-                        sum += p0 + p1;
-                        o[e / 2] = ptx::Pack2<T>::pack(p0, p1);
+                        sum2[(e / 2) & 1] = ptx::f2_add(sum2[(e / 2) & 1], ptx::f2_pack(pr.x, pr.y));
+                        o[e / 2] = ptx::Pack2<T>::pack(pr.x, pr.y);
                     }
-                    ptx::tmem_st16(s_cols + c * 16, o);
+                    ptx::tmem_st16(p_cols + c * 16, o);
+                    if (c == 1) {
+                        ptx::tmem_st_wait();
+                        arrive(kFwdPFirst);
+                    }
                 }
-                l += sum;
                 ptx::tmem_st_wait();
-                ptx::tc_fence_before();
-                ptx::mbar_arrive(bar(kFwdPReady + x));
+                arrive(kFwdPReady);
+                const float2 sum = ptx::f2_unpack(ptx::f2_add(sum2[0], sum2[1]));
+                l += sum.x + sum.y;
+                mask_from -= C::kTile;
+                mask_to -= C::kTile;
             }
+            // (m_ref, not l, says whether the row saw a key: exp2_poly leaves 2^-126 on a masked one)
+            const bool any_key = q_valid && m_ref != -INFINITY;
+            const float inv = any_key ? 1.0f / l : 0.0f;
+            // ln(sum exp(s*scale)) = (m_ref*scale_log2 + log2 l) * ln 2
+            float* lse_dst = a.lse + int64_t(w.b_coord * a.heads_q + w.hq) * a.lse_rows + w.q_base + qi;
+            if (a.splits > 1) {
+                // This CTA's share of the keys: unnormalised O, fp32, and {m in log2 units, l} go to shared
+                // memory, over the K / V rings, for the merge below.
+                if (ok && w.n_iter > 0) ok = warp_wait(bar(kFwdAllDone), 0, abort_flag);
+                ptx::tc_fence_after();
+                *reinterpret_cast<float2*>(smem + C::kOffStats + (x * 128 + i) * 8) =
+                    make_float2(any_key ? m_ref * sl : -INFINITY, any_key ? l : 0.0f);
+                const uint32_t row_addr = sbase + C::kOffMerge + (x * 128 + i) * (D * 4);
+#pragma unroll 1
+                for (int c = 0; c < D / 32; ++c) {
+                    uint32_t r[32];
+                    if (n_steps > 0) {
+                        ptx::tmem_ld32(o_cols + c * 32, r);
+                        ptx::tmem_ld_wait();
+                    }
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const int chunk = (c * 8 + e) ^ (i & 7);  // (rows are 256 or 512 bytes apart: spread over the banks)
+                        const bool keep = n_steps > 0 && any_key;
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(row_addr + chunk * 16), "r"(keep ? r[4 * e] : 0u), "r"(keep ? r[4 * e + 1] : 0u),
+                                       "r"(keep ? r[4 * e + 2] : 0u), "r"(keep ? r[4 * e + 3] : 0u) : "memory");
+                    }
+                }
+            } else {
             if (ok && n_steps > 0) ok = warp_wait(bar(kFwdPvDone + x), (n_steps - 1) & 1, abort_flag);
-            T* dst = reinterpret_cast<T*>(a.out) + b_coord * a.o_strides.batch + hq * a.o_strides.head +
-                     int64_t(q_base + qi) * a.o_strides.row;
-            float* lse_dst = a.lse + int64_t(b_coord * a.heads_q + hq) * a.lse_rows + q_base + qi;
-            if (ok && ((q_valid && n_steps == 0) || (!q_valid && qi < slot_q))) {
+            T* dst = reinterpret_cast<T*>(a.out) + w.b_coord * a.o_strides.batch + w.hq * a.o_strides.head +
+                     int64_t(w.q_base + qi) * a.o_strides.row;
+            if (ok && ((q_valid && n_steps == 0) || (!q_valid && qi < w.slot_q))) {
                 // no visible key at all, or a row behind the used length: O = 0, lse = -inf
                 uint4* d4 = reinterpret_cast<uint4*>(dst);
 #pragma unroll
@@ -422,11 +651,42 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 // (tensor-memory loads are warp-wide: every lane runs them, only the stores of query rows
                 // past the end of the sequence are skipped)
                 ptx::tc_fence_after();
-                const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-                if (q_valid) {
-                    // ln(sum exp(s*scale)) = (m_ref*scale_log2 + log2 l) * ln 2
-                    *lse_dst = l > 0.0f ? (m_ref * sl + __log2f(l)) * 0.69314718055994531f : -INFINITY;
-                }
+                if (q_valid) *lse_dst = any_key ? (m_ref * sl + __log2f(l)) * 0.69314718055994531f : -INFINITY;
+                if (a.staged_store) {
+                    // through shared memory (the Q tile is dead: its last S completed before this O) and the copy
+                    // engine: whole lines instead of 16 bytes of 32 rows per instruction, rows past the end clipped
+                    const int w4 = warp & 3;
+                    const uint32_t stage = sbase + C::kOffQ + x * C::kOperandBytes + w4 * (C::kBoxes * 4096);
+                    const float scale_row = q_valid ? inv : 0.0f;  // (rows behind a used length hold zeros)
+#pragma unroll
+                    for (int c = 0; c < D / 32; ++c) {
+                        uint32_t r[32];
+                        ptx::tmem_ld32(o_cols + c * 32, r);
+                        ptx::tmem_ld_wait();
+                        const uint32_t row_addr = stage + (c >> 1) * 4096 + lane * 128;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            uint32_t o[4];
+#pragma unroll
+                            for (int h = 0; h < 4; ++h) {
+                                const float lo = __uint_as_float(r[8 * e + 2 * h]) * scale_row, hi = __uint_as_float(r[8 * e + 2 * h + 1]) * scale_row;
+                                o[h] = scale_row != 0.0f ? ptx::Pack2<T>::pack(lo, hi) : 0u;
+                            }
+                            const int chunk = ((c & 1) * 4 + e) ^ (lane & 7);
+                            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                                         ::"r"(row_addr + (chunk << 4)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+                        }
+                    }
+                    ptx::fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0 && qt * C::kTile + w4 * 32 < w.slot_q) {
+#pragma unroll
+                        for (int bx = 0; bx < C::kBoxes; ++bx)
+                            ptx::tma_store_4d(&tm_o, stage + bx * 4096, bx * 64, qt * C::kTile + w4 * 32, w.hq, w.b);
+                        ptx::bulk_commit_group();
+                        ptx::bulk_wait_group_read<0>();
+                    }
+                } else {
 #pragma unroll
                 for (int c = 0; c < D / 32; ++c) {
                     uint32_t r[32];
@@ -446,6 +706,19 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                     }
                     __syncwarp();  // reconverge before the next warp-wide load
                 }
+                }
+            }
+            }
+            if (a.splits > 1) {
+                // ---- merge of the cluster's shares: every CTA finishes 256 / splits of the w.pair's rows, reading
+                // the partial outputs of all peers through distributed shared memory
+                __syncwarp();
+                ptx::cluster_sync();
+                if (a.splits == 2) fwd_merge<T, D, 2>(a, w, sbase);
+                else if (a.splits == 4) fwd_merge<T, D, 4>(a, w, sbase);
+                else fwd_merge<T, D, 8>(a, w, sbase);
+                __syncwarp();
+                ptx::cluster_sync();  // the peers read this CTA's shared memory until here
             }
         }
     }
@@ -455,7 +728,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     __syncthreads();
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem, C::kTmemCols);
+        ptx::tmem_dealloc(flag_value(tmem_slot), C::kTmemCols);
     }
 }
 

@@ -40,6 +40,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return done != 0;
 }
 
+// The same question without waiting.
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
 // Generic-proxy writes to shared memory -> visible to the async proxy (TMA,
 // tcgen05.mma operand reads).
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -64,6 +77,26 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, uint3
         " [%0], [%1, {%3, %4, %5, %6}], [%2];"
         ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
+}
+// The producer's step for a converged warp (one lane is elected): expect the bytes of kBoxes boxes of
+// [128 rows][64 x 16 bit] on the barrier and request them, boxes 64 columns and 16 KiB apart.
+template <int kBoxes>
+__device__ __forceinline__ void tma_load_tile_elect(uint32_t dst, const void* map, uint32_t bar, int row, int head, int batch) {
+    static_assert(kBoxes == 1 || kBoxes == 2, "head dimension 64 or 128");
+    if (kBoxes == 1) {
+        asm volatile(
+            "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+            "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], 16384;\n\t"
+            "@q cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%6, %3, %4, %5}], [%2];\n\t}"
+            ::"r"(dst), "l"(map), "r"(bar), "r"(row), "r"(head), "r"(batch), "r"(0) : "memory");
+    } else {
+        asm volatile(
+            "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+            "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%2], 32768;\n\t"
+            "@q cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%6, %3, %4, %5}], [%2];\n\t"
+            "@q cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%8], [%1, {%7, %3, %4, %5}], [%2];\n\t}"
+            ::"r"(dst), "l"(map), "r"(bar), "r"(row), "r"(head), "r"(batch), "r"(0), "r"(64), "r"(dst + 16384) : "memory");
+    }
 }
 // 3-D tiled reduce-add shared -> global; elements outside the tensor are dropped.
 __device__ __forceinline__ void tma_reduce_add_3d(const void* map, uint32_t src, int c0, int c1,
@@ -135,115 +168,101 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// Single thread: arrive on an mbarrier when all MMAs issued so far by this
-// thread have completed.
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                 ::"r"(bar) : "memory");
-}
 // Whole converged warp: the elected lane arrives on an mbarrier when all MMAs it issued so far
-// have completed (the election is deterministic, so it is the lane the lean MMA forms elect).
+// have completed (the election is deterministic, so it is the lane the MMA forms below elect).
 __device__ __forceinline__ void tc_commit_elect(uint32_t bar) {
     asm volatile(
         "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
         ::"r"(bar) : "memory");
 }
-// Single thread: D[tmem] (+)= A[smem] * B[smem].
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                       uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// Single thread: D[tmem] (+)= A[tmem] * B[smem].  A is K-major by definition.
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc,
-                                       uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// Lean issue forms for the MMA-issuing warp.  They are executed by the whole, converged warp and
-// elect the issuing lane inside the asm block: with a converged warp the descriptors live in uniform
-// registers and one MMA costs a couple of issue slots, whereas a single divergent lane needs many
-// more and is starved by the math warps that share its scheduler (measured: 122 instead of 333
-// cycles per MMA with two busy math warps on the same scheduler).  A descriptor is passed as its two 32-bit
-// halves: `lo` (start address >> 4 | LBO field) advances by a compile-time constant per K step,
-// `hi` (SBO, version, swizzle) is one constant per layout.  kAcc is the accumulate flag.
+// Issue forms for the MMA-issuing warp.  They are executed by the whole, converged warp and elect the
+// issuing lane inside the asm block: with a converged warp the descriptors live in uniform registers and
+// one MMA costs a couple of issue slots, whereas a single divergent lane needs many more and is starved by
+// the math warps that share its scheduler.  One block issues the whole chain of K steps of a tile behind
+// one election: with two busy math warps on every scheduler, M128 N128 K16 MMAs go out every 64.2 cycles,
+// the rate of the pipe, against 79.6 when every MMA elects and builds its descriptors for itself.
+// A descriptor is passed as its low 32 bits (start address >> 4 | LBO field); the high half (SBO, version,
+// swizzle) is one constant, and a K step adds a compile-time constant.
 constexpr uint32_t kDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO 1024 B, version 1, 128-B swizzle
 __host__ __device__ constexpr uint32_t desc_lo_k_major(uint32_t addr) { return ((addr & 0x3FFFF) >> 4) | (1u << 16); }
 __host__ __device__ constexpr uint32_t desc_lo_mn_major(uint32_t addr, uint32_t lbo_bytes) {
     return ((addr & 0x3FFFF) >> 4) | (((lbo_bytes >> 4) & 0x3FFF) << 16);
 }
-template <bool kAcc>
-__device__ __forceinline__ void mma_ss_lean(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi,
-                                            uint32_t idesc) {
-    if (kAcc) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-            "setp.eq.u32 p, 0, 0;\n\t"
-            "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-            ".reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}"
-            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc) : "memory");
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-            "setp.ne.u32 p, 0, 0;\n\t"
-            "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-            ".reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}"
-            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc) : "memory");
-    }
-}
-__device__ __forceinline__ void mma_ss_lean_rt(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi,
-                                               uint32_t idesc, uint32_t accumulate) {
+// What K step kk (16 elements) adds to an operand: a K-major tile of [128 rows][64 columns] boxes, an
+// MN-major tile, and a 16-bit operand in tensor memory (two elements per column, contiguous or with columns
+// 64-127 of the tile 64 columns on).
+struct KMajor { __host__ __device__ static constexpr int step(int kk) { return (kk >> 2) * ((128 * 128) >> 4) + (kk & 3) * 2; } };
+struct MnMajor { __host__ __device__ static constexpr int step(int kk) { return kk * 128; } };
+struct TmemPacked { __host__ __device__ static constexpr int step(int kk) { return kk * 8; } };
+struct TmemHalves { __host__ __device__ static constexpr int step(int kk) { return (kk >> 2) * 64 + (kk & 3) * 8; } };
+
+#define FA3_MMA_SS_STEP(A, B) \
+    "add.s64 ea, da, %" A ";\n\tadd.s64 eb, db, %" B ";\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], ea, eb, %4, t;\n\t"
+// D[tmem] (+)= A[smem] * B[smem] over K steps 0..7 (or 0..3); accumulate = 0: the first one overwrites D.
+template <typename A, typename B>
+__device__ __forceinline__ void mma_ss_8(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-        ".reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 da, db, ea, eb;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\tsetp.eq.u32 t, 0, 0;\n\tmov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t"
+        FA3_MMA_SS_STEP("6", "7") FA3_MMA_SS_STEP("8", "9") FA3_MMA_SS_STEP("10", "11") FA3_MMA_SS_STEP("12", "13")
+        FA3_MMA_SS_STEP("14", "15") FA3_MMA_SS_STEP("16", "17") FA3_MMA_SS_STEP("18", "19") "}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kDescHiSw128), "r"(idesc), "r"(accumulate),
+          "n"(A::step(1)), "n"(B::step(1)), "n"(A::step(2)), "n"(B::step(2)), "n"(A::step(3)), "n"(B::step(3)), "n"(A::step(4)),
+          "n"(B::step(4)), "n"(A::step(5)), "n"(B::step(5)), "n"(A::step(6)), "n"(B::step(6)), "n"(A::step(7)), "n"(B::step(7))
+        : "memory");
 }
-template <bool kAcc>
-__device__ __forceinline__ void mma_ts_lean(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi,
-                                            uint32_t idesc) {
-    if (kAcc) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-            "setp.eq.u32 p, 0, 0;\n\t"
-            "mov.b64 db, {%2, %3};\n\t"
-            ".reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-            ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc) : "memory");
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-            "setp.ne.u32 p, 0, 0;\n\t"
-            "mov.b64 db, {%2, %3};\n\t"
-            ".reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-            "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-            ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc) : "memory");
-    }
-}
-__device__ __forceinline__ void mma_ts_lean_rt(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi,
-                                               uint32_t idesc, uint32_t accumulate) {
+template <typename A, typename B>
+__device__ __forceinline__ void mma_ss_4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 db, {%2, %3};\n\t"
-        ".reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 da, db, ea, eb;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\tsetp.eq.u32 t, 0, 0;\n\tmov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t"
+        FA3_MMA_SS_STEP("6", "7") FA3_MMA_SS_STEP("8", "9") FA3_MMA_SS_STEP("10", "11") "}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(kDescHiSw128), "r"(idesc), "r"(accumulate),
+          "n"(A::step(1)), "n"(B::step(1)), "n"(A::step(2)), "n"(B::step(2)), "n"(A::step(3)), "n"(B::step(3))
+        : "memory");
 }
+// K = 16 * kSteps elements.
+template <int kSteps, typename A, typename B>
+__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    static_assert(kSteps == 4 || kSteps == 8, "K of 64 or 128");
+    if (kSteps == 8) mma_ss_8<A, B>(d_tmem, a_lo, b_lo, idesc, accumulate);
+    else mma_ss_4<A, B>(d_tmem, a_lo, b_lo, idesc, accumulate);
+}
+#undef FA3_MMA_SS_STEP
+
+#define FA3_MMA_TS_STEP(A, B) \
+    "add.u32 ea, %1, %" A ";\n\tadd.s64 eb, db, %" B ";\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [ea], eb, %4, t;\n\t"
+// D[tmem] (+)= A[tmem] * B[smem] over the K steps kFirst .. kFirst + 3 of 16 elements.
+template <int kFirst, typename A, typename B>
+__device__ __forceinline__ void mma_ts_4(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 db, eb;\n\t.reg .b32 ea;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %3, 0;\n\tsetp.eq.u32 t, 0, 0;\n\tmov.b64 db, {%2, %5};\n\t"
+        "add.u32 ea, %1, %6;\n\tadd.s64 eb, db, %7;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], [ea], eb, %4, p;\n\t"
+        FA3_MMA_TS_STEP("8", "9") FA3_MMA_TS_STEP("10", "11") FA3_MMA_TS_STEP("12", "13") "}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(accumulate), "r"(idesc), "r"(kDescHiSw128),
+          "n"(A::step(kFirst)), "n"(B::step(kFirst)), "n"(A::step(kFirst + 1)), "n"(B::step(kFirst + 1)),
+          "n"(A::step(kFirst + 2)), "n"(B::step(kFirst + 2)), "n"(A::step(kFirst + 3)), "n"(B::step(kFirst + 3))
+        : "memory");
+}
+// ... over the eight K steps of 128 elements.
+template <typename A, typename B>
+__device__ __forceinline__ void mma_ts_8(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 db, eb;\n\t.reg .b32 ea;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %3, 0;\n\tsetp.eq.u32 t, 0, 0;\n\tmov.b64 db, {%2, %5};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t"
+        FA3_MMA_TS_STEP("6", "7") FA3_MMA_TS_STEP("8", "9") FA3_MMA_TS_STEP("10", "11") FA3_MMA_TS_STEP("12", "13")
+        FA3_MMA_TS_STEP("14", "15") FA3_MMA_TS_STEP("16", "17") FA3_MMA_TS_STEP("18", "19") "}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(accumulate), "r"(idesc), "r"(kDescHiSw128),
+          "n"(A::step(1)), "n"(B::step(1)), "n"(A::step(2)), "n"(B::step(2)), "n"(A::step(3)), "n"(B::step(3)), "n"(A::step(4)),
+          "n"(B::step(4)), "n"(A::step(5)), "n"(B::step(5)), "n"(A::step(6)), "n"(B::step(6)), "n"(A::step(7)), "n"(B::step(7))
+        : "memory");
+}
+#undef FA3_MMA_TS_STEP
 
 // 32 lanes x 32 consecutive 32-bit columns: thread l of the warp receives the
 // 32 columns of TMEM lane (lane_base + l).
@@ -351,6 +370,30 @@ __device__ __forceinline__ void launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Thread-block clusters.
+// All threads of all CTAs of the cluster; shared-memory writes before it are visible to the peers after it.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// Address of this CTA's shared-memory location `addr` in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
+    uint32_t d;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(rank));
+    return d;
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+    float4 v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ float2 ld_cluster_f2(uint32_t addr) {
+    float2 v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
+    return v;
+}
+
 // Per-warpgroup register re-allocation (all 128 threads of the warpgroup).
 template <int N>
 __device__ __forceinline__ void setmaxnreg_inc() {
@@ -366,6 +409,56 @@ __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
+}
+
+// Two fp32 values in one 64-bit register: one issue slot for both (the FMA pipe takes two cycles).
+__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 f2_unpack(uint64_t d) {
+    float2 v;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(d));
+    return v;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// 2^x of two values on the FMA and integer pipes, for code that the special-function unit bounds (a warp's
+// ex2 keeps it busy for 8 cycles, these 24 instructions for two values keep the FMA pipe busy for 16).
+// x = n + f with n the nearest integer (rounded by adding 1.5 * 2^23, which also leaves n in the low bits),
+// 2^f by a polynomial of degree 5 on [-1/2, 1/2] (Remez exchange on the relative error: 7.5e-8, 2.1e-7 as
+// evaluated in fp32; ex2.approx is good to 2.4e-7), then n added to the exponent field.  x above 127 is not
+// expected; below -126 the result stays at 2^-126.
+__device__ __forceinline__ float2 exp2_poly(uint64_t x2) {
+    const float kMagic = 12582912.0f;
+    float2 x = f2_unpack(x2);
+    x2 = f2_pack(fmaxf(x.x, -126.0f), fmaxf(x.y, -126.0f));
+    const uint64_t t2 = f2_add(x2, f2_pack(kMagic, kMagic));
+    const uint64_t f2 = f2_add(x2, f2_fma(t2, f2_pack(-1.0f, -1.0f), f2_pack(kMagic, kMagic)));  // x - n
+    uint64_t p2 = f2_pack(0x1.5c08e6p-10f, 0x1.5c08e6p-10f);
+    p2 = f2_fma(p2, f2, f2_pack(0x1.3d0c52p-7f, 0x1.3d0c52p-7f));
+    p2 = f2_fma(p2, f2, f2_pack(0x1.c6b6e4p-5f, 0x1.c6b6e4p-5f));
+    p2 = f2_fma(p2, f2, f2_pack(0x1.ebf918p-3f, 0x1.ebf918p-3f));
+    p2 = f2_fma(p2, f2, f2_pack(0x1.62e428p-1f, 0x1.62e428p-1f));
+    p2 = f2_fma(p2, f2, f2_pack(0x1.000002p+0f, 0x1.000002p+0f));
+    const float2 t = f2_unpack(t2), p = f2_unpack(p2);
+    return make_float2(__uint_as_float(__float_as_uint(p.x) + (__float_as_uint(t.x) << 23)),
+                       __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(t.y) << 23)));
 }
 
 // tanh(x) = 1 - 2 / (exp(2x) + 1) with the exp2 and reciprocal approximations: absolute error of a few

@@ -1,0 +1,58 @@
+"""GPU parity of the forward where a cluster of CTAs shares the key tiles of a pair of query tiles: every
+cluster size, key tiles that do not divide evenly, a ragged last pair, masks that leave a CTA without keys."""
+import numpy as np
+import pytest
+import torch
+
+from flash_attention3_b200 import ops
+from oracle import golden
+from tests.helpers import Problem, dev, host
+from tests.test_gpu_forward import check_forward
+
+pytestmark = pytest.mark.gpu
+
+# (b, hq, hkv, sq, sk, d, dtype, causal, layout, window)
+CASES = [
+    (1, 1, 1, 1024, 1024, 128, "bf16", True, "bhsd", (-1, -1)),    # clusters of 8, early pairs with fewer keys than CTAs
+    (1, 4, 2, 2048, 2048, 64, "fp16", True, "bshd", (-1, -1)),     # clusters of 4
+    (1, 9, 9, 2048, 2048, 128, "bf16", False, "bhsd", (-1, -1)),   # clusters of 2
+    (1, 2, 1, 130, 2000, 64, "bf16", False, "bshd", (-1, -1)),     # 16 key tiles, ragged; a pair with two rows in tile B
+    (1, 1, 1, 129, 1153, 128, "fp16", True, "bhsd", (-1, -1)),     # 10 key tiles over 8 CTAs: the last ones get none
+    (1, 2, 2, 1500, 1500, 128, "bf16", True, "bhsd", (700, -1)),   # a window: pairs see a part of the keys
+    (1, 2, 2, 1700, 1100, 64, "fp16", True, "bhsd", (-1, -1)),     # leading queries without a key
+]
+
+
+@pytest.mark.parametrize("b,hq,hkv,sq,sk,d,dtype,causal,layout,window", CASES)
+def test_split_keys(b, hq, hkv, sq, sk, d, dtype, causal, layout, window):
+    prob = Problem(b, hq, hkv, sq, d, dtype, causal, seed=700 + sq + sk, sk=sk, layout=layout, window=window)
+    x = prob.device_inputs()
+    out, lse = ops.fa3_fwd(x["q"], x["k"], x["v"], causal, prob.scale, layout=layout, window=window, sync=True)
+    check_forward(prob.from_layout(host(out)), host(lse), prob.ref["out"], prob.ref["lse"], dtype, (sq, sk, d, causal, window))
+
+
+def test_used_lengths_with_split_keys():
+    """Rows behind the used length are zero and do not disturb the merge."""
+    b, h, s, d, dtype = 1, 2, 1280, 64, "bf16"
+    used_q, used_k = 1000, 1111
+    q, k, v, do = golden.seeded_inputs(41, b, h, h, s, d, dtype)
+    ref = golden.backward(q[:, :, :used_q], k[:, :, :used_k], v[:, :, :used_k], do[:, :, :used_q], False, 1.0 / np.sqrt(d), dtype)
+    used = [torch.tensor([n], dtype=torch.int32, device="cuda") for n in (used_q, used_k)]
+    out, lse = ops.fa3_fwd(dev(q, dtype), dev(k, dtype), dev(v, dtype), False, seqused_q=used[0], seqused_k=used[1], sync=True)
+    out, lse = host(out), host(lse)
+    check_forward(out[:, :, :used_q], lse[:, :, :used_q], ref["out"], ref["lse"], dtype, "used lengths")
+    assert (out[:, :, used_q:] == 0).all() and np.isneginf(lse[:, :, used_q:]).all()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_exponentials_far_below_the_maximum(d):
+    """One key dominates every row: the other scores are hundreds of log2 units below it."""
+    s = 384
+    rng = np.random.default_rng(3)
+    q = golden.round_to("fp16", np.abs(rng.standard_normal((1, 2, s, d), dtype=np.float32)) + 1.0)
+    k = golden.round_to("fp16", -np.abs(rng.standard_normal((1, 2, s, d), dtype=np.float32)) * 8.0)
+    k[:, :, 200] = 8.0
+    v = golden.round_to("fp16", rng.standard_normal((1, 2, s, d), dtype=np.float32))
+    ref = golden.backward(q, k, v, v * 0, False, 1.0, "fp16")
+    out, lse = ops.fa3_fwd(dev(q, "fp16"), dev(k, "fp16"), dev(v, "fp16"), False, 1.0, sync=True)
+    check_forward(host(out), np.where(np.abs(host(lse)) < 1e9, host(lse), np.nan) / 1e3, ref["out"], ref["lse"] / 1e3, "fp16", "far below")

@@ -29,10 +29,12 @@
 namespace fa3b200 {
 
 struct DqArgs {
-    // Row statistics: the packed sidecar [B,Hq,Sq,3] = {m, r, delta}, or, when it is null, the three
+    // Row statistics: {log2 r - m, -delta} as [B,Hq,Sq,2] (the v2 call), or, when that is null, the packed
+    // sidecar [B,Hq,Sq,3] = {m, r, delta}, or, when both are null, the three
     // arrays of the reference's calling convention (reference src/dq_kernel.cpp:1515-1549): aux0 and
     // aux1 = row maximum of the unscaled scores and row sum (or aux0 = log-sum-exp and aux1 = null),
     // and delta, each [B,Hq,Sq].
+    const float2* stats;
     const float* sidecar;
     const float* aux0;
     const float* aux1;
@@ -141,8 +143,8 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         ptx::mbar_init(bar(kDqbSFull), 1);
         ptx::mbar_init(bar(kDqbDpFull), 1);
-        ptx::mbar_init(bar(kDqbSFree), 128);
-        ptx::mbar_init(bar(kDqbDsReady), 128);
+        ptx::mbar_init(bar(kDqbSFree), 4);  // (one arrival per warp)
+        ptx::mbar_init(bar(kDqbDsReady), 4);
         ptx::mbar_init(bar(kDqbDone), 1);
         flag_set(abort_flag, 0);
         ptx::fence_mbar_init();
@@ -243,7 +245,11 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             const int64_t stat_row = int64_t(b_coord * a.heads_q + hq) * a.sidecar_rows + q_base + (q_valid ? qi : 0);
             float neg = -INFINITY, delta = 0.0f;
             if (q_valid) {
-                if (a.sidecar != nullptr) {
+                if (a.stats != nullptr) {
+                    const float2 v = a.stats[stat_row];
+                    neg = v.x;
+                    delta = -v.y;
+                } else if (a.sidecar != nullptr) {
                     const float* side = a.sidecar + stat_row * 3;
                     neg = __log2f(side[1]) - side[0];
                     delta = side[2];
@@ -292,7 +298,8 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     }
                 }
                 ptx::tc_fence_before();
-                ptx::mbar_arrive(bar(kDqbSFree));
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar(kDqbSFree));
                 if (!(ok = warp_wait(bar(kDqbDpFull), t & 1, abort_flag))) break;
                 ptx::tc_fence_after();
 #pragma unroll
@@ -321,7 +328,8 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                 }
                 ptx::tmem_st_wait();
                 ptx::tc_fence_before();
-                ptx::mbar_arrive(bar(kDqbDsReady));
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar(kDqbDsReady));
             }
             if (ok && n_steps > 0) ok = warp_wait(bar(kDqbDone), 0, abort_flag);
             TOut* dst = reinterpret_cast<TOut*>(a.dq) + b_coord * a.q_strides.batch + hq * a.q_strides.head +

@@ -221,7 +221,7 @@ int finish(const ShaoboFa3Params* p, bool sync) {
 // ------------------------------------------------------------------ delta
 template <typename T, int D>
 void launch_delta_t(const void* dout, const void* out, const float* aux0, const float* aux1,
-                    float* delta, float* sidecar, float* zero_rows, int64_t rows, bool lse,
+                    float* delta, float* sidecar, float2* stats, float* zero_rows, int64_t rows, bool lse,
                     float scale_log2, const RowLayout& layout, cudaStream_t st) {
     constexpr int kRowsPerBlock = 8 * (32 / (D / 8));
     int64_t blocks = (rows + kRowsPerBlock - 1) / kRowsPerBlock;
@@ -241,18 +241,18 @@ void launch_delta_t(const void* dout, const void* out, const float* aux0, const 
     const T* dout_t = static_cast<const T*>(dout);
     const T* out_t = static_cast<const T*>(out);
     if (lse) {
-        cudaLaunchKernelEx(&cfg, delta_sidecar_kernel<T, D, true>, dout_t, out_t, aux0, aux1, delta, sidecar,
+        cudaLaunchKernelEx(&cfg, delta_sidecar_kernel<T, D, true>, dout_t, out_t, aux0, aux1, delta, sidecar, stats,
                            zero_rows, rows, scale_log2, layout);
     } else {
-        cudaLaunchKernelEx(&cfg, delta_sidecar_kernel<T, D, false>, dout_t, out_t, aux0, aux1, delta, sidecar,
+        cudaLaunchKernelEx(&cfg, delta_sidecar_kernel<T, D, false>, dout_t, out_t, aux0, aux1, delta, sidecar, stats,
                            zero_rows, rows, scale_log2, layout);
     }
 }
 
-// sidecar may be null (only delta is written); zero_rows, when non-null, is the fp32 dQ accumulator
-// that the same pass clears.
+// Row statistics go to sidecar or to stats, whichever is not null; zero_rows, when non-null, is the fp32 dQ
+// accumulator that the same pass clears.
 void launch_delta(const ShaoboFa3Params* p, const void* dout, const void* out, const float* aux0,
-                  const float* aux1, float* delta, float* sidecar, float* zero_rows, bool lse) {
+                  const float* aux1, float* delta, float* sidecar, float2* stats, float* zero_rows, bool lse) {
     const TensorShape shape = shape_of(p);
     const int64_t rows = int64_t(shape.batch) * p->num_heads_q * shape.rows_q;
     const float scale_log2 = p->softmax_scale * kLog2E;
@@ -260,11 +260,11 @@ void launch_delta(const ShaoboFa3Params* p, const void* dout, const void* out, c
     const bool bf = p->dtype == SHAOBO_FA3_DTYPE_BF16;
     const RowLayout layout = row_layout(p, p->num_heads_q, shape.rows_q, shape.bshd);
     if (p->head_dim_qk == 128) {
-        if (bf) launch_delta_t<__nv_bfloat16, 128>(dout, out, aux0, aux1, delta, sidecar, zero_rows, rows, lse, scale_log2, layout, st);
-        else launch_delta_t<__half, 128>(dout, out, aux0, aux1, delta, sidecar, zero_rows, rows, lse, scale_log2, layout, st);
+        if (bf) launch_delta_t<__nv_bfloat16, 128>(dout, out, aux0, aux1, delta, sidecar, stats, zero_rows, rows, lse, scale_log2, layout, st);
+        else launch_delta_t<__half, 128>(dout, out, aux0, aux1, delta, sidecar, stats, zero_rows, rows, lse, scale_log2, layout, st);
     } else {
-        if (bf) launch_delta_t<__nv_bfloat16, 64>(dout, out, aux0, aux1, delta, sidecar, zero_rows, rows, lse, scale_log2, layout, st);
-        else launch_delta_t<__half, 64>(dout, out, aux0, aux1, delta, sidecar, zero_rows, rows, lse, scale_log2, layout, st);
+        if (bf) launch_delta_t<__nv_bfloat16, 64>(dout, out, aux0, aux1, delta, sidecar, stats, zero_rows, rows, lse, scale_log2, layout, st);
+        else launch_delta_t<__half, 64>(dout, out, aux0, aux1, delta, sidecar, stats, zero_rows, rows, lse, scale_log2, layout, st);
     }
 }
 
@@ -402,7 +402,7 @@ struct FusedLaunch {
 };
 
 FusedLaunch prepare_fused(const ShaoboFa3Params* p, const void* dout, const void* q, const void* k,
-                          const void* v, const float* sidecar, float* dq_accum, void* dk, void* dv,
+                          const void* v, const float2* stats, const float* sidecar, float* dq_accum, void* dk, void* dv,
                           bool with_dq, bool dkv_f32 = false, void* dkv_slabs = nullptr) {
     FusedLaunch L;
     L.with_dq = with_dq;
@@ -460,6 +460,7 @@ FusedLaunch prepare_fused(const ShaoboFa3Params* p, const void* dout, const void
     const long long dq_bytes_per_head =
         with_dq ? (long long)group * plan_seqlen_q(p) * p->head_dim_qk * 4 : 0;
     const CtaOrderPlan plan = cached_plan(work, bh, group, sm_count(), dq_bytes_per_head);
+    args.stats = stats;
     args.sidecar = sidecar;
     args.dk = dk;
     args.dv = dv;
@@ -529,9 +530,9 @@ int run_fused(const ShaoboFa3Params* p, const FusedLaunch& L, bool pdl) {
 }
 
 int launch_fused(const ShaoboFa3Params* p, const void* dout, const void* q, const void* k,
-                 const void* v, const float* sidecar, float* dq_accum, void* dk, void* dv,
+                 const void* v, const float2* stats, const float* sidecar, float* dq_accum, void* dk, void* dv,
                  bool with_dq, bool dkv_f32 = false, void* dkv_slabs = nullptr, bool pdl = false) {
-    return run_fused(p, prepare_fused(p, dout, q, k, v, sidecar, dq_accum, dk, dv, with_dq, dkv_f32, dkv_slabs), pdl);
+    return run_fused(p, prepare_fused(p, dout, q, k, v, stats, sidecar, dq_accum, dk, dv, with_dq, dkv_f32, dkv_slabs), pdl);
 }
 
 // -------------------------------------------------------------- dQ kernel
@@ -569,9 +570,9 @@ int launch_dq_d(const ShaoboFa3Params* p, const CUtensorMap& mq, const CUtensorM
 }
 
 // Three-GEMM dQ kernel (split path).  out_f32 selects fp32 or input-dtype dq.  The row statistics
-// are the packed sidecar, or (sidecar null) aux0 / aux1 / delta as three arrays.
+// are stats, or the packed sidecar, or (both null) aux0 / aux1 / delta as three arrays.
 int launch_dq(const ShaoboFa3Params* p, const void* dout, const void* q, const void* k,
-              const void* v, const float* sidecar, void* dq, bool out_f32,
+              const void* v, const float2* stats, const float* sidecar, void* dq, bool out_f32,
               const float* aux0 = nullptr, const float* aux1 = nullptr, const float* delta = nullptr) {
     const bool bf = p->dtype == SHAOBO_FA3_DTYPE_BF16;
     const CUtensorMapDataType type = bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -586,6 +587,7 @@ int launch_dq(const ShaoboFa3Params* p, const void* dout, const void* q, const v
         return SHAOBO_FA3_STATUS_HIP_ERROR;
     }
     DqArgs args;
+    args.stats = stats;
     args.sidecar = sidecar;
     args.aux0 = aux0;
     args.aux1 = aux1;
@@ -808,7 +810,7 @@ extern "C" int shaobo_fa3_bwd_dot_do_o(const void* dout, const void* out, const 
     }
     launch_delta(params, dout, out, static_cast<const float*>(aux0),
                  static_cast<const float*>(aux1), static_cast<float*>(delta),
-                 static_cast<float*>(packed_sidecar), nullptr, lse);
+                 static_cast<float*>(packed_sidecar), nullptr, nullptr, lse);
     return finish(params, params->sync_after_launch != 0);
 }
 
@@ -832,7 +834,7 @@ extern "C" int shaobo_fa3_bwd_fused5(const void* dout, const void* q, const void
     if (cudaMemsetAsync(accum, 0, dq_bytes, stream_of(params)) != cudaSuccess) {  // (the slabs are written, not added into)
         return SHAOBO_FA3_STATUS_HIP_ERROR;
     }
-    int status = launch_fused(params, dout, q, k, v, static_cast<const float*>(packed_sidecar),
+    int status = launch_fused(params, dout, q, k, v, nullptr, static_cast<const float*>(packed_sidecar),
                               accum, dk, dv, true, false, dkv_slabs);
     if (status != SHAOBO_FA3_STATUS_SUCCESS) return status;
     launch_convert(params, accum, dq, dkv_slabs, dk, dv);
@@ -854,7 +856,7 @@ extern "C" int shaobo_fa3_bwd_dkv(const void* dout, const void* q, const void* k
         dv == nullptr || sidecar == nullptr) {
         return SHAOBO_FA3_STATUS_INVALID_VALUE;
     }
-    const int status = launch_fused(params, dout, q, k, v, static_cast<const float*>(sidecar),
+    const int status = launch_fused(params, dout, q, k, v, nullptr, static_cast<const float*>(sidecar),
                                     nullptr, dk, dv, false, true);
     if (status != SHAOBO_FA3_STATUS_SUCCESS) return status;
     return finish(params, params->sync_after_launch != 0);
@@ -890,9 +892,9 @@ extern "C" int shaobo_fa3_bwd_dq(const void* dout, const void* q, const void* k,
     }
     const int status =
         arrays_complete
-            ? launch_dq(params, dout, q, k, v, nullptr, dq, true, static_cast<const float*>(aux0),
+            ? launch_dq(params, dout, q, k, v, nullptr, nullptr, dq, true, static_cast<const float*>(aux0),
                         lse ? nullptr : static_cast<const float*>(aux1), delta)
-            : launch_dq(params, dout, q, k, v, sidecar, dq, true);
+            : launch_dq(params, dout, q, k, v, nullptr, sidecar, dq, true);
     if (status != SHAOBO_FA3_STATUS_SUCCESS) return status;
     return finish(params, params->sync_after_launch != 0);
 }
@@ -915,7 +917,7 @@ extern "C" int shaobo_fa3_bwd_v2(const void* dout, const void* q, const void* k,
     float* accum = reinterpret_cast<float*>(base);
     float* delta = softmax_d != nullptr ? static_cast<float*>(softmax_d)
                                         : reinterpret_cast<float*>(base + ws.delta_offset);
-    float* sidecar = reinterpret_cast<float*>(base + ws.sidecar_offset);
+    float2* stats = reinterpret_cast<float2*>(base + ws.sidecar_offset);  // (fits: 8 of the sidecar's 12 bytes per row)
 
     ShaoboFa3Params launch = *params;
     launch.softmax_aux_mode = SHAOBO_FA3_SOFTMAX_AUX_LSE;
@@ -929,11 +931,11 @@ extern "C" int shaobo_fa3_bwd_v2(const void* dout, const void* q, const void* k,
         cudaStream_t st = stream_of(&launch);
         void* dkv_slabs = ws.dkv_accum_bytes != 0 ? base + ws.dq_accum_bytes : nullptr;
         // host work of the second launch first, then the three launches back to back
-        const FusedLaunch fused = prepare_fused(&launch, dout, q, k, v, sidecar, accum, dk, dv, true, false, dkv_slabs);
+        const FusedLaunch fused = prepare_fused(&launch, dout, q, k, v, stats, nullptr, accum, dk, dv, true, false, dkv_slabs);
         if (fused.status != SHAOBO_FA3_STATUS_SUCCESS) return fused.status;
         stage_mark(0, st);
         launch_delta(&launch, dout, out, static_cast<const float*>(softmax_lse), nullptr, delta,
-                     sidecar, accum, true);
+                     nullptr, stats, accum, true);
         stage_mark(1, st);
         status = run_fused(&launch, fused, true);
         stage_mark(2, st);
@@ -945,12 +947,12 @@ extern "C" int shaobo_fa3_bwd_v2(const void* dout, const void* q, const void* k,
         cudaStream_t st = stream_of(&launch);
         stage_mark(0, st);
         launch_delta(&launch, dout, out, static_cast<const float*>(softmax_lse), nullptr, delta,
-                     sidecar, nullptr, true);
+                     nullptr, stats, nullptr, true);
         stage_mark(1, st);
-        status = launch_fused(&launch, dout, q, k, v, sidecar, nullptr, dk, dv, false, false);
+        status = launch_fused(&launch, dout, q, k, v, stats, nullptr, nullptr, dk, dv, false, false);
         stage_mark(2, st);
         if (status == SHAOBO_FA3_STATUS_SUCCESS) {
-            status = launch_dq(&launch, dout, q, k, v, sidecar, dq, false);
+            status = launch_dq(&launch, dout, q, k, v, stats, nullptr, dq, false);
         }
         stage_mark(3, st);
     }

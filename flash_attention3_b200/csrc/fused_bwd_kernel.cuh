@@ -25,10 +25,10 @@
 // kernel adds the slabs of a tile in chunk order.
 //
 // Warp roles (512 threads, four warpgroups): warp 0 = TMA producer, warp 1 = MMA
-// issuer and TMEM owner; warps 4-7 and 8-11 = two softmax / dS warpgroups (thread
+// issuer and TMEM owner, warp 2 = row statistics; warps 4-7 and 8-11 = two softmax / dS warpgroups (thread
 // j of each owns TMEM lane j = key j; the first takes queries 0-63 of the tile,
 // the second queries 64-127); warps 12-15 = dQ drain warpgroup.  Registers are
-// re-split with setmaxnreg (96 / 112 / 112 / 176 per thread at D=128).  All hand-offs go
+// re-split with setmaxnreg (96 / 120 / 120 / 176 per thread at D=128).  All hand-offs go
 // through mbarriers; every wait is bounded and a time-out raises an error flag
 // instead of hanging.
 //
@@ -46,9 +46,16 @@
 //     dO              1 stage (D=128) or 2 stages (D=64) x D*256
 //     dS^T            32 KiB               [128 keys][128 queries]
 //     dQ staging      32 KiB               4 warps x 2 boxes of [32 rows][32 fp32]
-//     row statistics  2 KiB / 3 KiB        {-m + log2 r, delta} x 128 rows x 2 buffers (D=128) / 3 (D=64)
+//     row statistics  2 KiB                {log2 r - m, -delta} x 128 rows x 2 buffers
 //     mbarriers       256
-//     total           231,680 (D=128) / 167,168 (D=64)   of 232,448 available
+//     total           231,680 (D=128) / 166,144 (D=64)   of 232,448 available
+//
+// What bounds it: at D=64 the softmax / dS warpgroups (2630 clk per step, 1664 of MMA): one instruction per two
+// elements wherever packed arithmetic allows, statistics brought by a warp of their own, one arrival per warp
+// and uniform votes at the barriers took the step from 2980; B=4,H=16,S=4096 full: kernel 859 -> 791 us.  At
+// D=128 the copy engine (64 KB of loads and 64 KB of fp32 reduce-adds per step, 2900 clk for the latter) and the
+// chain dS -> dQ -> drain -> dP -> dS, 3800-4000 clk per step (2560 of MMA), under a power limit that holds the
+// clock near 1.55 GHz: 1295 -> 1289 us for the same shape.
 #pragma once
 
 #include <cuda.h>
@@ -89,7 +96,11 @@ __device__ __forceinline__ long long trace_globaltimer() {
 #endif
 
 struct FusedArgs {
-    const float* sidecar;  // [B,Hq,Sq,3] = {m, r, delta} per query row (packed sequences: [Hq, total_q, 3])
+    // Row statistics of query row i, one of the two: {log2 r - m, -delta} as [B,Hq,Sq,2] (packed sequences:
+    // [Hq,total_q,2]), what the v2 call's delta stage leaves, or the packed sidecar {m, r, delta} as
+    // [B,Hq,Sq,3] of the component entry points.
+    const float2* stats;
+    const float* sidecar;
     void* dk;              // [B,Hkv,Sk,D] or [B,Sk,Hkv,D], see kv_strides
     void* dv;
     void* dkv_slabs;       // split tiles: a CTA writes its partial dK (scaled) to slab 2x and dV to slab 2x+1,
@@ -157,18 +168,15 @@ struct FusedCfg {
     static constexpr int kOffDS = kOffDO + kDoStages * kOperandBytes;
     static constexpr int kOffStage = kOffDS + kDsBytes;
     static constexpr int kOffStats = kOffStage + kStageBytes;
-    // Row statistics: kStatsBufs buffers of 128 x {log2 r - m} followed by as many of 128 x {delta}.  With three
-    // buffers (D=64, where the softmax warpgroups bound the step) a step's statistics are written one
-    // step ahead, so nobody waits for the writers; D=128 has no shared memory left for a third.
-    static constexpr int kStatsBufs = D == 64 ? 3 : 2;
-    static constexpr int kOffBar = kOffStats + kStatsBufs * 1024;
+    // Row statistics: two buffers of 128 x {log2 r - m}, then two of 128 x {-delta}
+    static constexpr int kOffBar = kOffStats + 2 * 1024;
     static constexpr int kSmemBytes = kOffBar + 256;
     static_assert(kSmemBytes <= 232448, "shared-memory ledger exceeds 227 KiB");
     static_assert(kOffStage % 1024 == 0 && kOffDS % 1024 == 0, "swizzled regions need 1 KiB alignment");
 
     // setmaxnreg split per warpgroup (producer+MMA / softmax x2 / drain); sums to <= 512
     static constexpr int kRegsControl = 96;
-    static constexpr int kRegsCompute = D == 128 ? 112 : 136;
+    static constexpr int kRegsCompute = D == 128 ? 120 : 136;
     static constexpr int kRegsDrain = D == 128 ? 176 : 136;
     static_assert(kRegsControl + 2 * kRegsCompute + kRegsDrain <= 512, "register file over-committed");
 
@@ -195,8 +203,9 @@ enum Bar : int {
     kDqFull = 13,
     kDqEmpty = 14,
     kDkvFull = 15,
-    kStatsFull = 16,  // 2 buffers (not used where the statistics are published a step ahead)
-    kNumBars = 18,
+    kStatsFull = 16,   // 2 buffers
+    kStatsEmpty = 18,  // 2 buffers
+    kNumBars = 20,
 };
 
 constexpr uint32_t kWaitTimeoutCycles = 2000000000u;  // about one second, of a 32-bit cycle counter
@@ -260,6 +269,115 @@ __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, uint32_
     }
 }
 
+// Two barriers at once (one round trip when both have completed).
+__device__ __forceinline__ bool warp_wait2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1, uint32_t abort_flag) {
+    const bool d0 = ptx::mbar_try_wait(bar0, parity0);
+    const bool d1 = ptx::mbar_try_wait(bar1, parity1);
+    if (__all_sync(0xffffffffu, d0 && d1)) return true;
+    return warp_wait(bar0, parity0, abort_flag) && warp_wait(bar1, parity1, abort_flag);
+}
+
+// Which key tile and which of its steps a CTA works on.
+struct FusedWork {
+    int kt, b, kvh, slab;
+    Band band;            // this batch entry's own lengths
+    int q_base, k_base, b_coord;
+    int slot_k;           // rows of dK / dV this batch entry owns
+    int q_tiles;          // query tiles of the sequence
+    int q_begin;          // first query tile that sees the key tile
+    int steps_per_head;
+    int first_head;       // first query head of the KV head's group
+    int t_begin, n_steps; // this CTA's share of the tile's steps (all of them unless the tile is split)
+    int rotation;
+};
+
+// (Each role works this out for itself behind its setmaxnreg: values carried across a change of the register
+// budget were spilled.)
+template <bool kCausal>
+__device__ __forceinline__ FusedWork fused_work(const FusedArgs& a) {
+    FusedWork w;
+    const int n_tiles = tiles_of(a.band.seqlen_k);      // key tiles (of the longest sequence)
+    const int bh_count = a.batch * a.heads_kv;
+    const bool split = a.chunk_steps > 0;
+    const int group = a.heads_q / a.heads_kv;
+    int bhi;
+    w.t_begin = w.slab = 0;
+    if (!split) {
+        // groups of head_group heads; inside a group tile slot major, head minor (see cta_order.h)
+        const int per_group = n_tiles * a.head_group;
+        const int hg = int(blockIdx.x) / per_group;
+        const int rem = int(blockIdx.x) - hg * per_group;
+        const int heads_here = min(a.head_group, bh_count - hg * a.head_group);
+        const int tile_slot = rem / heads_here;
+        bhi = hg * a.head_group + (rem - tile_slot * heads_here);
+        w.kt = remap_k_tile(tile_slot, n_tiles, a.order_mode, a.order_width);
+    } else {
+        const uint32_t entry = a.cta_table[blockIdx.x];
+        w.kt = int(entry & 0xffu);
+        w.t_begin = int((entry >> 8) & 0xffu) * a.chunk_steps;
+        w.slab = int(entry >> 16);
+        bhi = w.slab / a.chunks_per_head;
+    }
+    w.b = bhi / a.heads_kv;
+    w.kvh = bhi % a.heads_kv;
+    w.first_head = w.kvh * group;
+    // Packed sequences: this batch entry's own lengths and first rows; tensors are addressed as one
+    // batch of `total` rows, so rows past the end of a sequence belong to its neighbour (or read as
+    // zero past the end of the tensor) and are masked like any ragged tile end.
+    Band band = a.band;
+    w.q_base = w.k_base = 0;
+    w.b_coord = w.b;
+    if (a.cu_seqlens_q != nullptr) {
+        w.q_base = a.cu_seqlens_q[w.b];
+        w.k_base = a.cu_seqlens_k[w.b];
+        band.seqlen_q = a.cu_seqlens_q[w.b + 1] - w.q_base;
+        band.seqlen_k = a.cu_seqlens_k[w.b + 1] - w.k_base;
+        band.off = band.seqlen_k - band.seqlen_q;
+        w.b_coord = 0;
+    }
+    w.slot_k = band.seqlen_k;
+    if (a.seqused_q != nullptr || a.seqused_k != nullptr) {
+        if (a.seqused_q != nullptr) band.seqlen_q = max(0, min(band.seqlen_q, a.seqused_q[w.b]));
+        if (a.seqused_k != nullptr) band.seqlen_k = max(0, min(band.seqlen_k, a.seqused_k[w.b]));
+        band.off = band.seqlen_k - band.seqlen_q;
+    }
+    w.band = band;
+    w.q_tiles = tiles_of(band.seqlen_q);
+    const bool tile_exists = w.kt * kTileRows < band.seqlen_k;  // false only with packed sequences
+    w.q_begin = first_q_tile(w.kt, band);
+    w.steps_per_head = tile_exists ? q_tiles_of_k_tile(w.kt, band) : 0;
+    const int total_steps = group * w.steps_per_head;
+    w.n_steps = (split ? min(total_steps, w.t_begin + a.chunk_steps) : total_steps) - w.t_begin;
+    // Query tiles are visited in ascending order starting at the diagonal (causal) or at a
+    // per-CTA rotation (non-causal), so that CTAs of one head that run together add into
+    // different dQ tiles at any moment.
+    w.rotation = (kCausal || w.q_tiles == 0) ? 0 : w.kt % w.q_tiles;
+    return w;
+}
+
+// The walk over a CTA's steps: query head, query tile, place inside the head.
+template <bool kCausal>
+struct StepWalk {
+    int hq, qt, r;
+    __device__ __forceinline__ explicit StepWalk(const FusedWork& w) {
+        const int g = w.steps_per_head > 0 ? w.t_begin / w.steps_per_head : 0;
+        hq = w.first_head + g;
+        r = w.t_begin - g * w.steps_per_head;
+        qt = r + (kCausal ? w.q_begin : w.rotation);
+        if (!kCausal && qt >= w.q_tiles) qt -= w.q_tiles;
+    }
+    __device__ __forceinline__ void next(const FusedWork& w) {
+        ++r;
+        ++qt;
+        if (!kCausal && qt == w.q_tiles) qt = 0;
+        if (r == w.steps_per_head) {
+            r = 0;
+            ++hq;
+            qt = kCausal ? w.q_begin : w.rotation;
+        }
+    }
+};
+
 // kCausal: general form -- the visible band may be bounded (causal mask, sliding window) and the
 // sequence lengths need not be multiples of 128; tiles that need it are masked in registers and the
 // query tiles of a key tile are walked in ascending order from the first one that sees it.
@@ -292,67 +410,10 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         TRACE(0, 0);
         TRACE_GT(0, 1);
     }
-    // ---- which tile is ours ------------------------------------------------
-    const int n_tiles = tiles_of(a.band.seqlen_k);      // key tiles (of the longest sequence)
-    const int bh_count = a.batch * a.heads_kv;
-    const bool split = a.chunk_steps > 0;
-    const int group = a.heads_q / a.heads_kv;
-    int kt, bhi, t_begin_split = 0, slab = 0;
-    if (!split) {
-        // groups of head_group heads; inside a group tile slot major, head minor (see cta_order.h)
-        const int per_group = n_tiles * a.head_group;
-        const int hg = int(blockIdx.x) / per_group;
-        const int rem = int(blockIdx.x) - hg * per_group;
-        const int heads_here = min(a.head_group, bh_count - hg * a.head_group);
-        const int tile_slot = rem / heads_here;
-        bhi = hg * a.head_group + (rem - tile_slot * heads_here);
-        kt = remap_k_tile(tile_slot, n_tiles, a.order_mode, a.order_width);
-    } else {
-        const uint32_t entry = a.cta_table[blockIdx.x];
-        kt = int(entry & 0xffu);
-        t_begin_split = int((entry >> 8) & 0xffu) * a.chunk_steps;
-        slab = int(entry >> 16);
-        bhi = slab / a.chunks_per_head;
-    }
-    const int b = bhi / a.heads_kv;
-    const int kvh = bhi % a.heads_kv;
-    // Packed sequences: this batch entry's own lengths and first rows; tensors are addressed as one
-    // batch of `total` rows, so rows past the end of a sequence belong to its neighbour (or read as
-    // zero past the end of the tensor) and are masked like any ragged tile end.
-    Band band = a.band;
-    int q_base = 0, k_base = 0, b_coord = b;
-    if (a.cu_seqlens_q != nullptr) {
-        q_base = a.cu_seqlens_q[b];
-        k_base = a.cu_seqlens_k[b];
-        band.seqlen_q = a.cu_seqlens_q[b + 1] - q_base;
-        band.seqlen_k = a.cu_seqlens_k[b + 1] - k_base;
-        band.off = band.seqlen_k - band.seqlen_q;
-        b_coord = 0;
-    }
-    const int slot_k = band.seqlen_k;  // rows of dK / dV this batch entry owns
-    if (a.seqused_q != nullptr || a.seqused_k != nullptr) {
-        if (a.seqused_q != nullptr) band.seqlen_q = max(0, min(band.seqlen_q, a.seqused_q[b]));
-        if (a.seqused_k != nullptr) band.seqlen_k = max(0, min(band.seqlen_k, a.seqused_k[b]));
-        band.off = band.seqlen_k - band.seqlen_q;
-    }
-    const int n_q_tiles = tiles_of(band.seqlen_q);
-    const bool tile_exists = kt * C::kTile < band.seqlen_k;  // false only with packed sequences
-    const int q_begin = first_q_tile(kt, band);
-    const int steps_per_head = tile_exists ? q_tiles_of_k_tile(kt, band) : 0;
-    // this CTA's share of the tile's steps (all of them unless the tile is split)
-    const int total_steps = group * steps_per_head;
-    const int t_begin = t_begin_split;
-    const int t_end = split ? min(total_steps, t_begin + a.chunk_steps) : total_steps;
-    const int n_steps = t_end - t_begin;
-    // "misaligned" also covers a CTA without work: every role is skipped, set-up and teardown still run
-    const bool misaligned = (sbase & 1023u) != 0 || n_steps == 0;
-    // an unsplit key tile that no query sees (possible with a left-bounded window) still owes zeros
-    // to dK / dV
-    const bool owes_zeros = !split && n_steps == 0 && (sbase & 1023u) == 0;
-
+    const bool misaligned = (sbase & 1023u) != 0;
     if (threadIdx.x == 0) {
         TRACE(0, 4);
-        if ((sbase & 1023u) != 0) atomicCAS(&g_device_error, kDevOk, kDevSmemMisaligned);
+        if (misaligned) atomicCAS(&g_device_error, kDevOk, kDevSmemMisaligned);
         ptx::mbar_init(bar(kKvFull), 1);
         for (int s = 0; s < 2; ++s) {
             ptx::mbar_init(bar(kQFull + s), 1);
@@ -360,13 +421,17 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             ptx::mbar_init(bar(kDoFull + s), 1);
             ptx::mbar_init(bar(kDoEmpty + s), 1);
         }
-        for (int s = 0; s < 2; ++s) ptx::mbar_init(bar(kStatsFull + s), 128);  // (unused with three buffers)
+        // (the math warps arrive once per warp)
+        for (int s = 0; s < 2; ++s) {
+            ptx::mbar_init(bar(kStatsFull + s), 1);
+            ptx::mbar_init(bar(kStatsEmpty + s), 8);
+        }
         ptx::mbar_init(bar(kSFull), 1);
         ptx::mbar_init(bar(kDpFull), 1);
-        ptx::mbar_init(bar(kPReady), 256);
-        ptx::mbar_init(bar(kDsReady), 256);
+        ptx::mbar_init(bar(kPReady), 8);
+        ptx::mbar_init(bar(kDsReady), 8);
         ptx::mbar_init(bar(kDqFull), 1);
-        ptx::mbar_init(bar(kDqEmpty), 128);
+        ptx::mbar_init(bar(kDqEmpty), 4);
         ptx::mbar_init(bar(kDkvFull), 1);
         flag_set(abort_flag, 0);
         ptx::fence_mbar_init();
@@ -376,33 +441,23 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         ptx::tmem_alloc(tmem_slot, C::kTmemCols);
         ptx::tmem_relinquish();
     }
-    ptx::tc_fence_before();
-    __syncthreads();
-    ptx::tc_fence_after();
-    const uint32_t tmem = flag_value(tmem_slot);
     // The kernel behind this one (dQ convert) may begin to launch; it waits for our completion itself.
     ptx::launch_dependents();
-
-    // Query tiles are visited in ascending order starting at the diagonal (causal) or at a
-    // per-CTA rotation (non-causal), so that CTAs of one head that run together add into
-    // different dQ tiles at any moment.
-    const int rotation = (kCausal || n_q_tiles == 0) ? 0 : kt % n_q_tiles;
-    auto step_coords = [&](int t_local, int& hq, int& qt) {
-        const int t = t_begin + t_local;
-        const int g = t / steps_per_head;
-        hq = kvh * group + g;
-        const int r = t - g * steps_per_head;
-        if (kCausal) {
-            qt = q_begin + r;
-        } else {
-            qt = r + rotation;
-            if (qt >= n_q_tiles) qt -= n_q_tiles;
-        }
+    // (all threads: barriers initialised, tensor memory allocated)
+    auto set_up_done = [&] {
+        ptx::tc_fence_before();
+        asm volatile("bar.sync 0;" ::: "memory");
+        ptx::tc_fence_after();
+        return flag_value(tmem_slot);
     };
 
     if (wg == 0) {
         ptx::setmaxnreg_dec<C::kRegsControl>();
-        if (!misaligned && warp == 0) {
+        const FusedWork w = fused_work<kCausal>(a);
+        const uint32_t tmem = set_up_done();
+        const bool idle = misaligned || w.n_steps == 0;  // a CTA without work: set-up and teardown still run
+        const int n_steps = w.n_steps;
+        if (!idle && warp == 0) {
             // =================================================== TMA producer
             if (lane == 0) {
                 ptx::prefetch_tensormap(&tm_q);
@@ -414,23 +469,23 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
                 for (int bx = 0; bx < C::kBoxes; ++bx) {
                     ptx::tma_load_4d(sbase + C::kOffK + bx * C::kBoxBytes, &tm_k, bar(kKvFull), bx * 64,
-                                     k_base + kt * C::kTile, kvh, b_coord);
+                                     w.k_base + w.kt * C::kTile, w.kvh, w.b_coord);
                     ptx::tma_load_4d(sbase + C::kOffV + bx * C::kBoxBytes, &tm_v, bar(kKvFull), bx * 64,
-                                     k_base + kt * C::kTile, kvh, b_coord);
+                                     w.k_base + w.kt * C::kTile, w.kvh, w.b_coord);
                 }
                 TRACE(0, 3);
+                StepWalk<kCausal> st(w);
 #pragma unroll 1
-                for (int t = 0; t < n_steps; ++t) {
-                    int hq, qt;
-                    step_coords(t, hq, qt);
-                    const int q_row = q_base + qt * C::kTile;
+                for (int t = 0; t < n_steps; ++t, st.next(w)) {
+                    const int hq = st.hq;
+                    const int q_row = w.q_base + st.qt * C::kTile;
                     const int s = t % C::kQStages;
                     if (!bounded_wait<true>(bar(kQEmpty + s), ((t / C::kQStages) & 1) ^ 1, abort_flag)) break;
                     ptx::mbar_arrive_expect_tx(bar(kQFull + s), C::kOperandBytes);
 #pragma unroll
                     for (int bx = 0; bx < C::kBoxes; ++bx) {
                         ptx::tma_load_4d(sbase + C::kOffQ + s * C::kOperandBytes + bx * C::kBoxBytes, &tm_q,
-                                         bar(kQFull + s), bx * 64, q_row, hq, b_coord);
+                                         bar(kQFull + s), bx * 64, q_row, hq, w.b_coord);
                     }
                     const int sd = t % C::kDoStages;
                     if (!bounded_wait<true>(bar(kDoEmpty + sd), ((t / C::kDoStages) & 1) ^ 1, abort_flag)) break;
@@ -438,11 +493,11 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
                     for (int bx = 0; bx < C::kBoxes; ++bx) {
                         ptx::tma_load_4d(sbase + C::kOffDO + sd * C::kOperandBytes + bx * C::kBoxBytes, &tm_do,
-                                         bar(kDoFull + sd), bx * 64, q_row, hq, b_coord);
+                                         bar(kDoFull + sd), bx * 64, q_row, hq, w.b_coord);
                     }
                 }
             }
-        } else if (!misaligned && warp == 1) {
+        } else if (!idle && warp == 1) {
             // ===================================================== MMA issuer
             // The whole warp runs this role converged; MMAs and commits elect their lane inside the asm.
             {
@@ -540,100 +595,93 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 TRACE(1, 62);
             }
         }
+        else if (!idle && warp == 2) {
+            // ============================================== row statistics
+            // One warp fetches the statistics of the next step's 128 query rows while the math warps work and
+            // hands them over in shared memory, two steps deep.  (A softmax warpgroup that fetched its own spent
+            // 300-700 clk of every step on it.)  P = exp2(x - m) * r = exp2(x + (log2 r - m)); a row past the end
+            // of the sequence gets -inf, which makes its P, and with it dS, exactly zero.
+            // The statistics come from the delta kernel, which may still be running (programmatic launch); Q, K,
+            // V, dO are inputs of the call, so the TMA and MMA warps did not have to wait.
+            ptx::grid_dependency_wait();
+            float* stats = reinterpret_cast<float*>(smem + C::kOffStats);
+            float neg[4], ndel[4];
+            auto fetch = [&](const StepWalk<kCausal>& st) {
+                const int64_t row0 = int64_t(w.b_coord * a.heads_q + st.hq) * a.sidecar_rows + w.q_base;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int qi = st.qt * C::kTile + k * 32 + lane;
+                    const bool valid = !kCausal || qi < w.band.seqlen_q;
+                    neg[k] = -INFINITY;
+                    ndel[k] = 0.0f;
+                    if (valid && a.stats != nullptr) {
+                        const float2 v = a.stats[row0 + qi];
+                        neg[k] = v.x;
+                        ndel[k] = v.y;
+                    } else if (valid) {
+                        const float* v = a.sidecar + (row0 + qi) * 3;
+                        neg[k] = __log2f(v[1]) - v[0];
+                        ndel[k] = -v[2];
+                    }
+                }
+            };
+            StepWalk<kCausal> st(w);
+            fetch(st);
+#pragma unroll 1
+            for (int t = 0; t < n_steps; ++t) {
+                const int buf = t & 1;
+                if (!warp_wait(bar(kStatsEmpty + buf), ((t >> 1) & 1) ^ 1, abort_flag)) break;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    stats[buf * 128 + k * 32 + lane] = neg[k];
+                    stats[256 + buf * 128 + k * 32 + lane] = ndel[k];
+                }
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar(kStatsFull + buf));
+                if (t + 1 < n_steps) {
+                    st.next(w);
+                    fetch(st);
+                }
+            }
+        }
     } else if (wg == 1 || wg == 2) {
         // ============================================ softmax / dS warpgroups
         if (C::kRegsCompute < 128) ptx::setmaxnreg_dec<C::kRegsCompute>();
         else ptx::setmaxnreg_inc<C::kRegsCompute>();
-        if (!misaligned) {
+        const FusedWork w = fused_work<kCausal>(a);
+        const uint32_t tmem = set_up_done();
+        const bool idle = misaligned || w.n_steps == 0;  // a CTA without work: set-up and teardown still run
+        const int n_steps = w.n_steps;
+        if (!idle) {
             const int half = wg - 1;          // which 64 queries of the tile
             const int j = threadIdx.x & 127;  // key row inside the tile == TMEM lane
             const uint32_t tl = tmem + (uint32_t((warp & 3) * 32) << 16);
             const uint32_t s_cols = tl + C::kColS + half * 64;
             const uint32_t dp_cols = tl + C::kColDP + half * 64;
-            float* stats = reinterpret_cast<float*>(smem + C::kOffStats);
+            const uint32_t stats = sbase + C::kOffStats + half * 256;  // this half's 64 queries
+            const uint64_t scale2 = ptx::f2_pack(a.scale_log2, a.scale_log2);
             uint32_t ppk[32];
-            const float* side_base = a.sidecar;
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-            bool s_valid = false;
-            // Statistics of query row qi of head hq, fetched one step ahead.  The loaded values are
-            // not touched here (their first use, one step later, is what waits for the loads); rows
-            // past the end of the sequence read row 0 instead and are replaced at that first use.
-            auto load_stats = [&](int hq, int qt) {
-                const int qi = qt * C::kTile + j;
-                s_valid = qi < band.seqlen_q;
-                const int64_t row = int64_t(b_coord * a.heads_q + hq) * a.sidecar_rows + q_base + (s_valid ? qi : 0);
-                s0 = side_base[row * 3 + 0];
-                s1 = side_base[row * 3 + 1];
-                s2 = side_base[row * 3 + 2];
+            // one arrival per warp: every lane's accesses are ordered before it by the fence and the warp barrier
+            auto arrive = [&](int which) {
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar(which));
             };
-            // the sidecar comes from the delta kernel, which may still be running (programmatic launch);
-            // Q, K, V, dO are inputs of the call, so the TMA and MMA warps did not have to wait
-            ptx::grid_dependency_wait();
-            constexpr int kNB = C::kStatsBufs;
-            constexpr bool kStatsAhead = kNB == 3;
-            // row statistics of query row j of a tile, for both warpgroups:
-            // P = exp2(x - m) * r = exp2(x + (log2 r - m)); a row past the end of the sequence
-            // gets -inf, which makes its P (and with it dS) exactly zero
-            auto publish_stats = [&](int buf) {
-                stats[buf * 128 + j] = (!kCausal || s_valid) ? __log2f(s1) - s0 : -INFINITY;
-                stats[kNB * 128 + buf * 128 + j] = (!kCausal || s_valid) ? s2 : 0.f;
-                if (!kStatsAhead) ptx::mbar_arrive(bar(kStatsFull + buf));
-            };
-            if (half == 0) {
-                int hq, qt;
-                step_coords(0, hq, qt);
-                load_stats(hq, qt);
-                if (kStatsAhead) {
-                    publish_stats(0);
-                    if (n_steps > 1) {
-                        step_coords(1, hq, qt);
-                        load_stats(hq, qt);
-                    }
-                }
-            }
-            // (step 0's statistics are the exception: one meeting of the two warpgroups)
-            if (kStatsAhead) asm volatile("bar.sync 1, 256;" ::: "memory");
             bool ok = true;
+            StepWalk<kCausal> st(w);
 #pragma unroll 1
-            for (int t = 0; t < n_steps; ++t) {
+            for (int t = 0; t < n_steps; ++t, st.next(w)) {
                 if (warp == 4 && t == 3) TRACE(2, 0);
-                int hq, qt;
-                step_coords(t, hq, qt);
-                if (warp == 4 && t == 3) TRACE(2, 1);
-                const int buf = t % kNB;
-                const float* negp = stats + buf * 128 + half * 64;
-                const float* delp = stats + kNB * 128 + buf * 128 + half * 64;
-                if (half == 0) {
-                    if (kStatsAhead) {
-                        // the registers hold step t+1: publish it now (its buffer was last read in step
-                        // t-2, which every warp has left: this warpgroup could not have written dS(t-1)
-                        // before dS(t-2) of both was consumed), then fetch step t+2
-                        if (t + 1 < n_steps) publish_stats((t + 1) % kNB);
-                        if (warp == 4 && t == 3) TRACE(2, 2);
-                    } else {
-                        publish_stats(buf);
-                        if (warp == 4 && t == 3) TRACE(2, 2);
-                        if (t + 1 < n_steps) {
-                            int hq1, qt1;
-                            step_coords(t + 1, hq1, qt1);
-                            load_stats(hq1, qt1);
-                        }
-                    }
-                }
-                if (warp == 4 && t == 3) TRACE(2, 3);
-                // Published one step ahead, the statistics of step t need no barrier of their own: their
-                // writers arrived at "P ready" of step t-1 after writing them, S(t) was issued after that
-                // barrier completed, and every reader waits for S(t) below.
-                if (!kStatsAhead) {
-                    if (!(ok = warp_wait(bar(kStatsFull + buf), (t / kNB) & 1, abort_flag))) break;
-                }
-                if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 0);
-                if (!(ok = warp_wait(bar(kSFull), t & 1, abort_flag))) break;
+                const int qt = st.qt;
+                const int buf = t & 1;
+                const uint32_t negp = stats + buf * 512;
+                const uint32_t delp = stats + 1024 + buf * 512;
+                if (!(ok = warp_wait2(bar(kStatsFull + buf), (t >> 1) & 1, bar(kSFull), t & 1, abort_flag))) break;
                 if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 1);
                 ptx::tc_fence_after();
-                // A tile that crosses an edge of the band or holds keys past the end of the sequence is
+                // A tile that crosses an edge of the w.band or holds keys past the end of the sequence is
                 // masked: element (key j, query i) survives iff mask_from <= i <= mask_to.
-                const bool diagonal = kCausal && tile_needs_mask(kt, qt, band);
+                const bool diagonal = kCausal && tile_needs_mask(w.kt, qt, w.band);
                 int mask_from = 0, mask_to = 0;  // set only on masked tiles
                 // ---- P^T = exp2(S^T * scale_log2 + neg_i), masked as above.
                 // (two copies of the chunk code, so that unmasked tiles carry no per-element test)
@@ -647,26 +695,37 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     constexpr bool kMasked = decltype(masked_tag)::value;
 #pragma unroll
                     for (int e = 0; e < 32; e += 4) {
-                        const float4 n4 = *reinterpret_cast<const float4*>(negp + c * 32 + e);
-                        float p0 = ptx::ex2_approx(log2_score(r[e + 0], n4.x));
-                        float p1 = ptx::ex2_approx(log2_score(r[e + 1], n4.y));
-                        float p2 = ptx::ex2_approx(log2_score(r[e + 2], n4.z));
-                        float p3 = ptx::ex2_approx(log2_score(r[e + 3], n4.w));
-                        if (kMasked) {
-                            const int i = half * 64 + c * 32 + e;
-                            p0 = (i + 0 >= mask_from && i + 0 <= mask_to) ? p0 : 0.0f;
-                            p1 = (i + 1 >= mask_from && i + 1 <= mask_to) ? p1 : 0.0f;
-                            p2 = (i + 2 >= mask_from && i + 2 <= mask_to) ? p2 : 0.0f;
-                            p3 = (i + 3 >= mask_from && i + 3 <= mask_to) ? p3 : 0.0f;
+                        const ptx::F4Pairs n4 = ptx::f2_ld_shared(negp + (c * 32 + e) * 4);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const uint64_t neg2 = h == 0 ? n4.lo : n4.hi;
+                            const int el = e + 2 * h;
+                            float2 p2;
+                            if (kSoftcap) {
+                                const float2 neg = ptx::f2_unpack(neg2);
+                                p2.x = ptx::ex2_approx(log2_score(r[el], neg.x));
+                                p2.y = ptx::ex2_approx(log2_score(r[el + 1], neg.y));
+                            } else {
+                                const uint64_t x2 = ptx::f2_fma(ptx::f2_pack(__uint_as_float(r[el]), __uint_as_float(r[el + 1])), scale2, neg2);
+                                // (exp2_poly for a part of these changed nothing: B=4,H=16,S=4096,D=64 791, 792, 795, 810 us for 0 to 3
+                                // pairs of 8)
+                                p2 = ptx::f2_unpack(x2);
+                                p2.x = ptx::ex2_approx(p2.x);
+                                p2.y = ptx::ex2_approx(p2.y);
+                            }
+                            if (kMasked) {
+                                const int i = half * 64 + c * 32 + el;
+                                p2.x = (i + 0 >= mask_from && i + 0 <= mask_to) ? p2.x : 0.0f;
+                                p2.y = (i + 1 >= mask_from && i + 1 <= mask_to) ? p2.y : 0.0f;
+                            }
+                            ppk[c * 16 + el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
                         }
-                        ppk[c * 16 + e / 2 + 0] = ptx::Pack2<T>::pack(p0, p1);
-                        ppk[c * 16 + e / 2 + 1] = ptx::Pack2<T>::pack(p2, p3);
                     }
                     // P chunk c -> columns [16c, 16c+16) of this half's S columns (already read)
                     ptx::tmem_st16(s_cols + c * 16, &ppk[c * 16]);
                 };
                 if (diagonal) {
-                    query_range_of_key(kt * C::kTile + j, qt * C::kTile, band, &mask_from, &mask_to);
+                    query_range_of_key(w.kt * C::kTile + j, qt * C::kTile, w.band, &mask_from, &mask_to);
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {
                         uint32_t r[32];
@@ -685,14 +744,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 }
                 if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 2);
                 ptx::tmem_st_wait();
-                ptx::tc_fence_before();
-                ptx::mbar_arrive(bar(kPReady));
-                if (kStatsAhead && half == 0 && t + 2 < n_steps) {
-                    // (requested here, where the warp is about to wait for dP anyway)
-                    int hq2, qt2;
-                    step_coords(t + 2, hq2, qt2);
-                    load_stats(hq2, qt2);
-                }
+                arrive(kPReady);
                 if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 3);
                 // ---- dS^T = P^T * (dP^T - delta_i), stored [key][query] in the 128-byte swizzle
                 if (!(ok = warp_wait(bar(kDpFull), t & 1, abort_flag))) break;
@@ -706,40 +758,39 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 auto ds_chunk = [&](int c, const uint32_t* r) {
 #pragma unroll
                     for (int e = 0; e < 32; e += 8) {
-                        const float4 d0 = *reinterpret_cast<const float4*>(delp + c * 32 + e);
-                        const float4 d1 = *reinterpret_cast<const float4*>(delp + c * 32 + e + 4);
-                        const float2 pa = ptx::Pack2<T>::unpack(ppk[c * 16 + e / 2 + 0]);
-                        const float2 pb = ptx::Pack2<T>::unpack(ppk[c * 16 + e / 2 + 1]);
-                        const float2 pc = ptx::Pack2<T>::unpack(ppk[c * 16 + e / 2 + 2]);
-                        const float2 pd = ptx::Pack2<T>::unpack(ppk[c * 16 + e / 2 + 3]);
-                        uint4 o;
-                        if (kSoftcap) {
-                            // dS = P (dP - delta) (1 - t^2), t recovered from P and the row's reference
-                            const float4 n0 = *reinterpret_cast<const float4*>(negp + c * 32 + e);
-                            const float4 n1 = *reinterpret_cast<const float4*>(negp + c * 32 + e + 4);
-                            auto capped = [&](float p, uint32_t dp, float del, float neg) {
-                                const float t = (__log2f(p) - neg) * inv_post;
-                                const float slope = fmaxf(1.0f - t * t, 0.0f);
-                                return p > 0.0f ? p * (__uint_as_float(dp) - del) * slope : 0.0f;
-                            };
-                            o.x = ptx::Pack2<T>::pack(capped(pa.x, r[e + 0], d0.x, n0.x), capped(pa.y, r[e + 1], d0.y, n0.y));
-                            o.y = ptx::Pack2<T>::pack(capped(pb.x, r[e + 2], d0.z, n0.z), capped(pb.y, r[e + 3], d0.w, n0.w));
-                            o.z = ptx::Pack2<T>::pack(capped(pc.x, r[e + 4], d1.x, n1.x), capped(pc.y, r[e + 5], d1.y, n1.y));
-                            o.w = ptx::Pack2<T>::pack(capped(pd.x, r[e + 6], d1.z, n1.z), capped(pd.y, r[e + 7], d1.w, n1.w));
-                        } else {
-                        o.x = ptx::Pack2<T>::pack(pa.x * (__uint_as_float(r[e + 0]) - d0.x),
-                                                  pa.y * (__uint_as_float(r[e + 1]) - d0.y));
-                        o.y = ptx::Pack2<T>::pack(pb.x * (__uint_as_float(r[e + 2]) - d0.z),
-                                                  pb.y * (__uint_as_float(r[e + 3]) - d0.w));
-                        o.z = ptx::Pack2<T>::pack(pc.x * (__uint_as_float(r[e + 4]) - d1.x),
-                                                  pc.y * (__uint_as_float(r[e + 5]) - d1.y));
-                        o.w = ptx::Pack2<T>::pack(pd.x * (__uint_as_float(r[e + 6]) - d1.z),
-                                                  pd.y * (__uint_as_float(r[e + 7]) - d1.w));
+                        uint32_t o[4];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const ptx::F4Pairs d4 = ptx::f2_ld_shared(delp + (c * 32 + e + 4 * h) * 4);  // -delta
+                            const int el = e + 4 * h;
+                            if (kSoftcap) {
+                                // dS = P (dP - delta) (1 - t^2), t recovered from P and the row's reference
+                                const ptx::F4Pairs n4 = ptx::f2_ld_shared(negp + (c * 32 + el) * 4);
+                                auto capped = [&](float p, uint32_t dp, float ndel, float neg) {
+                                    const float t = (__log2f(p) - neg) * inv_post;
+                                    const float slope = fmaxf(1.0f - t * t, 0.0f);
+                                    return p > 0.0f ? p * (__uint_as_float(dp) + ndel) * slope : 0.0f;
+                                };
+#pragma unroll
+                                for (int g = 0; g < 2; ++g) {
+                                    const float2 p = ptx::Pack2<T>::unpack(ppk[c * 16 + el / 2 + g]);
+                                    const float2 d = ptx::f2_unpack(g == 0 ? d4.lo : d4.hi), n = ptx::f2_unpack(g == 0 ? n4.lo : n4.hi);
+                                    o[2 * h + g] = ptx::Pack2<T>::pack(capped(p.x, r[el + 2 * g], d.x, n.x), capped(p.y, r[el + 2 * g + 1], d.y, n.y));
+                                }
+                            } else {
+#pragma unroll
+                                for (int g = 0; g < 2; ++g) {
+                                    const float2 p = ptx::Pack2<T>::unpack(ppk[c * 16 + el / 2 + g]);
+                                    const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[el + 2 * g]), __uint_as_float(r[el + 2 * g + 1]));
+                                    const float2 ds = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, g == 0 ? d4.lo : d4.hi)));
+                                    o[2 * h + g] = ptx::Pack2<T>::pack(ds.x, ds.y);
+                                }
+                            }
                         }
                         const int chunk = c * 4 + e / 8;  // 16-byte chunk inside this half's box
                         const uint32_t addr = ds_row + ((chunk ^ (j & 7)) << 4);
-                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(o.x),
-                                     "r"(o.y), "r"(o.z), "r"(o.w) : "memory");
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(o[0]),
+                                     "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
                     }
                 };
 #pragma unroll
@@ -751,8 +802,8 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 }
                 if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 6);
                 ptx::fence_proxy_async_smem();
-                ptx::tc_fence_before();
-                ptx::mbar_arrive(bar(kDsReady));
+                arrive(kDsReady);
+                if (lane == 0) ptx::mbar_arrive(bar(kStatsEmpty + buf));
                 if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 7);
             }
             // ---- epilogue: the first warpgroup writes dK (scaled), the second dV
@@ -770,9 +821,10 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 const int w4 = warp & 3;  // which 32 rows of the tile
                 // packed sequences: the rows behind this sequence's end belong to its neighbour, which the
                 // copy engine cannot know; fp32 outputs of the split path: plain rows.  Both keep per-thread stores.
+                const bool split = a.chunk_steps > 0;
                 const bool staged = split || (sizeof(TOut) == 2 && a.cu_seqlens_q == nullptr);
                 if (staged && split && !kBf16) {
-                    // fp16 inputs: the partial sums go to this CTA's slabs (slab 2x: dK, 2x+1: dV) as fp16,
+                    // fp16 inputs: the partial sums go to this CTA's slabs (w.slab 2x: dK, 2x+1: dV) as fp16,
                     // boxes of [32 rows][64 x 16 bit].  (fp16 keeps 11 significant bits, three more than a
                     // bf16 result would; the bytes written, not the arithmetic, bound this epilogue.)
                     const uint32_t scratch = sbase + C::kOffQ + (half * 4 + w4) * (C::kBoxes * C::kStageBoxBytes);
@@ -799,7 +851,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     if (lane == 0) {
 #pragma unroll
                         for (int bx = 0; bx < C::kBoxes; ++bx)
-                            ptx::tma_store_4d(&tm_dk, scratch + bx * C::kStageBoxBytes, bx * 64, w4 * 32, slab * 2 + half, 0);
+                            ptx::tma_store_4d(&tm_dk, scratch + bx * C::kStageBoxBytes, bx * 64, w4 * 32, w.slab * 2 + half, 0);
                         ptx::bulk_commit_group();
                         ptx::bulk_wait_group_read<0>();
                     }
@@ -828,7 +880,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
                         for (int c = 0; c < kBoxesPerWarp; ++c)
                             ptx::tma_store_3d(&tm_dk, scratch + c * C::kStageBoxBytes, c * 32, w4 * 32,
-                                              slab * 2 + half);
+                                              w.slab * 2 + half);
                         ptx::bulk_commit_group();
                         ptx::bulk_wait_group_read<0>();
                     }
@@ -861,7 +913,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
                         for (int bx = 0; bx < C::kBoxes; ++bx)
                             ptx::tma_store_4d(map, scratch + bx * C::kStageBoxBytes, bx * 64,
-                                              kt * C::kTile + w4 * 32, kvh, b);
+                                              w.kt * C::kTile + w4 * 32, w.kvh, w.b);
                         ptx::bulk_commit_group();
                         ptx::bulk_wait_group_read<0>();
                     }
@@ -869,9 +921,9 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     // (tensor-memory loads are warp-wide: every lane runs them, only the stores of key rows
                     // past the end of the sequence are skipped)
                     // (rows between the used length and the end of the slot hold exact zeros)
-                    const bool key_valid = kt * C::kTile + j < slot_k;
-                    const int64_t off = b_coord * a.kv_strides.batch + kvh * a.kv_strides.head +
-                                        int64_t(k_base + kt * C::kTile + j) * a.kv_strides.row;
+                    const bool key_valid = w.kt * C::kTile + j < w.slot_k;
+                    const int64_t off = w.b_coord * a.kv_strides.batch + w.kvh * a.kv_strides.head +
+                                        int64_t(w.k_base + w.kt * C::kTile + j) * a.kv_strides.row;
                     TOut* dst = reinterpret_cast<TOut*>(half == 0 ? a.dk : a.dv) + off;
 #pragma unroll
                     for (int c = 0; c < D / 32; ++c) {
@@ -903,12 +955,12 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 }
             }
             if (warp == 4) TRACE(2, 61);
-        } else if (owes_zeros) {
-            // nobody attends to these keys: the first warpgroup clears dK, the second dV
+        } else if (!misaligned && a.chunk_steps == 0) {
+            // nobody attends to these keys (possible with a left-bounded window), but dK / dV still owe zeros: the first warpgroup clears dK, the second dV
             const int j = threadIdx.x & 127;
-            if (kt * C::kTile + j < slot_k) {
-                const int64_t off = b_coord * a.kv_strides.batch + kvh * a.kv_strides.head +
-                                    int64_t(k_base + kt * C::kTile + j) * a.kv_strides.row;
+            if (w.kt * C::kTile + j < w.slot_k) {
+                const int64_t off = w.b_coord * a.kv_strides.batch + w.kvh * a.kv_strides.head +
+                                    int64_t(w.k_base + w.kt * C::kTile + j) * a.kv_strides.row;
                 uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<TOut*>(wg == 1 ? a.dk : a.dv) + off);
 #pragma unroll
                 for (int e = 0; e < int(D * sizeof(TOut) / 16); ++e) d4[e] = make_uint4(0u, 0u, 0u, 0u);
@@ -918,21 +970,25 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // ==================================================== dQ drain warpgroup
         if (!kWithDq) {
             ptx::setmaxnreg_dec<C::kRegsControl>();
+            set_up_done();
         } else {
             ptx::setmaxnreg_inc<C::kRegsDrain>();
-            if (!misaligned) {
+            const FusedWork w = fused_work<kCausal>(a);
+            const uint32_t tmem = set_up_done();
+            const bool idle = misaligned || w.n_steps == 0;  // a CTA without work: set-up and teardown still run
+            const int n_steps = w.n_steps;
+            if (!idle) {
                 const int qd = warp & 3;
                 const uint32_t tl = tmem + (uint32_t(qd * 32) << 16);
                 const uint32_t stage = sbase + C::kOffStage + qd * 2 * C::kStageBoxBytes;
                 bool pending = false;
                 // the accumulators are cleared by the delta kernel: do not add into them before it is done
                 ptx::grid_dependency_wait();
+                StepWalk<kCausal> st(w);
 #pragma unroll 1
-                for (int t = 0; t < n_steps; ++t) {
-                    int hq, qt;
-                    step_coords(t, hq, qt);
-                    const int q_row = qt * C::kTile + qd * 32;  // row inside the head
-                    const int q_head = b_coord * a.heads_q + hq;
+                for (int t = 0; t < n_steps; ++t, st.next(w)) {
+                    const int q_row = st.qt * C::kTile + qd * 32;  // row inside the head
+                    const int q_head = w.b_coord * a.heads_q + st.hq;
                     if (!warp_wait(bar(kDqFull), t & 1, abort_flag)) break;
                     if (warp == 12 && t < 12) TRACE(3, 4 + 4 * t + 0);
                     ptx::tc_fence_after();
@@ -942,7 +998,8 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     for (int c = 0; c < D / 32; ++c) ptx::tmem_ld32(tl + C::kColDQ + c * 32, r[c]);
                     ptx::tmem_ld_wait();
                     ptx::tc_fence_before();
-                    ptx::mbar_arrive(bar(kDqEmpty));
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(bar(kDqEmpty));
                     if (warp == 12 && t < 12) TRACE(3, 4 + 4 * t + 1);
 #pragma unroll
                     for (int hf = 0; hf < D / 64; ++hf) {
@@ -965,9 +1022,9 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                         ptx::fence_proxy_async_smem();
                         __syncwarp();
                         // accumulator map: [batch*head][row][D]; rows past the sequence end are dropped
-                        if (lane == 0 && q_row < band.seqlen_q) {
-                            ptx::tma_reduce_add_3d(&tm_dqacc, stage, hf * 64, q_base + q_row, q_head);
-                            ptx::tma_reduce_add_3d(&tm_dqacc, stage + C::kStageBoxBytes, hf * 64 + 32, q_base + q_row, q_head);
+                        if (lane == 0 && q_row < w.band.seqlen_q) {
+                            ptx::tma_reduce_add_3d(&tm_dqacc, stage, hf * 64, w.q_base + q_row, q_head);
+                            ptx::tma_reduce_add_3d(&tm_dqacc, stage + C::kStageBoxBytes, hf * 64 + 32, w.q_base + q_row, q_head);
                             ptx::bulk_commit_group();
                         }
                         pending = true;
@@ -987,7 +1044,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     __syncthreads();
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem, C::kTmemCols);
+        ptx::tmem_dealloc(flag_value(tmem_slot), C::kTmemCols);
     }
     if (threadIdx.x == 0) {
         TRACE(0, 63);

@@ -51,7 +51,8 @@ __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, float hi) {
 // and of O, so a warp reads 512 contiguous bytes per tensor per instruction.
 // When zero_rows is non-null the same lanes also clear the row of the fp32 dQ
 // accumulator (row pitch D floats), which saves a separate memset pass.  The
-// sidecar is optional (null: only delta is written).
+// v2 call gets {log2 r - m, -delta} per row instead of the sidecar (stats
+// non-null), the form its kernels use.
 //
 // Rows are numbered in [batch, head, row] order (the order of aux0, delta and
 // the sidecar); RowLayout says where row r of dO and O lives, so that both the
@@ -80,7 +81,7 @@ template <typename T, int D, bool kLseInput>
 __global__ void __launch_bounds__(256)
 delta_sidecar_kernel(const T* __restrict__ dout, const T* __restrict__ out,
                      const float* __restrict__ aux0, const float* __restrict__ aux1,
-                     float* __restrict__ delta, float* __restrict__ sidecar,
+                     float* __restrict__ delta, float* __restrict__ sidecar, float2* __restrict__ stats,
                      float* __restrict__ zero_rows, int64_t rows, float scale_log2, RowLayout layout) {
     constexpr int kLanesPerRow = D / 8;
     constexpr int kRowsPerWarp = 32 / kLanesPerRow;
@@ -132,7 +133,7 @@ delta_sidecar_kernel(const T* __restrict__ dout, const T* __restrict__ out,
             }
         }
         if (valid && col == 0) delta[row] = acc;
-        if (valid && col == 0 && sidecar != nullptr) {
+        if (valid && col == 0 && (sidecar != nullptr || stats != nullptr)) {
             float m, r;
             if (kLseInput) {
                 m = aux0[row] * kLog2E;
@@ -146,10 +147,14 @@ delta_sidecar_kernel(const T* __restrict__ dout, const T* __restrict__ out,
                 m = 0.0f;
                 r = 0.0f;
             }
-            float* s = sidecar + row * 3;
-            s[0] = m;
-            s[1] = r;
-            s[2] = acc;
+            if (stats != nullptr) {
+                stats[row] = make_float2(__log2f(r) - m, -acc);
+            } else {
+                float* s = sidecar + row * 3;
+                s[0] = m;
+                s[1] = r;
+                s[2] = acc;
+            }
         }
     }
 #ifdef FA3B200_TRACE

@@ -4,6 +4,7 @@
 // without a GPU.  Behaviour follows reference src/shaobo_fa3_bwd_api.cpp
 // (validation order and status codes, lines 70-120; workspace carving, lines
 // 122-156), widened to BF16 and head_dim 64.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -144,9 +145,9 @@ SplitPlan split_plan(const ShaoboFa3Params* p) {
     const int tiles = tiles_of(p->seqlen_k);
     const Band band = band_of(p);
     const long long heads = (long long)p->batch * p->num_heads_kv;
-    if (tiles * heads >= kSplitSmCount) return SplitPlan{};
+    if (tiles * heads >= kMaxSplitCtas || tiles > kSplitSmCount) return SplitPlan{};
     const long long group = p->num_heads_q / p->num_heads_kv;
-    const SplitKey key{band.seqlen_q, band.seqlen_k, band.left, band.right, band.off, heads, group};
+    const SplitKey key{band.seqlen_q, band.seqlen_k, band.left, band.right, p->head_dim_qk * 2 + (p->dtype == SHAOBO_FA3_DTYPE_FP16), heads, group};
     {
         std::lock_guard<std::mutex> lock(g_split_mu);
         auto it = g_split_cache.find(key);
@@ -160,7 +161,6 @@ SplitPlan split_plan(const ShaoboFa3Params* p) {
 }
 
 static SplitPlan search_split_plan(const ShaoboFa3Params* p, int tiles, const Band& band, long long heads, long long group) {
-    (void)p;
     SplitPlan plan;
     long long longest = 0;  // steps of the heaviest key tile
     for (int kt = 0; kt < tiles; ++kt) {
@@ -205,6 +205,28 @@ static SplitPlan search_split_plan(const ShaoboFa3Params* p, int tiles, const Ba
         }
     }
     if (plan.chunk_steps >= longest) return SplitPlan{};  // a chunk as long as the heaviest tile is no split at all
+    if (tiles * heads >= kSplitSmCount) {
+        // Every SM has a tile anyway: splitting pays only where the last wave is nearly empty (160 equal tiles of 40
+        // steps: 174 half steps unsplit, 123 in chunks of 17), and the partial sums are many.  They are counted at what
+        // writing and reading them costs the whole GPU: about 4 MB per half step (1 us).
+        std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free_at;
+        for (int i = 0; i < kSplitSmCount; ++i) free_at.push(0);
+        std::vector<long long> steps_of;
+        for (int kt = 0; kt < tiles; ++kt) steps_of.push_back(group * q_tiles_of_k_tile(kt, band));
+        std::sort(steps_of.begin(), steps_of.end(), std::greater<long long>());
+        long long unsplit = 0;
+        for (const long long n : steps_of) {
+            for (long long h = 0; h < heads; ++h) {
+                const long long end = free_at.top() + 7 + 2 * n;
+                free_at.pop();
+                free_at.push(end);
+                unsplit = std::max(unsplit, end);
+            }
+        }
+        const long long slab_bytes = 2LL * kSequenceAlignment * p->head_dim_qk * (p->dtype == SHAOBO_FA3_DTYPE_FP16 ? 2 : 4);
+        const long long sums = 2 * slab_bytes * plan.chunks_per_head * heads / (4 << 20);
+        if ((best_cost + sums) * 10 > unsplit * 9) return SplitPlan{};
+    }
     return plan;
 }
 

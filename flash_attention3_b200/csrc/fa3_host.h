@@ -64,8 +64,9 @@ bool fused_shape_ok(const ShaoboFa3Params* p);
 size_t dq_accum_bytes(const ShaoboFa3Params* p);
 
 // Splitting of key tiles on small problems.  Shapes with fewer (batch x KV head x key tile) units
-// than a B200 has SMs would leave most of the chip idle, so the query steps of every key tile are
-// cut into chunks of `chunk_steps` steps, one CTA per chunk; every CTA writes its dK/dV partial sums
+// than a B200 has SMs would leave most of the chip idle (and up to 511 units the last wave may be
+// nearly empty: those are split where the model below gains more than the partial sums cost), so the
+// query steps of every key tile are cut into chunks of `chunk_steps` steps, one CTA per chunk; every CTA writes its dK/dV partial sums
 // to its own fp32 slab and the convert kernel adds the slabs of a tile in chunk order.  The chunk
 // size is the one with the smallest modelled makespan when the CTAs, longest first, are handed to
 // 148 SMs as they free up (a CTA costs a fixed part worth 3.5 steps plus its steps); that may be

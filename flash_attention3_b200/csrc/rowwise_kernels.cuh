@@ -167,7 +167,7 @@ delta_sidecar_kernel(const T* __restrict__ dout, const T* __restrict__ out,
 // per-CTA slabs its chunks wrote ([128 rows][D] fp32 each, dK slab then dV slab per CTA), added here
 // in chunk order, so these two outputs do not depend on the order in which the CTAs ran.  The slabs
 // hold fp16 when the inputs are fp16 and fp32 when they are bf16.
-constexpr int kMaxSplitTiles = 148;  // tiles are only split while tiles x heads < 148
+constexpr int kMaxSplitTiles = 148;  // heads with more key tiles are not split
 struct ConvertSegments {
     const float* src[3];   // [0]: fp32 dQ accumulator [batch, head, row, D] contiguous; [1],[2] unused
     void* dst[3];

@@ -120,3 +120,16 @@ def test_softcap(b, hq, hkv, sq, sk, d, dtype, causal, window, softcap, determin
         ref_lse = prob.ref["lse"]
         finite = np.isfinite(ref_lse)
         assert np.abs(host(lse)[finite] - ref_lse[finite]).max() <= 3e-3
+
+
+# (b, hq, hkv, s, d, dtype, causal): at least 148 key tiles, split all the same because the last wave is nearly empty
+MANY_TILES_SPLIT = [
+    (1, 100, 25, 700, 64, "bf16", False),    # 150 tiles as 300 CTAs, fp32 partial sums
+    (1, 100, 25, 700, 128, "fp16", True),    # 150 tiles as 200 CTAs of unequal length, fp16 partial sums
+]
+
+
+@pytest.mark.parametrize("b,hq,hkv,s,d,dtype,causal", MANY_TILES_SPLIT)
+def test_split_with_a_nearly_empty_last_wave(b, hq, hkv, s, d, dtype, causal):
+    prob = Problem(b, hq, hkv, s, d, dtype, causal, seed=4321 + s)
+    assert_parity(run_v2(prob), prob, label=f"{(b, hq, hkv, s, d, dtype, causal)}")

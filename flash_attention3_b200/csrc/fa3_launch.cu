@@ -457,8 +457,11 @@ FusedLaunch prepare_fused(const ShaoboFa3Params* p, const void* dout, const void
     const int bh = p->batch * p->num_heads_kv;
     const int group = p->num_heads_q / p->num_heads_kv;
     // bytes of dQ accumulator behind one (batch, KV head): only the fused path adds into it
+    // (packed sequences are planned as if all were the longest one: grouping heads for the L2 then costs more balance
+    // than the model sees, so they are issued heaviest tile first over everything while the accumulators fit in the L2)
+    const bool packed_in_l2 = is_varlen(p) && p->total_q * p->num_heads_q * p->head_dim_qk * 4 <= (128LL << 20);
     const long long dq_bytes_per_head =
-        with_dq ? (long long)group * plan_seqlen_q(p) * p->head_dim_qk * 4 : 0;
+        with_dq && !packed_in_l2 ? (long long)group * plan_seqlen_q(p) * p->head_dim_qk * 4 : 0;
     const CtaOrderPlan plan = cached_plan(work, bh, group, sm_count(), dq_bytes_per_head);
     args.stats = stats;
     args.sidecar = sidecar;

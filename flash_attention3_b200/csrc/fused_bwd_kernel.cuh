@@ -659,7 +659,10 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const uint32_t s_cols = tl + C::kColS + half * 64;
             const uint32_t dp_cols = tl + C::kColDP + half * 64;
             const uint32_t stats = sbase + C::kOffStats + half * 256;  // this half's 64 queries
-            const uint64_t scale2 = ptx::f2_pack(a.scale_log2, a.scale_log2);
+            // what a raw score is multiplied with: scale*log2e, or, capped, what makes it 2*log2e * (argument of tanh)
+            const float score_mul = kSoftcap ? a.softcap_pre * ptx::kTanhArg : a.scale_log2;
+            const uint64_t scale2 = ptx::f2_pack(score_mul, score_mul);
+            const uint64_t post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
             uint32_t ppk[32];
             // one arrival per warp: every lane's accesses are ordered before it by the fence and the warp barrier
             auto arrive = [&](int which) {
@@ -685,12 +688,6 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 int mask_from = 0, mask_to = 0;  // set only on masked tiles
                 // ---- P^T = exp2(S^T * scale_log2 + neg_i), masked as above.
                 // (two copies of the chunk code, so that unmasked tiles carry no per-element test)
-                // score in log2 units, relative to the row's reference: s * scale*log2e + (log2 r - m), or the
-                // capped score + (log2 r - m)
-                auto log2_score = [&](uint32_t raw, float neg) {
-                    return kSoftcap ? fmaf(a.softcap_post, ptx::tanh_approx(__uint_as_float(raw) * a.softcap_pre), neg)
-                                    : fmaf(__uint_as_float(raw), a.scale_log2, neg);
-                };
                 auto softmax_chunk = [&](int c, const uint32_t* r, auto masked_tag) {
                     constexpr bool kMasked = decltype(masked_tag)::value;
 #pragma unroll
@@ -701,12 +698,12 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                             const uint64_t neg2 = h == 0 ? n4.lo : n4.hi;
                             const int el = e + 2 * h;
                             float2 p2;
-                            if (kSoftcap) {
-                                const float2 neg = ptx::f2_unpack(neg2);
-                                p2.x = ptx::ex2_approx(log2_score(r[el], neg.x));
-                                p2.y = ptx::ex2_approx(log2_score(r[el + 1], neg.y));
-                            } else {
-                                const uint64_t x2 = ptx::f2_fma(ptx::f2_pack(__uint_as_float(r[el]), __uint_as_float(r[el + 1])), scale2, neg2);
+                            {
+                                // score in log2 units, relative to the row's reference: s * scale*log2e + (log2 r - m), or the
+                                // capped score + (log2 r - m)
+                                const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[el]), __uint_as_float(r[el + 1]));
+                                const uint64_t x2 = kSoftcap ? ptx::f2_fma(ptx::tanh_pair(ptx::f2_mul(s2, scale2)), post2, neg2)
+                                                             : ptx::f2_fma(s2, scale2, neg2);
                                 // (exp2_poly for a part of these changed nothing: B=4,H=16,S=4096,D=64 791, 792, 795, 810 us for 0 to 3
                                 // pairs of 8)
                                 p2 = ptx::f2_unpack(x2);
@@ -766,16 +763,14 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                             if (kSoftcap) {
                                 // dS = P (dP - delta) (1 - t^2), t recovered from P and the row's reference
                                 const ptx::F4Pairs n4 = ptx::f2_ld_shared(negp + (c * 32 + el) * 4);
-                                auto capped = [&](float p, uint32_t dp, float ndel, float neg) {
-                                    const float t = (__log2f(p) - neg) * inv_post;
-                                    const float slope = fmaxf(1.0f - t * t, 0.0f);
-                                    return p > 0.0f ? p * (__uint_as_float(dp) + ndel) * slope : 0.0f;
-                                };
 #pragma unroll
                                 for (int g = 0; g < 2; ++g) {
                                     const float2 p = ptx::Pack2<T>::unpack(ppk[c * 16 + el / 2 + g]);
-                                    const float2 d = ptx::f2_unpack(g == 0 ? d4.lo : d4.hi), n = ptx::f2_unpack(g == 0 ? n4.lo : n4.hi);
-                                    o[2 * h + g] = ptx::Pack2<T>::pack(capped(p.x, r[el + 2 * g], d.x, n.x), capped(p.y, r[el + 2 * g + 1], d.y, n.y));
+                                    const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[el + 2 * g]), __uint_as_float(r[el + 2 * g + 1]));
+                                    const float2 slope = ptx::cap_slope(p, g == 0 ? n4.lo : n4.hi, inv_post);
+                                    const uint64_t x2 = ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, g == 0 ? d4.lo : d4.hi));
+                                    const float2 ds = ptx::f2_unpack(ptx::f2_mul(x2, ptx::f2_pack(slope.x, slope.y)));
+                                    o[2 * h + g] = ptx::Pack2<T>::pack(ds.x, ds.y);
                                 }
                             } else {
 #pragma unroll

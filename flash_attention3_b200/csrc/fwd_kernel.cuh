@@ -512,12 +512,16 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 if (C::kOwnP) arrive(kFwdSFree);
                 if (kSoftcap) {
                     // capped scores, already in log2 units: from here on they are used with a scale of 1
+                    const float pre = a.softcap_pre * ptx::kTanhArg;
+                    const uint64_t pre2 = ptx::f2_pack(pre, pre), post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
 #pragma unroll
-                        for (int e = 0; e < 32; ++e) {
-                            r[c][e] = __float_as_uint(a.softcap_post *
-                                                      ptx::tanh_approx(__uint_as_float(r[c][e]) * a.softcap_pre));
+                        for (int e = 0; e < 32; e += 2) {
+                            const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
+                            const float2 capped = ptx::f2_unpack(ptx::f2_mul(ptx::tanh_pair(ptx::f2_mul(s2, pre2)), post2));
+                            r[c][e] = __float_as_uint(capped.x);
+                            r[c][e + 1] = __float_as_uint(capped.y);
                         }
                     }
                 }

@@ -475,14 +475,29 @@ __device__ __forceinline__ float2 exp2_poly(uint64_t x2) {
                        __uint_as_float(__float_as_uint(p.y) + (__float_as_uint(t.y) << 23)));
 }
 
-// tanh(x) = 1 - 2 / (exp(2x) + 1) with the exp2 and reciprocal approximations: absolute error of a few
-// 1e-7.  (tanh.approx.f32 has a relative error of 2^-11; the softcap multiplies it by softcap*log2(e),
-// which for a cap of 50 already costs P a quarter of a percent.)
-__device__ __forceinline__ float tanh_approx(float x) {
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * 2.8853900817779268f));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(e + 1.0f));
-    return fmaf(-2.0f, r, 1.0f);
+// tanh of two values, 1 - 2 / (exp(2x) + 1), absolute error of a few 1e-7; the argument is x * kTanhArg.
+// (tanh.approx.f32 has a relative error of 2^-11; the softcap multiplies it by softcap*log2(e), which for a cap
+// of 50 already costs P a quarter of a percent.)  The special-function unit bounds code that caps scores, so
+// two values share one reciprocal: 1/a = b * 1/(ab).  Beyond 2^60 the quotient no longer counts, and the
+// product of two such values is still finite.
+constexpr float kTanhArg = 2.8853900817779268f;  // 2 * log2(e)
+__device__ __forceinline__ uint64_t tanh_pair(uint64_t x_arg2) {
+    const float2 x = f2_unpack(x_arg2);
+    const float2 d = f2_unpack(f2_add(f2_pack(ex2_approx(fminf(x.x, 60.0f)), ex2_approx(fminf(x.y, 60.0f))), f2_pack(1.0f, 1.0f)));
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d.x * d.y));
+    r *= -2.0f;
+    return f2_fma(f2_pack(r, r), f2_pack(d.y, d.x), f2_pack(1.0f, 1.0f));
+}
+// Slope 1 - t^2 of the cap at two probabilities, t = (log2 P - neg) * inv_post.  P = 0 gives 0 (also where neg is
+// -inf: the maximum drops a NaN).
+__device__ __forceinline__ float2 cap_slope(float2 p, uint64_t neg2, float inv_post) {
+    float lx, ly;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(lx) : "f"(p.x));
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(ly) : "f"(p.y));
+    const uint64_t diff2 = f2_fma(neg2, f2_pack(-1.0f, -1.0f), f2_pack(lx, ly));
+    const float2 t = f2_unpack(f2_mul(diff2, f2_pack(inv_post, inv_post)));
+    return make_float2(fmaxf(fmaf(-t.x, t.x, 1.0f), 0.0f), fmaxf(fmaf(-t.y, t.y, 1.0f), 0.0f));
 }
 
 template <typename T>

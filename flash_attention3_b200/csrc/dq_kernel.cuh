@@ -59,7 +59,7 @@ struct DqArgs {
 template <int D>
 struct DqCfg {
     static constexpr int kTile = 128;
-    static constexpr int kThreads = 256;
+    static constexpr int kThreads = 384;
     static constexpr int kBoxBytes = 128 * 128;
     static constexpr int kBoxes = D / 64;
     static constexpr int kOperandBytes = kBoxes * kBoxBytes;
@@ -89,7 +89,7 @@ enum DqBar : int {
 };
 
 template <typename T, int D, bool kCausal, typename TOut, bool kSoftcap = false>
-__global__ void __launch_bounds__(256, 1)
+__global__ void __launch_bounds__(384, 1)
 dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
               const DqArgs a) {
@@ -143,8 +143,8 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         ptx::mbar_init(bar(kDqbSFull), 1);
         ptx::mbar_init(bar(kDqbDpFull), 1);
-        ptx::mbar_init(bar(kDqbSFree), 4);  // (one arrival per warp)
-        ptx::mbar_init(bar(kDqbDsReady), 4);
+        ptx::mbar_init(bar(kDqbSFree), 8);  // (one arrival per warp)
+        ptx::mbar_init(bar(kDqbDsReady), 8);
         ptx::mbar_init(bar(kDqbDone), 1);
         flag_set(abort_flag, 0);
         ptx::fence_mbar_init();
@@ -153,6 +153,7 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         ptx::tmem_alloc(tmem_slot, C::kTmemCols);
         ptx::tmem_relinquish();
     }
+    ptx::launch_dependents();  // (what follows waits for this kernel itself)
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
@@ -228,7 +229,7 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     ptx::tc_fence_after();
                     {
                         const uint32_t loK = ptx::desc_lo_mn_major(sK(t), C::kBoxBytes);
-                        ptx::mma_ts_8<ptx::TmemPacked, ptx::MnMajor>(tmem + C::kColDQ, tmem + C::kColDP, loK, kIdDq, t > 0 ? 1u : 0u);
+                        ptx::mma_ts_8<ptx::TmemHalves, ptx::MnMajor>(tmem + C::kColDQ, tmem + C::kColDP, loK, kIdDq, t > 0 ? 1u : 0u);
                     }
                     if (more) issue_dp(t + 1);  // after dQ(t) in issue order: dS(t) is consumed first
                     ptx::tc_commit_elect(bar(kDqbKvEmpty + (t & 1)));
@@ -236,8 +237,11 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                 if (ok) ptx::tc_commit_elect(bar(kDqbDone));  // never reached without steps: nobody waits then
             }
         } else if (warp >= 4) {
-            const int i = threadIdx.x - 128;  // query row inside the tile == TMEM lane
+            const int half = (warp - 4) >> 2;     // which 64 keys of a key tile, and which half of the columns of dQ
+            const int i = threadIdx.x & 127;      // query row inside the tile == TMEM lane
             const uint32_t tl = tmem + (uint32_t((warp & 3) * 32) << 16);
+            const uint32_t s_cols = tl + C::kColS + half * 64;
+            const uint32_t dp_cols = tl + C::kColDP + half * 64;
             const int qi = q_row + i;  // query row inside the head
             const bool q_valid = qi < band.seqlen_q;
             // rows past the end of the sequence: P = exp2(-inf) = 0
@@ -246,7 +250,7 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             float neg = -INFINITY, delta = 0.0f;
             if (q_valid) {
                 if (a.stats != nullptr) {
-                    const float2 v = a.stats[stat_row];
+                    const float2 v = __ldcg(a.stats + stat_row);  // (from the L2: see the launch)
                     neg = v.x;
                     delta = -v.y;
                 } else if (a.sidecar != nullptr) {
@@ -264,81 +268,82 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     delta = a.delta[stat_row];
                 }
             }
-            uint32_t ppk[64];
+            uint32_t ppk[32];
+            const float score_mul = kSoftcap ? a.softcap_pre * ptx::kTanhArg : a.scale_log2;
+            const uint64_t scale2 = ptx::f2_pack(score_mul, score_mul);
+            const uint64_t post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
+            const uint64_t neg2 = ptx::f2_pack(neg, neg), ndel2 = ptx::f2_pack(-delta, -delta);
+            const float inv_post = kSoftcap ? 1.0f / a.softcap_post : 0.0f;
+            auto arrive = [&](int which) {
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar(which));
+            };
+            // element (query i, key j of this half) survives iff mask_from <= j <= mask_to (band edges, end of keys)
+            int mask_from = 0, mask_to = 0;
+            key_range_of_query(qi, k_begin * C::kTile + half * 64, band, &mask_from, &mask_to);
             bool ok = true;
 #pragma unroll 1
-            for (int t = 0; t < n_steps; ++t) {
+            for (int t = 0; t < n_steps; ++t, mask_from -= C::kTile, mask_to -= C::kTile) {
                 if (!(ok = warp_wait(bar(kDqbSFull), t & 1, abort_flag))) break;
                 ptx::tc_fence_after();
-                // element (query i, key j) survives iff mask_from <= j <= mask_to (band edges, end of keys)
-                const bool diagonal = kCausal && tile_needs_mask(k_begin + t, qt, band);
-                int mask_from, mask_to;
-                key_range_of_query(qi, (k_begin + t) * C::kTile, band, &mask_from, &mask_to);
+                const bool diagonal = kCausal && __any_sync(0xffffffffu, mask_from > 0 || mask_to < 63);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < 2; ++c) {
                     uint32_t r[32];
-                    ptx::tmem_ld32(tl + C::kColS + c * 32, r);
+                    ptx::tmem_ld32(s_cols + c * 32, r);
                     ptx::tmem_ld_wait();
 #pragma unroll
                     for (int e = 0; e < 32; e += 2) {
-                        float p0, p1;
-                        if (kSoftcap) {
-                            p0 = ptx::ex2_approx(fmaf(a.softcap_post, ptx::tanh_approx(__uint_as_float(r[e + 0]) * a.softcap_pre), neg));
-                            p1 = ptx::ex2_approx(fmaf(a.softcap_post, ptx::tanh_approx(__uint_as_float(r[e + 1]) * a.softcap_pre), neg));
-                        } else {
-                            p0 = ptx::ex2_approx(fmaf(__uint_as_float(r[e + 0]), a.scale_log2, neg));
-                            p1 = ptx::ex2_approx(fmaf(__uint_as_float(r[e + 1]), a.scale_log2, neg));
-                        }
+                        const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
+                        float2 p = ptx::f2_unpack(kSoftcap ? ptx::f2_fma(ptx::tanh_pair(ptx::f2_mul(s2, scale2)), post2, neg2)
+                                                           : ptx::f2_fma(s2, scale2, neg2));
+                        p.x = ptx::ex2_approx(p.x);
+                        p.y = ptx::ex2_approx(p.y);
                         if (diagonal) {
                             const int j = c * 32 + e;
-                            p0 = (j + 0 >= mask_from && j + 0 <= mask_to) ? p0 : 0.0f;
-                            p1 = (j + 1 >= mask_from && j + 1 <= mask_to) ? p1 : 0.0f;
+                            p.x = (j + 0 >= mask_from && j + 0 <= mask_to) ? p.x : 0.0f;
+                            p.y = (j + 1 >= mask_from && j + 1 <= mask_to) ? p.y : 0.0f;
                         }
-                        ppk[c * 16 + e / 2] = ptx::Pack2<T>::pack(p0, p1);
+                        ppk[c * 16 + e / 2] = ptx::Pack2<T>::pack(p.x, p.y);
                     }
                 }
-                ptx::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(bar(kDqbSFree));
+                arrive(kDqbSFree);
                 if (!(ok = warp_wait(bar(kDqbDpFull), t & 1, abort_flag))) break;
                 ptx::tc_fence_after();
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < 2; ++c) {
                     uint32_t r[32];
-                    ptx::tmem_ld32(tl + C::kColDP + c * 32, r);
+                    ptx::tmem_ld32(dp_cols + c * 32, r);
                     ptx::tmem_ld_wait();
                     uint32_t o[16];
 #pragma unroll
                     for (int e = 0; e < 32; e += 2) {
                         const float2 p = ptx::Pack2<T>::unpack(ppk[c * 16 + e / 2]);
-                        float ds0 = p.x * (__uint_as_float(r[e + 0]) - delta);
-                        float ds1 = p.y * (__uint_as_float(r[e + 1]) - delta);
+                        const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
+                        uint64_t ds2 = ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, ndel2));
                         if (kSoftcap) {
-                            // slope 1 - tanh^2 of the cap, with tanh recovered from P and the row's reference
-                            const float inv_post = 1.0f / a.softcap_post;
-                            const float t0 = (__log2f(p.x) - neg) * inv_post, t1 = (__log2f(p.y) - neg) * inv_post;
-                            ds0 = p.x > 0.0f ? ds0 * fmaxf(1.0f - t0 * t0, 0.0f) : 0.0f;
-                            ds1 = p.y > 0.0f ? ds1 * fmaxf(1.0f - t1 * t1, 0.0f) : 0.0f;
+                            const float2 slope = ptx::cap_slope(p, neg2, inv_post);
+                            ds2 = ptx::f2_mul(ds2, ptx::f2_pack(slope.x, slope.y));
                         }
-                        o[e / 2] = ptx::Pack2<T>::pack(ds0, ds1);
+                        const float2 ds = ptx::f2_unpack(ds2);
+                        o[e / 2] = ptx::Pack2<T>::pack(ds.x, ds.y);
                     }
-                    // dS chunk c lands on columns [16c, 16c+16) of the dP region,
-                    // all of which were read by chunk loads <= c
-                    ptx::tmem_st16(tl + C::kColDP + c * 16, o);
+                    // dS chunk c lands on columns [16c, 16c+16) of this half's dP columns, all of which were read by
+                    // chunk loads <= c
+                    ptx::tmem_st16(dp_cols + c * 16, o);
                 }
                 ptx::tmem_st_wait();
-                ptx::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(bar(kDqbDsReady));
+                arrive(kDqbDsReady);
             }
             if (ok && n_steps > 0) ok = warp_wait(bar(kDqbDone), 0, abort_flag);
             TOut* dst = reinterpret_cast<TOut*>(a.dq) + b_coord * a.q_strides.batch + hq * a.q_strides.head +
-                        int64_t(q_base + qi) * a.q_strides.row;
+                        int64_t(q_base + qi) * a.q_strides.row + half * (D / 2);
             if (ok && ((q_valid && n_steps == 0) || (!q_valid && qi < slot_q))) {
                 // no visible key at all, or a row behind the used length: the gradient is zero
                 uint4* d4 = reinterpret_cast<uint4*>(dst);
 #pragma unroll
-                for (int e = 0; e < int(D * sizeof(TOut) / 16); ++e) d4[e] = make_uint4(0u, 0u, 0u, 0u);
+                for (int e = 0; e < int(D / 2 * sizeof(TOut) / 16); ++e) d4[e] = make_uint4(0u, 0u, 0u, 0u);
             }
             __syncwarp();
             if (ok && n_steps > 0) {
@@ -346,9 +351,9 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                 // rows past the end of the sequence are skipped)
                 ptx::tc_fence_after();
 #pragma unroll
-                for (int c = 0; c < D / 32; ++c) {
+                for (int c = 0; c < D / 64; ++c) {
                     uint32_t r[32];
-                    ptx::tmem_ld32(tl + C::kColDQ + c * 32, r);
+                    ptx::tmem_ld32(tl + C::kColDQ + half * (D / 2) + c * 32, r);
                     ptx::tmem_ld_wait();
                     if (q_valid) {
                     if (sizeof(TOut) == 4) {
@@ -376,6 +381,8 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
     }
 
+    // This kernel may run beside the dK/dV kernel in front of it; it must not complete before that one.
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) ptx::grid_dependency_wait();
     __syncwarp();
     ptx::tc_fence_before();
     __syncthreads();

@@ -541,7 +541,7 @@ int launch_fused(const ShaoboFa3Params* p, const void* dout, const void* q, cons
 // -------------------------------------------------------------- dQ kernel
 template <typename T, int D, bool kCausal, typename TOut, bool kSoftcap = false>
 int launch_dq_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                const CUtensorMap& mdo, const DqArgs& args, int blocks, cudaStream_t st) {
+                const CUtensorMap& mdo, const DqArgs& args, int blocks, cudaStream_t st, bool pdl) {
     auto kernel = dq_bwd_kernel<T, D, kCausal, TOut, kSoftcap>;
     static DeviceOnce configured;
     if (!configured.done()) {
@@ -551,32 +551,42 @@ int launch_dq_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap&
         }
         configured.mark();
     }
-    kernel<<<blocks, DqCfg<D>::kThreads, DqCfg<D>::kSmemBytes, st>>>(mq, mk, mv, mdo, args);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(DqCfg<D>::kThreads);
+    cfg.dynamicSmemBytes = DqCfg<D>::kSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, mdo, args) != cudaSuccess) return SHAOBO_FA3_STATUS_HIP_ERROR;
     return SHAOBO_FA3_STATUS_SUCCESS;
 }
 
 template <typename T, typename TOut>
 int launch_dq_d(const ShaoboFa3Params* p, const CUtensorMap& mq, const CUtensorMap& mk,
-                const CUtensorMap& mv, const CUtensorMap& mdo, const DqArgs& args, int blocks) {
+                const CUtensorMap& mv, const CUtensorMap& mdo, const DqArgs& args, int blocks, bool pdl) {
     cudaStream_t st = stream_of(p);
     const bool banded = needs_general_form(p);
     if (p->softcap > 0.0f) {
-        return p->head_dim_qk == 128 ? launch_dq_t<T, 128, true, TOut, true>(mq, mk, mv, mdo, args, blocks, st)
-                                     : launch_dq_t<T, 64, true, TOut, true>(mq, mk, mv, mdo, args, blocks, st);
+        return p->head_dim_qk == 128 ? launch_dq_t<T, 128, true, TOut, true>(mq, mk, mv, mdo, args, blocks, st, pdl)
+                                     : launch_dq_t<T, 64, true, TOut, true>(mq, mk, mv, mdo, args, blocks, st, pdl);
     }
     if (p->head_dim_qk == 128) {
-        return banded ? launch_dq_t<T, 128, true, TOut>(mq, mk, mv, mdo, args, blocks, st)
-                         : launch_dq_t<T, 128, false, TOut>(mq, mk, mv, mdo, args, blocks, st);
+        return banded ? launch_dq_t<T, 128, true, TOut>(mq, mk, mv, mdo, args, blocks, st, pdl)
+                         : launch_dq_t<T, 128, false, TOut>(mq, mk, mv, mdo, args, blocks, st, pdl);
     }
-    return banded ? launch_dq_t<T, 64, true, TOut>(mq, mk, mv, mdo, args, blocks, st)
-                     : launch_dq_t<T, 64, false, TOut>(mq, mk, mv, mdo, args, blocks, st);
+    return banded ? launch_dq_t<T, 64, true, TOut>(mq, mk, mv, mdo, args, blocks, st, pdl)
+                     : launch_dq_t<T, 64, false, TOut>(mq, mk, mv, mdo, args, blocks, st, pdl);
 }
 
 // Three-GEMM dQ kernel (split path).  out_f32 selects fp32 or input-dtype dq.  The row statistics
 // are stats, or the packed sidecar, or (both null) aux0 / aux1 / delta as three arrays.
 int launch_dq(const ShaoboFa3Params* p, const void* dout, const void* q, const void* k,
               const void* v, const float2* stats, const float* sidecar, void* dq, bool out_f32,
-              const float* aux0 = nullptr, const float* aux1 = nullptr, const float* delta = nullptr) {
+              const float* aux0 = nullptr, const float* aux1 = nullptr, const float* delta = nullptr, bool pdl = false) {
     const bool bf = p->dtype == SHAOBO_FA3_DTYPE_BF16;
     const CUtensorMapDataType type = bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     const int d = p->head_dim_qk;
@@ -615,11 +625,11 @@ int launch_dq(const ShaoboFa3Params* p, const void* dout, const void* q, const v
     if (blocks64 > 0x7fffffffLL) return SHAOBO_FA3_STATUS_UNSUPPORTED;
     const int blocks = int(blocks64);
     if (out_f32) {
-        return bf ? launch_dq_d<__nv_bfloat16, float>(p, mq, mk, mv, mdo, args, blocks)
-                  : launch_dq_d<__half, float>(p, mq, mk, mv, mdo, args, blocks);
+        return bf ? launch_dq_d<__nv_bfloat16, float>(p, mq, mk, mv, mdo, args, blocks, pdl)
+                  : launch_dq_d<__half, float>(p, mq, mk, mv, mdo, args, blocks, pdl);
     }
-    return bf ? launch_dq_d<__nv_bfloat16, __nv_bfloat16>(p, mq, mk, mv, mdo, args, blocks)
-              : launch_dq_d<__half, __half>(p, mq, mk, mv, mdo, args, blocks);
+    return bf ? launch_dq_d<__nv_bfloat16, __nv_bfloat16>(p, mq, mk, mv, mdo, args, blocks, pdl)
+              : launch_dq_d<__half, __half>(p, mq, mk, mv, mdo, args, blocks, pdl);
 }
 
 // ---------------------------------------------------------- forward kernel
@@ -952,10 +962,14 @@ extern "C" int shaobo_fa3_bwd_v2(const void* dout, const void* q, const void* k,
         launch_delta(&launch, dout, out, static_cast<const float*>(softmax_lse), nullptr, delta,
                      nullptr, stats, nullptr, true);
         stage_mark(1, st);
-        status = launch_fused(&launch, dout, q, k, v, stats, nullptr, nullptr, dk, dv, false, false);
+        // The dQ kernel needs the delta stage only, not dK / dV: launched programmatically it fills the SMs that the
+        // last wave of the dK/dV kernel leaves idle.  It starts when every CTA of that kernel has seen the delta stage
+        // complete (or has exited), reads the statistics from the L2, and its last CTA waits for the dK/dV kernel, so
+        // that what follows on the stream waits for both.
+        status = launch_fused(&launch, dout, q, k, v, stats, nullptr, nullptr, dk, dv, false, false, nullptr, true);
         stage_mark(2, st);
         if (status == SHAOBO_FA3_STATUS_SUCCESS) {
-            status = launch_dq(&launch, dout, q, k, v, stats, nullptr, dq, false);
+            status = launch_dq(&launch, dout, q, k, v, stats, nullptr, dq, false, nullptr, nullptr, nullptr, true);
         }
         stage_mark(3, st);
     }

@@ -441,8 +441,9 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         ptx::tmem_alloc(tmem_slot, C::kTmemCols);
         ptx::tmem_relinquish();
     }
-    // The kernel behind this one (dQ convert) may begin to launch; it waits for our completion itself.
-    ptx::launch_dependents();
+    // The kernel behind this one (dQ convert) may begin to launch; it waits for our completion itself.  (The dQ kernel
+    // of the split path does not: it is let go by the statistics warp, below, once the delta stage has completed.)
+    if (kWithDq) ptx::launch_dependents();
     // (all threads: barriers initialised, tensor memory allocated)
     auto set_up_done = [&] {
         ptx::tc_fence_before();
@@ -604,6 +605,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             // The statistics come from the delta kernel, which may still be running (programmatic launch); Q, K,
             // V, dO are inputs of the call, so the TMA and MMA warps did not have to wait.
             ptx::grid_dependency_wait();
+            if (!kWithDq) ptx::launch_dependents();
             float* stats = reinterpret_cast<float*>(smem + C::kOffStats);
             float neg[4], ndel[4];
             auto fetch = [&](const StepWalk<kCausal>& st) {

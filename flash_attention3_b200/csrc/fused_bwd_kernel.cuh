@@ -42,13 +42,13 @@
 // Shared-memory ledger (bytes; every tile is made of 16 KiB boxes of
 // [128 rows][64 x 16 bit] in the 128-byte swizzle):
 //     K, V            2 x D*256            resident for the CTA
-//     Q               2 stages x D*256
+//     Q               2 stages (D=128) or 3 (D=64) x D*256
 //     dO              1 stage (D=128) or 2 stages (D=64) x D*256
 //     dS^T            32 KiB               [128 keys][128 queries]
 //     dQ staging      32 KiB               4 warps x 2 boxes of [32 rows][32 fp32]
 //     row statistics  2 KiB                {log2 r - m, -delta} x 128 rows x 2 buffers
 //     mbarriers       256
-//     total           231,680 (D=128) / 166,144 (D=64)   of 232,448 available
+//     total           231,680 (D=128) / 182,528 (D=64)   of 232,448 available
 //
 // What bounds it: at D=64 the softmax / dS warpgroups (2630 clk per step, 1664 of MMA): one instruction per two
 // elements wherever packed arithmetic allows, statistics brought by a warp of their own, one arrival per warp
@@ -155,7 +155,8 @@ struct FusedCfg {
     static constexpr int kBoxBytes = 128 * 128;
     static constexpr int kBoxes = D / 64;
     static constexpr int kOperandBytes = kBoxes * kBoxBytes;
-    static constexpr int kQStages = 2;
+    // (a third Q stage at D=64: 904 -> 865 us per call of B=4,H=16,S=4096 full; a fourth, or a third of dO, no more)
+    static constexpr int kQStages = D == 64 ? 3 : 2;
     static constexpr int kDoStages = D == 128 ? 1 : 2;
     static constexpr int kDsBytes = 2 * kBoxBytes;
     static constexpr int kStageBoxBytes = 32 * 128;
@@ -192,20 +193,20 @@ struct FusedCfg {
 
 enum Bar : int {
     kKvFull = 0,
-    kQFull = 1,     // 2 stages
-    kQEmpty = 3,    // 2 stages
-    kDoFull = 5,    // up to 2 stages
-    kDoEmpty = 7,   // up to 2 stages
-    kSFull = 9,
-    kDpFull = 10,
-    kPReady = 11,
-    kDsReady = 12,
-    kDqFull = 13,
-    kDqEmpty = 14,
-    kDkvFull = 15,
-    kStatsFull = 16,   // 2 buffers
-    kStatsEmpty = 18,  // 2 buffers
-    kNumBars = 20,
+    kQFull = 1,        // up to 3 stages
+    kQEmpty = 4,       // up to 3 stages
+    kDoFull = 7,       // up to 2 stages
+    kDoEmpty = 9,      // up to 2 stages
+    kSFull = 11,
+    kDpFull = 12,
+    kPReady = 13,
+    kDsReady = 14,
+    kDqFull = 15,
+    kDqEmpty = 16,
+    kDkvFull = 17,
+    kStatsFull = 18,   // 2 buffers
+    kStatsEmpty = 20,  // 2 buffers
+    kNumBars = 22,
 };
 
 constexpr uint32_t kWaitTimeoutCycles = 2000000000u;  // about one second, of a 32-bit cycle counter
@@ -415,9 +416,11 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         TRACE(0, 4);
         if (misaligned) atomicCAS(&g_device_error, kDevOk, kDevSmemMisaligned);
         ptx::mbar_init(bar(kKvFull), 1);
-        for (int s = 0; s < 2; ++s) {
+        for (int s = 0; s < C::kQStages; ++s) {
             ptx::mbar_init(bar(kQFull + s), 1);
             ptx::mbar_init(bar(kQEmpty + s), 1);
+        }
+        for (int s = 0; s < C::kDoStages; ++s) {
             ptx::mbar_init(bar(kDoFull + s), 1);
             ptx::mbar_init(bar(kDoEmpty + s), 1);
         }

@@ -280,7 +280,6 @@ void launch_convert(const ShaoboFa3Params* p, const float* accum, void* dq,
     seg.n_vec8[0] = int64_t(shape.batch) * p->num_heads_q * shape.rows_q * p->head_dim_qk / 8;
     seg.scale[0] = p->softmax_scale;
     seg.layout[0] = row_layout(p, p->num_heads_q, shape.rows_q, shape.bshd);
-    seg.head_dim = p->head_dim_qk;
     seg.count = 1;
     int64_t total = seg.n_vec8[0];
     const SplitPlan split = dkv_slabs != nullptr ? split_plan(p) : SplitPlan{};
@@ -289,7 +288,6 @@ void launch_convert(const ShaoboFa3Params* p, const float* accum, void* dq,
         seg.dst[1] = dk;
         seg.dst[2] = dv;
         seg.n_vec8[1] = seg.n_vec8[2] = n / 8;
-        seg.scale[1] = seg.scale[2] = 1.0f;
         seg.layout[1] = seg.layout[2] = row_layout(p, p->num_heads_kv, shape.rows_k, shape.bshd);
         seg.count = 3;
         seg.slabs = dkv_slabs;
@@ -322,14 +320,14 @@ void launch_convert(const ShaoboFa3Params* p, const float* accum, void* dq,
     attr[0].val.programmaticStreamSerializationAllowed = 1;  // the kernel waits for the GEMM kernel itself
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const bool slabs = seg.count == 3;
-    if (p->dtype == SHAOBO_FA3_DTYPE_BF16) {
-        if (slabs) cudaLaunchKernelEx(&cfg, dq_convert_kernel<__nv_bfloat16, true>, seg);
-        else cudaLaunchKernelEx(&cfg, dq_convert_kernel<__nv_bfloat16, false>, seg);
-    } else {
-        if (slabs) cudaLaunchKernelEx(&cfg, dq_convert_kernel<__half, true>, seg);
-        else cudaLaunchKernelEx(&cfg, dq_convert_kernel<__half, false>, seg);
-    }
+    const bool slabs = seg.count == 3, bf = p->dtype == SHAOBO_FA3_DTYPE_BF16;
+    auto launch = [&](auto d) {
+        constexpr int D = decltype(d)::value;
+        if (bf) cudaLaunchKernelEx(&cfg, slabs ? dq_convert_kernel<__nv_bfloat16, D, true> : dq_convert_kernel<__nv_bfloat16, D, false>, seg);
+        else cudaLaunchKernelEx(&cfg, slabs ? dq_convert_kernel<__half, D, true> : dq_convert_kernel<__half, D, false>, seg);
+    };
+    if (p->head_dim_qk == 128) launch(std::integral_constant<int, 128>{});
+    else launch(std::integral_constant<int, 64>{});
 }
 
 // ------------------------------------------------------- fused / dKV kernel

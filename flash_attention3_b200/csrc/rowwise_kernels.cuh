@@ -68,13 +68,14 @@ struct RowLayout {
     int contiguous;         // 1: row r starts at element r*D ([B,H,S,D] contiguous)
 };
 
-__device__ __forceinline__ int64_t row_offset(const RowLayout& l, int64_t row, int d) {
-    if (l.contiguous) return row * d;
-    const int64_t bh = row / l.seqlen;
-    const int s = int(row - bh * l.seqlen);
-    const int64_t b = bh / l.heads;
-    const int h = int(bh - b * l.heads);
-    return b * l.strides.batch + h * l.strides.head + s * l.strides.row;
+// (a tensor that fits the GPU has fewer than 2^31 rows: 32-bit divisions, 64-bit ones cost several times as much)
+__device__ __forceinline__ int64_t row_offset(const RowLayout& l, uint32_t row, int d) {
+    if (l.contiguous) return int64_t(row) * d;
+    const uint32_t bh = row / uint32_t(l.seqlen);
+    const uint32_t s = row - bh * uint32_t(l.seqlen);
+    const uint32_t b = bh / uint32_t(l.heads);
+    const uint32_t h = bh - b * uint32_t(l.heads);
+    return int64_t(b) * l.strides.batch + int64_t(h) * l.strides.head + int64_t(s) * l.strides.row;
 }
 
 template <typename T, int D, bool kLseInput>
@@ -107,7 +108,7 @@ delta_sidecar_kernel(const T* __restrict__ dout, const T* __restrict__ out,
         const bool valid = row < rows;
         uint4 a = make_uint4(0u, 0u, 0u, 0u), b = a;
         if (valid) {
-            const int64_t src = row_offset(layout, row, D) + col * 8;
+            const int64_t src = row_offset(layout, uint32_t(row), D) + col * 8;
             a = ld_stream_16B(dout + src);
             b = ld_stream_16B(out + src);
         }
@@ -172,10 +173,9 @@ struct ConvertSegments {
     const float* src[3];   // [0]: fp32 dQ accumulator [batch, head, row, D] contiguous; [1],[2] unused
     void* dst[3];
     int64_t n_vec8[3];
-    float scale[3];
+    float scale[1];        // of dQ (dK was scaled before its partial sums were written)
     RowLayout layout[3];   // where the rows of dst live
     int count;
-    int head_dim;
     const void* slabs;     // count == 3: slab base; chunk x of the GEMM kernel owns slabs 2x (dK) and 2x+1 (dV)
     int slabs_f16;         // the slabs hold fp16 (fp16 inputs) instead of fp32
     int rows_k;            // key rows per (batch, KV head)
@@ -186,29 +186,32 @@ struct ConvertSegments {
 // dst[i] = T(scale * accum[i]).  8 elements per thread: 32 B in, 16 B out.
 // Algorithmic HBM bytes per element: 4 read + 2 written.
 // kSlabs = false: dQ alone (every problem whose key tiles are not split), a lean single-segment loop.
-template <typename T, bool kSlabs>
+// Small problems are latency-bound here: one load -> store trip per thread, 32-bit index arithmetic (the 64-bit
+// divisions of the strided layout took 1 us of 45 at B=2,Hq=16,Hkv=8,S=1111).
+template <typename T, int D, bool kSlabs>
 __global__ void __launch_bounds__(256)
 dq_convert_kernel(const __grid_constant__ ConvertSegments seg) {
 #ifdef FA3B200_TRACE
     if (threadIdx.x == 0) atomicMin(reinterpret_cast<unsigned long long*>(&g_trace_rowwise[2]), (unsigned long long)trace_globaltimer());
 #endif
-    // launched programmatically behind the GEMM kernel: wait until all of it has completed
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    // (a following call's first kernel may take its place now; it waits for this one itself)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // The segments form one index space, so that with enough blocks every thread makes a single
-    // load -> store trip whatever the number of segments (small problems are latency-bound here).
+    constexpr int kVecs = D / 8;  // per row
+    // The segments form one index space, so that with enough blocks every thread makes a single trip whatever the
+    // number of segments.
     const int64_t n0 = seg.n_vec8[0];
     const int64_t n01 = n0 + (kSlabs ? seg.n_vec8[1] : 0);
     const int64_t total = n01 + (kSlabs ? seg.n_vec8[2] : 0);
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    const int vec_per_row = seg.head_dim / 8;
+    // launched programmatically behind the GEMM kernel: wait until all of it has completed
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // (a following call's first kernel may take its place now; it waits for this one itself)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     for (int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; g < total; g += stride) {
         // (selects instead of indexing: the parameter arrays stay in constant memory)
         const int sgi = !kSlabs ? 0 : (g < n0 ? 0 : (g < n01 ? 1 : 2));
         const int64_t i = g - (sgi == 0 ? 0 : (sgi == 1 ? n0 : n01));
+        const uint32_t row_all = uint32_t(i / kVecs);
+        const int col = int(i % kVecs) * 8;
         T* __restrict__ dst = static_cast<T*>(sgi == 0 ? seg.dst[0] : (sgi == 1 ? seg.dst[1] : seg.dst[2]));
-        const float scale = sgi == 0 ? seg.scale[0] : (sgi == 1 ? seg.scale[1] : seg.scale[2]);
         float v[8];
         if (sgi == 0) {
             const uint4 lo = ld_stream_16B(seg.src[0] + i * 8);
@@ -218,21 +221,18 @@ dq_convert_kernel(const __grid_constant__ ConvertSegments seg) {
             v[4] = __uint_as_float(hi.x); v[5] = __uint_as_float(hi.y);
             v[6] = __uint_as_float(hi.z); v[7] = __uint_as_float(hi.w);
         } else {
-            // element (head, row, col) of dK / dV: add the slabs of the chunks of key tile row / 128
-            const int64_t row_all = i / vec_per_row;
-            const int col = int(i - row_all * vec_per_row) * 8;
-            const int64_t bh = row_all / seg.rows_k;
-            const int row = int(row_all - bh * seg.rows_k);
+            // element (head, row, col) of dK / dV: add the slabs of the chunks of key tile row / 128, in chunk order
+            const uint32_t bh = row_all / uint32_t(seg.rows_k);
+            const int row = int(row_all - bh * uint32_t(seg.rows_k));
             const int kt = row >> 7;
             const int c0 = seg.chunk_begin[kt], c1 = seg.chunk_begin[kt + 1];
-            const int64_t slab_elems = int64_t(kTileRows) * seg.head_dim;
-            const int64_t first = ((bh * seg.chunks_per_head + c0) * 2 + (sgi - 1)) * slab_elems +
-                                  int64_t(row & 127) * seg.head_dim + col;
+            constexpr int kSlab = kTileRows * D;  // elements
+            const int64_t first = ((int64_t(bh) * seg.chunks_per_head + c0) * 2 + (sgi - 1)) * kSlab + (row & 127) * D + col;
 #pragma unroll
             for (int e = 0; e < 8; ++e) v[e] = 0.0f;
             if (seg.slabs_f16) {
                 const __half* src = static_cast<const __half*>(seg.slabs) + first;
-                for (int c = c0; c < c1; ++c, src += 2 * slab_elems) {
+                for (int c = c0; c < c1; ++c, src += 2 * kSlab) {
                     const uint4 x = ld_stream_16B(src);
                     const float2 a0 = unpack2<__half>(x.x), a1 = unpack2<__half>(x.y);
                     const float2 a2 = unpack2<__half>(x.z), a3 = unpack2<__half>(x.w);
@@ -241,7 +241,7 @@ dq_convert_kernel(const __grid_constant__ ConvertSegments seg) {
                 }
             } else {
                 const float* src = static_cast<const float*>(seg.slabs) + first;
-                for (int c = c0; c < c1; ++c, src += 2 * slab_elems) {
+                for (int c = c0; c < c1; ++c, src += 2 * kSlab) {
                     const uint4 lo = ld_stream_16B(src);
                     const uint4 hi = ld_stream_16B(src + 4);
                     v[0] += __uint_as_float(lo.x); v[1] += __uint_as_float(lo.y);
@@ -251,6 +251,7 @@ dq_convert_kernel(const __grid_constant__ ConvertSegments seg) {
                 }
             }
         }
+        const float scale = sgi == 0 ? seg.scale[0] : 1.0f;
         uint4 o;
         o.x = pack2<T>(v[0] * scale, v[1] * scale);
         o.y = pack2<T>(v[2] * scale, v[3] * scale);
@@ -261,10 +262,8 @@ dq_convert_kernel(const __grid_constant__ ConvertSegments seg) {
         if (contiguous) {
             reinterpret_cast<uint4*>(dst)[i] = o;
         } else {
-            const RowLayout layout = sgi == 0 ? seg.layout[0] : (sgi == 1 ? seg.layout[1] : seg.layout[2]);
-            const int64_t row = i / vec_per_row;
-            const int col = int(i - row * vec_per_row) * 8;
-            *reinterpret_cast<uint4*>(dst + row_offset(layout, row, seg.head_dim) + col) = o;
+            const RowLayout& layout = sgi == 0 ? seg.layout[0] : (sgi == 1 ? seg.layout[1] : seg.layout[2]);
+            *reinterpret_cast<uint4*>(dst + row_offset(layout, row_all, D) + col) = o;
         }
     }
 #ifdef FA3B200_TRACE

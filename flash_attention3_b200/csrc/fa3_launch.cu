@@ -1169,7 +1169,7 @@ bool host_call_supported(const ShaoboFa3Params* p) {
 int host_shard_count(const ShaoboFa3Params* p) {
     // Shards overlap the copies of one with the kernels and the copies back of another, but every copy costs about 5 us on
     // the copy engine besides its bytes, and twice that while the other direction is busy, so they are few and large: one
-    // below 16 MB of traffic, two below 96, four below 400, else eight.  us per call with 1, 2, 4 and 8: 17 MB 374, 365,
+    // below 16 MB of traffic, two below 80, four below 400, else eight.  us per call with 1, 2, 4 and 8: 17 MB 374, 365,
     // 402, 404; 34 MB 690, 610, 670, 787; 67 MB 1377, 1160, 1209, 1285; 168 MB 3267, 2866, 2795, 2943; 673 MB 14620, 11920,
     // 11020, 10570.  One more shard where that cuts evenly ((batch, KV head) units are not divided): 840 -> 805 us for
     // three units of 14 MB.
@@ -1177,7 +1177,7 @@ int host_shard_count(const ShaoboFa3Params* p) {
     const size_t total = (size_t(5) * p->num_heads_q + size_t(4) * p->num_heads_kv) * p->batch *
                          p->seqlen_q * p->head_dim_qk * elem;
     const long long units = (long long)p->batch * p->num_heads_kv;
-    long long n = total < (size_t(16) << 20) ? 1 : total < (size_t(96) << 20) ? 2 : total < (size_t(400) << 20) ? 4 : 8;
+    long long n = total < (size_t(16) << 20) ? 1 : total < (size_t(80) << 20) ? 2 : total < (size_t(400) << 20) ? 4 : 8;
     if (n > 1 && units % n != 0 && units % (n + 1) == 0) ++n;
     n = std::min(n, units);
     return int(n);

@@ -333,8 +333,8 @@ void launch_convert(const ShaoboFa3Params* p, const float* accum, void* dq,
 // ------------------------------------------------------- fused / dKV kernel
 template <typename T, int D, bool kCausal, bool kWithDq, typename TOut, bool kSoftcap = false>
 int launch_fused_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                   const CUtensorMap& mdo, const CUtensorMap& mdq, const CUtensorMap& mdk,
-                   const CUtensorMap& mdv, const FusedArgs& args, int blocks, cudaStream_t st, bool pdl) {
+                   const CUtensorMap& mdo, const CUtensorMap& mdq, const FusedArgs& args, int blocks,
+                   cudaStream_t st, bool pdl) {
     auto kernel = fused_bwd_kernel<T, D, kCausal, kWithDq, TOut, kSoftcap>;
     static DeviceOnce configured;  // per instantiation and device
     if (!configured.done()) {
@@ -356,7 +356,7 @@ int launch_fused_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
     attr[0].val.programmaticStreamSerializationAllowed = pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, mdo, mdq, mdk, mdv, args) != cudaSuccess) {
+    if (cudaLaunchKernelEx(&cfg, kernel, mq, mk, mv, mdo, mdq, args) != cudaSuccess) {
         return SHAOBO_FA3_STATUS_HIP_ERROR;
     }
     return SHAOBO_FA3_STATUS_SUCCESS;
@@ -365,21 +365,21 @@ int launch_fused_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
 template <typename T, bool kWithDq, typename TOut>
 int launch_fused_d(const ShaoboFa3Params* p, const CUtensorMap& mq, const CUtensorMap& mk,
                    const CUtensorMap& mv, const CUtensorMap& mdo, const CUtensorMap& mdq,
-                   const CUtensorMap& mdk, const CUtensorMap& mdv, const FusedArgs& args, int blocks,
+                   const FusedArgs& args, int blocks,
                    bool pdl) {
     cudaStream_t st = stream_of(p);
     const bool banded = needs_general_form(p);
     if (p->softcap > 0.0f) {  // softcapped scores: general form only
         return p->head_dim_qk == 128
-                   ? launch_fused_t<T, 128, true, kWithDq, TOut, true>(mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, st, pdl)
-                   : launch_fused_t<T, 64, true, kWithDq, TOut, true>(mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, st, pdl);
+                   ? launch_fused_t<T, 128, true, kWithDq, TOut, true>(mq, mk, mv, mdo, mdq, args, blocks, st, pdl)
+                   : launch_fused_t<T, 64, true, kWithDq, TOut, true>(mq, mk, mv, mdo, mdq, args, blocks, st, pdl);
     }
     if (p->head_dim_qk == 128) {
-        return banded ? launch_fused_t<T, 128, true, kWithDq, TOut>(mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, st, pdl)
-                         : launch_fused_t<T, 128, false, kWithDq, TOut>(mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, st, pdl);
+        return banded ? launch_fused_t<T, 128, true, kWithDq, TOut>(mq, mk, mv, mdo, mdq, args, blocks, st, pdl)
+                         : launch_fused_t<T, 128, false, kWithDq, TOut>(mq, mk, mv, mdo, mdq, args, blocks, st, pdl);
     }
-    return banded ? launch_fused_t<T, 64, true, kWithDq, TOut>(mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, st, pdl)
-                     : launch_fused_t<T, 64, false, kWithDq, TOut>(mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, st, pdl);
+    return banded ? launch_fused_t<T, 64, true, kWithDq, TOut>(mq, mk, mv, mdo, mdq, args, blocks, st, pdl)
+                     : launch_fused_t<T, 64, false, kWithDq, TOut>(mq, mk, mv, mdo, mdq, args, blocks, st, pdl);
 }
 
 // with_dq: fused five-GEMM kernel writing dK/dV in the input dtype and adding
@@ -392,7 +392,7 @@ int launch_fused_d(const ShaoboFa3Params* p, const CUtensorMap& mq, const CUtens
 // between the two launches while the host encodes the tensor maps.
 struct FusedLaunch {
     int status = SHAOBO_FA3_STATUS_SUCCESS;
-    CUtensorMap mq, mk, mv, mdo, mdq, mdk, mdv;
+    CUtensorMap mq, mk, mv, mdo, mdq;
     FusedArgs args;
     int blocks = 0;
     bool with_dq = false;
@@ -405,7 +405,7 @@ FusedLaunch prepare_fused(const ShaoboFa3Params* p, const void* dout, const void
     FusedLaunch L;
     L.with_dq = with_dq;
     L.dkv_f32 = dkv_f32;
-    CUtensorMap &mq = L.mq, &mk = L.mk, &mv = L.mv, &mdo = L.mdo, &mdq = L.mdq, &mdk = L.mdk, &mdv = L.mdv;
+    CUtensorMap &mq = L.mq, &mk = L.mk, &mv = L.mv, &mdo = L.mdo, &mdq = L.mdq;
     FusedArgs& args = L.args;
     auto fail = [&](int status) {
         L.status = status;
@@ -430,25 +430,8 @@ FusedLaunch prepare_fused(const ShaoboFa3Params* p, const void* dout, const void
         mdq = mq;  // unused by the kernel
     }
     const SplitPlan split = (with_dq && dkv_slabs != nullptr) ? split_plan(p) : SplitPlan{};
-    // Where the epilogue stores dK / dV through the copy engine: the fp32 slabs of split tiles
-    // ([slab][128 rows][D], two slabs per CTA), or dk / dv themselves in boxes of 32 rows (16-bit
-    // outputs of fixed-length batches).  Other cases (packed sequences, fp32 outputs) store from
-    // registers and do not use these maps.
-    if (split.chunk_steps > 0) {
-        const int64_t slabs = int64_t(split.chunks_per_head) * p->batch * p->num_heads_kv * 2;
-        const bool ok = bf ? make_map_accum(&mdk, static_cast<const float*>(dkv_slabs), slabs, kTileRows, d)
-                           : make_map_16(&mdk, type, dkv_slabs, 1, int(slabs), kTileRows, d, false, 32);
-        if (!ok) return fail(SHAOBO_FA3_STATUS_HIP_ERROR);
-        mdv = mdk;
-    } else if (!dkv_f32 && !is_varlen(p)) {
-        if (!make_map_16(&mdk, type, dk, shape.batch, p->num_heads_kv, shape.rows_k, d, bshd, 32) ||
-            !make_map_16(&mdv, type, dv, shape.batch, p->num_heads_kv, shape.rows_k, d, bshd, 32)) {
-            return fail(SHAOBO_FA3_STATUS_HIP_ERROR);
-        }
-    } else {
-        mdk = mq;
-        mdv = mq;
-    }
+    // (dK / dV are written in 16-byte units)
+    if (((reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 15) != 0) return fail(SHAOBO_FA3_STATUS_HIP_ERROR);
     const int n_tiles = tiles_of(plan_seqlen_k(p));
     const Band band = band_of(p);
     const TileWork work = TileWork::of(band);
@@ -487,24 +470,28 @@ FusedLaunch prepare_fused(const ShaoboFa3Params* p, const void* dout, const void
     args.chunk_steps = split.chunk_steps;
     args.chunks_per_head = split.chunks_per_head;
     if (split.chunk_steps > 0) {
-        // every chunk of every (batch, KV head), longest first (stable: equal lengths keep the order
-        // head, key tile, chunk), so that the CTAs beyond one wave are the shortest ones
-        struct Chunk { int steps; uint32_t entry; };
-        std::vector<Chunk> chunks;
+        // every chunk of every (batch, KV head), longest first (equal lengths keep the order head, key tile, chunk), so
+        // that the CTAs beyond one wave are the shortest ones
+        const int64_t ctas = int64_t(split.chunks_per_head) * bh;
+        if (ctas > kMaxSplitCtas || n_tiles > 255) return fail(SHAOBO_FA3_STATUS_UNSUPPORTED);
+        uint32_t entry[kMaxSplitCtas];
+        int steps_of[kMaxSplitCtas];
+        int n = 0;
         for (int h = 0; h < bh; ++h) {
             int place = 0;
             for (int kt = 0; kt < n_tiles; ++kt) {
                 const int steps = group * q_tiles_of_k_tile(kt, band);
-                for (int c = 0, t0 = 0; t0 < steps; ++c, t0 += split.chunk_steps, ++place) {
-                    const int n = std::min(split.chunk_steps, steps - t0);
+                for (int c = 0, t0 = 0; t0 < steps; ++c, t0 += split.chunk_steps, ++place, ++n) {
                     const uint32_t slab = uint32_t(h * split.chunks_per_head + place);
-                    chunks.push_back(Chunk{n, uint32_t(kt) | (uint32_t(c) << 8) | (slab << 16)});
+                    steps_of[n] = std::min(split.chunk_steps, steps - t0);
+                    entry[n] = uint32_t(kt) | (uint32_t(c) << 8) | (slab << 16);
                 }
             }
         }
-        if (chunks.size() > size_t(kMaxSplitCtas) || n_tiles > 255) return fail(SHAOBO_FA3_STATUS_UNSUPPORTED);
-        std::stable_sort(chunks.begin(), chunks.end(), [](const Chunk& x, const Chunk& y) { return x.steps > y.steps; });
-        for (size_t i = 0; i < chunks.size(); ++i) args.cta_table[i] = chunks[i].entry;
+        std::vector<int> place(size_t(split.chunk_steps) + 1, 0);  // first place of every length, longest first
+        for (int i = 0; i < n; ++i) ++place[size_t(steps_of[i]) - 1];
+        for (int len = split.chunk_steps - 1; len >= 0; --len) place[size_t(len)] += place[size_t(len) + 1];
+        for (int i = 0; i < n; ++i) args.cta_table[place[size_t(steps_of[i])]++] = entry[i];
     }
     const int64_t blocks64 = split.chunk_steps > 0 ? int64_t(split.chunks_per_head) * bh : int64_t(n_tiles) * bh;
     if (blocks64 > 0x7fffffffLL) return fail(SHAOBO_FA3_STATUS_UNSUPPORTED);
@@ -515,19 +502,19 @@ FusedLaunch prepare_fused(const ShaoboFa3Params* p, const void* dout, const void
 int run_fused(const ShaoboFa3Params* p, const FusedLaunch& L, bool pdl) {
     if (L.status != SHAOBO_FA3_STATUS_SUCCESS) return L.status;
     const bool bf = p->dtype == SHAOBO_FA3_DTYPE_BF16;
-    const CUtensorMap &mq = L.mq, &mk = L.mk, &mv = L.mv, &mdo = L.mdo, &mdq = L.mdq, &mdk = L.mdk, &mdv = L.mdv;
+    const CUtensorMap &mq = L.mq, &mk = L.mk, &mv = L.mv, &mdo = L.mdo, &mdq = L.mdq;
     const FusedArgs& args = L.args;
     const int blocks = L.blocks;
     if (L.with_dq) {
-        return bf ? launch_fused_d<__nv_bfloat16, true, __nv_bfloat16>(p, mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, pdl)
-                  : launch_fused_d<__half, true, __half>(p, mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, pdl);
+        return bf ? launch_fused_d<__nv_bfloat16, true, __nv_bfloat16>(p, mq, mk, mv, mdo, mdq, args, blocks, pdl)
+                  : launch_fused_d<__half, true, __half>(p, mq, mk, mv, mdo, mdq, args, blocks, pdl);
     }
     if (L.dkv_f32) {
-        return bf ? launch_fused_d<__nv_bfloat16, false, float>(p, mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, pdl)
-                  : launch_fused_d<__half, false, float>(p, mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, pdl);
+        return bf ? launch_fused_d<__nv_bfloat16, false, float>(p, mq, mk, mv, mdo, mdq, args, blocks, pdl)
+                  : launch_fused_d<__half, false, float>(p, mq, mk, mv, mdo, mdq, args, blocks, pdl);
     }
-    return bf ? launch_fused_d<__nv_bfloat16, false, __nv_bfloat16>(p, mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, pdl)
-              : launch_fused_d<__half, false, __half>(p, mq, mk, mv, mdo, mdq, mdk, mdv, args, blocks, pdl);
+    return bf ? launch_fused_d<__nv_bfloat16, false, __nv_bfloat16>(p, mq, mk, mv, mdo, mdq, args, blocks, pdl)
+              : launch_fused_d<__half, false, __half>(p, mq, mk, mv, mdo, mdq, args, blocks, pdl);
 }
 
 int launch_fused(const ShaoboFa3Params* p, const void* dout, const void* q, const void* k,

@@ -18,8 +18,7 @@
 // convert kernel) instead of per element of dS.
 //
 // Epilogue: when the last MMA has completed, every softmax warp stages its 32 key rows of dK
-// (scaled) or dV over the dead Q / dO / dS^T buffers in the layout of a swizzled TMA box and one
-// lane stores them with the copy engine.  On problems too small to fill the GPU the query steps
+// (scaled) or dV over the dead Q / dO / dS^T buffers and stores them in whole lines.  On problems too small to fill the GPU the query steps
 // of a key tile are cut into chunks, one CTA each (a table in the kernel parameters says which,
 // longest chunks first); such a CTA stores its partial dK / dV to its own slab and the convert
 // kernel adds the slabs of a tile in chunk order.
@@ -188,7 +187,7 @@ struct FusedCfg {
     static constexpr int kColDP = 2 * D + 128;
     static constexpr int kColDQ = D == 128 ? kColDP : kColDP + 128;
     static_assert(kColDQ + D <= kTmemCols, "tensor-memory ledger exceeds 512 columns");
-    static_assert(8 * (D / 32) * kStageBoxBytes <= kOffStage - kOffQ, "epilogue staging does not fit");
+    static_assert(8 * 32 * D * 4 <= kOffStage - kOffQ, "epilogue staging does not fit");
 };
 
 enum Bar : int {
@@ -394,8 +393,7 @@ template <typename T, int D, bool kCausal, bool kWithDq, typename TOut, bool kSo
 __global__ void __launch_bounds__(512, 1)
 fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                 const __grid_constant__ CUtensorMap tm_dqacc, const __grid_constant__ CUtensorMap tm_dk,
-                 const __grid_constant__ CUtensorMap tm_dv, const __grid_constant__ FusedArgs a) {
+                 const __grid_constant__ CUtensorMap tm_dqacc, const __grid_constant__ FusedArgs a) {
     using C = FusedCfg<D>;
     constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -810,148 +808,67 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             if (ok) ok = warp_wait(bar(kDkvFull), 0, abort_flag);
             if (warp == 4) TRACE(2, 60);
             if (ok) {
-                // Every MMA has completed, so the Q / dO / dS^T buffers are dead.  Each warp stages its
-                // 32 key rows there in the layout of a swizzled TMA box and one lane stores them with
-                // the copy engine: whole 128-byte lines, rows past the end of the tensor clipped by the
-                // hardware.  (A thread storing its own row straight from registers writes 16 bytes per
-                // line and instruction: measured 6 us per CTA instead of under 1.)
+                // Every MMA has completed, so the Q / dO / dS^T buffers are dead.  Each warp stages its 32 key rows
+                // there and stores them again in whole lines, 512 contiguous bytes (or two rows) per instruction.
+                // (Stores through the copy engine queue behind the drain's last reduce-adds, about 2700 clk at D=128;
+                // a thread storing its own row straight from registers writes 16 bytes per line and instruction.)
                 ptx::tc_fence_after();
                 const float mul = half == 0 ? a.scale : 1.0f;
                 const uint32_t col0 = tl + (half == 0 ? C::kColDK : C::kColDV);
                 const int w4 = warp & 3;  // which 32 rows of the tile
-                // packed sequences: the rows behind this sequence's end belong to its neighbour, which the
-                // copy engine cannot know; fp32 outputs of the split path: plain rows.  Both keep per-thread stores.
-                const bool split = a.chunk_steps > 0;
-                const bool staged = split || (sizeof(TOut) == 2 && a.cu_seqlens_q == nullptr);
-                if (staged && split && !kBf16) {
-                    // fp16 inputs: the partial sums go to this CTA's slabs (w.slab 2x: dK, 2x+1: dV) as fp16,
-                    // boxes of [32 rows][64 x 16 bit].  (fp16 keeps 11 significant bits, three more than a
-                    // bf16 result would; the bytes written, not the arithmetic, bound this epilogue.)
-                    const uint32_t scratch = sbase + C::kOffQ + (half * 4 + w4) * (C::kBoxes * C::kStageBoxBytes);
+                // rows of element type O at dst, `pitch` elements apart, of which the first `rows` are written
+                auto store_rows = [&](auto tag, void* dst_rows, int64_t pitch, int rows) {
+                    using O = decltype(tag);
+                    constexpr int kRowBytes = D * int(sizeof(O));
+                    constexpr int kChunks = kRowBytes / 16;
+                    constexpr int kPerLoad = 32 * int(sizeof(O)) / 16;  // 16-byte chunks of 32 columns
+                    const uint32_t scratch = sbase + C::kOffQ + (half * 4 + w4) * (32 * kRowBytes);
 #pragma unroll
                     for (int c = 0; c < D / 32; ++c) {
                         uint32_t r[32];
                         ptx::tmem_ld32(col0 + c * 32, r);
                         ptx::tmem_ld_wait();
-                        const uint32_t row_addr = scratch + (c >> 1) * C::kStageBoxBytes + lane * 128;
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const uint32_t o0 = ptx::Pack2<__half>::pack(__uint_as_float(r[8 * e + 0]) * mul, __uint_as_float(r[8 * e + 1]) * mul);
-                            const uint32_t o1 = ptx::Pack2<__half>::pack(__uint_as_float(r[8 * e + 2]) * mul, __uint_as_float(r[8 * e + 3]) * mul);
-                            const uint32_t o2 = ptx::Pack2<__half>::pack(__uint_as_float(r[8 * e + 4]) * mul, __uint_as_float(r[8 * e + 5]) * mul);
-                            const uint32_t o3 = ptx::Pack2<__half>::pack(__uint_as_float(r[8 * e + 6]) * mul, __uint_as_float(r[8 * e + 7]) * mul);
-                            const int chunk = (c & 1) * 4 + e;
-                            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
-                                         ::"r"(row_addr + ((chunk ^ (lane & 7)) << 4)), "r"(o0), "r"(o1), "r"(o2), "r"(o3)
-                                         : "memory");
-                        }
-                    }
-                    ptx::fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
+                        for (int e = 0; e < kPerLoad; ++e) {
+                            uint32_t o[4];
 #pragma unroll
-                        for (int bx = 0; bx < C::kBoxes; ++bx)
-                            ptx::tma_store_4d(&tm_dk, scratch + bx * C::kStageBoxBytes, bx * 64, w4 * 32, w.slab * 2 + half, 0);
-                        ptx::bulk_commit_group();
-                        ptx::bulk_wait_group_read<0>();
-                    }
-                } else if (staged && split) {
-                    // bf16 inputs: fp32 partial sums -> this CTA's slabs, boxes of [32 rows][32 fp32]
-                    constexpr int kBoxesPerWarp = D / 32;
-                    const uint32_t scratch = sbase + C::kOffQ + (half * 4 + w4) * (kBoxesPerWarp * C::kStageBoxBytes);
-#pragma unroll
-                    for (int c = 0; c < kBoxesPerWarp; ++c) {
-                        uint32_t r[32];
-                        ptx::tmem_ld32(col0 + c * 32, r);
-                        ptx::tmem_ld_wait();
-                        const uint32_t row_addr = scratch + c * C::kStageBoxBytes + lane * 128;
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};"
-                                         ::"r"(row_addr + ((e ^ (lane & 7)) << 4)),
-                                           "f"(__uint_as_float(r[4 * e]) * mul), "f"(__uint_as_float(r[4 * e + 1]) * mul),
-                                           "f"(__uint_as_float(r[4 * e + 2]) * mul), "f"(__uint_as_float(r[4 * e + 3]) * mul)
-                                         : "memory");
-                        }
-                    }
-                    ptx::fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
-#pragma unroll
-                        for (int c = 0; c < kBoxesPerWarp; ++c)
-                            ptx::tma_store_3d(&tm_dk, scratch + c * C::kStageBoxBytes, c * 32, w4 * 32,
-                                              w.slab * 2 + half);
-                        ptx::bulk_commit_group();
-                        ptx::bulk_wait_group_read<0>();
-                    }
-                } else if (staged) {
-                    // 16-bit outputs -> dk / dv through their tensor maps, boxes of [32 rows][64 x 16 bit]
-                    const uint32_t scratch = sbase + C::kOffQ + (half * 4 + w4) * (C::kBoxes * C::kStageBoxBytes);
-#pragma unroll
-                    for (int c = 0; c < D / 32; ++c) {
-                        uint32_t r[32];
-                        ptx::tmem_ld32(col0 + c * 32, r);
-                        ptx::tmem_ld_wait();
-                        // 32 columns = 64 bytes = chunks 4*(c&1) .. 4*(c&1)+3 of this row of box c/2
-                        const uint32_t row_addr = scratch + (c >> 1) * C::kStageBoxBytes + lane * 128;
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const uint32_t o0 = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 0]) * mul, __uint_as_float(r[8 * e + 1]) * mul);
-                            const uint32_t o1 = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 2]) * mul, __uint_as_float(r[8 * e + 3]) * mul);
-                            const uint32_t o2 = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 4]) * mul, __uint_as_float(r[8 * e + 5]) * mul);
-                            const uint32_t o3 = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 6]) * mul, __uint_as_float(r[8 * e + 7]) * mul);
-                            const int chunk = (c & 1) * 4 + e;
-                            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
-                                         ::"r"(row_addr + ((chunk ^ (lane & 7)) << 4)), "r"(o0), "r"(o1), "r"(o2), "r"(o3)
-                                         : "memory");
-                        }
-                    }
-                    ptx::fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0) {
-                        const void* map = half == 0 ? static_cast<const void*>(&tm_dk) : static_cast<const void*>(&tm_dv);
-#pragma unroll
-                        for (int bx = 0; bx < C::kBoxes; ++bx)
-                            ptx::tma_store_4d(map, scratch + bx * C::kStageBoxBytes, bx * 64,
-                                              w.kt * C::kTile + w4 * 32, w.kvh, w.b);
-                        ptx::bulk_commit_group();
-                        ptx::bulk_wait_group_read<0>();
-                    }
-                } else {
-                    // (tensor-memory loads are warp-wide: every lane runs them, only the stores of key rows
-                    // past the end of the sequence are skipped)
-                    // (rows between the used length and the end of the slot hold exact zeros)
-                    const bool key_valid = w.kt * C::kTile + j < w.slot_k;
-                    const int64_t off = w.b_coord * a.kv_strides.batch + w.kvh * a.kv_strides.head +
-                                        int64_t(w.k_base + w.kt * C::kTile + j) * a.kv_strides.row;
-                    TOut* dst = reinterpret_cast<TOut*>(half == 0 ? a.dk : a.dv) + off;
-#pragma unroll
-                    for (int c = 0; c < D / 32; ++c) {
-                        uint32_t r[32];
-                        ptx::tmem_ld32(col0 + c * 32, r);
-                        ptx::tmem_ld_wait();
-                        if (key_valid) {
-                            if (sizeof(TOut) == 4) {
-                                float4* d4 = reinterpret_cast<float4*>(dst + c * 32);
-#pragma unroll
-                                for (int e = 0; e < 8; ++e)
-                                    d4[e] = make_float4(__uint_as_float(r[4 * e]) * mul, __uint_as_float(r[4 * e + 1]) * mul,
-                                                        __uint_as_float(r[4 * e + 2]) * mul, __uint_as_float(r[4 * e + 3]) * mul);
-                            } else {
-                                uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    uint4 o;
-                                    o.x = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 0]) * mul, __uint_as_float(r[8 * e + 1]) * mul);
-                                    o.y = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 2]) * mul, __uint_as_float(r[8 * e + 3]) * mul);
-                                    o.z = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 4]) * mul, __uint_as_float(r[8 * e + 5]) * mul);
-                                    o.w = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 6]) * mul, __uint_as_float(r[8 * e + 7]) * mul);
-                                    d4[e] = o;
+                            for (int h = 0; h < 4; ++h) {
+                                if constexpr (sizeof(O) == 4) {
+                                    o[h] = __float_as_uint(__uint_as_float(r[4 * e + h]) * mul);
+                                } else {
+                                    o[h] = ptx::Pack2<O>::pack(__uint_as_float(r[8 * e + 2 * h]) * mul, __uint_as_float(r[8 * e + 2 * h + 1]) * mul);
                                 }
                             }
+                            const int chunk = (c * kPerLoad + e) ^ (lane & 7);  // (spread over the banks)
+                            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                                         ::"r"(scratch + lane * kRowBytes + chunk * 16), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
                         }
-                        __syncwarp();  // reconverge before the next warp-wide load
                     }
+                    __syncwarp();
+                    constexpr int kRowsPerPass = 32 / kChunks;  // 1, 2 or 4
+                    const int sub = lane / kChunks, ch = lane % kChunks;
+                    O* dst = static_cast<O*>(dst_rows) + ch * (16 / int(sizeof(O)));
+#pragma unroll 8
+                    for (int row = sub; row < 32; row += kRowsPerPass) {
+                        uint4 v;
+                        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                                     : "r"(scratch + row * kRowBytes + ((ch ^ (row & 7)) << 4)) : "memory");
+                        if (row < rows) *reinterpret_cast<uint4*>(dst + row * pitch) = v;
+                    }
+                };
+                if (kWithDq && a.chunk_steps > 0) {
+                    // a share of a split tile: the partial sums go to this CTA's slabs (slab 2x: dK, 2x+1: dV), fp16 for
+                    // fp16 inputs (11 significant bits, three more than a bf16 result would have; the bytes written, not
+                    // the arithmetic, bound this epilogue), fp32 for bf16 inputs
+                    using Slab = typename std::conditional<kBf16, float, __half>::type;
+                    Slab* slab = static_cast<Slab*>(a.dkv_slabs) + int64_t(w.slab * 2 + half) * (C::kTile * D) + w4 * 32 * D;
+                    store_rows(Slab{}, slab, D, 32);
+                } else {
+                    // (rows between the used length and the end of the slot hold exact zeros)
+                    TOut* dst = reinterpret_cast<TOut*>(half == 0 ? a.dk : a.dv) + w.b_coord * a.kv_strides.batch +
+                                w.kvh * a.kv_strides.head + int64_t(w.k_base + w.kt * C::kTile + w4 * 32) * a.kv_strides.row;
+                    store_rows(TOut{}, dst, a.kv_strides.row, w.slot_k - (w.kt * C::kTile + w4 * 32));
                 }
             }
             if (warp == 4) TRACE(2, 61);

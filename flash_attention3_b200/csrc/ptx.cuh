@@ -115,13 +115,7 @@ __device__ __forceinline__ void tma_reduce_add_2d(const void* map, uint32_t src,
         ::"l"(map), "r"(src), "r"(x), "r"(y)
         : "memory");
 }
-// 3-D / 4-D tiled store shared -> global; elements outside the tensor are dropped.
-__device__ __forceinline__ void tma_store_3d(const void* map, uint32_t src, int c0, int c1, int c2) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-        ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2)
-        : "memory");
-}
+// 4-D tiled store shared -> global; elements outside the tensor are dropped.
 __device__ __forceinline__ void tma_store_4d(const void* map, uint32_t src, int c0, int c1, int c2, int c3) {
     asm volatile(
         "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"

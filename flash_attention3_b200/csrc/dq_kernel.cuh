@@ -41,6 +41,9 @@ struct DqArgs {
     const float* delta;
     void* dq;              // [B,Hq,Sq,D] or [B,Sq,Hq,D], see q_strides
     TensorStrides q_strides;  // element strides of dq
+    FastDiv bh;               // batch * heads_q
+    FastDiv heads;            // heads_q
+    FastDiv group;            // heads_q / heads_kv
     int batch;
     int heads_q;
     int heads_kv;
@@ -104,13 +107,13 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const uint32_t abort_flag = tmem_slot + 4;
 
     const int n_q_tiles = tiles_of(a.band.seqlen_q);  // of the longest sequence
-    const int bh_count = a.batch * a.heads_q;
     // heaviest query tiles (most visible keys) are launched first
-    const int qt = kCausal ? n_q_tiles - 1 - int(blockIdx.x) / bh_count : int(blockIdx.x) / bh_count;
-    const int bhi = int(blockIdx.x) % bh_count;
-    const int b = bhi / a.heads_q;
-    const int hq = bhi % a.heads_q;
-    const int kvh = hq / (a.heads_q / a.heads_kv);
+    const int slot = fast_div(int(blockIdx.x), a.bh);
+    const int qt = kCausal ? n_q_tiles - 1 - slot : slot;
+    const int bhi = int(blockIdx.x) - slot * a.bh.divisor;
+    const int b = fast_div(bhi, a.heads);
+    const int hq = bhi - b * a.heads_q;
+    const int kvh = fast_div(hq, a.group);
     // packed sequences: this batch entry's own lengths and first rows (see the five-GEMM kernel)
     Band band = a.band;
     int q_base = 0, k_base = 0, b_coord = b;

@@ -467,6 +467,11 @@ FusedLaunch prepare_fused(const ShaoboFa3Params* p, const void* dout, const void
     args.order_mode = plan.mode;
     args.order_width = plan.width;
     args.head_group = plan.head_group;
+    args.per_group = fast_div_of(int64_t(n_tiles) * plan.head_group);
+    args.in_group = fast_div_of(plan.head_group);
+    args.kv_heads = fast_div_of(p->num_heads_kv);
+    args.chunks = fast_div_of(split.chunks_per_head);
+    args.group = group;
     args.chunk_steps = split.chunk_steps;
     args.chunks_per_head = split.chunks_per_head;
     if (split.chunk_steps > 0) {
@@ -593,6 +598,9 @@ int launch_dq(const ShaoboFa3Params* p, const void* dout, const void* q, const v
     args.dq = dq;
     // fp32 dQ of the split path is always [B,Hq,Sq,D]; 16-bit dQ follows the layout of Q
     args.q_strides = strides_of(bshd && !out_f32, p->num_heads_q, shape.rows_q, d);
+    args.bh = fast_div_of(int64_t(p->batch) * p->num_heads_q);
+    args.heads = fast_div_of(p->num_heads_q);
+    args.group = fast_div_of(p->num_heads_q / p->num_heads_kv);
     args.batch = p->batch;
     args.heads_q = p->num_heads_q;
     args.heads_kv = p->num_heads_kv;
@@ -683,6 +691,9 @@ int launch_fwd(const ShaoboFa3Params* p, const void* q, const void* k, const voi
     args.out = out;
     args.lse = lse;
     args.o_strides = strides_of(shape.bshd, p->num_heads_q, shape.rows_q, d);
+    args.bh = fast_div_of(int64_t(p->batch) * p->num_heads_q);
+    args.heads = fast_div_of(p->num_heads_q);
+    args.group = fast_div_of(p->num_heads_q / p->num_heads_kv);
     args.batch = p->batch;
     args.heads_q = p->num_heads_q;
     args.heads_kv = p->num_heads_kv;
@@ -699,6 +710,7 @@ int launch_fwd(const ShaoboFa3Params* p, const void* q, const void* k, const voi
     // one CTA per pair of query tiles, or a cluster of `splits` of them
     const int64_t units = int64_t((tiles_of(plan_seqlen_q(p)) + 1) / 2) * p->batch * p->num_heads_q;
     args.splits = cached_fwd_splits(args.band, int64_t(p->batch) * p->num_heads_q, sm_count());
+    args.split_shift = args.splits == 8 ? 3 : args.splits == 4 ? 2 : args.splits == 2 ? 1 : 0;
     const int64_t blocks64 = units * args.splits;
     if (blocks64 > 0x7fffffffLL) return SHAOBO_FA3_STATUS_UNSUPPORTED;
     L.blocks = int(blocks64);

@@ -123,6 +123,11 @@ struct FusedArgs {
     // softcap_post = softcap * log2(e)
     float softcap_pre;
     float softcap_post;
+    FastDiv per_group;     // key tiles * head_group
+    FastDiv in_group;      // head_group
+    FastDiv kv_heads;      // heads_kv
+    FastDiv chunks;        // chunks_per_head
+    int group;             // heads_q / heads_kv
     int order_mode;        // see cta_order.h
     int order_width;
     int head_group;        // heads per scheduling group: block = (group * n_tiles + tile slot) * head_group + head
@@ -299,16 +304,15 @@ __device__ __forceinline__ FusedWork fused_work(const FusedArgs& a) {
     const int n_tiles = tiles_of(a.band.seqlen_k);      // key tiles (of the longest sequence)
     const int bh_count = a.batch * a.heads_kv;
     const bool split = a.chunk_steps > 0;
-    const int group = a.heads_q / a.heads_kv;
+    const int group = a.group;
     int bhi;
     w.t_begin = w.slab = 0;
     if (!split) {
         // groups of head_group heads; inside a group tile slot major, head minor (see cta_order.h)
-        const int per_group = n_tiles * a.head_group;
-        const int hg = int(blockIdx.x) / per_group;
-        const int rem = int(blockIdx.x) - hg * per_group;
+        const int hg = fast_div(int(blockIdx.x), a.per_group);
+        const int rem = int(blockIdx.x) - hg * a.per_group.divisor;
         const int heads_here = min(a.head_group, bh_count - hg * a.head_group);
-        const int tile_slot = rem / heads_here;
+        const int tile_slot = heads_here == a.head_group ? fast_div(rem, a.in_group) : rem / heads_here;
         bhi = hg * a.head_group + (rem - tile_slot * heads_here);
         w.kt = remap_k_tile(tile_slot, n_tiles, a.order_mode, a.order_width);
     } else {
@@ -316,10 +320,10 @@ __device__ __forceinline__ FusedWork fused_work(const FusedArgs& a) {
         w.kt = int(entry & 0xffu);
         w.t_begin = int((entry >> 8) & 0xffu) * a.chunk_steps;
         w.slab = int(entry >> 16);
-        bhi = w.slab / a.chunks_per_head;
+        bhi = fast_div(w.slab, a.chunks);
     }
-    w.b = bhi / a.heads_kv;
-    w.kvh = bhi % a.heads_kv;
+    w.b = fast_div(bhi, a.kv_heads);
+    w.kvh = bhi - w.b * a.heads_kv;
     w.first_head = w.kvh * group;
     // Packed sequences: this batch entry's own lengths and first rows; tensors are addressed as one
     // batch of `total` rows, so rows past the end of a sequence belong to its neighbour (or read as
@@ -351,7 +355,7 @@ __device__ __forceinline__ FusedWork fused_work(const FusedArgs& a) {
     // Query tiles are visited in ascending order starting at the diagonal (causal) or at a
     // per-CTA rotation (non-causal), so that CTAs of one head that run together add into
     // different dQ tiles at any moment.
-    w.rotation = (kCausal || w.q_tiles == 0) ? 0 : w.kt % w.q_tiles;
+    w.rotation = (kCausal || w.q_tiles == 0) ? 0 : w.kt < w.q_tiles ? w.kt : w.kt % w.q_tiles;
     return w;
 }
 
@@ -360,7 +364,7 @@ template <bool kCausal>
 struct StepWalk {
     int hq, qt, r;
     __device__ __forceinline__ explicit StepWalk(const FusedWork& w) {
-        const int g = w.steps_per_head > 0 ? w.t_begin / w.steps_per_head : 0;
+        const int g = w.t_begin < w.steps_per_head || w.steps_per_head == 0 ? 0 : w.t_begin / w.steps_per_head;
         hq = w.first_head + g;
         r = w.t_begin - g * w.steps_per_head;
         qt = r + (kCausal ? w.q_begin : w.rotation);

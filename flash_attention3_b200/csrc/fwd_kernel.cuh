@@ -65,6 +65,10 @@ struct FwdArgs {
     float scale_log2;         // softmax scale * log2(e)
     float softcap_pre;        // softcap variant: scores become softcap_post * tanh(score * softcap_pre),
     float softcap_post;       // with softcap_pre = scale / softcap and softcap_post = softcap * log2(e)
+    FastDiv bh;               // batch * heads_q
+    FastDiv heads;            // heads_q
+    FastDiv group;            // heads_q / heads_kv
+    int split_shift;          // log2(splits)
     int splits;               // CTAs per pair of query tiles: a cluster of so many shares its key tiles
     int staged_store;         // out goes through tm_o (not packed: the copy engine cannot clip at a sequence's end)
 };
@@ -139,15 +143,15 @@ template <bool kMasked>
 __device__ __forceinline__ FwdWork fwd_work(const FwdArgs& a) {
     FwdWork w;
     const int n_pairs = (tiles_of(a.band.seqlen_q) + 1) / 2;  // of the longest sequence
-    const int bh_count = a.batch * a.heads_q;
-    const int unit = int(blockIdx.x) / a.splits;
-    w.rank = int(blockIdx.x) - unit * a.splits;       // == rank in the cluster
+    const int unit = int(blockIdx.x) >> a.split_shift;
+    w.rank = int(blockIdx.x) & (a.splits - 1);        // == rank in the cluster
+    const int slot = fast_div(unit, a.bh);
     // heaviest query tiles (most visible keys) are launched first
-    w.pair = kMasked ? n_pairs - 1 - unit / bh_count : unit / bh_count;
-    const int bhi = unit % bh_count;
-    w.b = bhi / a.heads_q;
-    w.hq = bhi % a.heads_q;
-    w.kvh = w.hq / (a.heads_q / a.heads_kv);
+    w.pair = kMasked ? n_pairs - 1 - slot : slot;
+    const int bhi = unit - slot * a.bh.divisor;
+    w.b = fast_div(bhi, a.heads);
+    w.hq = bhi - w.b * a.heads_q;
+    w.kvh = fast_div(w.hq, a.group);
     ptx::grid_dependency_wait();
     // packed sequences: this batch entry's own lengths and first rows
     Band band = a.band;
@@ -189,7 +193,7 @@ __device__ __forceinline__ FwdWork fwd_work(const FwdArgs& a) {
         t_end = first[1] + count[1] - 1;
     }
     if (a.splits > 1) {
-        const int share = (t_end - t_begin + a.splits) / a.splits;  // ceil(tiles / splits)
+        const int share = (t_end - t_begin + a.splits) >> a.split_shift;  // ceil(tiles / splits)
         t_begin += w.rank * share;
         t_end = min(t_end, t_begin + share - 1);
 #pragma unroll

@@ -288,6 +288,15 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     const uint32_t tmem_slot = sbase + C::kOffBar + 8 * kFwdNum;
     const uint32_t abort_flag = tmem_slot + 4;
 
+    // Packed sequences: the grid is sized for the longest one, so many CTAs have no rows; they leave before any set-up.
+    if (a.cu_seqlens_q != nullptr) {
+        ptx::grid_dependency_wait();
+        const int slot = fast_div(int(blockIdx.x) >> a.split_shift, a.bh);
+        const int first_pair = kMasked ? (tiles_of(a.band.seqlen_q) + 1) / 2 - 1 - slot : slot;
+        const int entry = fast_div((int(blockIdx.x) >> a.split_shift) - slot * a.bh.divisor, a.heads);
+        if (first_pair * 2 * C::kTile >= a.cu_seqlens_q[entry + 1] - a.cu_seqlens_q[entry]) return;
+    }
+
     // Set-up first: launched programmatically, it overlaps the end of the kernel in front, which
     // grid_dependency_wait() below waits for before any of its outputs is read.
     const bool misaligned = (sbase & 1023u) != 0;

@@ -13,6 +13,7 @@
 #pragma once
 
 #include <algorithm>
+#include <array>
 #include <functional>
 #include <queue>
 #include <vector>
@@ -148,31 +149,50 @@ inline CtaOrderPlan plan_cta_order(int n_tiles, int bh_count, int group, bool ca
     return plan_cta_order(TileWork::square(n_tiles, causal), bh_count, group, sms, dq_bytes_per_head);
 }
 
-// How many CTAs (a cluster of 1, 2, 4 or 8) share the key tiles of a pair of query tiles in the forward.
+// How the forward hands out its query tiles.  splits: how many CTAs (a cluster of 1, 2, 4 or 8) share the key tiles
+// of a pair of neighbouring query tiles.  fold: a CTA takes the last and the first query tile, the last but one and
+// the second, and so on, where a causal mask gives the later ones more keys.
 // Pairs are launched heaviest first when the mask makes them unequal; a cluster needs its SMs at the same
-// time, so the model hands the pairs to sms / splits gangs as these free up.  A CTA costs its key tiles plus
-// what corresponds to 3 of them (set-up, first loads, pipeline fill, output), and a split one 3 more (partial
-// outputs exchanged through distributed shared memory).  The fewest CTAs within 3 % of the best are taken.
-// us per call, one against the planned number: S=2048, 4 heads, D=128 causal 33.1 and 18.0; S=1024, 1 head 19.2
-// and 13.2; 300 queries x 8000 keys, 2 heads 156 and 24; S=512, 1 head 12.5 and 13.4 (not split).
-inline int plan_fwd_splits(const Band& band, long long bh_count, int sms) {
-    const int pairs = (tiles_of(band.seqlen_q) + 1) / 2;
-    if (pairs * bh_count > 8LL * sms) return 1;  // many waves: nothing stands idle for long
-    int best = 1;
+// time, so the model hands the pairs to as many gangs of SMs as the device holds clusters of that size (gangs[0 .. 3];
+// fewer than sms / splits, because a cluster does not cross a GPC) as these free up.  A CTA costs its key tiles plus
+// what corresponds to 3 of them (set-up, first loads, pipeline fill, output), and a split one 2 to 3 more (partial
+// outputs exchanged through distributed shared memory).  A key tile that only one of the two query tiles sees costs
+// 5/6, so folded pairs do more work in sum but are nearly equal: they pay for up to about one wave of CTAs.  (Of
+// 1.93 us per key tile at D=128, 1.47 at D=64, the model is within 5 % for 4 to 96 heads of 384 to 3072 rows.)  A plan
+// further down the list has to be 2 % better than those in front of it.
+// us per call, one CTA per pair of neighbours against the planned number: S=2048, 4 heads, D=128 causal 33.1 and 18.0;
+// S=1024, 1 head 19.2 and 13.2; 300 queries x 8000 keys, 2 heads 156 and 24.  Neighbours against folded pairs, causal:
+// 16 heads x 2048, D=128 37.1 and 32.3, D=64 29.8 and 24.7; 32 x 1024, D=128 21.9 and 19.1; 48 x 512 14.4 and 13.2.
+struct FwdPlan {
+    int splits = 1;
+    bool fold = false;
+};
+
+using FwdGangs = std::array<int, 4>;  // clusters of 1, 2, 4, 8 CTAs that run at the same time
+
+inline FwdPlan plan_fwd(const Band& band, long long bh_count, const FwdGangs& gangs) {
+    const int q_tiles = tiles_of(band.seqlen_q), pairs = (q_tiles + 1) / 2;
+    FwdPlan best;
+    if (pairs * bh_count > 8LL * gangs[0]) return best;  // many waves: nothing stands idle for long
+    const FwdPlan options[] = {{1, false}, {1, true}, {2, false}, {4, false}, {8, false}};
     long long best_cost = -1;
-    for (int splits = 1; splits <= 8; splits *= 2) {
+    for (const FwdPlan& option : options) {
+        if (option.fold && (band.left < kUnbounded || band.right >= kUnbounded)) continue;  // (every tile starts at the first key)
         std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free_at;
-        for (int i = 0; i < sms / splits; ++i) free_at.push(0);
+        const int gang = option.splits == 8 ? 3 : option.splits / 2;
+        for (int i = 0; i < std::max(1, gangs[size_t(gang)]); ++i) free_at.push(0);
         long long makespan = 0;
-        for (int pair = pairs - 1; pair >= 0; --pair) {
+        for (int slot = 0; slot < pairs; ++slot) {
+            const int heavy = q_tiles - 1 - slot;  // (of an odd number of tiles the middle one is alone)
+            const int a = option.fold ? heavy : 2 * (pairs - 1 - slot), b = option.fold ? (slot < heavy ? slot : q_tiles) : a + 1;
+            const int most_a = k_tiles_of_q_tile(a, band), most_b = b < q_tiles ? k_tiles_of_q_tile(b, band) : 0;
             int first = kUnbounded, last = -1;
-            for (int qt = 2 * pair; qt < 2 * pair + 2 && qt < tiles_of(band.seqlen_q); ++qt) {
-                if (k_tiles_of_q_tile(qt, band) == 0) continue;
-                first = std::min(first, first_k_tile(qt, band));
-                last = std::max(last, last_k_tile(qt, band));
-            }
-            const int tiles = last >= first ? last - first + 1 : 0;
-            const long long cost = 3 + (splits > 1 ? 3 : 0) + (tiles + splits - 1) / splits;
+            if (most_a > 0) first = first_k_tile(a, band), last = last_k_tile(a, band);
+            if (most_b > 0) first = std::min(first, first_k_tile(b, band)), last = std::max(last, last_k_tile(b, band));
+            const int tiles = last >= first ? last - first + 1 : 0, both = std::max(0, most_a + most_b - tiles);
+            // in sixths of a key tile
+            const long long cost = option.splits == 1 ? 6 * (3 + both) + 5 * (tiles - both)
+                                                      : 6 * (3 + (tiles + option.splits - 1) / option.splits) + (option.splits == 2 ? 13 : option.splits == 4 ? 15 : 18);
             for (long long i = 0; i < bh_count; ++i) {
                 const long long end = free_at.top() + cost;
                 free_at.pop();
@@ -180,9 +200,9 @@ inline int plan_fwd_splits(const Band& band, long long bh_count, int sms) {
                 makespan = std::max(makespan, end);
             }
         }
-        if (best_cost < 0 || makespan * 103 < best_cost * 100) {
+        if (best_cost < 0 || makespan * 102 < best_cost * 100) {
             best_cost = makespan;
-            best = splits;
+            best = option;
         }
     }
     return best;

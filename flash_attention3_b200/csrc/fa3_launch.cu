@@ -138,17 +138,6 @@ CtaOrderPlan cached_plan(const TileWork& work, int bh, int group, int sms, long 
     return plan;
 }
 
-int cached_fwd_splits(const Band& band, int64_t bh, int sms) {
-    static std::mutex mu;
-    static std::map<std::tuple<int, int, int, int, int64_t, int>, int> cache;
-    const auto key = std::make_tuple(band.seqlen_q, band.seqlen_k, band.left, band.right, bh, sms);
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(key);
-    if (it != cache.end()) return it->second;
-    if (cache.size() > 4096) cache.clear();
-    return cache[key] = plan_fwd_splits(band, bh, sms);
-}
-
 // Remembers, per CUDA device, that a one-time set-up step has been done
 // (function attributes are per device).
 struct DeviceOnce {
@@ -674,6 +663,46 @@ int launch_fwd_d(const ShaoboFa3Params* p, const FwdLaunch& L) {
     return masked ? launch_fwd_t<T, 64, true>(L, st) : launch_fwd_t<T, 64, false>(L, st);
 }
 
+// How many clusters of 1, 2, 4 and 8 CTAs of the forward kernel the current device runs at the same time (every variant
+// takes a whole SM).
+FwdGangs fwd_gangs() {
+    FwdGangs gangs;
+    const int sms = sm_count();
+    auto kernel = fwd_kernel<__nv_bfloat16, 64, true>;
+    const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<64>::kSmemBytes) == cudaSuccess;
+    for (int i = 0; i < 4; ++i) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(unsigned(sms / 8 * 8));
+        cfg.blockDim = dim3(FwdCfg<64>::kThreads);
+        cfg.dynamicSmemBytes = FwdCfg<64>::kSmemBytes;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1u << i;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        gangs[size_t(i)] = i > 0 && ok && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0
+                               ? std::min(n, sms >> i) : sms >> i;
+    }
+    return gangs;
+}
+
+FwdPlan cached_fwd_plan(const Band& band, int64_t bh) {
+    static std::mutex mu;
+    static std::map<int, FwdGangs> gangs;
+    static std::map<std::tuple<int, int, int, int, int64_t, int>, FwdPlan> cache;
+    const int dev = DeviceOnce::device();
+    const auto key = std::make_tuple(band.seqlen_q, band.seqlen_k, band.left, band.right, bh, dev);
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = cache.find(key);
+    if (it != cache.end()) return it->second;
+    if (gangs.find(dev) == gangs.end()) gangs[dev] = fwd_gangs();
+    if (cache.size() > 4096) cache.clear();
+    return cache[key] = plan_fwd(band, bh, gangs[dev]);
+}
+
 int launch_fwd(const ShaoboFa3Params* p, const void* q, const void* k, const void* v, void* out,
                float* lse) {
     const bool bf = p->dtype == SHAOBO_FA3_DTYPE_BF16;
@@ -709,7 +738,9 @@ int launch_fwd(const ShaoboFa3Params* p, const void* q, const void* k, const voi
     args.staged_store = is_varlen(p) ? 0 : 1;
     // one CTA per pair of query tiles, or a cluster of `splits` of them
     const int64_t units = int64_t((tiles_of(plan_seqlen_q(p)) + 1) / 2) * p->batch * p->num_heads_q;
-    args.splits = cached_fwd_splits(args.band, int64_t(p->batch) * p->num_heads_q, sm_count());
+    const FwdPlan plan = cached_fwd_plan(args.band, int64_t(p->batch) * p->num_heads_q);
+    args.splits = plan.splits;
+    args.fold = plan.fold && !is_varlen(p) ? 1 : 0;  // (packed sequences have different numbers of tiles)
     args.split_shift = args.splits == 8 ? 3 : args.splits == 4 ? 2 : args.splits == 2 ? 1 : 0;
     const int64_t blocks64 = units * args.splits;
     if (blocks64 > 0x7fffffffLL) return SHAOBO_FA3_STATUS_UNSUPPORTED;

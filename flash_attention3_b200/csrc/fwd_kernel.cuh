@@ -31,7 +31,7 @@
 // 1.6 GHz); B=2, Hq=32, Hkv=8, S=8192 causal, D=128 905 and 1150.
 //
 // When the pairs are too few to fill the GPU a cluster of 2, 4 or 8 CTAs shares the key tiles of a pair
-// (plan_fwd_splits) and merges the partial outputs through distributed shared memory.
+// (plan_fwd) and merges the partial outputs through distributed shared memory.
 //
 // Tensor-memory ledger: S_A [0,128)  S_B [128,256)  O_A [256,256+D)  O_B [256+D,256+2D); at D=64 also
 // P_A [384,448)  P_B [448,512).
@@ -70,6 +70,7 @@ struct FwdArgs {
     FastDiv group;            // heads_q / heads_kv
     int split_shift;          // log2(splits)
     int splits;               // CTAs per pair of query tiles: a cluster of so many shares its key tiles
+    int fold;                 // pairs are the last and the first query tile, the last but one and the second, ... (no split)
     int staged_store;         // out goes through tm_o (not packed: the copy engine cannot clip at a sequence's end)
 };
 
@@ -129,6 +130,7 @@ enum FwdBar : int {
 // Which query tiles and keys a CTA works on.
 struct FwdWork {
     int pair, rank, hq, kvh, b, b_coord, q_base, k_base;
+    int tile[2];         // query tiles A and B
     int slot_q;          // rows of out this batch entry owns
     int t_begin, n_iter; // the CTA walks key tiles t_begin .. t_begin + n_iter - 1;
     int lo[2], hi[2];    // query tile x takes part in iterations lo[x] .. hi[x] - 1 (none when it sees no key or
@@ -148,6 +150,13 @@ __device__ __forceinline__ FwdWork fwd_work(const FwdArgs& a) {
     const int slot = fast_div(unit, a.bh);
     // heaviest query tiles (most visible keys) are launched first
     w.pair = kMasked ? n_pairs - 1 - slot : slot;
+    w.tile[0] = 2 * w.pair;
+    w.tile[1] = 2 * w.pair + 1;
+    if (kMasked && a.fold) {  // (of an odd number of tiles the middle one is alone)
+        const int n_tiles = tiles_of(a.band.seqlen_q);
+        w.tile[0] = n_tiles - 1 - slot;
+        w.tile[1] = slot < w.tile[0] ? slot : n_tiles;
+    }
     const int bhi = unit - slot * a.bh.divisor;
     w.b = fast_div(bhi, a.heads);
     w.hq = bhi - w.b * a.heads_q;
@@ -177,7 +186,7 @@ __device__ __forceinline__ FwdWork fwd_work(const FwdArgs& a) {
     int first[2], count[2];
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
-        const int qt = 2 * w.pair + x;
+        const int qt = w.tile[x];
         first[x] = first_k_tile(qt, band);
         count[x] = qt * kTileRows < band.seqlen_q ? k_tiles_of_q_tile(qt, band) : 0;
     }
@@ -355,7 +364,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 for (int x = 0; x < 2; ++x) {
                     if (w.lo[x] >= w.hi[x]) continue;  // nothing is loaded for a tile that sees no key
                     ptx::tma_load_tile_elect<C::kBoxes>(sbase + C::kOffQ + x * C::kOperandBytes, &tm_q, bar(kFwdQFull + x),
-                                                        w.q_base + (2 * w.pair + x) * C::kTile, w.hq, w.b_coord);
+                                                        w.q_base + w.tile[x] * C::kTile, w.hq, w.b_coord);
                 }
 #pragma unroll 1
                 for (int it = 0; it < n_iter; ++it) {
@@ -487,7 +496,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         } else {
             const int x = (warp - 4) >> 2;      // which query tile
             const int i = threadIdx.x & 127;    // query row inside the tile == TMEM lane
-            const int qt = 2 * w.pair + x;
+            const int qt = x == 0 ? w.tile[0] : w.tile[1];
             const int n_steps = x == 0 ? w.hi[0] - w.lo[0] : w.hi[1] - w.lo[1];  // (selects, not indexing: no local array)
             const int k_begin = w.t_begin + (x == 0 ? w.lo[0] : w.lo[1]);
             const uint32_t tl = tmem + (uint32_t((warp & 3) * 32) << 16);

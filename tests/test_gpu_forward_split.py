@@ -20,6 +20,10 @@ CASES = [
     (1, 1, 1, 129, 1153, 128, "fp16", True, "bhsd", (-1, -1)),     # 10 key tiles over 8 CTAs: the last ones get none
     (1, 2, 2, 1500, 1500, 128, "bf16", True, "bhsd", (700, -1)),   # a window: pairs see a part of the keys
     (1, 2, 2, 1700, 1100, 64, "fp16", True, "bhsd", (-1, -1)),     # leading queries without a key
+    # CTAs that take the last and the first query tile, the last but one and the second, ... (no split)
+    (1, 2, 1, 449, 449, 128, "bf16", True, "bhsd", (-1, -1)),      # four tiles, the last one ragged
+    (2, 1, 1, 833, 333, 64, "fp16", True, "bshd", (-1, -1)),       # seven tiles: the middle one is alone; tiles without a key
+    (1, 12, 4, 769, 769, 64, "bf16", True, "bshd", (-1, -1)),
 ]
 
 
@@ -39,6 +43,18 @@ def test_used_lengths_with_split_keys():
     ref = golden.backward(q[:, :, :used_q], k[:, :, :used_k], v[:, :, :used_k], do[:, :, :used_q], False, 1.0 / np.sqrt(d), dtype)
     used = [torch.tensor([n], dtype=torch.int32, device="cuda") for n in (used_q, used_k)]
     out, lse = ops.fa3_fwd(dev(q, dtype), dev(k, dtype), dev(v, dtype), False, seqused_q=used[0], seqused_k=used[1], sync=True)
+    out, lse = host(out), host(lse)
+    check_forward(out[:, :, :used_q], lse[:, :, :used_q], ref["out"], ref["lse"], dtype, "used lengths")
+    assert (out[:, :, used_q:] == 0).all() and np.isneginf(lse[:, :, used_q:]).all()
+
+
+@pytest.mark.parametrize("used_q,used_k", [(500, 500), (130, 500), (500, 260), (60, 1)])
+def test_used_lengths_with_folded_pairs(used_q, used_k):
+    b, h, s, d, dtype = 1, 3, 500, 128, "fp16"
+    q, k, v, do = golden.seeded_inputs(43, b, h, h, s, d, dtype)
+    ref = golden.backward(q[:, :, :used_q], k[:, :, :used_k], v[:, :, :used_k], do[:, :, :used_q], True, 1.0 / np.sqrt(d), dtype)
+    used = [torch.tensor([n], dtype=torch.int32, device="cuda") for n in (used_q, used_k)]
+    out, lse = ops.fa3_fwd(dev(q, dtype), dev(k, dtype), dev(v, dtype), True, seqused_q=used[0], seqused_k=used[1], sync=True)
     out, lse = host(out), host(lse)
     check_forward(out[:, :, :used_q], lse[:, :, :used_q], ref["out"], ref["lse"], dtype, "used lengths")
     assert (out[:, :, used_q:] == 0).all() and np.isneginf(lse[:, :, used_q:]).all()

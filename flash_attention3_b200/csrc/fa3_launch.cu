@@ -271,6 +271,8 @@ void launch_convert(const ShaoboFa3Params* p, const float* accum, void* dq,
     seg.layout[0] = row_layout(p, p->num_heads_q, shape.rows_q, shape.bshd);
     seg.count = 1;
     int64_t total = seg.n_vec8[0];
+    constexpr int kShared = 8;  // lanes that share the partial sums of a vector where they are many
+    int lanes = 0;
     const SplitPlan split = dkv_slabs != nullptr ? split_plan(p) : SplitPlan{};
     if (split.chunk_steps > 0) {
         const int64_t n = int64_t(shape.batch) * p->num_heads_kv * shape.rows_k * p->head_dim_qk;
@@ -279,6 +281,7 @@ void launch_convert(const ShaoboFa3Params* p, const float* accum, void* dq,
         seg.n_vec8[1] = seg.n_vec8[2] = n / 8;
         seg.layout[1] = seg.layout[2] = row_layout(p, p->num_heads_kv, shape.rows_k, shape.bshd);
         seg.count = 3;
+        lanes = 1;
         seg.slabs = dkv_slabs;
         seg.slabs_f16 = p->dtype == SHAOBO_FA3_DTYPE_FP16 ? 1 : 0;
         seg.rows_k = shape.rows_k;
@@ -294,7 +297,11 @@ void launch_convert(const ShaoboFa3Params* p, const float* accum, void* dq,
             next += (steps + split.chunk_steps - 1) / split.chunk_steps;
         }
         seg.chunk_begin[tiles] = static_cast<unsigned short>(next);
-        total += 2 * (n / 8);
+        // (the line: bf16, 1 head, D=128 full, S=1024 with 8 slabs per tile 15.1 us alone and 15.4 shared, S=1536 with 12
+        // 22.9 and 18.8; fp16 8 slabs 17.2 and 19.9, 16 slabs 24.5 and 24.5, 32 slabs 19.5 and 16.5; and one trip per thread)
+        const bool deep = seg.slabs_f16 ? split.chunks_per_head >= 16 * tiles : split.chunks_per_head > 8 * tiles;
+        if (deep && total + 2 * (n / 8) * kShared <= int64_t(sm_count()) * 16 * 256) lanes = kShared;
+        total += 2 * (n / 8) * lanes + 96;  // (segments rounded up to warps)
     }
     int64_t blocks = (total + 255) / 256;  // one 8-element vector per thread while the grid allows it
     const int64_t cap = int64_t(sm_count()) * 16;
@@ -309,11 +316,13 @@ void launch_convert(const ShaoboFa3Params* p, const float* accum, void* dq,
     attr[0].val.programmaticStreamSerializationAllowed = 1;  // the kernel waits for the GEMM kernel itself
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const bool slabs = seg.count == 3, bf = p->dtype == SHAOBO_FA3_DTYPE_BF16;
+    const bool bf = p->dtype == SHAOBO_FA3_DTYPE_BF16;
     auto launch = [&](auto d) {
         constexpr int D = decltype(d)::value;
-        if (bf) cudaLaunchKernelEx(&cfg, slabs ? dq_convert_kernel<__nv_bfloat16, D, true> : dq_convert_kernel<__nv_bfloat16, D, false>, seg);
-        else cudaLaunchKernelEx(&cfg, slabs ? dq_convert_kernel<__half, D, true> : dq_convert_kernel<__half, D, false>, seg);
+        auto kernel = lanes == 0   ? (bf ? dq_convert_kernel<__nv_bfloat16, D, 0> : dq_convert_kernel<__half, D, 0>)
+                      : lanes == 1 ? (bf ? dq_convert_kernel<__nv_bfloat16, D, 1> : dq_convert_kernel<__half, D, 1>)
+                                   : (bf ? dq_convert_kernel<__nv_bfloat16, D, kShared> : dq_convert_kernel<__half, D, kShared>);
+        cudaLaunchKernelEx(&cfg, kernel, seg);
     };
     if (p->head_dim_qk == 128) launch(std::integral_constant<int, 128>{});
     else launch(std::integral_constant<int, 64>{});

@@ -133,3 +133,18 @@ MANY_TILES_SPLIT = [
 def test_split_with_a_nearly_empty_last_wave(b, hq, hkv, s, d, dtype, causal):
     prob = Problem(b, hq, hkv, s, d, dtype, causal, seed=4321 + s)
     assert_parity(run_v2(prob), prob, label=f"{(b, hq, hkv, s, d, dtype, causal)}")
+
+
+# (b, hq, hkv, sq, sk, d, dtype, causal, layout): key tiles in many chunks, whose partial sums eight lanes share
+MANY_CHUNKS = [
+    (1, 8, 1, 512, 512, 128, "bf16", False, "bhsd"),    # 32 per tile
+    (1, 8, 1, 500, 509, 64, "fp16", False, "bshd"),     # 32 per tile in fp16; ragged
+    (1, 3, 1, 1000, 129, 64, "bf16", True, "bshd"),     # a tile with one row, query rows that are no multiple of a warp
+    (1, 1, 1, 1537, 1537, 128, "bf16", True, "bhsd"),   # 1 to 13 per tile: lanes without any
+]
+
+
+@pytest.mark.parametrize("b,hq,hkv,sq,sk,d,dtype,causal,layout", MANY_CHUNKS)
+def test_many_partial_sums_per_tile(b, hq, hkv, sq, sk, d, dtype, causal, layout):
+    prob = Problem(b, hq, hkv, sq, d, dtype, causal, seed=99 + sq, sk=sk, layout=layout)
+    assert_parity(run_v2(prob), prob, label=f"{(b, hq, hkv, sq, sk, d, dtype, causal, layout)}")

@@ -170,14 +170,15 @@ struct FwdPlan {
 
 using FwdGangs = std::array<int, 4>;  // clusters of 1, 2, 4, 8 CTAs that run at the same time
 
-inline FwdPlan plan_fwd(const Band& band, long long bh_count, const FwdGangs& gangs) {
+// (packed sequences have different numbers of tiles: not folded)
+inline FwdPlan plan_fwd(const Band& band, long long bh_count, const FwdGangs& gangs, bool packed) {
     const int q_tiles = tiles_of(band.seqlen_q), pairs = (q_tiles + 1) / 2;
     FwdPlan best;
     if (pairs * bh_count > 8LL * gangs[0]) return best;  // many waves: nothing stands idle for long
     const FwdPlan options[] = {{1, false}, {1, true}, {2, false}, {4, false}, {8, false}};
     long long best_cost = -1;
     for (const FwdPlan& option : options) {
-        if (option.fold && (band.left < kUnbounded || band.right >= kUnbounded)) continue;  // (every tile starts at the first key)
+        if (option.fold && (packed || band.left < kUnbounded || band.right >= kUnbounded)) continue;  // (every tile starts at the first key)
         std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free_at;
         const int gang = option.splits == 8 ? 3 : option.splits / 2;
         for (int i = 0; i < std::max(1, gangs[size_t(gang)]); ++i) free_at.push(0);

@@ -698,18 +698,18 @@ FwdGangs fwd_gangs() {
     return gangs;
 }
 
-FwdPlan cached_fwd_plan(const Band& band, int64_t bh) {
+FwdPlan cached_fwd_plan(const Band& band, int64_t bh, bool packed) {
     static std::mutex mu;
     static std::map<int, FwdGangs> gangs;
-    static std::map<std::tuple<int, int, int, int, int64_t, int>, FwdPlan> cache;
+    static std::map<std::tuple<int, int, int, int, int64_t, int, bool>, FwdPlan> cache;
     const int dev = DeviceOnce::device();
-    const auto key = std::make_tuple(band.seqlen_q, band.seqlen_k, band.left, band.right, bh, dev);
+    const auto key = std::make_tuple(band.seqlen_q, band.seqlen_k, band.left, band.right, bh, dev, packed);
     std::lock_guard<std::mutex> lock(mu);
     auto it = cache.find(key);
     if (it != cache.end()) return it->second;
     if (gangs.find(dev) == gangs.end()) gangs[dev] = fwd_gangs();
     if (cache.size() > 4096) cache.clear();
-    return cache[key] = plan_fwd(band, bh, gangs[dev]);
+    return cache[key] = plan_fwd(band, bh, gangs[dev], packed);
 }
 
 int launch_fwd(const ShaoboFa3Params* p, const void* q, const void* k, const void* v, void* out,
@@ -747,9 +747,9 @@ int launch_fwd(const ShaoboFa3Params* p, const void* q, const void* k, const voi
     args.staged_store = is_varlen(p) ? 0 : 1;
     // one CTA per pair of query tiles, or a cluster of `splits` of them
     const int64_t units = int64_t((tiles_of(plan_seqlen_q(p)) + 1) / 2) * p->batch * p->num_heads_q;
-    const FwdPlan plan = cached_fwd_plan(args.band, int64_t(p->batch) * p->num_heads_q);
+    const FwdPlan plan = cached_fwd_plan(args.band, int64_t(p->batch) * p->num_heads_q, is_varlen(p));
     args.splits = plan.splits;
-    args.fold = plan.fold && !is_varlen(p) ? 1 : 0;  // (packed sequences have different numbers of tiles)
+    args.fold = plan.fold ? 1 : 0;
     args.split_shift = args.splits == 8 ? 3 : args.splits == 4 ? 2 : args.splits == 2 ? 1 : 0;
     const int64_t blocks64 = units * args.splits;
     if (blocks64 > 0x7fffffffLL) return SHAOBO_FA3_STATUS_UNSUPPORTED;

@@ -265,7 +265,7 @@ __device__ __forceinline__ void fwd_merge(const FwdArgs& a, const FwdWork& w, ui
             acc[4] = fmaf(f, part[s][1].x, acc[4]); acc[5] = fmaf(f, part[s][1].y, acc[5]);
             acc[6] = fmaf(f, part[s][1].z, acc[6]); acc[7] = fmaf(f, part[s][1].w, acc[7]);
         }
-        const float inv = l > 0.0f ? 1.0f / l : 0.0f;  // (l = 0: no visible key, or behind the used length)
+        const float inv = l == 0.0f ? 0.0f : 1.0f / l;  // (l = 0: no visible key, or behind the used length; NaN stays)
         uint4 o;
         o.x = ptx::Pack2<T>::pack(acc[0] * inv, acc[1] * inv);
         o.y = ptx::Pack2<T>::pack(acc[2] * inv, acc[3] * inv);
@@ -277,7 +277,7 @@ __device__ __forceinline__ void fwd_merge(const FwdArgs& a, const FwdWork& w, ui
         *reinterpret_cast<uint2*>(dst + D / 2) = make_uint2(o.z, o.w);
         if (col == 0)
             a.lse[int64_t(w.b_coord * a.heads_q + w.hq) * a.lse_rows + w.q_base + qi] =
-                l > 0.0f ? (m + __log2f(l)) * 0.69314718055994531f : -INFINITY;
+                l == 0.0f ? -INFINITY : (m + __log2f(l)) * 0.69314718055994531f;
     }
 }
 
@@ -557,23 +557,25 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                         }
                     }
                 }
-                // four chains of three-input maxima
+                // four chains of three-input maxima; a NaN among the visible scores makes the maximum NaN
                 float mx[4];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) mx[c] = fmaxf(__uint_as_float(r[c][0]), __uint_as_float(r[c][1]));
+                for (int c = 0; c < 4; ++c) mx[c] = ptx::max_nan(__uint_as_float(r[c][0]), __uint_as_float(r[c][1]));
 #pragma unroll
                 for (int e = 2; e < 32; e += 2) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) mx[c] = ptx::max3(mx[c], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
+                    for (int c = 0; c < 4; ++c) mx[c] = ptx::max3_nan(mx[c], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
                 }
-                const float mt = fmaxf(ptx::max3(mx[0], mx[1], mx[2]), mx[3]);
-                // ---- move the reference maximum only when it is more than 2^8 too small
-                const bool move = m_ref == -INFINITY ? mt != -INFINITY : (mt - m_ref) * sl > C::kRescaleThreshold;
+                const float mt = ptx::max_nan(ptx::max3_nan(mx[0], mx[1], mx[2]), mx[3]);
+                // ---- move the reference maximum only when it is more than 2^8 too small (or NaN)
+                const bool move = m_ref == -INFINITY ? mt != -INFINITY : !((mt - m_ref) * sl <= C::kRescaleThreshold);
                 if (__any_sync(0xffffffffu, move)) {
                     // exp2(-inf) = 0 on the first move
                     const float alpha = move ? ptx::ex2_approx((m_ref - mt) * sl) : 1.0f;
                     if (move) m_ref = mt;
-                    l *= alpha;
+                    // a NaN or +inf score makes l, and by it O and the log-sum-exp, NaN (mt - mt): not every exponential
+                    // of such a row would be NaN (exp2_poly)
+                    l = fmaf(l, alpha, move ? mt - mt : 0.0f);
                     if (u > 0) {
                         // O carries the old reference: wait for P V of step u-1, then rescale these 32 rows (16
                         // columns at a time: the score row is still held in registers)

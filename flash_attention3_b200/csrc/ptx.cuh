@@ -440,9 +440,15 @@ __device__ __forceinline__ F4Pairs f2_ld_shared(uint32_t addr) {
     asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(v.lo), "=l"(v.hi) : "r"(addr) : "memory");
     return v;
 }
-__device__ __forceinline__ float max3(float a, float b, float c) {
+// Maxima that are NaN if any operand is (fmaxf drops a NaN).
+__device__ __forceinline__ float max_nan(float a, float b) {
     float d;
-    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+    float d;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
 
@@ -450,8 +456,8 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // ex2 keeps it busy for 8 cycles, these 24 instructions for two values keep the FMA pipe busy for 16).
 // x = n + f with n the nearest integer (rounded by adding 1.5 * 2^23, which also leaves n in the low bits),
 // 2^f by a polynomial of degree 5 on [-1/2, 1/2] (Remez exchange on the relative error: 7.5e-8, 2.1e-7 as
-// evaluated in fp32; ex2.approx is good to 2.4e-7), then n added to the exponent field.  x above 127 is not
-// expected; below -126 the result stays at 2^-126.
+// evaluated in fp32; ex2.approx is good to 2.4e-7), then n added to the exponent field.  x above 127 and
+// NaN are not expected (the forward treats a row with such a score by its sum); below -126 the result stays at 2^-126.
 __device__ __forceinline__ float2 exp2_poly(uint64_t x2) {
     const float kMagic = 12582912.0f;
     float2 x = f2_unpack(x2);

@@ -86,3 +86,18 @@ def test_forward_packed_sequences():
         q0, q1 = cu_q[i], cu_q[i + 1]
         check_forward(out[q0:q1].transpose(1, 0, 2)[None], lse[:, q0:q1][None], ref["out"], ref["lse"], "bf16",
                       ("packed", i))
+
+
+@pytest.mark.parametrize("softcap", [15.0, 50.0])
+@pytest.mark.parametrize("d", [64, 128])
+def test_capped_scores_are_good_to_single_precision(d, softcap):
+    """Equal keys, so that the log-sum-exp is the capped score plus log(number of keys), with scores that are exact:
+    the error of tanh, in units of the cap, stays within one rounding of a 32-bit value near 1 (rms 2^-24)."""
+    rows, keys = 4096, 128
+    score = np.random.default_rng(9).uniform(-softcap, softcap, rows).astype(np.float16)
+    q, k = np.zeros((1, 1, rows, d), np.float32), np.zeros((1, 1, keys, d), np.float32)
+    q[0, 0, :, 0], k[..., 0] = score, 1.0
+    _, lse = ops.fa3_fwd(dev(q, "fp16"), dev(k, "fp16"), dev(k, "fp16"), False, 1.0, softcap=softcap, sync=True)
+    expected = softcap * np.tanh(score.astype(np.float64) / softcap) + np.log(keys)
+    error = (host(lse)[0, 0].astype(np.float64) - expected) / softcap
+    assert np.sqrt((error ** 2).mean()) <= 2.0 ** -24

@@ -43,13 +43,7 @@ def check_forward(heads, s, d, plant, softcap):
     assert np.isfinite(out[~bad]).all() and np.isfinite(lse[~bad]).all()
     if np.isnan(plant[2]):  # (an infinity also takes keys out of other rows)
         out0, lse0 = (host(t)[0] for t in run(clean))
-        if softcap == 0.0:
-            assert np.array_equal(out[~bad], out0[~bad]) and np.array_equal(lse[~bad], lse0[~bad])
-        else:
-            # capped scores share a reciprocal in pairs, so the value of a hidden neighbour may move the last bits of tanh:
-            # 4e-7 of softcap, twice (two scores) in the log-sum-exp, and with it at most one storage step in O
-            assert np.abs(lse[~bad] - lse0[~bad]).max() <= 2 * 4e-7 * softcap
-            assert np.abs(out[~bad] - out0[~bad]).max() <= golden.storage_ulp("fp16", np.abs(out0[~bad])).max()
+        assert np.array_equal(out[~bad], out0[~bad]) and np.array_equal(lse[~bad], lse0[~bad])
 
 
 @pytest.mark.parametrize("plant", PLANTS)

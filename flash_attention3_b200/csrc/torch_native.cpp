@@ -10,6 +10,7 @@
 //
 // Two front doors share the functions below: CPython fast calls for ops.py, and the dispatcher ops
 // fa3b200::attention_fwd / attention_bwd with a C++ autograd function over them for torch_binding.py.
+#include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
@@ -465,6 +466,9 @@ class Attention : public torch::autograd::Function<Attention> {
             c10::Dispatcher::singleton().findSchemaOrThrow("fa3b200::attention_bwd", "").typed<BwdSignature>();
         const auto saved = ctx->get_saved_variables();
         auto& d = ctx->saved_data;
+        // with create_graph the op goes through its Autograd kernel, which refuses a second derivative
+        std::optional<at::AutoDispatchBelowADInplaceOrView> below_autograd;
+        if (!at::GradMode::is_enabled()) below_autograd.emplace();
         auto [dq, dk, dv] = op.call(grads[0], saved[0], saved[1], saved[2], saved[3], saved[4], d["causal"].toBool(),
                                     d["scale"].toDouble(), d["deterministic"].toBool(), d["window_left"].toInt(),
                                     d["window_right"].toInt(), d["softcap"].toDouble(), d["layout"].toStringRef());
@@ -522,6 +526,12 @@ TORCH_LIBRARY(fa3b200, m) {
 TORCH_LIBRARY_IMPL(fa3b200, CUDA, m) {
     m.impl("attention_bwd", attention_bwd);
     m.impl("attention_fwd", attention_fwd);
+}
+// The ops themselves have no derivative (attention() has one, of first order): differentiating them raises.
+// Without these kernels torch warns and leaves their part of the gradient out.
+TORCH_LIBRARY_IMPL(fa3b200, Autograd, m) {
+    m.impl("attention_bwd", torch::autograd::autogradNotImplementedFallback());
+    m.impl("attention_fwd", torch::autograd::autogradNotImplementedFallback());
 }
 
 PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&kModule); }

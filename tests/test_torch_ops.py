@@ -1,0 +1,34 @@
+"""The torch front end without a GPU: what autograd is told about the two ops, on meta tensors."""
+import pytest
+import torch
+
+from flash_attention3_b200 import torch_binding
+
+
+@pytest.fixture
+def qkv():
+    return [torch.empty((1, h, 48, 64), dtype=torch.float16, device="meta", requires_grad=True) for h in (4, 2, 2)]
+
+
+def test_attention_has_a_first_derivative(qkv):
+    out = torch_binding.attention(*qkv, causal=True)
+    grads = torch.autograd.grad(out.float().square().sum(), qkv)
+    assert [g.shape for g in grads] == [t.shape for t in qkv]
+    assert not any(g.requires_grad for g in grads)
+
+
+def test_second_derivatives_are_refused(qkv):
+    out = torch_binding.attention(*qkv, causal=True)
+    dq, = torch.autograd.grad(out.float().square().sum(), qkv[:1], create_graph=True)
+    with pytest.raises(RuntimeError, match="attention_bwd is not implemented"):
+        torch.autograd.grad(dq.float().sum(), qkv)
+
+
+def test_differentiating_the_ops_is_refused(qkv):
+    out, lse = torch.ops.fa3b200.attention_fwd(*qkv, True, 0.125)
+    assert out.requires_grad and lse.requires_grad
+    for t in (out, lse):
+        with pytest.raises(RuntimeError, match="attention_fwd is not implemented"):
+            torch.autograd.grad(t.float().sum(), qkv[:1], retain_graph=True)
+    with torch.no_grad():
+        assert not torch.ops.fa3b200.attention_fwd(*qkv, True, 0.125)[0].requires_grad

@@ -14,6 +14,7 @@
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/utils/object_ptr.h>
 #include <torch/library.h>
 #include <ATen/ATen.h>
 #include <ATen/core/dispatch/Dispatcher.h>
@@ -385,7 +386,24 @@ PyObject* py_bwd_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 // ----------------------------------------------------------- dispatcher ops (torch_binding.py)
-[[noreturn]] void fail(const AbiError& e) { TORCH_CHECK(false, e.entry, " returned ", e.code, " (", shaobo_fa3_status_string(e.code), ")"); }
+PyObject* g_error_type = nullptr;  // ops.Fa3Error, for the life of the process
+
+PyObject* py_set_error_type(PyObject*, PyObject* type) {
+    Py_INCREF(type);
+    Py_XSETREF(g_error_type, type);
+    Py_RETURN_NONE;
+}
+
+// A call that the C ABI refused raises ops.Fa3Error, through the dispatcher and the autograd engine as well.
+[[noreturn]] void fail(const AbiError& e) {
+    TORCH_CHECK(g_error_type != nullptr, e.entry, " returned ", e.code, " (", shaobo_fa3_status_string(e.code), ")");
+    pybind11::gil_scoped_acquire gil;
+    THPObjectPtr error(PyObject_CallFunction(g_error_type, "si", e.entry, e.code));
+    if (error) PyErr_SetObject(g_error_type, error.get());
+    python_error raised;
+    raised.persist();
+    throw raised;
+}
 
 // (the kernels read dense tensors: strided views are copied)
 std::tuple<Tensor, Tensor> attention_fwd(const Tensor& q_in, const Tensor& k_in, const Tensor& v_in, bool causal, double scale,
@@ -508,6 +526,7 @@ PyMethodDef kMethods[] = {
     {"fwd_packed", fast<py_fwd_packed>(), METH_FASTCALL, nullptr},
     {"bwd_packed", fast<py_bwd_packed>(), METH_FASTCALL, nullptr},
     {"attention", fast<py_attention>(), METH_FASTCALL, nullptr},
+    {"set_error_type", py_set_error_type, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

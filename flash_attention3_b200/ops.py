@@ -20,6 +20,9 @@ class Fa3Error(RuntimeError):
         self.code = code
 
 
+_native.set_error_type(Fa3Error)  # (what the torch ops raise)
+
+
 class Fa3DeviceError(RuntimeError):
     """A kernel gave up a bounded wait (1) or found its shared memory misaligned (2): its outputs are
     not valid."""

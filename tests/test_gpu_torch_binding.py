@@ -194,3 +194,35 @@ def test_two_host_threads_with_separate_staging():
         for name, t in zip(("dq", "dk", "dv"), outs):
             m = golden.check_gradient(t.float().numpy(), prob.ref[name], "bf16")
             assert m["pass"], (name, m)
+
+
+def test_refused_calls_raise_the_library_error():
+    """A parameter set that the C ABI turns away (head dimension 32) raises Fa3Error with its status everywhere."""
+    from flash_attention3_b200 import capi, ops, torch_binding
+    q = torch.zeros((1, 2, 128, 32), dtype=torch.float16, device="cuda", requires_grad=True)
+    lse = torch.zeros((1, 2, 128), device="cuda")
+    for call in (lambda: torch_binding.attention(q, q, q, causal=True),
+                 lambda: torch.ops.fa3b200.attention_fwd(q, q, q, True, 0.1),
+                 lambda: torch.ops.fa3b200.attention_bwd(q, q, q, q, q, lse, True, 0.1, False),
+                 lambda: ops.fa3_fwd(q, q, q, True)):
+        with pytest.raises(ops.Fa3Error) as refused:
+            call()
+        assert refused.value.code == capi.STATUS_UNSUPPORTED
+
+
+def test_refused_backward_raises_the_library_error_through_autograd():
+    from flash_attention3_b200 import capi, ops
+    q = torch.zeros((1, 2, 128, 32), dtype=torch.float16, device="cuda", requires_grad=True)
+
+    class Backward(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return x * 1
+
+        @staticmethod
+        def backward(ctx, g):
+            return torch.ops.fa3b200.attention_bwd(g, g, g, g, g, torch.zeros((1, 2, 128), device="cuda"), True, 0.1, False)[0]
+
+    with pytest.raises(ops.Fa3Error) as refused:
+        Backward.apply(q).float().sum().backward()
+    assert refused.value.code == capi.STATUS_UNSUPPORTED

@@ -74,21 +74,21 @@ void same_kind(const char* name, const Tensor& t, const Tensor& q) {
 // Shapes, dtypes and devices of one fixed-length problem (the C ABI takes raw pointers, so a tensor of
 // the wrong size would be read or written out of bounds), and the parameter block that describes it.
 struct Options {
-    bool causal = false;
+    int64_t causal = 0;  // (flags other than 0 and 1 are turned away by the C ABI)
     std::optional<double> scale;
     bool bshd = false;
     int64_t window_left = -1, window_right = -1;
     Tensor seqused_q, seqused_k;
     double softcap = 0.0;
-    bool deterministic = false;
-    bool sync = false;
+    int64_t deterministic = 0;
+    int64_t sync = 0;
 };
 
 void set_common(ShaoboFa3Params* p, const Tensor& q, const Options& o) {
-    p->causal = o.causal;
+    p->causal = int32_t(o.causal);
     p->dtype = dtype_code(q);
-    p->deterministic = o.deterministic;
-    p->sync_after_launch = o.sync;
+    p->deterministic = int32_t(o.deterministic);
+    p->sync_after_launch = int32_t(o.sync);
     p->window_left = int32_t(o.window_left);
     p->window_right = int32_t(o.window_right);
     p->softcap = float(o.softcap);
@@ -205,34 +205,42 @@ bool arg_bool(PyObject* o) {
     if (v < 0) throw python_error();
     return v != 0;
 }
-int64_t arg_int(PyObject* o) {
-    PyObject* i = PyNumber_Long(o);  // (takes what int() takes)
-    if (i == nullptr) throw python_error();
-    const long long v = PyLong_AsLongLong(i);
-    Py_DECREF(i);
+// bool of a torch schema: None, or what says by itself whether it is true (a string does not)
+bool arg_schema_bool(PyObject* o, const char* name) {
+    const PyNumberMethods* number = Py_TYPE(o)->tp_as_number;
+    TORCH_CHECK_TYPE(o == Py_None || (number != nullptr && number->nb_bool != nullptr), name, " must be a bool");
+    return arg_bool(o);
+}
+int64_t long_value(THPObjectPtr i) {
+    if (!i) throw python_error();
+    const long long v = PyLong_AsLongLong(i.get());
     if (v == -1 && PyErr_Occurred()) throw python_error();
     return v;
 }
-double arg_double(PyObject* o) {
+int64_t arg_int(PyObject* o) { return long_value(THPObjectPtr(PyNumber_Long(o))); }           // int(o)
+int64_t arg_schema_int(PyObject* o) { return long_value(THPObjectPtr(PyNumber_Index(o))); }  // (no float)
+double arg_double(PyObject* o) {  // a number
     const double v = PyFloat_AsDouble(o);
     if (v == -1.0 && PyErr_Occurred()) throw python_error();
     return v;
+}
+double arg_float(PyObject* o) {  // float(o)
+    const THPObjectPtr f(PyNumber_Float(o));
+    if (!f) throw python_error();
+    return PyFloat_AS_DOUBLE(f.get());
 }
 const char* arg_str(PyObject* o) {
     const char* s = PyUnicode_AsUTF8(o);
     if (s == nullptr) throw python_error();
     return s;
 }
-void arg_window(PyObject* o, Options* opt) {
-    PyObject* seq = PySequence_Fast(o, "window must be a pair");
-    if (seq == nullptr) throw python_error();
-    const bool ok = PySequence_Fast_GET_SIZE(seq) >= 2;
-    if (ok) {
-        opt->window_left = arg_int(PySequence_Fast_GET_ITEM(seq, 0));
-        opt->window_right = arg_int(PySequence_Fast_GET_ITEM(seq, 1));
+void arg_window(PyObject* o, Options* opt) {  // int(o[0]), int(o[1])
+    for (const long i : {0, 1}) {
+        const THPObjectPtr index(PyLong_FromLong(i));
+        THPObjectPtr item(index ? PyObject_GetItem(o, const_cast<PyObject*>(index.get())) : nullptr);
+        if (!item) throw python_error();
+        (i == 0 ? opt->window_left : opt->window_right) = arg_int(item.get());
     }
-    Py_DECREF(seq);
-    TORCH_CHECK_VALUE(ok, "window must be a pair");
 }
 void arg_count(Py_ssize_t got, Py_ssize_t want) { TORCH_CHECK_TYPE(got == want, "expected ", want, " arguments, got ", got); }
 
@@ -254,14 +262,14 @@ PyObject* py_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const Tensor q = arg_required(a[0], "q"), k = arg_required(a[1], "k"), v = arg_required(a[2], "v");
     require_cuda({&q, &k, &v});
     Options o;
-    o.causal = arg_bool(a[3]);
-    if (a[4] != Py_None) o.scale = arg_double(a[4]);
+    o.causal = arg_int(a[3]);
+    if (a[4] != Py_None) o.scale = arg_float(a[4]);
     o.bshd = is_bshd(arg_str(a[5]));
     arg_window(a[6], &o);
-    o.sync = arg_bool(a[7]);
+    o.sync = arg_int(a[7]);
     o.seqused_q = arg_tensor(a[8], "seqused_q");
     o.seqused_k = arg_tensor(a[9], "seqused_k");
-    o.softcap = arg_double(a[10]);
+    o.softcap = arg_float(a[10]);
     ShaoboFa3Params p = fixed_problem(q, k, v, Tensor(), Tensor(), Tensor(), o);
     try {
         Tensor out, lse;
@@ -285,17 +293,17 @@ PyObject* py_bwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
                  v = arg_required(a[3], "v"), out = arg_required(a[4], "out"), lse = arg_required(a[5], "softmax_lse");
     require_cuda({&dout, &q, &k, &v, &out, &lse});
     Options o;
-    o.causal = arg_bool(a[6]);
-    if (a[7] != Py_None) o.scale = arg_double(a[7]);
-    o.deterministic = arg_bool(a[8]);
+    o.causal = arg_int(a[6]);
+    if (a[7] != Py_None) o.scale = arg_float(a[7]);
+    o.deterministic = arg_int(a[8]);
     const Tensor workspace = arg_tensor(a[9], "workspace");
     const bool return_delta = arg_bool(a[10]);
-    o.sync = arg_bool(a[11]);
+    o.sync = arg_int(a[11]);
     o.bshd = is_bshd(arg_str(a[12]));
     arg_window(a[13], &o);
     o.seqused_q = arg_tensor(a[14], "seqused_q");
     o.seqused_k = arg_tensor(a[15], "seqused_k");
-    o.softcap = arg_double(a[17]);
+    o.softcap = arg_float(a[17]);
     ShaoboFa3Params p = fixed_problem(q, k, v, out, dout, lse, o);
     Gradients g;
     if (a[16] != Py_None) {
@@ -336,10 +344,10 @@ PyObject* py_fwd_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
                  cu_q = arg_required(a[3], "cu_seqlens_q"), cu_k = arg_required(a[4], "cu_seqlens_k");
     require_cuda({&q, &k, &v, &cu_q, &cu_k});
     Options o;
-    o.causal = arg_bool(a[7]);
-    if (a[8] != Py_None) o.scale = arg_double(a[8]);
+    o.causal = arg_int(a[7]);
+    if (a[8] != Py_None) o.scale = arg_float(a[8]);
     arg_window(a[9], &o);
-    o.sync = arg_bool(a[10]);
+    o.sync = arg_int(a[10]);
     ShaoboFa3Params p = packed_problem(q, k, cu_q, cu_k, arg_int(a[5]), arg_int(a[6]), o);
     try {
         Tensor out, lse;
@@ -363,12 +371,12 @@ PyObject* py_bwd_packed(PyObject*, PyObject* const* a, Py_ssize_t n) {
                  cu_q = arg_required(a[6], "cu_seqlens_q"), cu_k = arg_required(a[7], "cu_seqlens_k");
     require_cuda({&dout, &q, &k, &v, &out, &lse, &cu_q, &cu_k});
     Options o;
-    o.causal = arg_bool(a[10]);
-    if (a[11] != Py_None) o.scale = arg_double(a[11]);
-    o.deterministic = arg_bool(a[12]);
+    o.causal = arg_int(a[10]);
+    if (a[11] != Py_None) o.scale = arg_float(a[11]);
+    o.deterministic = arg_int(a[12]);
     arg_window(a[13], &o);
     const bool return_delta = arg_bool(a[14]);
-    o.sync = arg_bool(a[15]);
+    o.sync = arg_int(a[15]);
     ShaoboFa3Params p = packed_problem(q, k, cu_q, cu_k, arg_int(a[8]), arg_int(a[9]), o);
     try {
         Tensor delta;
@@ -499,17 +507,23 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
     arg_count(n, 9);
     const Tensor q = arg_required(a[0], "q"), k = arg_required(a[1], "k"), v = arg_required(a[2], "v");
-    Options o;
-    o.causal = arg_bool(a[3]);
+    // (what the schema of the ops takes)
+    const bool causal = arg_schema_bool(a[3], "causal"), deterministic = arg_schema_bool(a[5], "deterministic");
     const double scale = a[4] != Py_None ? arg_double(a[4]) : 1.0 / std::sqrt(double(q.size(-1)));
-    o.deterministic = arg_bool(a[5]);
-    arg_window(a[6], &o);
-    o.softcap = arg_double(a[7]);
+    THPObjectPtr window(PySequence_Tuple(a[6]));
+    if (!window) throw python_error();
+    int64_t sides[2];
+    for (const int i : {0, 1}) {
+        PyObject* item = PyTuple_GetItem(window.get(), i);
+        if (item == nullptr) throw python_error();
+        sides[i] = arg_schema_int(item);
+    }
+    const double softcap = arg_float(a[7]);
     const std::string layout = arg_str(a[8]);
     Tensor out;
     {
         pybind11::gil_scoped_release no_gil;
-        out = Attention::apply(q, k, v, o.causal, scale, o.deterministic, o.window_left, o.window_right, o.softcap, layout);
+        out = Attention::apply(q, k, v, causal, scale, deterministic, sides[0], sides[1], softcap, layout);
     }
     return THPVariable_Wrap(out);
     END_HANDLE_TH_ERRORS

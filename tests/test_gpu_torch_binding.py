@@ -226,3 +226,22 @@ def test_refused_backward_raises_the_library_error_through_autograd():
     with pytest.raises(ops.Fa3Error) as refused:
         Backward.apply(q).float().sum().backward()
     assert refused.value.code == capi.STATUS_UNSUPPORTED
+
+
+def test_flags_and_numbers_of_the_tensor_calls():
+    """Flags go through int(), numbers through int() and float(), and flags other than 0 and 1 are refused."""
+    from flash_attention3_b200 import capi, ops
+    q = torch.randn((1, 2, 130, 64), dtype=torch.float16, device="cuda")
+    out, lse = ops.fa3_fwd(q, q, q, True, window=(5, 0))
+    for same in (dict(causal=1, window=(5, 0)), dict(causal=np.bool_(True), window=[5.9, "0"]),
+                 dict(causal=True, window=np.array([5, 0]), softcap="0")):
+        assert torch.equal(ops.fa3_fwd(q, q, q, **same)[0], out)
+    for causal in (2, -1):
+        for call in (lambda: ops.fa3_fwd(q, q, q, causal), lambda: ops.fa3_bwd(q, q, q, q, out, lse, causal),
+                     lambda: ops.fa3_bwd(q, q, q, q, out, lse, True, deterministic=causal)):
+            with pytest.raises(ops.Fa3Error) as refused:
+                call()
+            assert refused.value.code == capi.STATUS_INVALID_VALUE
+    for bad in (dict(causal=None), dict(causal="x"), dict(causal=True, window=(1,)), dict(causal=True, window={1, 2})):
+        with pytest.raises((TypeError, ValueError, IndexError)):
+            ops.fa3_fwd(q, q, q, **bad)

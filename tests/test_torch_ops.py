@@ -32,3 +32,14 @@ def test_differentiating_the_ops_is_refused(qkv):
             torch.autograd.grad(t.float().sum(), qkv[:1], retain_graph=True)
     with torch.no_grad():
         assert not torch.ops.fa3b200.attention_fwd(*qkv, True, 0.125)[0].requires_grad
+
+
+def test_attention_takes_the_arguments_that_the_ops_take(qkv):
+    """Numbers and flags as in the schema of the ops: what torch would turn away there is turned away."""
+    for accepted in (dict(causal=1), dict(causal=None), dict(window=[3, 0]), dict(window=torch.tensor([3, 0])),
+                     dict(softcap="0.5"), dict(softmax_scale=1), dict(deterministic=torch.tensor(True))):
+        assert torch_binding.attention(*qkv, **accepted).shape == qkv[0].shape
+    for refused in (dict(causal="x"), dict(causal=[]), dict(window=(1.5, 0)), dict(window=("1", "0")), dict(window=(1,)),
+                    dict(window=None), dict(softmax_scale="0.5"), dict(softcap=None), dict(layout=3), dict(deterministic="x")):
+        with pytest.raises((TypeError, ValueError, IndexError, RuntimeError)):
+            torch_binding.attention(*qkv, **refused)

@@ -27,6 +27,7 @@
 #include <optional>
 #include <string>
 #include <tuple>
+#include <vector>
 
 #include "shaobo_fa3_api.h"
 #include "shaobo_fa3_b200_ext.h"
@@ -548,13 +549,17 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, 
 }  // namespace
 
 TORCH_LIBRARY(fa3b200, m) {
+    // (with a fake implementation and dense results the ops are fit for torch.compile, also where it takes no others)
+    const std::vector<at::Tag> tags = {at::Tag::pt2_compliant_tag};
     m.def(
         "attention_bwd(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor out, Tensor softmax_lse, bool causal, "
         "float softmax_scale, bool deterministic, SymInt window_left=-1, SymInt window_right=-1, float softcap=0.0, "
-        "str layout=\"bhsd\") -> (Tensor, Tensor, Tensor)");
+        "str layout=\"bhsd\") -> (Tensor, Tensor, Tensor)",
+        tags);
     m.def(
         "attention_fwd(Tensor q, Tensor k, Tensor v, bool causal, float softmax_scale, SymInt window_left=-1, "
-        "SymInt window_right=-1, float softcap=0.0, str layout=\"bhsd\") -> (Tensor, Tensor)");
+        "SymInt window_right=-1, float softcap=0.0, str layout=\"bhsd\") -> (Tensor, Tensor)",
+        tags);
 }
 TORCH_LIBRARY_IMPL(fa3b200, CUDA, m) {
     m.impl("attention_bwd", attention_bwd);

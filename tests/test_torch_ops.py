@@ -43,3 +43,8 @@ def test_attention_takes_the_arguments_that_the_ops_take(qkv):
                     dict(window=None), dict(softmax_scale="0.5"), dict(softcap=None), dict(layout=3), dict(deterministic="x")):
         with pytest.raises((TypeError, ValueError, IndexError, RuntimeError)):
             torch_binding.attention(*qkv, **refused)
+
+
+def test_ops_are_marked_fit_for_compilation():
+    for op in (torch_binding.attention_fwd, torch_binding.attention_bwd):
+        assert torch.Tag.pt2_compliant_tag in op.tags

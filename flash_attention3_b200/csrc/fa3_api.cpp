@@ -205,7 +205,9 @@ static SplitPlan search_split_plan(const ShaoboFa3Params* p, int tiles, const Ba
         }
     }
     if (plan.chunk_steps >= longest) return SplitPlan{};  // a chunk as long as the heaviest tile is no split at all
-    if (tiles * heads >= kSplitSmCount) {
+    if (tiles * heads < kSplitSmCount) {
+        if (p->dtype == SHAOBO_FA3_DTYPE_FP16) plan.slab_elem_bytes = 2;
+    } else {
         // Every SM has a tile anyway: splitting pays only where the last wave is nearly empty (160 equal tiles of 40
         // steps: 174 half steps unsplit, 123 in chunks of 17), and the partial sums are many.  They are counted at what
         // writing and reading them costs the whole GPU: about 4 MB per half step (1 us).
@@ -223,7 +225,7 @@ static SplitPlan search_split_plan(const ShaoboFa3Params* p, int tiles, const Ba
                 unsplit = std::max(unsplit, end);
             }
         }
-        const long long slab_bytes = 2LL * kSequenceAlignment * p->head_dim_qk * (p->dtype == SHAOBO_FA3_DTYPE_FP16 ? 2 : 4);
+        const long long slab_bytes = 2LL * kSequenceAlignment * p->head_dim_qk * plan.slab_elem_bytes;
         const long long sums = 2 * slab_bytes * plan.chunks_per_head * heads / (4 << 20);
         if ((best_cost + sums) * 10 > unsplit * 9) return SplitPlan{};
     }
@@ -233,8 +235,8 @@ static SplitPlan search_split_plan(const ShaoboFa3Params* p, int tiles, const Ba
 size_t dkv_accum_bytes(const ShaoboFa3Params* p) {
     const SplitPlan plan = split_plan(p);
     if (plan.chunk_steps == 0) return 0;
-    // one dK slab and one dV slab of [128 rows][D] per CTA: fp16 for fp16 inputs, fp32 for bf16 inputs
-    const size_t elem = p->dtype == SHAOBO_FA3_DTYPE_FP16 ? 2 : sizeof(float);
+    // one dK slab and one dV slab of [128 rows][D] per CTA
+    const size_t elem = size_t(plan.slab_elem_bytes);
     size_t n = size_t(p->batch), out = 0;
     if (!mul_ok(n, size_t(p->num_heads_kv), &n) || !mul_ok(n, size_t(plan.chunks_per_head), &n) ||
         !mul_ok(n, size_t(kSequenceAlignment), &n) || !mul_ok(n, size_t(p->head_dim_qk), &n) ||

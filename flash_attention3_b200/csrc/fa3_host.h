@@ -67,7 +67,7 @@ size_t dq_accum_bytes(const ShaoboFa3Params* p);
 // than a B200 has SMs would leave most of the chip idle (and up to 511 units the last wave may be
 // nearly empty: those are split where the model below gains more than the partial sums cost), so the
 // query steps of every key tile are cut into chunks of `chunk_steps` steps, one CTA per chunk; every CTA writes its dK/dV partial sums
-// to its own fp32 slab and the convert kernel adds the slabs of a tile in chunk order.  The chunk
+// to its own slabs and the convert kernel adds the slabs of a tile in chunk order.  The chunk
 // size is the one with the smallest modelled makespan when the CTAs, longest first, are handed to
 // 148 SMs as they free up (a CTA costs a fixed part worth 3.5 steps plus its steps); that may be
 // more CTAs than SMs: the overflow are the shortest ones and run on the SMs that free up first.
@@ -77,16 +77,18 @@ constexpr int kSplitSmCount = 148;
 struct SplitPlan {
     int chunk_steps = 0;      // 0 = no splitting
     int chunks_per_head = 0;  // CTAs per (batch, KV head)
+    int slab_elem_bytes = 4;  // of the partial sums: fp32, or 2 (fp16 inputs on problems with too few units: there the
+                              // time to write them counts)
 };
 SplitPlan split_plan(const ShaoboFa3Params* p);
 
 // Bytes of the per-CTA partial-sum slabs of split tiles (one dK and one dV slab of [128][D] per CTA,
-// fp16 for fp16 inputs and fp32 for bf16 inputs); 0 when tiles are not split.
+// elements of slab_elem_bytes); 0 when tiles are not split.
 size_t dkv_accum_bytes(const ShaoboFa3Params* p);
 
 // Carving of the caller's workspace by shaobo_fa3_bwd_v2:
 //   [0, dq_accum)                fp32 dQ accumulator
-//   [dq_accum, +dkv_accum)       fp32 dK / dV partial-sum slabs (only when tiles are split)
+//   [dq_accum, +dkv_accum)       dK / dV partial-sum slabs (only when tiles are split)
 //   [delta_offset, +rows*4)      delta, used when softmax_d is NULL
 //   [sidecar_offset, +rows*12)   packed sidecar
 // Each region starts on a 256-byte boundary.

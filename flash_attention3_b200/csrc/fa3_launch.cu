@@ -283,7 +283,7 @@ void launch_convert(const ShaoboFa3Params* p, const float* accum, void* dq,
         seg.count = 3;
         lanes = 1;
         seg.slabs = dkv_slabs;
-        seg.slabs_f16 = p->dtype == SHAOBO_FA3_DTYPE_FP16 ? 1 : 0;
+        seg.slabs_f16 = split.slab_elem_bytes == 2 ? 1 : 0;
         seg.rows_k = shape.rows_k;
         seg.chunks_per_head = split.chunks_per_head;
         // the chunk list of a head, as the GEMM kernel numbers its CTAs: key tile 0 first
@@ -384,7 +384,7 @@ int launch_fused_d(const ShaoboFa3Params* p, const CUtensorMap& mq, const CUtens
 // dQ into dq_accum (already zero).  !with_dq: four-GEMM dK/dV kernel with fp32
 // outputs (split path).
 // dkv_slabs non-null (fused path only): key tiles are split as split_plan(p) says and every CTA
-// writes its partial dK/dV to its own pair of fp32 slabs instead of dk / dv.
+// writes its partial dK/dV to its own pair of slabs instead of dk / dv.
 // Everything the launch of the five-GEMM / dK-dV kernel needs, built on the host ahead of time: the
 // v2 entry prepares it before it launches the delta kernel, so that the GPU does not sit idle
 // between the two launches while the host encodes the tensor maps.
@@ -447,6 +447,7 @@ FusedLaunch prepare_fused(const ShaoboFa3Params* p, const void* dout, const void
     args.dk = dk;
     args.dv = dv;
     args.dkv_slabs = dkv_slabs;
+    args.slabs_f16 = split.slab_elem_bytes == 2 ? 1 : 0;
     // fp32 dK/dV of the split path are always [B,Hkv,Sk,D]; 16-bit outputs follow the layout of K/V
     args.kv_strides = strides_of(bshd && !dkv_f32, p->num_heads_kv, shape.rows_k, d);
     args.batch = p->batch;

@@ -103,8 +103,9 @@ struct FusedArgs {
     void* dk;              // [B,Hkv,Sk,D] or [B,Sk,Hkv,D], see kv_strides
     void* dv;
     void* dkv_slabs;       // split tiles: a CTA writes its partial dK (scaled) to slab 2x and dV to slab 2x+1,
-                           // each [128 rows][D], fp16 for fp16 inputs and fp32 for bf16 inputs; the convert
+                           // each [128 rows][D], fp32 or (slabs_f16, fp16 inputs only) fp16; the convert
                            // kernel adds the slabs of a tile
+    int slabs_f16;
     TensorStrides kv_strides;  // element strides of dk / dv
     int batch;
     int heads_q;
@@ -132,7 +133,7 @@ struct FusedArgs {
     int order_width;
     int head_group;        // heads per scheduling group: block = (group * n_tiles + tile slot) * head_group + head
     int chunk_steps;       // > 0: the steps of a key tile are cut into chunks of this many steps, one CTA
-                           // per chunk, and the partial dK/dV of every chunk go to its own fp32 slab
+                           // per chunk, and the partial dK/dV of every chunk go to its own slabs
     int chunks_per_head;   // number of chunks of one (batch, KV head) when chunk_steps > 0
     // chunk_steps > 0: which chunk CTA x runs, longest chunks first.  Entry = key tile | chunk index
     // inside the tile << 8 | slab << 16, where slab = (batch, KV head) * chunks_per_head + the chunk's
@@ -862,12 +863,13 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     }
                 };
                 if (kWithDq && a.chunk_steps > 0) {
-                    // a share of a split tile: the partial sums go to this CTA's slabs (slab 2x: dK, 2x+1: dV), fp16 for
-                    // fp16 inputs (11 significant bits, three more than a bf16 result would have; the bytes written, not
-                    // the arithmetic, bound this epilogue), fp32 for bf16 inputs
-                    using Slab = typename std::conditional<kBf16, float, __half>::type;
-                    Slab* slab = static_cast<Slab*>(a.dkv_slabs) + int64_t(w.slab * 2 + half) * (C::kTile * D) + w4 * 32 * D;
-                    store_rows(Slab{}, slab, D, 32);
+                    // a share of a split tile: the partial sums go to this CTA's slabs (slab 2x: dK, 2x+1: dV).  fp32, but
+                    // fp16 for fp16 inputs where the tiles are fewer than the SMs: the bytes written, not the arithmetic,
+                    // bound this epilogue.  (With as many tiles as SMs, fp16 slabs had taken dK and dV, whose sums stay in
+                    // tensor memory when their tile is not split, 1.16 and 1.23 times as far from the exact values.)
+                    const int64_t first = int64_t(w.slab * 2 + half) * (C::kTile * D) + w4 * 32 * D;
+                    if (!kBf16 && a.slabs_f16) store_rows(__half{}, static_cast<__half*>(a.dkv_slabs) + first, D, 32);
+                    else store_rows(float{}, static_cast<float*>(a.dkv_slabs) + first, D, 32);
                 } else {
                     // (rows between the used length and the end of the slot hold exact zeros)
                     TOut* dst = reinterpret_cast<TOut*>(half == 0 ? a.dk : a.dv) + w.b_coord * a.kv_strides.batch +

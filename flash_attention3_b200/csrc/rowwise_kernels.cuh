@@ -165,9 +165,8 @@ delta_sidecar_kernel(const T* __restrict__ dout, const T* __restrict__ out,
 
 // Up to three (fp32 -> storage dtype) conversions in one launch: dQ (scaled) from its accumulator
 // always; dK and dV as well when key tiles were split.  A split tile's dK / dV is the sum of the
-// per-CTA slabs its chunks wrote ([128 rows][D] fp32 each, dK slab then dV slab per CTA), added here
-// in a fixed order, so these two outputs do not depend on the order in which the CTAs ran.  The slabs
-// hold fp16 when the inputs are fp16 and fp32 when they are bf16.
+// per-CTA slabs its chunks wrote ([128 rows][D] each, dK slab then dV slab per CTA), added here
+// in a fixed order, so these two outputs do not depend on the order in which the CTAs ran.
 constexpr int kMaxSplitTiles = 148;  // heads with more key tiles are not split
 struct ConvertSegments {
     const float* src[3];   // [0]: fp32 dQ accumulator [batch, head, row, D] contiguous; [1],[2] unused
@@ -177,7 +176,7 @@ struct ConvertSegments {
     RowLayout layout[3];   // where the rows of dst live
     int count;
     const void* slabs;     // count == 3: slab base; chunk x of the GEMM kernel owns slabs 2x (dK) and 2x+1 (dV)
-    int slabs_f16;         // the slabs hold fp16 (fp16 inputs) instead of fp32
+    int slabs_f16;         // the slabs hold fp16 instead of fp32
     int rows_k;            // key rows per (batch, KV head)
     int chunks_per_head;   // CTAs per (batch, KV head)
     unsigned short chunk_begin[kMaxSplitTiles + 1];  // first chunk of key tile kt inside its head

@@ -4,7 +4,9 @@ bottom-right).  Same gates and the same oracle as the square cases; every call g
 shaobo_fa3_bwd_v2 with NaN-poisoned outputs and workspace."""
 import numpy as np
 import pytest
+import torch
 
+from flash_attention3_b200 import ops
 from oracle import golden
 
 from tests.helpers import Problem, assert_parity, run_v2
@@ -125,7 +127,8 @@ def test_softcap(b, hq, hkv, sq, sk, d, dtype, causal, window, softcap, determin
 # (b, hq, hkv, s, d, dtype, causal): at least 148 key tiles, split all the same because the last wave is nearly empty
 MANY_TILES_SPLIT = [
     (1, 100, 25, 700, 64, "bf16", False),    # 150 tiles as 300 CTAs, fp32 partial sums
-    (1, 100, 25, 700, 128, "fp16", True),    # 150 tiles as 200 CTAs of unequal length, fp16 partial sums
+    (1, 100, 25, 700, 128, "fp16", True),    # 150 tiles, not split: the partial sums would cost what it gains
+    (1, 200, 25, 700, 128, "fp16", True),    # 150 tiles as 200 CTAs of unequal length, fp32 partial sums of fp16 inputs
 ]
 
 
@@ -148,3 +151,22 @@ MANY_CHUNKS = [
 def test_many_partial_sums_per_tile(b, hq, hkv, sq, sk, d, dtype, causal, layout):
     prob = Problem(b, hq, hkv, sq, d, dtype, causal, seed=99 + sq, sk=sk, layout=layout)
     assert_parity(run_v2(prob), prob, label=f"{(b, hq, hkv, sq, sk, d, dtype, causal, layout)}")
+
+
+def test_partial_sums_beyond_the_range_of_fp16():
+    """160 key tiles in chunks whose partial dV are beyond 65504 and cancel: the first two of the four query heads of a
+    group carry +dO, the other two, with the same queries, -dO."""
+    hkv, s, sk, d, big = 160, 2048, 128, 64, 4000.0
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    q = torch.randn((1, hkv, 2, s, d), device="cuda", generator=gen)
+    q = torch.cat([q, q], dim=2).reshape(1, 4 * hkv, s, d).half()
+    k, v = (torch.randn((1, hkv, sk, d), device="cuda", generator=gen).half() for _ in range(2))
+    dout = torch.full((1, hkv, 4, s, d), big, device="cuda")
+    dout[:, :, 2:] *= -1
+    dout = dout.reshape(1, 4 * hkv, s, d).half()
+    out, lse = ops.fa3_fwd(q, k, v, False)
+    dq, dk, dv = ops.fa3_bwd(dout, q, k, v, out, lse, False, sync=True)
+    assert all(torch.isfinite(t).all() for t in (dq, dk, dv))
+    # a sum of 4 s probabilities that average 1 / sk reaches 2 s / sk * big = 128000 before it returns to zero; each of
+    # the 4 s / 16 products of 16 terms rounds it to 24 bits, and no more than their sum can be left
+    assert dv.abs().max().item() <= 2 * s / sk * big * 2.0 ** -24 * (4 * s / 16)

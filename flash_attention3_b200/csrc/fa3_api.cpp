@@ -208,6 +208,7 @@ static SplitPlan search_split_plan(const ShaoboFa3Params* p, int tiles, const Ba
     if (tiles * heads < kSplitSmCount) {
         if (p->dtype == SHAOBO_FA3_DTYPE_FP16) plan.slab_elem_bytes = 2;
     } else {
+        plan.optional = true;
         // Every SM has a tile anyway: splitting pays only where the last wave is nearly empty (160 equal tiles of 40
         // steps: 174 half steps unsplit, 123 in chunks of 17), and the partial sums are many.  They are counted at what
         // writing and reading them costs the whole GPU: about 4 MB per half step (1 us).
@@ -246,12 +247,16 @@ size_t dkv_accum_bytes(const ShaoboFa3Params* p) {
     return out;
 }
 
-V2Workspace v2_workspace(const ShaoboFa3Params* p) {
+size_t dkv_accum_bytes_within(const ShaoboFa3Params* p, size_t room) {
+    const size_t bytes = dkv_accum_bytes(p);
+    return bytes > room && split_plan(p).optional ? 0 : bytes;
+}
+
+static V2Workspace lay_out(const ShaoboFa3Params* p, size_t dkv_bytes) {
     V2Workspace w;
-    if (validate_v2(p) != SHAOBO_FA3_STATUS_SUCCESS) return w;
     w.dq_accum_bytes = dq_accum_bytes(p);
     if (w.dq_accum_bytes == 0) return w;
-    w.dkv_accum_bytes = dkv_accum_bytes(p);
+    w.dkv_accum_bytes = dkv_bytes;
     if (!add_ok(w.dq_accum_bytes, w.dkv_accum_bytes, &w.delta_offset)) return V2Workspace{};
     bool ok = false;
     const size_t rows = row_count(p, &ok);
@@ -265,6 +270,14 @@ V2Workspace v2_workspace(const ShaoboFa3Params* p) {
     }
     w.valid = true;
     return w;
+}
+
+V2Workspace v2_workspace(const ShaoboFa3Params* p, size_t available) {
+    if (validate_v2(p) != SHAOBO_FA3_STATUS_SUCCESS) return V2Workspace{};
+    const size_t dkv_bytes = dkv_accum_bytes(p);
+    const V2Workspace w = lay_out(p, dkv_bytes);
+    if (dkv_bytes == 0 || (w.valid && w.total_bytes <= available) || !split_plan(p).optional) return w;
+    return lay_out(p, 0);
 }
 
 size_t naive_reference_bytes(const ShaoboFa3Params* p) {

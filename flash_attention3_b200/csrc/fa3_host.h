@@ -72,11 +72,13 @@ size_t dq_accum_bytes(const ShaoboFa3Params* p);
 // 148 SMs as they free up (a CTA costs a fixed part worth 3.5 steps plus its steps); that may be
 // more CTAs than SMs: the overflow are the shortest ones and run on the SMs that free up first.
 // The decision depends on the parameters only, so the workspace formula and the launch always
-// agree.  The deterministic path never splits.
+// agree; an optional split is left out when the caller's workspace has no room for its partial sums.
+// The deterministic path never splits.
 constexpr int kSplitSmCount = 148;
 struct SplitPlan {
     int chunk_steps = 0;      // 0 = no splitting
     int chunks_per_head = 0;  // CTAs per (batch, KV head)
+    bool optional = false;    // every SM has a tile anyway: with too small a workspace the tiles stay whole
     int slab_elem_bytes = 4;  // of the partial sums: fp32, or 2 (fp16 inputs on problems with too few units: there the
                               // time to write them counts)
 };
@@ -85,6 +87,8 @@ SplitPlan split_plan(const ShaoboFa3Params* p);
 // Bytes of the per-CTA partial-sum slabs of split tiles (one dK and one dV slab of [128][D] per CTA,
 // elements of slab_elem_bytes); 0 when tiles are not split.
 size_t dkv_accum_bytes(const ShaoboFa3Params* p);
+// The same for a workspace that has `room` bytes for them: 0 where an optional split does not fit.
+size_t dkv_accum_bytes_within(const ShaoboFa3Params* p, size_t room);
 
 // Carving of the caller's workspace by shaobo_fa3_bwd_v2:
 //   [0, dq_accum)                fp32 dQ accumulator
@@ -100,7 +104,9 @@ struct V2Workspace {
     size_t total_bytes = 0;
     bool valid = false;
 };
-V2Workspace v2_workspace(const ShaoboFa3Params* p);
+// What the parameters ask for, or, where that is more than `available` and the split is optional, the
+// layout without partial sums.
+V2Workspace v2_workspace(const ShaoboFa3Params* p, size_t available = SIZE_MAX);
 
 // Workspace of the naive fp32 device reference used by dkv_path/dq_path == 1:
 // prob[rows,Sk] + dp[rows,Sk] + row_max + row_sum + delta

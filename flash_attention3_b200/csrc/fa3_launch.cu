@@ -875,7 +875,7 @@ extern "C" int shaobo_fa3_bwd_fused5(const void* dout, const void* q, const void
     }
     if (!stage_params_ok(params)) return SHAOBO_FA3_STATUS_UNSUPPORTED;
     const size_t dq_bytes = dq_accum_bytes(params);
-    const size_t dkv_bytes = dkv_accum_bytes(params);
+    const size_t dkv_bytes = dkv_accum_bytes_within(params, params->workspace_bytes < dq_bytes ? 0 : params->workspace_bytes - dq_bytes);
     const size_t need = dq_bytes + dkv_bytes;
     if (dq_bytes == 0 || params->workspace == nullptr || params->workspace_bytes < need) {
         return SHAOBO_FA3_STATUS_INVALID_VALUE;
@@ -960,7 +960,7 @@ extern "C" int shaobo_fa3_bwd_v2(const void* dout, const void* q, const void* k,
         softmax_lse == nullptr || dq == nullptr || dk == nullptr || dv == nullptr) {
         return SHAOBO_FA3_STATUS_INVALID_VALUE;
     }
-    const V2Workspace ws = v2_workspace(params);
+    const V2Workspace ws = v2_workspace(params, params->workspace_bytes);
     if (!ws.valid || params->workspace == nullptr || params->workspace_bytes < ws.total_bytes) {
         return SHAOBO_FA3_STATUS_INVALID_VALUE;
     }
@@ -1093,7 +1093,7 @@ extern "C" int shaobo_fa3_b200_bwd_v2_noalloc(const void* dout, const void* q, c
         softmax_lse == nullptr || dq == nullptr || dk == nullptr || dv == nullptr) {
         return SHAOBO_FA3_STATUS_INVALID_VALUE;
     }
-    const V2Workspace ws = v2_workspace(params);
+    const V2Workspace ws = v2_workspace(params, size_t(SHAOBO_FA3_B200_STATIC_SCRATCH_BYTES));
     if (!ws.valid) return SHAOBO_FA3_STATUS_INVALID_VALUE;
     if (ws.total_bytes > size_t(SHAOBO_FA3_B200_STATIC_SCRATCH_BYTES)) {
         // the problem needs more scratch than the built-in array holds

@@ -51,14 +51,18 @@ int shaobo_fa3_b200_last_stage_ms(float* ms3);
  * ignored: the scratch is a fixed array of
  * SHAOBO_FA3_B200_STATIC_SCRATCH_BYTES inside the library.  It holds what the
  * workspace of shaobo_fa3_bwd_v2 holds: the fp32 dQ accumulator
- * (4*B*Hq*Sq*D bytes), on small problems whose key tiles are split over
- * several thread blocks the partial dK/dV sums of those blocks (512*D bytes
- * per block for fp16 inputs, 1024*D for bf16 inputs, up to 148 blocks), delta
- * and the packed sidecar (16 bytes per query row).  The call performs no cudaMalloc, no cudaFree and no other
+ * (4*B*Hq*Sq*D bytes), on problems whose key tiles are split over several
+ * thread blocks the partial dK/dV sums of those blocks (512*D bytes per block
+ * for fp16 inputs, 1024*D for bf16 inputs and wherever there are 148 key tiles
+ * or more; up to 511 blocks), delta and the packed sidecar (16 bytes per query
+ * row).  The call performs no cudaMalloc, no cudaFree and no other
  * allocating runtime or library call.
  *
  * Limit: the problem must satisfy
  *     shaobo_fa3_bwd_v2_workspace_bytes(params) <= SHAOBO_FA3_B200_STATIC_SCRATCH_BYTES
+ * where partial sums do not count if there are 148 key tiles (B*Hkv*ceil(Sk/128))
+ * or more: such tiles stay whole when the sums do not fit, as they do in
+ * shaobo_fa3_bwd_v2 when the workspace has no room for them
  * (ask that function; e.g. B=1,H=4,S=2048,D=128 fp16 needs 13 MiB and
  * B=1,H=15,S=4096,D=128 31 MiB, B=2,H=16,S=2048,D=128 does not fit).  A larger
  * problem returns SHAOBO_FA3_STATUS_UNSUPPORTED and launches nothing.  Status

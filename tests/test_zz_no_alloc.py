@@ -112,3 +112,31 @@ def test_problem_larger_than_the_built_in_scratch_is_refused():
     p.struct_size = 0
     assert lib.shaobo_fa3_b200_bwd_v2_noalloc(vp(q), vp(q), vp(q), vp(q), vp(q), vp(q), vp(q), vp(q), vp(q), None,
                                                ctypes.byref(p)) == capi.STATUS_INVALID_VALUE
+
+
+def test_key_tiles_stay_whole_where_their_partial_sums_do_not_fit():
+    """150 key tiles, split when the workspace may be large (36 MiB with the partial sums): the built-in array, and a
+    workspace of the size without them, run them whole; one byte less is refused."""
+    lib = capi.load()
+    prob = helpers.Problem(1, 100, 25, 700, 64, "bf16", False, seed=905)
+    x = prob.device_inputs()
+    p = ops.make_params(x["q"], x["k"], prob.causal, prob.scale, sync_after_launch=1)
+    rows = 100 * 700
+    whole = rows * 64 * 4 + (rows * 4 + 255) // 256 * 256 + rows * 12
+    assert whole < capi.STATIC_SCRATCH_BYTES < lib.shaobo_fa3_bwd_v2_workspace_bytes(ctypes.byref(p))
+    helpers.assert_parity(_call_noalloc(prob, x), prob, "built-in array")
+    ws = torch.full((whole + 256,), 0xFF, dtype=torch.uint8, device="cuda")
+    out = [helpers.poison(x[n].shape, torch.bfloat16) for n in ("q", "k", "k")]
+    delta = helpers.poison(x["lse"].shape, torch.float32)
+    p.workspace = ws.data_ptr()
+    call = lambda: lib.shaobo_fa3_bwd_v2(*(vp(x[n]) for n in ("dout", "q", "k", "v", "out", "lse")), *map(vp, out), vp(delta),
+                                         ctypes.byref(p))
+    p.workspace_bytes = whole - 1
+    assert call() == capi.STATUS_INVALID_VALUE
+    p.workspace_bytes = whole
+    code = call()
+    torch.cuda.synchronize()
+    result = dict(zip(("dq", "dk", "dv"), map(helpers.host, out)), delta=helpers.host(delta), code=code,
+                  device_error=lib.shaobo_fa3_b200_device_error(1))
+    helpers.assert_parity(result, prob, "workspace without room for partial sums")
+    assert (ws[whole:] == 0xFF).all()

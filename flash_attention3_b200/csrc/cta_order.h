@@ -168,7 +168,7 @@ struct FwdPlan {
     bool fold = false;
 };
 
-using FwdGangs = std::array<int, 4>;  // clusters of 1, 2, 4, 8 CTAs that run at the same time
+using FwdGangs = std::array<int, 4>;  // clusters of 1, 2, 4, 8 CTAs that run at the same time; 0: the device runs none
 
 // (packed sequences have different numbers of tiles: not folded)
 inline FwdPlan plan_fwd(const Band& band, long long bh_count, const FwdGangs& gangs, bool packed) {
@@ -181,6 +181,7 @@ inline FwdPlan plan_fwd(const Band& band, long long bh_count, const FwdGangs& ga
         if (option.fold && (packed || band.left < kUnbounded || band.right >= kUnbounded)) continue;  // (every tile starts at the first key)
         std::priority_queue<long long, std::vector<long long>, std::greater<long long>> free_at;
         const int gang = option.splits == 8 ? 3 : option.splits / 2;
+        if (option.splits > 1 && gangs[size_t(gang)] <= 0) continue;
         for (int i = 0; i < std::max(1, gangs[size_t(gang)]); ++i) free_at.push(0);
         long long makespan = 0;
         for (int slot = 0; slot < pairs; ++slot) {

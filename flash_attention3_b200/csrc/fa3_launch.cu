@@ -674,7 +674,7 @@ int launch_fwd_d(const ShaoboFa3Params* p, const FwdLaunch& L) {
 }
 
 // How many clusters of 1, 2, 4 and 8 CTAs of the forward kernel the current device runs at the same time (every variant
-// takes a whole SM).
+// takes a whole SM); 0 where it runs none (a partition of the device) or does not say.
 FwdGangs fwd_gangs() {
     FwdGangs gangs;
     const int sms = sm_count();
@@ -693,9 +693,10 @@ FwdGangs fwd_gangs() {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        gangs[size_t(i)] = i > 0 && ok && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0
-                               ? std::min(n, sms >> i) : sms >> i;
+        const bool known = i > 0 && ok && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess;
+        gangs[size_t(i)] = i == 0 ? sms : known ? std::min(n, sms >> i) : 0;
     }
+    (void)cudaGetLastError();  // (a query that failed is no failure of the call)
     return gangs;
 }
 

@@ -185,8 +185,8 @@ inline FwdPlan plan_fwd(const Band& band, long long bh_count, const FwdGangs& ga
         for (int i = 0; i < std::max(1, gangs[size_t(gang)]); ++i) free_at.push(0);
         long long makespan = 0;
         for (int slot = 0; slot < pairs; ++slot) {
-            const int heavy = q_tiles - 1 - slot;  // (of an odd number of tiles the middle one is alone)
-            const int a = option.fold ? heavy : 2 * (pairs - 1 - slot), b = option.fold ? (slot < heavy ? slot : q_tiles) : a + 1;
+            const TilePair tiles_here = tile_pair_of_slot(slot, q_tiles, true, option.fold);
+            const int a = tiles_here.a, b = tiles_here.b;
             const int most_a = k_tiles_of_q_tile(a, band), most_b = b < q_tiles ? k_tiles_of_q_tile(b, band) : 0;
             int first = kUnbounded, last = -1;
             if (most_a > 0) first = first_k_tile(a, band), last = last_k_tile(a, band);

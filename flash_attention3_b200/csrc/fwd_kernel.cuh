@@ -129,7 +129,7 @@ enum FwdBar : int {
 
 // Which query tiles and keys a CTA works on.
 struct FwdWork {
-    int pair, rank, hq, kvh, b, b_coord, q_base, k_base;
+    int rank, hq, kvh, b, b_coord, q_base, k_base;
     int tile[2];         // query tiles A and B
     int slot_q;          // rows of out this batch entry owns
     int t_begin, n_iter; // the CTA walks key tiles t_begin .. t_begin + n_iter - 1;
@@ -144,19 +144,13 @@ struct FwdWork {
 template <bool kMasked>
 __device__ __forceinline__ FwdWork fwd_work(const FwdArgs& a) {
     FwdWork w;
-    const int n_pairs = (tiles_of(a.band.seqlen_q) + 1) / 2;  // of the longest sequence
     const int unit = int(blockIdx.x) >> a.split_shift;
     w.rank = int(blockIdx.x) & (a.splits - 1);        // == rank in the cluster
     const int slot = fast_div(unit, a.bh);
-    // heaviest query tiles (most visible keys) are launched first
-    w.pair = kMasked ? n_pairs - 1 - slot : slot;
-    w.tile[0] = 2 * w.pair;
-    w.tile[1] = 2 * w.pair + 1;
-    if (kMasked && a.fold) {  // (of an odd number of tiles the middle one is alone)
-        const int n_tiles = tiles_of(a.band.seqlen_q);
-        w.tile[0] = n_tiles - 1 - slot;
-        w.tile[1] = slot < w.tile[0] ? slot : n_tiles;
-    }
+    // heaviest query tiles (most visible keys) are launched first (packed: of the longest sequence)
+    const TilePair tiles = tile_pair_of_slot(slot, tiles_of(a.band.seqlen_q), kMasked, kMasked && a.fold);
+    w.tile[0] = tiles.a;
+    w.tile[1] = tiles.b;
     const int bhi = unit - slot * a.bh.divisor;
     w.b = fast_div(bhi, a.heads);
     w.hq = bhi - w.b * a.heads_q;
@@ -239,7 +233,7 @@ __device__ __forceinline__ void fwd_merge(const FwdArgs& a, const FwdWork& w, ui
 #pragma unroll 1
     for (int rr = tid / kLanes; rr < kRows; rr += 256 / kLanes) {
         const int row = w.rank * kRows + rr;  // row of the pair
-        const int qi = 2 * w.pair * kTileRows + row;
+        const int qi = w.tile[0] * kTileRows + row;  // (split pairs are neighbours)
         if (qi >= w.slot_q) break;
         float2 ml[kSplits];
         float4 part[kSplits][2];
@@ -301,9 +295,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     if (a.cu_seqlens_q != nullptr) {
         ptx::grid_dependency_wait();
         const int slot = fast_div(int(blockIdx.x) >> a.split_shift, a.bh);
-        const int first_pair = kMasked ? (tiles_of(a.band.seqlen_q) + 1) / 2 - 1 - slot : slot;
+        const int first_tile = tile_pair_of_slot(slot, tiles_of(a.band.seqlen_q), kMasked, false).a;
         const int entry = fast_div((int(blockIdx.x) >> a.split_shift) - slot * a.bh.divisor, a.heads);
-        if (first_pair * 2 * C::kTile >= a.cu_seqlens_q[entry + 1] - a.cu_seqlens_q[entry]) return;
+        if (first_tile * C::kTile >= a.cu_seqlens_q[entry + 1] - a.cu_seqlens_q[entry]) return;
     }
 
     // Set-up first: launched programmatically, it overlaps the end of the kernel in front, which

@@ -126,6 +126,21 @@ FA3B200_HD inline void key_range_of_query(int query, int key0, const Band& b, in
     *hi = h;
 }
 
+// The two query tiles of a forward CTA: the slot-th pair of neighbours, first (or, heaviest first, last) pair in
+// front, or, folded, the slot-th tile from the end with the slot-th from the start.  b == n_tiles: a is alone.
+struct TilePair {
+    int a;
+    int b;
+};
+FA3B200_HD inline TilePair tile_pair_of_slot(int slot, int n_tiles, bool heavy_first, bool fold) {
+    if (fold) {
+        const int heavy = n_tiles - 1 - slot;
+        return TilePair{heavy, slot < heavy ? slot : n_tiles};
+    }
+    const int pair = heavy_first ? (n_tiles + 1) / 2 - 1 - slot : slot;
+    return TilePair{2 * pair, 2 * pair + 1};
+}
+
 // Division by a divisor that the host knows: q = (hi(n * mul) + n) >> shift for 0 <= n < 2^31.  (A block works out
 // which tile is its own before anything else can start; a 32-bit division costs about 100 clk of that chain.)
 struct FastDiv {

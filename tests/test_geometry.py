@@ -27,6 +27,11 @@ int g_needs_mask(int kt, int qt, int sq, int sk, int c, int wl, int wr) {
 void g_query_range(int key, int q0, int sq, int sk, int c, int wl, int wr, int* lo, int* hi) {
     query_range_of_key(key, q0, make_band(sq, sk, c, wl, wr), lo, hi);
 }
+int g_fast_div(int n, long long d) { return fast_div(n, fast_div_of(d)); }
+void g_pair(int slot, int n, int heavy_first, int fold, int* a, int* b) {
+    const TilePair t = tile_pair_of_slot(slot, n, heavy_first != 0, fold != 0);
+    *a = t.a; *b = t.b;
+}
 void g_key_range(int query, int k0, int sq, int sk, int c, int wl, int wr, int* lo, int* hi) {
     key_range_of_query(query, k0, make_band(sq, sk, c, wl, wr), lo, hi);
 }
@@ -90,3 +95,30 @@ def test_tile_walks_cover_the_band_and_masks_match(lib, sq, sk, causal, window):
                 assert not keep[block.shape[1]:].any()
             covered[qt * 128:(qt + 1) * 128, kt * 128:(kt + 1) * 128] = True
     assert not (visible & ~covered).any()
+
+
+def test_division_by_multiplication(lib):
+    top = 2**31 - 1
+    rng = np.random.default_rng(0)
+    divisors = [1, 2, 3, 5, 7, 64, 148, 641, 46341, 2**16 - 1, 2**16 + 1, 2**30 - 1, 2**30, 2**30 + 1, top - 1, top]
+    for d in divisors + [int(x) for x in np.exp(rng.uniform(0, np.log(top), 200))]:
+        numbers = {0, 1, d - 1, d, d + 1, 2 * d - 1, 2 * d, top // d * d - 1, top // d * d, top - 1, top}
+        numbers.update(int(x) for x in rng.integers(0, top, 20))
+        for n in numbers:
+            if 0 <= n <= top:
+                assert lib.g_fast_div(n, ctypes.c_longlong(d)) == n // d, (n, d)
+    assert lib.g_fast_div(top - 1, ctypes.c_longlong(2**40)) == 0
+
+
+@pytest.mark.parametrize("n_tiles", [1, 2, 3, 4, 7, 8, 63])
+def test_every_query_tile_is_in_one_pair(lib, n_tiles):
+    a, b = ctypes.c_int(), ctypes.c_int()
+    for heavy_first, fold in ((0, 0), (1, 0), (1, 1)):
+        seen = []
+        for slot in range((n_tiles + 1) // 2):
+            lib.g_pair(slot, n_tiles, heavy_first, fold, ctypes.byref(a), ctypes.byref(b))
+            seen += [t for t in (a.value, b.value) if t < n_tiles]
+            assert fold or b.value == a.value + 1
+        assert sorted(seen) == list(range(n_tiles)), (heavy_first, fold)
+        if heavy_first:
+            assert seen[0] >= n_tiles - 2

@@ -41,3 +41,25 @@ def test_clusters_that_the_device_does_not_run_are_not_planned(plan, sq, sk, cau
     assert abs(plan(sq, sk, causal, heads, gangs=(148, 0, 0, 0))) == 1
     for size, gangs in ((2, (148, 74, 0, 0)), (4, (148, 0, 36, 0)), (8, (148, 0, 0, 16))):
         assert plan(sq, sk, causal, heads, gangs=gangs) in (-1, 1, size)
+
+
+def test_gpu_cases_reach_the_form_they_name(plan):
+    """Clusters of 8, 4 and 2, folded pairs and neighbours, on devices with more or fewer clusters per GPC."""
+    from tests.test_gpu_forward_split import CASES
+    expected = [8, 4, 2, 8, 8, 8, 8, -1, -1, -1, -1, 1]
+    for gangs in (B200, (148, 74, 36, 18)):
+        assert [plan(sq, sk, causal, b * hq, window, gangs) for b, hq, _, sq, sk, _, _, causal, _, window in CASES] == expected
+        assert plan(1280, 1280, False, 2, gangs=gangs) == 8  # (used lengths)
+    assert plan(500, 500, True, 3) == -1  # (used lengths, folded)
+
+
+def test_non_finite_problems_cover_the_forms(plan):
+    from tests.test_gpu_nonfinite import PROBLEMS
+    assert [plan(s, s, True, heads) for heads, s in PROBLEMS] == [8, -1, 1]
+
+
+def test_only_causal_masks_fold_and_packed_sequences_do_not(plan):
+    assert plan(449, 449, True, 12) == -1
+    assert plan(449, 449, True, 12, packed=True) > 0 and plan(449, 449, False, 12) > 0
+    assert plan(449, 449, True, 12, window=(200, -1)) > 0
+    assert plan(8192, 8192, True, 64) == 1  # many waves

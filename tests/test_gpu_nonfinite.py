@@ -11,7 +11,7 @@ from tests.helpers import dev, host
 pytestmark = pytest.mark.gpu
 
 # (heads, length): pairs of query tiles whose keys a cluster shares; pairs of the last and the first tile; neighbours
-PROBLEMS = [(1, 640), (60, 300), (200, 1100)]
+PROBLEMS = [(1, 640), (12, 449), (200, 1100)]
 # tensor, row, value: rows of the first and of later tiles, keys with either form of the exponential at D=64
 PLANTS = [("q", 3, np.nan), ("q", 200, np.nan), ("k", 3, np.nan), ("k", 14, np.nan), ("k", 159, np.nan),
           ("k", 14, np.inf), ("k", 64, np.inf)]

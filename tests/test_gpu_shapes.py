@@ -142,8 +142,12 @@ def test_split_with_a_nearly_empty_last_wave(b, hq, hkv, s, d, dtype, causal):
 MANY_CHUNKS = [
     (1, 8, 1, 512, 512, 128, "bf16", False, "bhsd"),    # 32 per tile
     (1, 8, 1, 500, 509, 64, "fp16", False, "bshd"),     # 32 per tile in fp16; ragged
-    (1, 3, 1, 1000, 129, 64, "bf16", True, "bshd"),     # a tile with one row, query rows that are no multiple of a warp
-    (1, 1, 1, 1537, 1537, 128, "bf16", True, "bhsd"),   # 1 to 13 per tile: lanes without any
+    (1, 9, 1, 333, 129, 64, "bf16", False, "bshd"),     # a tile with one row; dQ vectors that are no multiple of a warp
+    (1, 7, 1, 397, 500, 128, "bf16", True, "bhsd"),     # 14 to 28 per tile: lanes without any
+    (1, 33, 1, 301, 300, 64, "fp16", True, "bhsd"),     # all of this in fp16
+    # few enough for one lane
+    (1, 3, 1, 1000, 129, 64, "bf16", True, "bshd"),     # a tile with one row
+    (1, 1, 1, 1537, 1537, 128, "bf16", True, "bhsd"),   # 1 to 13 per tile
 ]
 
 

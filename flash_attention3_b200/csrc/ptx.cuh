@@ -455,9 +455,10 @@ __device__ __forceinline__ float max3_nan(float a, float b, float c) {
 // 2^x of two values on the FMA and integer pipes, for code that the special-function unit bounds (a warp's
 // ex2 keeps it busy for 8 cycles, these 24 instructions for two values keep the FMA pipe busy for 16).
 // x = n + f with n the nearest integer (rounded by adding 1.5 * 2^23, which also leaves n in the low bits),
-// 2^f by a polynomial of degree 5 on [-1/2, 1/2] (Remez exchange on the relative error: 7.5e-8, 2.2e-7 as
-// evaluated in fp32; ex2.approx is good to 2.4e-7), then n added to the exponent field.  x above 127 and
-// NaN are not expected (the forward treats a row with such a score by its sum); below -126 the result stays at 2^-126.
+// 2^f by a polynomial of degree 5 on [-1/2, 1/2] (Remez exchange on the relative error: 7.5e-8, or 2.2e-7 with
+// coefficients and arithmetic in fp32; ex2.approx is good to 2.4e-7), then n added to the exponent field.  x above
+// 127 and NaN are not expected (the forward treats a row with such a score by its sum); below -126 the result stays
+// at 2^-126.
 __device__ __forceinline__ float2 exp2_poly(uint64_t x2) {
     const float kMagic = 12582912.0f;
     float2 x = f2_unpack(x2);

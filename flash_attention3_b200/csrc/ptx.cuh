@@ -60,15 +60,6 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 }
 
 // ----------------------------------------------------------------------- TMA
-// 2-D tiled load global -> shared, completion on an mbarrier (this CTA only).
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* map, uint32_t bar, int x,
-                                            int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
-        : "memory");
-}
 // 4-D tiled load (coordinates innermost first); rows outside the tensor read as zero.
 __device__ __forceinline__ void tma_load_4d(uint32_t dst, const void* map, uint32_t bar, int c0,
                                             int c1, int c2, int c3) {
@@ -107,25 +98,11 @@ __device__ __forceinline__ void tma_reduce_add_3d(const void* map, uint32_t src,
         ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2)
         : "memory");
 }
-// 2-D tiled reduce-add shared -> global (element type comes from the map).
-__device__ __forceinline__ void tma_reduce_add_2d(const void* map, uint32_t src, int x, int y) {
-    asm volatile(
-        "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group"
-        " [%0, {%2, %3}], [%1];"
-        ::"l"(map), "r"(src), "r"(x), "r"(y)
-        : "memory");
-}
 // 4-D tiled store shared -> global; elements outside the tensor are dropped.
 __device__ __forceinline__ void tma_store_4d(const void* map, uint32_t src, int c0, int c1, int c2, int c3) {
     asm volatile(
         "cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
         ::"l"(map), "r"(src), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-__device__ __forceinline__ void tma_store_2d(const void* map, uint32_t src, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];"
-        ::"l"(map), "r"(src), "r"(x), "r"(y)
         : "memory");
 }
 __device__ __forceinline__ void bulk_commit_group() {
@@ -273,14 +250,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
         : "r"(taddr)
         : "memory");
 }
-// 32 lanes x 64 consecutive columns in one instruction (one TMEM round trip).
-__device__ __forceinline__ void tmem_ld64(uint32_t taddr, uint32_t (&r)[64]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31]), "=r"(r[32]), "=r"(r[33]), "=r"(r[34]), "=r"(r[35]), "=r"(r[36]), "=r"(r[37]), "=r"(r[38]), "=r"(r[39]), "=r"(r[40]), "=r"(r[41]), "=r"(r[42]), "=r"(r[43]), "=r"(r[44]), "=r"(r[45]), "=r"(r[46]), "=r"(r[47]), "=r"(r[48]), "=r"(r[49]), "=r"(r[50]), "=r"(r[51]), "=r"(r[52]), "=r"(r[53]), "=r"(r[54]), "=r"(r[55]), "=r"(r[56]), "=r"(r[57]), "=r"(r[58]), "=r"(r[59]), "=r"(r[60]), "=r"(r[61]), "=r"(r[62]), "=r"(r[63])
-        : "r"(taddr)
-        : "memory");
-}
 // 32 lanes x 16 columns load.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
@@ -304,24 +273,12 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
           "r"(r[13]), "r"(r[14]), "r"(r[15])
         : "memory");
 }
-// 32 lanes x 32 columns store (one register per column).
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
-        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
-          "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
-          "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-        : "memory");
-}
 __device__ __forceinline__ void tmem_st_wait() {
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
 // --------------------------------------------------------------- descriptors
-// 64-bit shared-memory matrix descriptor, 128-byte swizzle, version 1.
+// 64-bit shared-memory matrix descriptor, 128-byte swizzle, version 1 (kDescHiSw128 and desc_lo_* above are its halves).
 //   bits  0-13  start address >> 4
 //   bits 16-29  leading-dimension byte offset >> 4
 //   bits 32-45  stride-dimension byte offset >> 4
@@ -335,12 +292,6 @@ __device__ __forceinline__ void tmem_st_wait() {
 //  MN-major operand (the 64 contiguous elements run along M or N): LBO = box
 //    bytes (next 64 M/N elements), SBO = 1024 (next 8 K rows).  K advances by
 //    2048 B per 16 rows.
-__host__ __device__ constexpr uint64_t smem_desc_sw128(uint32_t addr, uint32_t lbo_bytes,
-                                                       uint32_t sbo_bytes) {
-    return uint64_t((addr & 0x3FFFF) >> 4) | (uint64_t((lbo_bytes >> 4) & 0x3FFF) << 16) |
-           (uint64_t((sbo_bytes >> 4) & 0x3FFF) << 32) | (uint64_t(1) << 46) |
-           (uint64_t(2) << 61);
-}
 
 // 32-bit instruction descriptor for kind::f16, fp32 accumulate.
 //   bits 4-5 D format (1 = f32); 7-9 A format; 10-12 B format (0 f16, 1 bf16);

@@ -437,10 +437,16 @@ FusedLaunch prepare_fused(const ShaoboFa3Params* p, const void* dout, const void
     const int group = p->num_heads_q / p->num_heads_kv;
     // bytes of dQ accumulator behind one (batch, KV head): only the fused path adds into it
     // (packed sequences are planned as if all were the longest one: grouping heads for the L2 then costs more balance
-    // than the model sees, so they are issued heaviest tile first over everything while the accumulators fit in the L2)
-    const bool packed_in_l2 = is_varlen(p) && p->total_q * p->num_heads_q * p->head_dim_qk * 4 <= (128LL << 20);
+    // than the model sees, so they are issued heaviest tile first over everything while what the kernel works on, dQ
+    // accumulators, Q, dO, K and V, is little more than the L2.  us per call, heads grouped and not, causal, mean length
+    // about half of the maximum, MiB in front: 51 (9 sequences of up to 2048, 8 heads, D=64) 83 and 76; 144 (9 x 2048, 16
+    // heads on 4, D=128) 230 and 219; 155 (9 x 2048, 32 on 8, D=64) 257 and 246; 202 (2 x 4096, 32 on 8, D=128) 469 and 448;
+    // 207 (9 x 2048, 16 on 16, D=128) 233 and 257; 236 (24 x 1024, 16 on 4) 243 and 259; 259 (2 x 8192, 16 on 4) 1181 and
+    // 1269; 441 (9 x 4096, 16 on 16) 738 and 912; 915 (24 x 2048, 32 on 8) 1208 and 1563.)
+    const bool packed_near_l2 =
+        is_varlen(p) && (p->total_q * p->num_heads_q * 8 + p->total_k * p->num_heads_kv * 4) * p->head_dim_qk <= (176LL << 20);
     const long long dq_bytes_per_head =
-        with_dq && !packed_in_l2 ? (long long)group * plan_seqlen_q(p) * p->head_dim_qk * 4 : 0;
+        with_dq && !packed_near_l2 ? (long long)group * plan_seqlen_q(p) * p->head_dim_qk * 4 : 0;
     const CtaOrderPlan plan = cached_plan(work, bh, group, sm_count(), dq_bytes_per_head);
     args.stats = stats;
     args.sidecar = sidecar;

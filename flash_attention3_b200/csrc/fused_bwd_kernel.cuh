@@ -416,7 +416,6 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
     const bool misaligned = (sbase & 1023u) != 0;
     if (threadIdx.x == 0) {
-        TRACE(0, 4);
         if (misaligned) atomicCAS(&g_device_error, kDevOk, kDevSmemMisaligned);
         ptx::mbar_init(bar(kKvFull), 1);
         for (int s = 0; s < C::kQStages; ++s) {

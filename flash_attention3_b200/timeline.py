@@ -128,10 +128,9 @@ def main():
 
 
     print("-- set-up (clk from CTA start)")
-    stat("index arithmetic done (tile known)", [rel(c, 0, 4) for c in ctas])
     stat("barriers initialised", [rel(c, 0, 2) for c in ctas])
     stat("first loads issued (K,V,Q0,dO0)", [rel(c, 0, 3) for c in ctas])
-    stat("set-up barrier passed (TMEM allocated)", [rel(c, 1, 0) for c in ctas])
+    stat("set-up barrier passed (tile known, TMEM allocated)", [rel(c, 1, 0) for c in ctas])
     stat("K,V,Q(0) landed (seen by MMA warp)", [rel(c, 1, 1) for c in ctas])
     stat("S(0) issued", [rel(c, 1, 2) for c in ctas])
     stat("dP(0) issued", [rel(c, 1, 4) for c in ctas])

@@ -49,12 +49,12 @@
 //     mbarriers       256
 //     total           231,680 (D=128) / 182,528 (D=64)   of 232,448 available
 //
-// What bounds it: at D=64 the softmax / dS warpgroups (2630 clk per step, 1664 of MMA): one instruction per two
+// What bounds it: at D=64 the softmax / dS warpgroups (2650 clk per step, 1664 of MMA): one instruction per two
 // elements wherever packed arithmetic allows, statistics brought by a warp of their own, one arrival per warp
-// and uniform votes at the barriers took the step from 2980; B=4,H=16,S=4096 full: kernel 859 -> 791 us.  At
-// D=128 the copy engine (64 KB of loads and 64 KB of fp32 reduce-adds per step, 2900 clk for the latter) and the
-// chain dS -> dQ -> drain -> dP -> dS, 3800-4000 clk per step (2560 of MMA), under a power limit that holds the
-// clock near 1.55 GHz: 1295 -> 1289 us for the same shape.
+// and uniform votes at the barriers took the step from 2980; B=4,H=16,S=4096 full, kernel alone after a pause:
+// 859-867 -> 788 us.  At D=128 the copy engine (64 KB of loads and 64 KB of fp32 reduce-adds per step, 2400-3000 clk
+// for the latter) and the chain dS -> dQ -> drain -> dP -> dS, 3800-4000 clk per step (2560 of MMA): 1197 -> 1188 us for
+// the same shape, 1270-1320 both under the power limit, which holds the clock near 1.55 GHz.
 #pragma once
 
 #include <cuda.h>
@@ -160,7 +160,8 @@ struct FusedCfg {
     static constexpr int kBoxBytes = 128 * 128;
     static constexpr int kBoxes = D / 64;
     static constexpr int kOperandBytes = kBoxes * kBoxBytes;
-    // (a third Q stage at D=64: 904 -> 865 us per call of B=4,H=16,S=4096 full; a fourth, or a third of dO, no more)
+    // (a third Q stage at D=64: us per call of B=4,H=16,S=4096 full, back to back, 877-899 with two and 873 with three;
+    // the kernel alone after a pause 782 and 788; a fourth, or a third of dO, no more)
     static constexpr int kQStages = D == 64 ? 3 : 2;
     static constexpr int kDoStages = D == 128 ? 1 : 2;
     static constexpr int kDsBytes = 2 * kBoxBytes;

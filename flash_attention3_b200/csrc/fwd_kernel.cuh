@@ -26,9 +26,9 @@
 // busy warp of a scheduler issues an instruction every 1.9 clk, so the softmax is written for few
 // instructions: packed two-value arithmetic, three-input maxima, at D=64 every eighth exponential on the FMA
 // pipe (more of them cost more issue slots than they free), votes instead of divergent polling at the
-// barriers (see warp_wait), P's barrier asked for ahead of its use.  TFLOP/s, before and after: B=4, H=16,
-// S=4096 full, D=64 560 and 811, D=128 1050 and 1130-1180 (there the power limit holds the clock near
-// 1.6 GHz); B=2, Hq=32, Hkv=8, S=8192 causal, D=128 905 and 1150.
+// barriers (see warp_wait), P's barrier asked for ahead of its use.  TFLOP/s, back to back, before and
+// after: B=4, H=16, S=4096 full, D=64 567 and 823, D=128 930-990 and 1155-1170 (there the power limit holds the
+// clock near 1.6 GHz); B=2, Hq=32, Hkv=8, S=8192 causal, D=128 857 and 1063.
 //
 // When the pairs are too few to fill the GPU a cluster of 2, 4 or 8 CTAs shares the key tiles of a pair
 // (plan_fwd) and merges the partial outputs through distributed shared memory.

@@ -212,20 +212,31 @@ bool arg_schema_bool(PyObject* o, const char* name) {
     TORCH_CHECK_TYPE(o == Py_None || (number != nullptr && number->nb_bool != nullptr), name, " must be a bool");
     return arg_bool(o);
 }
-int64_t long_value(THPObjectPtr i) {
-    if (!i) throw python_error();
-    const long long v = PyLong_AsLongLong(i.get());
+// (the conversions of ints, bools, floats and tuples, what nearly every call passes, need no object of their own)
+int64_t long_value(PyObject* i) {
+    const long long v = PyLong_AsLongLong(i);
     if (v == -1 && PyErr_Occurred()) throw python_error();
     return v;
 }
-int64_t arg_int(PyObject* o) { return long_value(THPObjectPtr(PyNumber_Long(o))); }           // int(o)
-int64_t arg_schema_int(PyObject* o) { return long_value(THPObjectPtr(PyNumber_Index(o))); }  // (no float)
+int64_t arg_int(PyObject* o) {  // int(o)
+    if (PyLong_CheckExact(o) || PyBool_Check(o)) return long_value(o);
+    THPObjectPtr i(PyNumber_Long(o));
+    if (!i) throw python_error();
+    return long_value(i.get());
+}
+int64_t arg_schema_int(PyObject* o) {  // (no float)
+    if (PyLong_CheckExact(o)) return long_value(o);
+    THPObjectPtr i(PyNumber_Index(o));
+    if (!i) throw python_error();
+    return long_value(i.get());
+}
 double arg_double(PyObject* o) {  // a number
     const double v = PyFloat_AsDouble(o);
     if (v == -1.0 && PyErr_Occurred()) throw python_error();
     return v;
 }
 double arg_float(PyObject* o) {  // float(o)
+    if (PyFloat_CheckExact(o)) return PyFloat_AS_DOUBLE(o);
     const THPObjectPtr f(PyNumber_Float(o));
     if (!f) throw python_error();
     return PyFloat_AS_DOUBLE(f.get());
@@ -236,6 +247,11 @@ const char* arg_str(PyObject* o) {
     return s;
 }
 void arg_window(PyObject* o, Options* opt) {  // int(o[0]), int(o[1])
+    if (PyTuple_CheckExact(o) && PyTuple_GET_SIZE(o) >= 2) {
+        opt->window_left = arg_int(PyTuple_GET_ITEM(o, 0));
+        opt->window_right = arg_int(PyTuple_GET_ITEM(o, 1));
+        return;
+    }
     for (const long i : {0, 1}) {
         const THPObjectPtr index(PyLong_FromLong(i));
         THPObjectPtr item(index ? PyObject_GetItem(o, const_cast<PyObject*>(index.get())) : nullptr);

@@ -271,12 +271,11 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     delta = a.delta[stat_row];
                 }
             }
-            uint32_t ppk[32];
-            const float score_mul = kSoftcap ? a.softcap_pre * ptx::kTanhArg : a.scale_log2;
-            const uint64_t scale2 = ptx::f2_pack(score_mul, score_mul);
+            uint32_t ppk[32];  // what dP - delta is multiplied with, in 16 bits: P, or, capped, P (1 - t^2)
+            const uint64_t scale2 = ptx::f2_pack(a.scale_log2, a.scale_log2);
             const uint64_t post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
             const uint64_t neg2 = ptx::f2_pack(neg, neg), ndel2 = ptx::f2_pack(-delta, -delta);
-            const float inv_post = kSoftcap ? 1.0f / a.softcap_post : 0.0f;
+            const float small_score = kSoftcap ? ptx::kTanhPolyMax / fabsf(a.softcap_pre) : 0.0f;
             auto arrive = [&](int which) {
                 ptx::tc_fence_before();
                 __syncwarp();
@@ -296,19 +295,33 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     uint32_t r[32];
                     ptx::tmem_ld32(s_cols + c * 32, r);
                     ptx::tmem_ld_wait();
+                    auto softmax_chunk = [&](auto small_tag) {
 #pragma unroll
-                    for (int e = 0; e < 32; e += 2) {
-                        const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
-                        float2 p = ptx::f2_unpack(kSoftcap ? ptx::f2_fma(ptx::tanh_pair(ptx::f2_mul(s2, scale2)), post2, neg2)
-                                                           : ptx::f2_fma(s2, scale2, neg2));
-                        p.x = ptx::ex2_approx(p.x);
-                        p.y = ptx::ex2_approx(p.y);
-                        if (diagonal) {
-                            const int j = c * 32 + e;
-                            p.x = (j + 0 >= mask_from && j + 0 <= mask_to) ? p.x : 0.0f;
-                            p.y = (j + 1 >= mask_from && j + 1 <= mask_to) ? p.y : 0.0f;
+                        for (int e = 0; e < 32; e += 2) {
+                            const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
+                            uint64_t t2 = 0;
+                            if constexpr (kSoftcap) t2 = ptx::tanh_score<decltype(small_tag)::value>(s2, a.softcap_pre, small_score);
+                            float2 p = ptx::f2_unpack(kSoftcap ? ptx::f2_fma(t2, post2, neg2) : ptx::f2_fma(s2, scale2, neg2));
+                            p.x = ptx::ex2_approx(p.x);
+                            p.y = ptx::ex2_approx(p.y);
+                            if constexpr (kSoftcap) {
+                                const float2 tt = ptx::f2_unpack(t2);
+                                p = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y),
+                                                               ptx::f2_pack(fmaf(-tt.x, tt.x, 1.0f), fmaf(-tt.y, tt.y, 1.0f))));
+                            }
+                            if (diagonal) {
+                                const int j = c * 32 + e;
+                                p.x = (j + 0 >= mask_from && j + 0 <= mask_to) ? p.x : 0.0f;
+                                p.y = (j + 1 >= mask_from && j + 1 <= mask_to) ? p.y : 0.0f;
+                            }
+                            ppk[c * 16 + e / 2] = ptx::Pack2<T>::pack(p.x, p.y);
                         }
-                        ppk[c * 16 + e / 2] = ptx::Pack2<T>::pack(p.x, p.y);
+                    };
+                    if constexpr (kSoftcap) {
+                        if (__all_sync(0xffffffffu, ptx::all_small<32>(r, small_score))) softmax_chunk(std::true_type{});
+                        else softmax_chunk(std::false_type{});
+                    } else {
+                        softmax_chunk(std::false_type{});
                     }
                 }
                 arrive(kDqbSFree);
@@ -324,12 +337,7 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     for (int e = 0; e < 32; e += 2) {
                         const float2 p = ptx::Pack2<T>::unpack(ppk[c * 16 + e / 2]);
                         const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
-                        uint64_t ds2 = ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, ndel2));
-                        if (kSoftcap) {
-                            const float2 slope = ptx::cap_slope(p, neg2, inv_post);
-                            ds2 = ptx::f2_mul(ds2, ptx::f2_pack(slope.x, slope.y));
-                        }
-                        const float2 ds = ptx::f2_unpack(ds2);
+                        const float2 ds = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, ndel2)));
                         o[e / 2] = ptx::Pack2<T>::pack(ds.x, ds.y);
                     }
                     // dS chunk c lands on columns [16c, 16c+16) of this half's dP columns, all of which were read by

@@ -185,7 +185,9 @@ struct FusedCfg {
     static constexpr int kRegsControl = 96;
     static constexpr int kRegsCompute = D == 128 ? 120 : 136;
     static constexpr int kRegsDrain = D == 128 ? 176 : 136;
+    static constexpr int kRegsComputeNoDq = 160;  // without dQ the drain warpgroup idles at kRegsControl
     static_assert(kRegsControl + 2 * kRegsCompute + kRegsDrain <= 512, "register file over-committed");
+    static_assert(2 * kRegsControl + 2 * kRegsComputeNoDq <= 512, "register file over-committed");
 
     static constexpr int kTmemCols = 512;
     static constexpr int kColDK = 0;
@@ -392,9 +394,8 @@ struct StepWalk {
 // T: storage type of Q/K/V/dO (__half or __nv_bfloat16).  TOut: type of the dK
 // and dV outputs (T for the fused path, float for the split path).  kWithDq:
 // false turns the kernel into the four-GEMM dK/dV half of the split path.
-// kSoftcap: softcapped scores (general form only).  dS then carries the slope 1 - tanh^2 of the cap,
-// which the second softmax phase recovers from P itself (t = (log2 P - (log2 r - m)) / softcap_post)
-// instead of keeping it in registers between the phases.
+// kSoftcap: softcapped scores (general form only).  dS then carries the slope 1 - t^2 of the cap, t the tanh: the second
+// softmax phase needs P only in that product, so P (1 - t^2) is what it is handed in registers, in P's place.
 template <typename T, int D, bool kCausal, bool kWithDq, typename TOut, bool kSoftcap = false>
 __global__ void __launch_bounds__(512, 1)
 fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -654,7 +655,8 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
     } else if (wg == 1 || wg == 2) {
         // ============================================ softmax / dS warpgroups
-        if (C::kRegsCompute < 128) ptx::setmaxnreg_dec<C::kRegsCompute>();
+        if (!kWithDq) ptx::setmaxnreg_inc<C::kRegsComputeNoDq>();
+        else if (C::kRegsCompute < 128) ptx::setmaxnreg_dec<C::kRegsCompute>();
         else ptx::setmaxnreg_inc<C::kRegsCompute>();
         const FusedWork w = fused_work<kCausal>(a);
         const uint32_t tmem = set_up_done();
@@ -667,11 +669,10 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const uint32_t s_cols = tl + C::kColS + half * 64;
             const uint32_t dp_cols = tl + C::kColDP + half * 64;
             const uint32_t stats = sbase + C::kOffStats + half * 256;  // this half's 64 queries
-            // what a raw score is multiplied with: scale*log2e, or, capped, what makes it 2*log2e * (argument of tanh)
-            const float score_mul = kSoftcap ? a.softcap_pre * ptx::kTanhArg : a.scale_log2;
-            const uint64_t scale2 = ptx::f2_pack(score_mul, score_mul);
+            const uint64_t scale2 = ptx::f2_pack(a.scale_log2, a.scale_log2);
             const uint64_t post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
-            uint32_t ppk[32];
+            const float small_score = kSoftcap ? ptx::kTanhPolyMax / fabsf(a.softcap_pre) : 0.0f;
+            uint32_t ppk[32];  // what dP - delta is multiplied with, in 16 bits: P, or P (1 - t^2)
             // one arrival per warp: every lane's accesses are ordered before it by the fence and the warp barrier
             auto arrive = [&](int which) {
                 ptx::tc_fence_before();
@@ -696,8 +697,9 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 int mask_from = 0, mask_to = 0;  // set only on masked tiles
                 // ---- P^T = exp2(S^T * scale_log2 + neg_i), masked as above.
                 // (two copies of the chunk code, so that unmasked tiles carry no per-element test)
-                auto softmax_chunk = [&](int c, const uint32_t* r, auto masked_tag) {
+                auto softmax_chunk = [&](int c, const uint32_t* r, auto masked_tag, auto small_tag) {
                     constexpr bool kMasked = decltype(masked_tag)::value;
+                    uint32_t capped_p[16];  // P where ppk holds P (1 - t^2)
 #pragma unroll
                     for (int e = 0; e < 32; e += 4) {
                         const ptx::F4Pairs n4 = ptx::f2_ld_shared(negp + (c * 32 + e) * 4);
@@ -705,47 +707,63 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                         for (int h = 0; h < 2; ++h) {
                             const uint64_t neg2 = h == 0 ? n4.lo : n4.hi;
                             const int el = e + 2 * h;
-                            float2 p2;
-                            {
-                                // score in log2 units, relative to the row's reference: s * scale*log2e + (log2 r - m), or the
-                                // capped score + (log2 r - m)
-                                const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[el]), __uint_as_float(r[el + 1]));
-                                const uint64_t x2 = kSoftcap ? ptx::f2_fma(ptx::tanh_pair(ptx::f2_mul(s2, scale2)), post2, neg2)
-                                                             : ptx::f2_fma(s2, scale2, neg2);
-                                // (exp2_poly for a part of these changed nothing: B=4,H=16,S=4096,D=64 791, 792, 795, 810 us for 0 to 3
-                                // pairs of 8)
-                                p2 = ptx::f2_unpack(x2);
-                                p2.x = ptx::ex2_approx(p2.x);
-                                p2.y = ptx::ex2_approx(p2.y);
+                            // score in log2 units, relative to the row's reference: s * scale*log2e + (log2 r - m), or the
+                            // capped score + (log2 r - m)
+                            const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[el]), __uint_as_float(r[el + 1]));
+                            uint64_t t2 = 0;
+                            if constexpr (kSoftcap) t2 = ptx::tanh_score<decltype(small_tag)::value>(s2, a.softcap_pre, small_score);
+                            // (exp2_poly for a part of these changed nothing: B=4,H=16,S=4096,D=64 791, 792, 795, 810 us for 0 to 3
+                            // pairs of 8)
+                            float2 p2 = ptx::f2_unpack(kSoftcap ? ptx::f2_fma(t2, post2, neg2) : ptx::f2_fma(s2, scale2, neg2));
+                            p2.x = ptx::ex2_approx(p2.x);
+                            p2.y = ptx::ex2_approx(p2.y);
+                            float2 w2;
+                            if constexpr (kSoftcap) {
+                                const float2 tt = ptx::f2_unpack(t2);
+                                w2 = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p2.x, p2.y),
+                                                                ptx::f2_pack(fmaf(-tt.x, tt.x, 1.0f), fmaf(-tt.y, tt.y, 1.0f))));
                             }
                             if (kMasked) {
                                 const int i = half * 64 + c * 32 + el;
-                                p2.x = (i + 0 >= mask_from && i + 0 <= mask_to) ? p2.x : 0.0f;
-                                p2.y = (i + 1 >= mask_from && i + 1 <= mask_to) ? p2.y : 0.0f;
+                                const bool sees0 = i + 0 >= mask_from && i + 0 <= mask_to, sees1 = i + 1 >= mask_from && i + 1 <= mask_to;
+                                p2.x = sees0 ? p2.x : 0.0f;
+                                p2.y = sees1 ? p2.y : 0.0f;
+                                if constexpr (kSoftcap) {
+                                    w2.x = sees0 ? w2.x : 0.0f;
+                                    w2.y = sees1 ? w2.y : 0.0f;
+                                }
                             }
-                            ppk[c * 16 + el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
+                            if constexpr (kSoftcap) {
+                                capped_p[el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
+                                ppk[c * 16 + el / 2] = ptx::Pack2<T>::pack(w2.x, w2.y);
+                            } else {
+                                ppk[c * 16 + el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
+                            }
                         }
                     }
                     // P chunk c -> columns [16c, 16c+16) of this half's S columns (already read)
-                    ptx::tmem_st16(s_cols + c * 16, &ppk[c * 16]);
+                    if constexpr (kSoftcap) ptx::tmem_st16(s_cols + c * 16, capped_p);
+                    else ptx::tmem_st16(s_cols + c * 16, &ppk[c * 16]);
+                };
+                auto softmax_phase = [&](auto masked_tag) {
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        uint32_t r[32];
+                        ptx::tmem_ld32(s_cols + c * 32, r);
+                        ptx::tmem_ld_wait();
+                        if constexpr (kSoftcap) {
+                            if (__all_sync(0xffffffffu, ptx::all_small<32>(r, small_score))) softmax_chunk(c, r, masked_tag, std::true_type{});
+                            else softmax_chunk(c, r, masked_tag, std::false_type{});
+                        } else {
+                            softmax_chunk(c, r, masked_tag, std::false_type{});
+                        }
+                    }
                 };
                 if (diagonal) {
                     query_range_of_key(w.kt * C::kTile + j, qt * C::kTile, w.band, &mask_from, &mask_to);
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        uint32_t r[32];
-                        ptx::tmem_ld32(s_cols + c * 32, r);
-                        ptx::tmem_ld_wait();
-                        softmax_chunk(c, r, std::true_type{});
-                    }
+                    softmax_phase(std::true_type{});
                 } else {
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        uint32_t r[32];
-                        ptx::tmem_ld32(s_cols + c * 32, r);
-                        ptx::tmem_ld_wait();
-                        softmax_chunk(c, r, std::false_type{});
-                    }
+                    softmax_phase(std::false_type{});
                 }
                 if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 2);
                 ptx::tmem_st_wait();
@@ -759,7 +777,6 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 5);
                 ptx::tc_fence_after();
                 const uint32_t ds_row = sbase + C::kOffDS + half * C::kBoxBytes + j * 128;
-                const float inv_post = kSoftcap ? 1.0f / a.softcap_post : 0.0f;
                 auto ds_chunk = [&](int c, const uint32_t* r) {
 #pragma unroll
                     for (int e = 0; e < 32; e += 8) {
@@ -768,26 +785,12 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                         for (int h = 0; h < 2; ++h) {
                             const ptx::F4Pairs d4 = ptx::f2_ld_shared(delp + (c * 32 + e + 4 * h) * 4);  // -delta
                             const int el = e + 4 * h;
-                            if (kSoftcap) {
-                                // dS = P (dP - delta) (1 - t^2), t recovered from P and the row's reference
-                                const ptx::F4Pairs n4 = ptx::f2_ld_shared(negp + (c * 32 + el) * 4);
 #pragma unroll
-                                for (int g = 0; g < 2; ++g) {
-                                    const float2 p = ptx::Pack2<T>::unpack(ppk[c * 16 + el / 2 + g]);
-                                    const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[el + 2 * g]), __uint_as_float(r[el + 2 * g + 1]));
-                                    const float2 slope = ptx::cap_slope(p, g == 0 ? n4.lo : n4.hi, inv_post);
-                                    const uint64_t x2 = ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, g == 0 ? d4.lo : d4.hi));
-                                    const float2 ds = ptx::f2_unpack(ptx::f2_mul(x2, ptx::f2_pack(slope.x, slope.y)));
-                                    o[2 * h + g] = ptx::Pack2<T>::pack(ds.x, ds.y);
-                                }
-                            } else {
-#pragma unroll
-                                for (int g = 0; g < 2; ++g) {
-                                    const float2 p = ptx::Pack2<T>::unpack(ppk[c * 16 + el / 2 + g]);
-                                    const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[el + 2 * g]), __uint_as_float(r[el + 2 * g + 1]));
-                                    const float2 ds = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, g == 0 ? d4.lo : d4.hi)));
-                                    o[2 * h + g] = ptx::Pack2<T>::pack(ds.x, ds.y);
-                                }
+                            for (int g = 0; g < 2; ++g) {
+                                const float2 p = ptx::Pack2<T>::unpack(ppk[c * 16 + el / 2 + g]);
+                                const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[el + 2 * g]), __uint_as_float(r[el + 2 * g + 1]));
+                                const float2 ds = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, g == 0 ? d4.lo : d4.hi)));
+                                o[2 * h + g] = ptx::Pack2<T>::pack(ds.x, ds.y);
                             }
                         }
                         const int chunk = c * 4 + e / 8;  // 16-byte chunk inside this half's box

@@ -528,17 +528,21 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 if (C::kOwnP) arrive(kFwdSFree);
                 if (kSoftcap) {
                     // capped scores, already in log2 units: from here on they are used with a scale of 1
-                    const float pre = a.softcap_pre * ptx::kTanhArg;
-                    const uint64_t pre2 = ptx::f2_pack(pre, pre), post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
+                    const uint64_t post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
+                    const float small_score = ptx::kTanhPolyMax / fabsf(a.softcap_pre);
+                    auto cap_chunk = [&](uint32_t (&chunk)[32], auto small_tag) {
 #pragma unroll
                         for (int e = 0; e < 32; e += 2) {
-                            const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
-                            const float2 capped = ptx::f2_unpack(ptx::f2_mul(ptx::tanh_pair(ptx::f2_mul(s2, pre2)), post2));
-                            r[c][e] = __float_as_uint(capped.x);
-                            r[c][e + 1] = __float_as_uint(capped.y);
+                            const uint64_t s2 = ptx::f2_pack(__uint_as_float(chunk[e]), __uint_as_float(chunk[e + 1]));
+                            const float2 capped = ptx::f2_unpack(ptx::f2_mul(ptx::tanh_score<decltype(small_tag)::value>(s2, a.softcap_pre, small_score), post2));
+                            chunk[e] = __float_as_uint(capped.x);
+                            chunk[e + 1] = __float_as_uint(capped.y);
                         }
+                    };
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        if (__all_sync(0xffffffffu, ptx::all_small<32>(r[c], small_score))) cap_chunk(r[c], std::true_type{});
+                        else cap_chunk(r[c], std::false_type{});
                     }
                 }
                 if (diagonal) {

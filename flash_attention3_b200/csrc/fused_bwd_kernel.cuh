@@ -18,18 +18,25 @@
 // convert kernel) instead of per element of dS.
 //
 // Epilogue: when the last MMA has completed, every softmax warp stages its 32 key rows of dK
-// (scaled) or dV over the dead Q / dO / dS^T buffers and stores them in whole lines.  On problems too small to fill the GPU the query steps
+// (scaled) or dV in shared memory and stores them in whole lines.  On problems too small to fill the GPU the query steps
 // of a key tile are cut into chunks, one CTA each (a table in the kernel parameters says which,
 // longest chunks first); such a CTA stores its partial dK / dV to its own slab and the convert
 // kernel adds the slabs of a tile in chunk order.
 //
 // Warp roles (512 threads, four warpgroups): warp 0 = TMA producer, warp 1 = MMA
-// issuer and TMEM owner, warp 2 = row statistics; warps 4-7 and 8-11 = two softmax / dS warpgroups (thread
+// issuer and TMEM owner, warp 2 = row statistics, warp 3 = which tile; warps 4-7 and 8-11 = two softmax / dS warpgroups (thread
 // j of each owns TMEM lane j = key j; the first takes queries 0-63 of the tile,
 // the second queries 64-127); warps 12-15 = dQ drain warpgroup.  Registers are
 // re-split with setmaxnreg (96 / 120 / 120 / 176 per thread at D=128).  All hand-offs go
 // through mbarriers; every wait is bounded and a time-out raises an error flag
 // instead of hanging.
+//
+// Tiles (kPersist): a CTA that is about to finish its tile asks for the block index of a CTA that has not started, warp 3
+// works out what that is and hands it to the other roles in shared memory, and the roles, rings and hand-offs run on: K, V, Q
+// and dO of the next tile are loaded and its first S is computed beside the epilogue, and the set-up (barriers, tensor memory,
+// cold instruction cache: 1300-2800 clk until the first loads, 3000-5000 until they have landed) is paid once.  Where every SM
+// has several tiles; the rule and what it measured stand beside the launch.  One warp works the tile out for all, in either
+// form, because the index arithmetic inlined in five roles was 1400 clk of cold code in front of the first loads.
 //
 // Tensor-memory ledger (512 columns x 128 lanes x 32 bit):
 //     D = 128:  dK [0,128)  dV [128,256)  S/P [256,384)  dP and dQ share [384,512)
@@ -47,7 +54,8 @@
 //     dQ staging      32 KiB               4 warps x 2 boxes of [32 rows][32 fp32]
 //     row statistics  2 KiB                {log2 r - m, -delta} x 128 rows x 2 buffers
 //     mbarriers       256
-//     total           231,680 (D=128) / 182,528 (D=64)   of 232,448 available
+//     work of a tile  256                  two buffers
+//     total           231,936 (D=128) / 182,784 (D=64)   of 232,448 available
 //
 // What bounds it: at D=64 the softmax / dS warpgroups (2650 clk per step, 1664 of MMA): one instruction per two
 // elements wherever packed arithmetic allows, statistics brought by a warp of their own, one arrival per warp
@@ -177,7 +185,8 @@ struct FusedCfg {
     static constexpr int kOffStats = kOffStage + kStageBytes;
     // Row statistics: two buffers of 128 x {log2 r - m}, then two of 128 x {-delta}
     static constexpr int kOffBar = kOffStats + 2 * 1024;
-    static constexpr int kSmemBytes = kOffBar + 256;
+    static constexpr int kOffWork = kOffBar + 256;  // two buffers
+    static constexpr int kSmemBytes = kOffWork + 256;
     static_assert(kSmemBytes <= 232448, "shared-memory ledger exceeds 227 KiB");
     static_assert(kOffStage % 1024 == 0 && kOffDS % 1024 == 0, "swizzled regions need 1 KiB alignment");
 
@@ -214,7 +223,10 @@ enum Bar : int {
     kDkvFull = 17,
     kStatsFull = 18,   // 2 buffers
     kStatsEmpty = 20,  // 2 buffers
-    kNumBars = 22,
+    kAnswer = 22,      // which block comes next
+    kWorkFull = 23,    // 2 buffers: the work of a block
+    kWorkEmpty = 25,   // 2 buffers
+    kNumBars = 27,
 };
 
 constexpr uint32_t kWaitTimeoutCycles = 2000000000u;  // about one second, of a 32-bit cycle counter
@@ -286,8 +298,9 @@ __device__ __forceinline__ bool warp_wait2(uint32_t bar0, uint32_t parity0, uint
     return warp_wait(bar0, parity0, abort_flag) && warp_wait(bar1, parity1, abort_flag);
 }
 
-// Which key tile and which of its steps a CTA works on.
-struct FusedWork {
+// Which key tile and which of its steps a CTA works on.  One warp works it out and hands it to the others in shared memory.
+struct alignas(16) FusedWork {
+    int block;            // place in the launch order, -1: there is none
     int kt, b, kvh, slab;
     Band band;            // this batch entry's own lengths
     int q_base, k_base, b_coord;
@@ -299,12 +312,26 @@ struct FusedWork {
     int t_begin, n_steps; // this CTA's share of the tile's steps (all of them unless the tile is split)
     int rotation;
 };
-
-// (Each role works this out for itself behind its setmaxnreg: values carried across a change of the register
-// budget were spilled.)
-template <bool kCausal>
-__device__ __forceinline__ FusedWork fused_work(const FusedArgs& a) {
+static_assert(sizeof(FusedWork) == 96, "six 16-byte words");
+__device__ __forceinline__ void store_work(uint32_t addr, const FusedWork& w) {
+    const uint32_t* v = reinterpret_cast<const uint32_t*>(&w);
+#pragma unroll
+    for (int i = 0; i < 24; i += 4)
+        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr + 4 * i), "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]) : "memory");
+}
+__device__ __forceinline__ FusedWork load_work(uint32_t addr) {
     FusedWork w;
+    uint32_t* v = reinterpret_cast<uint32_t*>(&w);
+#pragma unroll
+    for (int i = 0; i < 24; i += 4)
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v[i]), "=r"(v[i + 1]), "=r"(v[i + 2]), "=r"(v[i + 3]) : "r"(addr + 4 * i) : "memory");
+    return w;
+}
+
+template <bool kCausal>
+__device__ __forceinline__ FusedWork fused_work(const FusedArgs& a, int block) {
+    FusedWork w;
+    w.block = block;
     const int n_tiles = tiles_of(a.band.seqlen_k);      // key tiles (of the longest sequence)
     const int bh_count = a.batch * a.heads_kv;
     const bool split = a.chunk_steps > 0;
@@ -313,14 +340,14 @@ __device__ __forceinline__ FusedWork fused_work(const FusedArgs& a) {
     w.t_begin = w.slab = 0;
     if (!split) {
         // groups of head_group heads; inside a group tile slot major, head minor (see cta_order.h)
-        const int hg = fast_div(int(blockIdx.x), a.per_group);
-        const int rem = int(blockIdx.x) - hg * a.per_group.divisor;
+        const int hg = fast_div(block, a.per_group);
+        const int rem = block - hg * a.per_group.divisor;
         const int heads_here = min(a.head_group, bh_count - hg * a.head_group);
         const int tile_slot = heads_here == a.head_group ? fast_div(rem, a.in_group) : rem / heads_here;
         bhi = hg * a.head_group + (rem - tile_slot * heads_here);
         w.kt = remap_k_tile(tile_slot, n_tiles, a.order_mode, a.order_width);
     } else {
-        const uint32_t entry = a.cta_table[blockIdx.x];
+        const uint32_t entry = a.cta_table[block];
         w.kt = int(entry & 0xffu);
         w.t_begin = int((entry >> 8) & 0xffu) * a.chunk_steps;
         w.slab = int(entry >> 16);
@@ -394,9 +421,10 @@ struct StepWalk {
 // T: storage type of Q/K/V/dO (__half or __nv_bfloat16).  TOut: type of the dK
 // and dV outputs (T for the fused path, float for the split path).  kWithDq:
 // false turns the kernel into the four-GEMM dK/dV half of the split path.
+// kPersist: CTAs take over the tiles of CTAs that have not started (see above).
 // kSoftcap: softcapped scores (general form only).  dS then carries the slope 1 - t^2 of the cap, t the tanh: the second
 // softmax phase needs P only in that product, so P (1 - t^2) is what it is handed in registers, in P's place.
-template <typename T, int D, bool kCausal, bool kWithDq, typename TOut, bool kSoftcap = false>
+template <typename T, int D, bool kCausal, bool kWithDq, typename TOut, bool kSoftcap = false, bool kPersist = false>
 __global__ void __launch_bounds__(512, 1)
 fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -411,6 +439,25 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     auto bar = [&](int i) -> uint32_t { return sbase + C::kOffBar + 8 * i; };
     const uint32_t tmem_slot = sbase + C::kOffBar + 8 * kNumBars;
     const uint32_t abort_flag = tmem_slot + 4;
+    const uint32_t answer = sbase + C::kOffBar + 240;
+    static_assert(8 * kNumBars + 8 <= 240, "barriers and the answer share 256 bytes");
+    const uint32_t work = sbase + C::kOffWork;
+    // (a converged warp) the first tile, and the tile after this one; n: how many this CTA has done before
+    auto first_tile = [&]() -> FusedWork {
+        const FusedWork w = load_work(work);
+        __syncwarp();
+        if (kPersist && lane == 0) ptx::mbar_arrive(bar(kWorkEmpty));
+        return w;
+    };
+    auto next_tile = [&](uint32_t n, FusedWork* w) -> bool {
+        if (!kPersist) return false;
+        const uint32_t buf = (n + 1) & 1;
+        if (!warp_wait(bar(kWorkFull + buf), (n >> 1) & 1, abort_flag)) return false;
+        *w = load_work(work + 128 * buf);
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(bar(kWorkEmpty + buf));
+        return w->block >= 0;
+    };
 
     if (threadIdx.x == 0) {
         TRACE(0, 0);
@@ -432,7 +479,10 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         for (int s = 0; s < 2; ++s) {
             ptx::mbar_init(bar(kStatsFull + s), 1);
             ptx::mbar_init(bar(kStatsEmpty + s), 8);
+            ptx::mbar_init(bar(kWorkFull + s), 1);
+            ptx::mbar_init(bar(kWorkEmpty + s), kWithDq ? 15 : 11);  // every warp that does the work
         }
+        ptx::mbar_init(bar(kAnswer), 1);
         ptx::mbar_init(bar(kSFull), 1);
         ptx::mbar_init(bar(kDpFull), 1);
         ptx::mbar_init(bar(kPReady), 8);
@@ -451,159 +501,191 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     // The kernel behind this one (dQ convert) may begin to launch; it waits for our completion itself.  (The dQ kernel
     // of the split path does not: it is let go by the statistics warp, below, once the delta stage has completed.)
     if (kWithDq) ptx::launch_dependents();
-    // (all threads: barriers initialised, tensor memory allocated)
+    // (all threads: barriers initialised, tensor memory allocated, first tile known)
     auto set_up_done = [&] {
         ptx::tc_fence_before();
         asm volatile("bar.sync 0;" ::: "memory");
         ptx::tc_fence_after();
-        return flag_value(tmem_slot);
     };
 
+    // Every role walks the tiles of this CTA, and keeps count of the steps of all of them (g0 in front of a tile): the rings and
+    // hand-offs run on from tile to tile.
     if (wg == 0) {
         ptx::setmaxnreg_dec<C::kRegsControl>();
-        const FusedWork w = fused_work<kCausal>(a);
-        const uint32_t tmem = set_up_done();
-        const bool idle = misaligned || w.n_steps == 0;  // a CTA without work: set-up and teardown still run
-        const int n_steps = w.n_steps;
-        if (!idle && warp == 0) {
+        if (warp == 0) {
             // =================================================== TMA producer
-            if (lane == 0) {
-                ptx::prefetch_tensormap(&tm_q);
-                ptx::prefetch_tensormap(&tm_k);
-                ptx::prefetch_tensormap(&tm_v);
-                ptx::prefetch_tensormap(&tm_do);
-                // tensor maps are [batch][head][row][D]; rows past the end of a sequence read as zero
-                ptx::mbar_arrive_expect_tx(bar(kKvFull), 2 * C::kOperandBytes);
-#pragma unroll
-                for (int bx = 0; bx < C::kBoxes; ++bx) {
-                    ptx::tma_load_4d(sbase + C::kOffK + bx * C::kBoxBytes, &tm_k, bar(kKvFull), bx * 64,
-                                     w.k_base + w.kt * C::kTile, w.kvh, w.b_coord);
-                    ptx::tma_load_4d(sbase + C::kOffV + bx * C::kBoxBytes, &tm_v, bar(kKvFull), bx * 64,
-                                     w.k_base + w.kt * C::kTile, w.kvh, w.b_coord);
-                }
-                TRACE(0, 3);
-                StepWalk<kCausal> st(w);
+            set_up_done();
+            FusedWork w = first_tile();
+            uint32_t n = 0, used = 0;  // tiles, tiles with steps
+            int g0 = 0;
 #pragma unroll 1
-                for (int t = 0; t < n_steps; ++t, st.next(w)) {
-                    const int hq = st.hq;
-                    const int q_row = w.q_base + st.qt * C::kTile;
-                    const int s = t % C::kQStages;
-                    if (!bounded_wait<true>(bar(kQEmpty + s), ((t / C::kQStages) & 1) ^ 1, abort_flag)) break;
-                    ptx::mbar_arrive_expect_tx(bar(kQFull + s), C::kOperandBytes);
+            for (bool more = !misaligned; more; ++n) {
+                if (lane == 0) {
+                    // K and V, when the MMAs of the tile before have completed.  (Tensor maps are [batch][head][row][D]; rows
+                    // past the end of a sequence read as zero.)
+                    if (w.n_steps > 0 && (used == 0 || bounded_wait<true>(bar(kDkvFull), (used - 1) & 1, abort_flag))) {
+                        ptx::mbar_arrive_expect_tx(bar(kKvFull), 2 * C::kOperandBytes);
 #pragma unroll
-                    for (int bx = 0; bx < C::kBoxes; ++bx) {
-                        ptx::tma_load_4d(sbase + C::kOffQ + s * C::kOperandBytes + bx * C::kBoxBytes, &tm_q,
-                                         bar(kQFull + s), bx * 64, q_row, hq, w.b_coord);
+                        for (int bx = 0; bx < C::kBoxes; ++bx) {
+                            ptx::tma_load_4d(sbase + C::kOffK + bx * C::kBoxBytes, &tm_k, bar(kKvFull), bx * 64,
+                                             w.k_base + w.kt * C::kTile, w.kvh, w.b_coord);
+                            ptx::tma_load_4d(sbase + C::kOffV + bx * C::kBoxBytes, &tm_v, bar(kKvFull), bx * 64,
+                                             w.k_base + w.kt * C::kTile, w.kvh, w.b_coord);
+                        }
                     }
-                    const int sd = t % C::kDoStages;
-                    if (!bounded_wait<true>(bar(kDoEmpty + sd), ((t / C::kDoStages) & 1) ^ 1, abort_flag)) break;
-                    ptx::mbar_arrive_expect_tx(bar(kDoFull + sd), C::kOperandBytes);
+                    if (n == 0) TRACE(0, 3);
+                    StepWalk<kCausal> st(w);
+#pragma unroll 1
+                    for (int t = 0; t < w.n_steps; ++t, st.next(w)) {
+                        const int hq = st.hq;
+                        const int q_row = w.q_base + st.qt * C::kTile;
+                        const int g = g0 + t;
+                        const int s = g % C::kQStages;
+                        if (!bounded_wait<true>(bar(kQEmpty + s), ((g / C::kQStages) & 1) ^ 1, abort_flag)) break;
+                        ptx::mbar_arrive_expect_tx(bar(kQFull + s), C::kOperandBytes);
 #pragma unroll
-                    for (int bx = 0; bx < C::kBoxes; ++bx) {
-                        ptx::tma_load_4d(sbase + C::kOffDO + sd * C::kOperandBytes + bx * C::kBoxBytes, &tm_do,
-                                         bar(kDoFull + sd), bx * 64, q_row, hq, w.b_coord);
+                        for (int bx = 0; bx < C::kBoxes; ++bx) {
+                            ptx::tma_load_4d(sbase + C::kOffQ + s * C::kOperandBytes + bx * C::kBoxBytes, &tm_q,
+                                             bar(kQFull + s), bx * 64, q_row, hq, w.b_coord);
+                        }
+                        const int sd = g % C::kDoStages;
+                        if (!bounded_wait<true>(bar(kDoEmpty + sd), ((g / C::kDoStages) & 1) ^ 1, abort_flag)) break;
+                        ptx::mbar_arrive_expect_tx(bar(kDoFull + sd), C::kOperandBytes);
+#pragma unroll
+                        for (int bx = 0; bx < C::kBoxes; ++bx) {
+                            ptx::tma_load_4d(sbase + C::kOffDO + sd * C::kOperandBytes + bx * C::kBoxBytes, &tm_do,
+                                             bar(kDoFull + sd), bx * 64, q_row, hq, w.b_coord);
+                        }
+                    }
+                    // Asks for the next tile, as late as it does not hold that up: tiles are to go to the CTAs in the order in
+                    // which these become free.  (Warp 3 has used the answer before this one.)
+                    if (kPersist) {
+                        ptx::mbar_arrive_expect_tx(bar(kAnswer), 16);
+                        ptx::request_block(answer, bar(kAnswer));
                     }
                 }
+                __syncwarp();
+                g0 += w.n_steps;
+                used += w.n_steps > 0 ? 1 : 0;
+                more = next_tile(n, &w);
             }
-        } else if (!idle && warp == 1) {
+        } else if (warp == 1) {
             // ===================================================== MMA issuer
             // The whole warp runs this role converged; MMAs and commits elect their lane inside the asm.
-            {
-                TRACE(1, 0);
-                constexpr uint32_t kIdSdP = ptx::instr_desc_f16(kBf16, 128, 128, false, false);
-                constexpr uint32_t kIdDkv = ptx::instr_desc_f16(kBf16, 128, D, false, true);
-                constexpr uint32_t kIdDq = ptx::instr_desc_f16(kBf16, 128, D, true, true);
-                // Descriptor low words (address >> 4 | LBO) of every operand tile.
-                const uint32_t loK_k = ptx::desc_lo_k_major(sbase + C::kOffK);
-                const uint32_t loV_k = ptx::desc_lo_k_major(sbase + C::kOffV);
-                const uint32_t loDS_k = ptx::desc_lo_k_major(sbase + C::kOffDS);
-                const uint32_t loK_mn = ptx::desc_lo_mn_major(sbase + C::kOffK, C::kBoxBytes);
-                const uint32_t loDS_mn = ptx::desc_lo_mn_major(sbase + C::kOffDS, C::kBoxBytes);
-                auto sQ = [&](int t) { return sbase + C::kOffQ + (t % C::kQStages) * C::kOperandBytes; };
-                auto sDO = [&](int t) { return sbase + C::kOffDO + (t % C::kDoStages) * C::kOperandBytes; };
-                auto issue_s = [&](int t) {
-                    const uint32_t loQ = ptx::desc_lo_k_major(sQ(t));
-                    ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(tmem + C::kColS, loK_k, loQ, kIdSdP, 0);
-                    ptx::tc_commit_elect(bar(kSFull));
-                };
-                auto issue_dp = [&](int t) {
-                    const uint32_t loDO = ptx::desc_lo_k_major(sDO(t));
-                    ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(tmem + C::kColDP, loV_k, loDO, kIdSdP, 0);
-                    ptx::tc_commit_elect(bar(kDpFull));
-                };
-                bool ok = warp_wait<false>(bar(kKvFull), 0, abort_flag) &&
-                          warp_wait<false>(bar(kQFull + 0), 0, abort_flag);
-                TRACE(1, 1);
-                if (ok) {
-                    ptx::tc_fence_after();
-                    issue_s(0);
-                    TRACE(1, 2);
-                    ok = warp_wait<false>(bar(kDoFull + 0), 0, abort_flag);
-                }
-                if (ok) {
-                    ptx::tc_fence_after();
-                    issue_dp(0);
-                    TRACE(1, 4);
+            set_up_done();
+            const uint32_t tmem = flag_value(tmem_slot);
+            FusedWork w = first_tile();
+            TRACE(1, 0);
+            constexpr uint32_t kIdSdP = ptx::instr_desc_f16(kBf16, 128, 128, false, false);
+            constexpr uint32_t kIdDkv = ptx::instr_desc_f16(kBf16, 128, D, false, true);
+            constexpr uint32_t kIdDq = ptx::instr_desc_f16(kBf16, 128, D, true, true);
+            // Descriptor low words (address >> 4 | LBO) of every operand tile.
+            const uint32_t loK_k = ptx::desc_lo_k_major(sbase + C::kOffK);
+            const uint32_t loV_k = ptx::desc_lo_k_major(sbase + C::kOffV);
+            const uint32_t loDS_k = ptx::desc_lo_k_major(sbase + C::kOffDS);
+            const uint32_t loK_mn = ptx::desc_lo_mn_major(sbase + C::kOffK, C::kBoxBytes);
+            const uint32_t loDS_mn = ptx::desc_lo_mn_major(sbase + C::kOffDS, C::kBoxBytes);
+            // (g: step counted over all tiles)
+            auto sQ = [&](int g) { return sbase + C::kOffQ + (g % C::kQStages) * C::kOperandBytes; };
+            auto sDO = [&](int g) { return sbase + C::kOffDO + (g % C::kDoStages) * C::kOperandBytes; };
+            auto wait_q = [&](int g) { return warp_wait<false>(bar(kQFull + g % C::kQStages), (g / C::kQStages) & 1, abort_flag); };
+            auto wait_do = [&](int g) { return warp_wait<false>(bar(kDoFull + g % C::kDoStages), (g / C::kDoStages) & 1, abort_flag); };
+            auto issue_s = [&](int g) {
+                const uint32_t loQ = ptx::desc_lo_k_major(sQ(g));
+                ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(tmem + C::kColS, loK_k, loQ, kIdSdP, 0);
+                ptx::tc_commit_elect(bar(kSFull));
+            };
+            auto issue_dp = [&](int g) {
+                const uint32_t loDO = ptx::desc_lo_k_major(sDO(g));
+                ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(tmem + C::kColDP, loV_k, loDO, kIdSdP, 0);
+                ptx::tc_commit_elect(bar(kDpFull));
+            };
+            uint32_t n = 0, used = 0;
+            int g0 = 0;
+            bool ok = true;
+#pragma unroll 1
+            for (bool next = !misaligned; next; ++n) {
+                const int n_steps = w.n_steps;
+                if (n_steps > 0) {
+                    ok = warp_wait<false>(bar(kKvFull), used & 1, abort_flag) && wait_q(g0);
+                    if (n == 0) TRACE(1, 1);
+                    if (ok) {
+                        ptx::tc_fence_after();
+                        issue_s(g0);
+                        if (n == 0) TRACE(1, 2);
+                        ok = wait_do(g0);
+                        // (dP takes the columns of dQ of the last step)
+                        if (kWithDq && D == 128) ok = ok && warp_wait<false>(bar(kDqEmpty), (g0 & 1) ^ 1, abort_flag);
+                    }
+                    if (ok) {
+                        ptx::tc_fence_after();
+                        issue_dp(g0);
+                        if (n == 0) TRACE(1, 4);
+                    }
+                    ++used;
                 }
 #pragma unroll 1
                 for (int t = 0; ok && t < n_steps; ++t) {
+                    const int g = g0 + t;
                     const bool more = t + 1 < n_steps;
+                    const bool traced = n == 0 && t < 6;
                     // dV += P^T dO.  P^T of queries 0-63 sits on columns [0,32) of the S
                     // region, of queries 64-127 on columns [64,96).
-                    if (!(ok = warp_wait<false>(bar(kPReady), t & 1, abort_flag))) break;
-                    if (t < 6) TRACE(1, 8 + 8 * t + 0);
+                    // (the softmax warps have stored dK / dV of the tile before when they hand over their first P)
+                    if (!(ok = warp_wait<false>(bar(kPReady), g & 1, abort_flag))) break;
+                    if (traced) TRACE(1, 8 + 8 * t + 0);
                     ptx::tc_fence_after();
                     {
-                        const uint32_t loDO = ptx::desc_lo_mn_major(sDO(t), C::kBoxBytes);
+                        const uint32_t loDO = ptx::desc_lo_mn_major(sDO(g), C::kBoxBytes);
                         ptx::mma_ts_8<ptx::TmemHalves, ptx::MnMajor>(tmem + C::kColDV, tmem + C::kColS, loDO, kIdDkv, t > 0 ? 1u : 0u);
                     }
-                    ptx::tc_commit_elect(bar(kDoEmpty + t % C::kDoStages));
-                    if (t < 6) TRACE(1, 8 + 8 * t + 1);
-                    // S(t+1) may overwrite S/P(t): MMAs execute in issue order.
+                    ptx::tc_commit_elect(bar(kDoEmpty + g % C::kDoStages));
+                    if (traced) TRACE(1, 8 + 8 * t + 1);
+                    // S of the next step may overwrite S/P of this one: MMAs execute in issue order.
                     if (more) {
-                        if (!(ok = warp_wait<false>(bar(kQFull + (t + 1) % C::kQStages),
-                                                ((t + 1) / C::kQStages) & 1, abort_flag))) break;
+                        if (!(ok = wait_q(g + 1))) break;
                         ptx::tc_fence_after();
-                        issue_s(t + 1);
+                        issue_s(g + 1);
                     }
-                    if (t < 6) TRACE(1, 8 + 8 * t + 2);
+                    if (traced) TRACE(1, 8 + 8 * t + 2);
                     // dK += dS^T Q
-                    if (!(ok = warp_wait<false>(bar(kDsReady), t & 1, abort_flag))) break;
-                    if (t < 6) TRACE(1, 8 + 8 * t + 3);
+                    if (!(ok = warp_wait<false>(bar(kDsReady), g & 1, abort_flag))) break;
+                    if (traced) TRACE(1, 8 + 8 * t + 3);
                     ptx::tc_fence_after();
                     {
-                        const uint32_t loQ = ptx::desc_lo_mn_major(sQ(t), C::kBoxBytes);
+                        const uint32_t loQ = ptx::desc_lo_mn_major(sQ(g), C::kBoxBytes);
                         ptx::mma_ss_8<ptx::KMajor, ptx::MnMajor>(tmem + C::kColDK, loDS_k, loQ, kIdDkv, t > 0 ? 1u : 0u);
                     }
-                    ptx::tc_commit_elect(bar(kQEmpty + t % C::kQStages));
+                    ptx::tc_commit_elect(bar(kQEmpty + g % C::kQStages));
                     if (kWithDq) {
-                        if (D == 64) {  // own dQ region: wait for the drain of step t-1
-                            if (!(ok = warp_wait<false>(bar(kDqEmpty), (t & 1) ^ 1, abort_flag))) break;
+                        if (D == 64) {  // own dQ region: wait for the drain of the step before
+                            if (!(ok = warp_wait<false>(bar(kDqEmpty), (g & 1) ^ 1, abort_flag))) break;
                             ptx::tc_fence_after();
                         }
-                        // dQ = dS K  (overwrites dP(t) when D = 128: dP(t) was consumed before kDsReady)
+                        // dQ = dS K  (overwrites dP when D = 128: it was consumed before kDsReady)
                         ptx::mma_ss_8<ptx::MnMajor, ptx::MnMajor>(tmem + C::kColDQ, loDS_mn, loK_mn, kIdDq, 0);
                         ptx::tc_commit_elect(bar(kDqFull));
                     }
-                    if (t < 6) TRACE(1, 8 + 8 * t + 4);
+                    if (traced) TRACE(1, 8 + 8 * t + 4);
                     if (more) {
-                        if (!(ok = warp_wait<false>(bar(kDoFull + (t + 1) % C::kDoStages),
-                                                ((t + 1) / C::kDoStages) & 1, abort_flag))) break;
-                        if (t < 6) TRACE(1, 8 + 8 * t + 5);
-                        if (kWithDq && D == 128) {  // dP(t+1) reuses the dQ(t) columns
-                            if (!(ok = warp_wait<false>(bar(kDqEmpty), t & 1, abort_flag))) break;
+                        if (!(ok = wait_do(g + 1))) break;
+                        if (traced) TRACE(1, 8 + 8 * t + 5);
+                        if (kWithDq && D == 128) {  // dP of the next step reuses the dQ columns
+                            if (!(ok = warp_wait<false>(bar(kDqEmpty), g & 1, abort_flag))) break;
                         }
-                        if (t < 6) TRACE(1, 8 + 8 * t + 6);
+                        if (traced) TRACE(1, 8 + 8 * t + 6);
                         ptx::tc_fence_after();
-                        issue_dp(t + 1);
-                        if (t < 6) TRACE(1, 8 + 8 * t + 7);
+                        issue_dp(g + 1);
+                        if (traced) TRACE(1, 8 + 8 * t + 7);
                     }
                 }
-                if (ok) ptx::tc_commit_elect(bar(kDkvFull));
-                TRACE(1, 62);
+                if (!ok) break;
+                if (n_steps > 0) ptx::tc_commit_elect(bar(kDkvFull));
+                if (n == 0) TRACE(1, 62);
+                g0 += n_steps;
+                next = next_tile(n, &w);
             }
-        }
-        else if (!idle && warp == 2) {
+        } else if (warp == 2) {
             // ============================================== row statistics
             // One warp fetches the statistics of the next step's 128 query rows while the math warps work and
             // hands them over in shared memory, two steps deep.  (A softmax warpgroup that fetched its own spent
@@ -611,11 +693,9 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             // of the sequence gets -inf, which makes its P, and with it dS, exactly zero.
             // The statistics come from the delta kernel, which may still be running (programmatic launch); Q, K,
             // V, dO are inputs of the call, so the TMA and MMA warps did not have to wait.
-            ptx::grid_dependency_wait();
-            if (!kWithDq) ptx::launch_dependents();
             float* stats = reinterpret_cast<float*>(smem + C::kOffStats);
             float neg[4], ndel[4];
-            auto fetch = [&](const StepWalk<kCausal>& st) {
+            auto fetch = [&](const FusedWork& w, const StepWalk<kCausal>& st) {
                 const int64_t row0 = int64_t(w.b_coord * a.heads_q + st.hq) * a.sidecar_rows + w.q_base;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -634,22 +714,76 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     }
                 }
             };
-            StepWalk<kCausal> st(w);
-            fetch(st);
+            if (lane == 0) {
+                ptx::prefetch_tensormap(&tm_k);
+                ptx::prefetch_tensormap(&tm_v);
+                ptx::prefetch_tensormap(&tm_q);
+                ptx::prefetch_tensormap(&tm_do);
+            }
+            __syncwarp();
+            set_up_done();
+            FusedWork w = first_tile();
+            ptx::grid_dependency_wait();
+            if (!kWithDq) ptx::launch_dependents();
+            uint32_t n = 0;
+            int g = 0;
+            bool ok = true;
 #pragma unroll 1
-            for (int t = 0; t < n_steps; ++t) {
-                const int buf = t & 1;
-                if (!warp_wait(bar(kStatsEmpty + buf), ((t >> 1) & 1) ^ 1, abort_flag)) break;
+            for (bool more = !misaligned; more; ++n) {
+                StepWalk<kCausal> st(w);
+                if (w.n_steps > 0) fetch(w, st);
+#pragma unroll 1
+                for (int t = 0; t < w.n_steps; ++t, ++g) {
+                    const int buf = g & 1;
+                    if (!(ok = warp_wait(bar(kStatsEmpty + buf), ((g >> 1) & 1) ^ 1, abort_flag))) break;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    stats[buf * 128 + k * 32 + lane] = neg[k];
-                    stats[256 + buf * 128 + k * 32 + lane] = ndel[k];
+                    for (int k = 0; k < 4; ++k) {
+                        stats[buf * 128 + k * 32 + lane] = neg[k];
+                        stats[256 + buf * 128 + k * 32 + lane] = ndel[k];
+                    }
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(bar(kStatsFull + buf));
+                    if (t + 1 < w.n_steps) {
+                        st.next(w);
+                        fetch(w, st);
+                    }
                 }
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(bar(kStatsFull + buf));
-                if (t + 1 < n_steps) {
-                    st.next(w);
-                    fetch(st);
+                if (!ok) break;
+                more = next_tile(n, &w);
+            }
+        } else {
+            // ================================================== which tile next
+            {
+                const FusedWork w = fused_work<kCausal>(a, int(blockIdx.x));
+                if (lane == 0) store_work(work, w);
+            }
+            set_up_done();
+            if (kPersist && !misaligned) {
+#pragma unroll 1
+                for (uint32_t n = 0, answers = 0;; ++n) {  // the work of tile n + 1
+                    const uint32_t buf = (n + 1) & 1;
+                    FusedWork w;
+                    bool ok;
+                    while ((ok = warp_wait(bar(kAnswer), answers & 1, abort_flag))) {
+                        ++answers;
+                        const int block = ptx::answered_block(answer);
+                        ptx::fence_proxy_async_smem();  // (it is written through the async proxy again)
+                        if (block >= 0) w = fused_work<kCausal>(a, block);
+                        w.block = block;
+                        // (packed sequences: the grid is sized for the longest one, and many blocks have no rows)
+                        if (block < 0 || w.kt * C::kTile < w.slot_k) break;
+                        __syncwarp();
+                        if (lane == 0) {
+                            ptx::mbar_arrive_expect_tx(bar(kAnswer), 16);
+                            ptx::request_block(answer, bar(kAnswer));
+                        }
+                    }
+                    // (that of tile n - 1 has been read)
+                    if (!ok || (n >= 1 && !warp_wait(bar(kWorkEmpty + buf), ((n - 1) >> 1) & 1, abort_flag))) break;
+                    if (lane == 0) store_work(work + 128 * buf, w);
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(bar(kWorkFull + buf));
+                    if (w.block < 0) break;
                 }
             }
         }
@@ -658,11 +792,10 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         if (!kWithDq) ptx::setmaxnreg_inc<C::kRegsComputeNoDq>();
         else if (C::kRegsCompute < 128) ptx::setmaxnreg_dec<C::kRegsCompute>();
         else ptx::setmaxnreg_inc<C::kRegsCompute>();
-        const FusedWork w = fused_work<kCausal>(a);
-        const uint32_t tmem = set_up_done();
-        const bool idle = misaligned || w.n_steps == 0;  // a CTA without work: set-up and teardown still run
-        const int n_steps = w.n_steps;
-        if (!idle) {
+        set_up_done();
+        const uint32_t tmem = flag_value(tmem_slot);
+        FusedWork w = first_tile();
+        {
             const int half = wg - 1;          // which 64 queries of the tile
             const int j = threadIdx.x & 127;  // key row inside the tile == TMEM lane
             const uint32_t tl = tmem + (uint32_t((warp & 3) * 32) << 16);
@@ -680,16 +813,21 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 if (lane == 0) ptx::mbar_arrive(bar(which));
             };
             bool ok = true;
+            uint32_t n = 0, used = 0;
+            int g = 0;  // step, counted over all tiles
+#pragma unroll 1
+            for (bool more = !misaligned; more; ++n) {
             StepWalk<kCausal> st(w);
 #pragma unroll 1
-            for (int t = 0; t < n_steps; ++t, st.next(w)) {
-                if (warp == 4 && t == 3) TRACE(2, 0);
+            for (int t = 0; t < w.n_steps; ++t, ++g, st.next(w)) {
+                const bool traced = warp == 4 && n == 0 && t < 7;
+                if (traced && t == 3) TRACE(2, 0);
                 const int qt = st.qt;
-                const int buf = t & 1;
+                const int buf = g & 1;
                 const uint32_t negp = stats + buf * 512;
                 const uint32_t delp = stats + 1024 + buf * 512;
-                if (!(ok = warp_wait2(bar(kStatsFull + buf), (t >> 1) & 1, bar(kSFull), t & 1, abort_flag))) break;
-                if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 1);
+                if (!(ok = warp_wait2(bar(kStatsFull + buf), (g >> 1) & 1, bar(kSFull), g & 1, abort_flag))) break;
+                if (traced) TRACE(2, 4 + 8 * t + 1);
                 ptx::tc_fence_after();
                 // A tile that crosses an edge of the w.band or holds keys past the end of the sequence is
                 // masked: element (key j, query i) survives iff mask_from <= i <= mask_to.
@@ -765,16 +903,16 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 } else {
                     softmax_phase(std::false_type{});
                 }
-                if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 2);
+                if (traced) TRACE(2, 4 + 8 * t + 2);
                 ptx::tmem_st_wait();
                 arrive(kPReady);
-                if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 3);
+                if (traced) TRACE(2, 4 + 8 * t + 3);
                 // ---- dS^T = P^T * (dP^T - delta_i), stored [key][query] in the 128-byte swizzle
-                if (!(ok = warp_wait(bar(kDpFull), t & 1, abort_flag))) break;
-                if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 4);
-                // (the dS buffer is free: dP(t) was issued behind dK(t-1), dQ(t-1), the readers of dS(t-1),
+                if (!(ok = warp_wait(bar(kDpFull), g & 1, abort_flag))) break;
+                if (traced) TRACE(2, 4 + 8 * t + 4);
+                // (the dS buffer is free: dP was issued behind dK and dQ of the step before, the readers of its dS,
                 // and the barrier just passed completes only when every MMA issued before it has)
-                if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 5);
+                if (traced) TRACE(2, 4 + 8 * t + 5);
                 ptx::tc_fence_after();
                 const uint32_t ds_row = sbase + C::kOffDS + half * C::kBoxBytes + j * 128;
                 auto ds_chunk = [&](int c, const uint32_t* r) {
@@ -806,63 +944,79 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     ptx::tmem_ld_wait();
                     ds_chunk(c, r);
                 }
-                if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 6);
+                if (traced) TRACE(2, 4 + 8 * t + 6);
                 ptx::fence_proxy_async_smem();
                 arrive(kDsReady);
                 if (lane == 0) ptx::mbar_arrive(bar(kStatsEmpty + buf));
-                if (warp == 4 && t < 7) TRACE(2, 4 + 8 * t + 7);
+                if (traced) TRACE(2, 4 + 8 * t + 7);
             }
             // ---- epilogue: the first warpgroup writes dK (scaled), the second dV
-            if (ok) ok = warp_wait(bar(kDkvFull), 0, abort_flag);
-            if (warp == 4) TRACE(2, 60);
-            if (ok) {
-                // Every MMA has completed, so the Q / dO / dS^T buffers are dead.  Each warp stages its 32 key rows
-                // there and stores them again in whole lines, 512 contiguous bytes (or two rows) per instruction.
-                // (Stores through the copy engine queue behind the drain's last reduce-adds, about 2700 clk at D=128;
-                // a thread storing its own row straight from registers writes 16 bytes per line and instruction.)
+            if (!ok) break;
+            const int w4 = warp & 3;  // which 32 rows of the tile
+            const bool has_steps = w.n_steps > 0;
+            const int64_t slab = int64_t(w.slab * 2 + half) * (C::kTile * D) + w4 * 32 * D;
+            const int rows = w.slot_k - (w.kt * C::kTile + w4 * 32);
+            // (rows between the used length and the end of the slot hold exact zeros)
+            TOut* out = reinterpret_cast<TOut*>(half == 0 ? a.dk : a.dv) + w.b_coord * a.kv_strides.batch +
+                        w.kvh * a.kv_strides.head + int64_t(w.k_base + w.kt * C::kTile + w4 * 32) * a.kv_strides.row;
+            more = next_tile(n, &w);  // (while the last MMAs of this one run)
+            if (has_steps && !(ok = warp_wait(bar(kDkvFull), used & 1, abort_flag))) break;
+            if (warp == 4 && n == 0) TRACE(2, 60);
+            if (has_steps) {
+                // Every MMA of the tile has completed.  Each warp stages its 32 key rows in shared memory and stores them again in
+                // whole lines: over the dead Q / dO / dS^T buffers, 512 contiguous bytes (or two rows) per instruction, or, where
+                // the next tile's Q and dO are being loaded, over its own rows of dS^T, 128 bytes of each row at a time.
+                // (Stores through the copy engine queue behind the drain's last reduce-adds, about 2700 clk at D=128; a thread
+                // storing its own row straight from registers writes 16 bytes per line and instruction.)
+                ++used;
                 ptx::tc_fence_after();
                 const float mul = half == 0 ? a.scale : 1.0f;
                 const uint32_t col0 = tl + (half == 0 ? C::kColDK : C::kColDV);
-                const int w4 = warp & 3;  // which 32 rows of the tile
-                // rows of element type O at dst, `pitch` elements apart, of which the first `rows` are written
-                auto store_rows = [&](auto tag, void* dst_rows, int64_t pitch, int rows) {
+                // rows of element type O at dst, `pitch` elements apart, of which the first `rows_here` are written
+                auto store_rows = [&](auto tag, void* dst_rows, int64_t pitch, int rows_here) {
                     using O = decltype(tag);
-                    constexpr int kRowBytes = D * int(sizeof(O));
-                    constexpr int kChunks = kRowBytes / 16;
+                    constexpr int kPass = kPersist ? 128 : D * int(sizeof(O));  // bytes of a row
+                    constexpr int kCols = kPass / int(sizeof(O));
+                    constexpr int kChunks = kPass / 16;
                     constexpr int kPerLoad = 32 * int(sizeof(O)) / 16;  // 16-byte chunks of 32 columns
-                    const uint32_t scratch = sbase + C::kOffQ + (half * 4 + w4) * (32 * kRowBytes);
-#pragma unroll
-                    for (int c = 0; c < D / 32; ++c) {
-                        uint32_t r[32];
-                        ptx::tmem_ld32(col0 + c * 32, r);
-                        ptx::tmem_ld_wait();
-#pragma unroll
-                        for (int e = 0; e < kPerLoad; ++e) {
-                            uint32_t o[4];
-#pragma unroll
-                            for (int h = 0; h < 4; ++h) {
-                                if constexpr (sizeof(O) == 4) {
-                                    o[h] = __float_as_uint(__uint_as_float(r[4 * e + h]) * mul);
-                                } else {
-                                    o[h] = ptx::Pack2<O>::pack(__uint_as_float(r[8 * e + 2 * h]) * mul, __uint_as_float(r[8 * e + 2 * h + 1]) * mul);
-                                }
-                            }
-                            const int chunk = (c * kPerLoad + e) ^ (lane & 7);  // (spread over the banks)
-                            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
-                                         ::"r"(scratch + lane * kRowBytes + chunk * 16), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-                        }
-                    }
-                    __syncwarp();
-                    constexpr int kRowsPerPass = 32 / kChunks;  // 1, 2 or 4
+                    constexpr int kRowsAtOnce = 32 / kChunks;
+                    const uint32_t scratch = sbase + (kPersist ? C::kOffDS + half * C::kBoxBytes + w4 * 32 * kPass
+                                                               : C::kOffQ + (half * 4 + w4) * 32 * kPass);
                     const int sub = lane / kChunks, ch = lane % kChunks;
                     O* dst = static_cast<O*>(dst_rows) + ch * (16 / int(sizeof(O)));
+#pragma unroll 1
+                    for (int col = 0; col < D; col += kCols) {
+#pragma unroll
+                        for (int c = 0; c < kCols / 32; ++c) {
+                            uint32_t r[32];
+                            ptx::tmem_ld32(col0 + col + c * 32, r);
+                            ptx::tmem_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < kPerLoad; ++e) {
+                                uint32_t o[4];
+#pragma unroll
+                                for (int h = 0; h < 4; ++h) {
+                                    if constexpr (sizeof(O) == 4) {
+                                        o[h] = __float_as_uint(__uint_as_float(r[4 * e + h]) * mul);
+                                    } else {
+                                        o[h] = ptx::Pack2<O>::pack(__uint_as_float(r[8 * e + 2 * h]) * mul, __uint_as_float(r[8 * e + 2 * h + 1]) * mul);
+                                    }
+                                }
+                                const int chunk = (c * kPerLoad + e) ^ (lane & 7);  // (spread over the banks)
+                                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                                             ::"r"(scratch + lane * kPass + chunk * 16), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+                            }
+                        }
+                        __syncwarp();
 #pragma unroll 8
-                    for (int row = sub; row < 32; row += kRowsPerPass) {
-                        uint4 v;
-                        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                                     : "r"(scratch + row * kRowBytes + ((ch ^ (row & 7)) << 4)) : "memory");
-                        if (row < rows) *reinterpret_cast<uint4*>(dst + row * pitch) = v;
+                        for (int row = sub; row < 32; row += kRowsAtOnce) {
+                            uint4 v;
+                            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                                         : "r"(scratch + row * kPass + ((ch ^ (row & 7)) << 4)) : "memory");
+                            if (row < rows_here) *reinterpret_cast<uint4*>(dst + row * pitch + col) = v;
+                        }
+                        __syncwarp();
                     }
                 };
                 if (kWithDq && a.chunk_steps > 0) {
@@ -870,26 +1024,20 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     // fp16 for fp16 inputs where the tiles are fewer than the SMs: the bytes written, not the arithmetic,
                     // bound this epilogue.  (With as many tiles as SMs, fp16 slabs had taken dK and dV, whose sums stay in
                     // tensor memory when their tile is not split, 1.16 and 1.23 times as far from the exact values.)
-                    const int64_t first = int64_t(w.slab * 2 + half) * (C::kTile * D) + w4 * 32 * D;
-                    if (!kBf16 && a.slabs_f16) store_rows(__half{}, static_cast<__half*>(a.dkv_slabs) + first, D, 32);
-                    else store_rows(float{}, static_cast<float*>(a.dkv_slabs) + first, D, 32);
+                    if (!kBf16 && a.slabs_f16) store_rows(__half{}, static_cast<__half*>(a.dkv_slabs) + slab, D, 32);
+                    else store_rows(float{}, static_cast<float*>(a.dkv_slabs) + slab, D, 32);
                 } else {
-                    // (rows between the used length and the end of the slot hold exact zeros)
-                    TOut* dst = reinterpret_cast<TOut*>(half == 0 ? a.dk : a.dv) + w.b_coord * a.kv_strides.batch +
-                                w.kvh * a.kv_strides.head + int64_t(w.k_base + w.kt * C::kTile + w4 * 32) * a.kv_strides.row;
-                    store_rows(TOut{}, dst, a.kv_strides.row, w.slot_k - (w.kt * C::kTile + w4 * 32));
+                    store_rows(TOut{}, out, a.kv_strides.row, rows);
+                }
+            } else if (a.chunk_steps == 0) {
+                // nobody attends to these keys (possible with a left-bounded window), but dK / dV still owe zeros
+                if (lane < rows) {
+                    uint4* d4 = reinterpret_cast<uint4*>(out + lane * a.kv_strides.row);
+#pragma unroll
+                    for (int e = 0; e < int(D * sizeof(TOut) / 16); ++e) d4[e] = make_uint4(0u, 0u, 0u, 0u);
                 }
             }
-            if (warp == 4) TRACE(2, 61);
-        } else if (!misaligned && a.chunk_steps == 0) {
-            // nobody attends to these keys (possible with a left-bounded window), but dK / dV still owe zeros: the first warpgroup clears dK, the second dV
-            const int j = threadIdx.x & 127;
-            if (w.kt * C::kTile + j < w.slot_k) {
-                const int64_t off = w.b_coord * a.kv_strides.batch + w.kvh * a.kv_strides.head +
-                                    int64_t(w.k_base + w.kt * C::kTile + j) * a.kv_strides.row;
-                uint4* d4 = reinterpret_cast<uint4*>(reinterpret_cast<TOut*>(wg == 1 ? a.dk : a.dv) + off);
-#pragma unroll
-                for (int e = 0; e < int(D * sizeof(TOut) / 16); ++e) d4[e] = make_uint4(0u, 0u, 0u, 0u);
+            if (warp == 4 && n == 0) TRACE(2, 61);
             }
         }
     } else {
@@ -899,24 +1047,29 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             set_up_done();
         } else {
             ptx::setmaxnreg_inc<C::kRegsDrain>();
-            const FusedWork w = fused_work<kCausal>(a);
-            const uint32_t tmem = set_up_done();
-            const bool idle = misaligned || w.n_steps == 0;  // a CTA without work: set-up and teardown still run
-            const int n_steps = w.n_steps;
-            if (!idle) {
+            set_up_done();
+            const uint32_t tmem = flag_value(tmem_slot);
+            FusedWork w = first_tile();
+            {
                 const int qd = warp & 3;
                 const uint32_t tl = tmem + (uint32_t(qd * 32) << 16);
                 const uint32_t stage = sbase + C::kOffStage + qd * 2 * C::kStageBoxBytes;
                 bool pending = false;
                 // the accumulators are cleared by the delta kernel: do not add into them before it is done
                 ptx::grid_dependency_wait();
+                bool ok = true;
+                uint32_t n = 0;
+                int g = 0;
+#pragma unroll 1
+                for (bool more = !misaligned; more; ++n) {
                 StepWalk<kCausal> st(w);
 #pragma unroll 1
-                for (int t = 0; t < n_steps; ++t, st.next(w)) {
+                for (int t = 0; t < w.n_steps; ++t, ++g, st.next(w)) {
+                    const bool traced = warp == 12 && n == 0 && t < 12;
                     const int q_row = st.qt * C::kTile + qd * 32;  // row inside the head
                     const int q_head = w.b_coord * a.heads_q + st.hq;
-                    if (!warp_wait(bar(kDqFull), t & 1, abort_flag)) break;
-                    if (warp == 12 && t < 12) TRACE(3, 4 + 4 * t + 0);
+                    if (!(ok = warp_wait(bar(kDqFull), g & 1, abort_flag))) break;
+                    if (traced) TRACE(3, 4 + 4 * t + 0);
                     ptx::tc_fence_after();
                     // pull the whole dQ tile row into registers and hand the columns back at once
                     uint32_t r[D / 32][32];
@@ -926,7 +1079,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     ptx::tc_fence_before();
                     __syncwarp();
                     if (lane == 0) ptx::mbar_arrive(bar(kDqEmpty));
-                    if (warp == 12 && t < 12) TRACE(3, 4 + 4 * t + 1);
+                    if (traced) TRACE(3, 4 + 4 * t + 1);
 #pragma unroll
                     for (int hf = 0; hf < D / 64; ++hf) {
                         if (pending) {
@@ -955,7 +1108,10 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                         }
                         pending = true;
                     }
-                    if (warp == 12 && t < 12) TRACE(3, 4 + 4 * t + 2);
+                    if (traced) TRACE(3, 4 + 4 * t + 2);
+                }
+                if (!ok) break;
+                more = next_tile(n, &w);
                 }
                 if (lane == 0) ptx::bulk_wait_group<0>();
                 if (warp == 12) TRACE(3, 59);

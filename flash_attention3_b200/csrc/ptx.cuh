@@ -315,6 +315,23 @@ __device__ __forceinline__ void launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Taking over the work of a block that has not started (a running block asks for the index of one; the block that had it is
+// never launched).  The answer, 16 bytes in shared memory, is counted by the barrier; after a refusal nothing more is asked.
+__device__ __forceinline__ void request_block(uint32_t answer, uint32_t bar) {
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(answer), "r"(bar) : "memory");
+}
+// blockIdx.x of the block taken over, -1 for a refusal.
+__device__ __forceinline__ int answered_block(uint32_t answer) {
+    uint32_t taken, x;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\tld.shared.b128 r, [%2];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\tselp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, r;\n\t}"
+        : "=r"(taken), "=r"(x) : "r"(answer) : "memory");
+    return taken != 0 ? int(x) : -1;
+}
+
 // Thread-block clusters.
 // All threads of all CTAs of the cluster; shared-memory writes before it are visible to the peers after it.
 __device__ __forceinline__ void cluster_sync() {

@@ -20,14 +20,16 @@ CASES = [
 ]
 
 
+@pytest.mark.parametrize("deterministic", [False, True])
 @pytest.mark.parametrize("b,hq,hkv,sq,sk,d,dtype,causal,layout,window", CASES)
-def test_tiles_taken_over(b, hq, hkv, sq, sk, d, dtype, causal, layout, window):
+def test_tiles_taken_over(b, hq, hkv, sq, sk, d, dtype, causal, layout, window, deterministic):
     from tests.helpers import Problem, assert_parity, run_v2
     prob = Problem(b, hq, hkv, sq, d, dtype, causal, seed=31 + sq + sk, sk=sk, layout=layout, window=window)
-    first = run_v2(prob)
+    first = run_v2(prob, deterministic=deterministic)
     assert_parity(first, prob, label=f"{(b, hq, hkv, sq, sk, d, dtype, causal, layout, window)}")
     for _ in range(3):
-        again = run_v2(prob)
+        again = run_v2(prob, deterministic=deterministic)
+        assert not deterministic or np.array_equal(again["dq"], first["dq"])
         assert np.array_equal(again["dk"], first["dk"]) and np.array_equal(again["dv"], first["dv"])
 
 

@@ -312,15 +312,18 @@ struct alignas(16) FusedWork {
     int t_begin, n_steps; // this CTA's share of the tile's steps (all of them unless the tile is split)
     int rotation;
 };
-static_assert(sizeof(FusedWork) == 96, "six 16-byte words");
-__device__ __forceinline__ void store_work(uint32_t addr, const FusedWork& w) {
+// (the forward's work, too)
+template <typename W>
+__device__ __forceinline__ void store_work(uint32_t addr, const W& w) {
+    static_assert(sizeof(W) == 96, "six 16-byte words");
     const uint32_t* v = reinterpret_cast<const uint32_t*>(&w);
 #pragma unroll
     for (int i = 0; i < 24; i += 4)
         asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr + 4 * i), "r"(v[i]), "r"(v[i + 1]), "r"(v[i + 2]), "r"(v[i + 3]) : "memory");
 }
-__device__ __forceinline__ FusedWork load_work(uint32_t addr) {
-    FusedWork w;
+template <typename W = FusedWork>
+__device__ __forceinline__ W load_work(uint32_t addr) {
+    W w;
     uint32_t* v = reinterpret_cast<uint32_t*>(&w);
 #pragma unroll
     for (int i = 0; i < 24; i += 4)
@@ -557,12 +560,6 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                                              bar(kDoFull + sd), bx * 64, q_row, hq, w.b_coord);
                         }
                     }
-                    // Asks for the next tile, as late as it does not hold that up: tiles are to go to the CTAs in the order in
-                    // which these become free.  (Warp 3 has used the answer before this one.)
-                    if (kPersist) {
-                        ptx::mbar_arrive_expect_tx(bar(kAnswer), 16);
-                        ptx::request_block(answer, bar(kAnswer));
-                    }
                 }
                 __syncwarp();
                 g0 += w.n_steps;
@@ -600,12 +597,27 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(tmem + C::kColDP, loV_k, loDO, kIdSdP, 0);
                 ptx::tc_commit_elect(bar(kDpFull));
             };
+            // Asks for the next tile, in front of the last dK and dQ of this one: late enough that tiles go to the CTAs in the order in
+            // which these become free, early enough that its K and V, which wait for those MMAs, are there when dK and dV are
+            // stored.  (Warp 3 has used the answer before.  Asked for when the last Q and dO were requested, one or two steps
+            // earlier: us, causal, 80 heads x 512, D=128 45.3 and 44.4, B=8, 32 x 300 84.2 and 80.9, packed 9 x 2048, 16 heads 277 and 271;
+            // full, 80 x 512 56.3 and 57.1; with a mask at D=64 slower than one CTA per tile, now faster.)
+            auto request = [&] {
+                if constexpr (kPersist) {
+                    if (lane == 0) {
+                        ptx::mbar_arrive_expect_tx(bar(kAnswer), 16);
+                        ptx::request_block(answer, bar(kAnswer));
+                    }
+                    __syncwarp();
+                }
+            };
             uint32_t n = 0, used = 0;
             int g0 = 0;
             bool ok = true;
 #pragma unroll 1
             for (bool next = !misaligned; next; ++n) {
                 const int n_steps = w.n_steps;
+                if (n_steps == 0) request();
                 if (n_steps > 0) {
                     ok = warp_wait<false>(bar(kKvFull), used & 1, abort_flag) && wait_q(g0);
                     if (n == 0) TRACE(1, 1);
@@ -651,6 +663,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     // dK += dS^T Q
                     if (!(ok = warp_wait<false>(bar(kDsReady), g & 1, abort_flag))) break;
                     if (traced) TRACE(1, 8 + 8 * t + 3);
+                    if (!more) request();
                     ptx::tc_fence_after();
                     {
                         const uint32_t loQ = ptx::desc_lo_mn_major(sQ(g), C::kBoxBytes);

@@ -87,8 +87,11 @@ struct FwdCfg {
     static constexpr int kOffV = kOffK + kStages * kOperandBytes;
     static constexpr int kOffMerge = kOffK;                          // split: [2 tiles][128 rows][D] fp32 over the dead rings
     static constexpr int kOffStats = kOffV + kStages * kOperandBytes;  // split: [2 tiles][128 rows] {m, l}
-    static constexpr int kOffBar = kOffStats + 2 * 128 * 8;
-    static constexpr int kSmemBytes = kOffBar + 256;
+    static constexpr int kOffOut = kOffStats + 2 * 128 * 8;            // tiles taken over: [8 warps][32 rows][64 columns] of O
+    static constexpr int kOffBar = kOffOut + 8 * 4096;
+    static constexpr int kOffWork = kOffBar + 288;                   // two buffers
+    static constexpr int kSmemBytes = kOffWork + 256;
+    static_assert(kOffOut % 1024 == 0, "swizzled region");
     static_assert(kSmemBytes <= 232448, "shared-memory ledger exceeds 227 KiB");
     static_assert(2 * 128 * D * 4 <= kOffStats - kOffMerge, "partial outputs do not fit over the rings");
     // P in columns of its own where they are free (D=64): the scores of the next key tile are then computed
@@ -124,11 +127,16 @@ enum FwdBar : int {
     kFwdPReady = 20,  // per query tile: all of P is written
     kFwdPvDone = 22,  // per query tile
     kFwdAllDone = 24, // every MMA of the CTA has completed
-    kFwdNum = 25,
+    kFwdAnswer = 25,     // tiles taken over, as in the backward: which block comes next
+    kFwdWorkFull = 26,   // 2 buffers
+    kFwdWorkEmpty = 28,  // 2 buffers
+    kFwdQEmpty = 30,     // per query tile: its last scores have been computed
+    kFwdNum = 32,
 };
 
-// Which query tiles and keys a CTA works on.
-struct FwdWork {
+// Which query tiles and keys a CTA works on.  One warp works it out and hands it to the others in shared memory.
+struct alignas(16) FwdWork {
+    int block;           // place in the launch order, -1: there is none
     int rank, hq, kvh, b, b_coord, q_base, k_base;
     int tile[2];         // query tiles A and B
     int slot_q;          // rows of out this batch entry owns
@@ -139,13 +147,13 @@ struct FwdWork {
     __device__ __forceinline__ bool active(int x, int it) const { return it >= lo[x] && it < hi[x]; }
 };
 
-// (Each role works this out for itself behind its setmaxnreg: values carried across a change of the register
-// budget were spilled.)
+// (behind grid_dependency_wait)
 template <bool kMasked>
-__device__ __forceinline__ FwdWork fwd_work(const FwdArgs& a) {
+__device__ __forceinline__ FwdWork fwd_work(const FwdArgs& a, int block) {
     FwdWork w;
-    const int unit = int(blockIdx.x) >> a.split_shift;
-    w.rank = int(blockIdx.x) & (a.splits - 1);        // == rank in the cluster
+    w.block = block;
+    const int unit = block >> a.split_shift;
+    w.rank = block & (a.splits - 1);        // == rank in the cluster
     const int slot = fast_div(unit, a.bh);
     // heaviest query tiles (most visible keys) are launched first (packed: of the longest sequence)
     const TilePair tiles = tile_pair_of_slot(slot, tiles_of(a.band.seqlen_q), kMasked, kMasked && a.fold);
@@ -155,7 +163,6 @@ __device__ __forceinline__ FwdWork fwd_work(const FwdArgs& a) {
     w.b = fast_div(bhi, a.heads);
     w.hq = bhi - w.b * a.heads_q;
     w.kvh = fast_div(w.hq, a.group);
-    ptx::grid_dependency_wait();
     // packed sequences: this batch entry's own lengths and first rows
     Band band = a.band;
     w.q_base = w.k_base = 0;
@@ -276,7 +283,9 @@ __device__ __forceinline__ void fwd_merge(const FwdArgs& a, const FwdWork& w, ui
 }
 
 // kSoftcap: the scaled scores go through softcap * tanh(x / softcap) before the softmax.
-template <typename T, int D, bool kMasked, bool kSoftcap = false>
+// kPersist: CTAs take over the tiles of CTAs that have not started (no clusters).  K, V and Q of the next tile are loaded and its
+// first scores computed beside the output of this one, which is staged in a region of its own.
+template <typename T, int D, bool kMasked, bool kSoftcap = false, bool kPersist = false>
 __global__ void __launch_bounds__(384, 1)
 fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
            const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
@@ -300,6 +309,26 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         if (first_tile * C::kTile >= a.cu_seqlens_q[entry + 1] - a.cu_seqlens_q[entry]) return;
     }
 
+    const uint32_t answer = sbase + C::kOffBar + 272;
+    static_assert(8 * kFwdNum + 8 <= 272, "barriers, then the answer");
+    const uint32_t work = sbase + C::kOffWork;
+    // (a converged warp) the first tile, and the tile after this one; n: how many this CTA has done before
+    auto first_tile = [&]() -> FwdWork {
+        const FwdWork w = load_work<FwdWork>(work);
+        __syncwarp();
+        if (kPersist && lane == 0) ptx::mbar_arrive(bar(kFwdWorkEmpty));
+        return w;
+    };
+    auto next_tile = [&](uint32_t n, FwdWork* w) -> bool {
+        if (!kPersist) return false;
+        const uint32_t buf = (n + 1) & 1;
+        if (!warp_wait<false>(bar(kFwdWorkFull + buf), (n >> 1) & 1, abort_flag)) return false;
+        *w = load_work<FwdWork>(work + 128 * buf);
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(bar(kFwdWorkEmpty + buf));
+        return w->block >= 0;
+    };
+
     // Set-up first: launched programmatically, it overlaps the end of the kernel in front, which
     // grid_dependency_wait() below waits for before any of its outputs is read.
     const bool misaligned = (sbase & 1023u) != 0;
@@ -312,6 +341,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             ptx::mbar_init(bar(kFwdPFirst + x), 4);
             ptx::mbar_init(bar(kFwdPReady + x), 4);
             ptx::mbar_init(bar(kFwdPvDone + x), 1);
+            ptx::mbar_init(bar(kFwdQEmpty + x), 1);
         }
         for (int s = 0; s < C::kStages; ++s) {
             ptx::mbar_init(bar(kFwdKFull + s), 1);
@@ -320,6 +350,11 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             ptx::mbar_init(bar(kFwdVEmpty + s), 1);
         }
         ptx::mbar_init(bar(kFwdAllDone), 1);
+        ptx::mbar_init(bar(kFwdAnswer), 1);
+        for (int s = 0; s < 2; ++s) {
+            ptx::mbar_init(bar(kFwdWorkFull + s), 1);
+            ptx::mbar_init(bar(kFwdWorkEmpty + s), 10);  // producer, MMA issuer, softmax warps
+        }
         flag_set(abort_flag, 0);
         ptx::fence_mbar_init();
     }
@@ -334,8 +369,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     }
     ptx::launch_dependents();
 
-    // (all threads: barriers initialised, tensor memory allocated)
+    // (all threads: barriers initialised, tensor memory allocated, first tile known)
     auto set_up_done = [&] {
+        ptx::grid_dependency_wait();
         ptx::tc_fence_before();
         asm volatile("bar.sync 0;" ::: "memory");
         ptx::tc_fence_after();
@@ -346,52 +382,77 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
     // which code runs under which budget)
     if (warp < 4) {
         ptx::setmaxnreg_dec<C::kRegsControl>();
-        const FwdWork w = fwd_work<kMasked>(a);
+        if (warp == 2) {
+            ptx::grid_dependency_wait();
+            const FwdWork w = fwd_work<kMasked>(a, int(blockIdx.x));
+            if (lane == 0) store_work(work, w);
+            __syncwarp();
+        }
         const uint32_t tmem = set_up_done();
-        const int n_iter = w.n_iter;
         if (misaligned) {
             // nothing to do
         } else if (warp == 0) {
             // TMA producer, converged like the MMA issuer
-            if (n_iter > 0) {
+            FwdWork w = first_tile();
+            uint32_t n = 0;
+            int g0 = 0, used[2] = {0, 0};  // iterations of the tiles before; how often Q of either query tile was loaded
+            bool ok = true;
+#pragma unroll 1
+            for (bool more = true; ok && more; ++n) {
+                auto load_k = [&](int it) {
+                    const int g = g0 + it, s = g % C::kStages;
+                    if (!warp_wait(bar(kFwdKEmpty + s), ((g / C::kStages) & 1) ^ 1, abort_flag)) return false;
+                    ptx::tma_load_tile_elect<C::kBoxes>(sbase + C::kOffK + s * C::kOperandBytes, &tm_k, bar(kFwdKFull + s),
+                                                        w.k_base + (w.t_begin + it) * C::kTile, w.kvh, w.b_coord);
+                    return true;
+                };
+                auto load_v = [&](int it) {
+                    const int g = g0 + it, s = g % C::kStages;
+                    if (!warp_wait(bar(kFwdVEmpty + s), ((g / C::kStages) & 1) ^ 1, abort_flag)) return false;
+                    ptx::tma_load_tile_elect<C::kBoxes>(sbase + C::kOffV + s * C::kOperandBytes, &tm_v, bar(kFwdVFull + s),
+                                                        w.k_base + (w.t_begin + it) * C::kTile, w.kvh, w.b_coord);
+                    return true;
+                };
+                if (n > 0 && w.n_iter > 0) ok = load_k(0);
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    if (w.lo[x] >= w.hi[x]) continue;  // nothing is loaded for a tile that sees no key
-                    ptx::tma_load_tile_elect<C::kBoxes>(sbase + C::kOffQ + x * C::kOperandBytes, &tm_q, bar(kFwdQFull + x),
-                                                        w.q_base + w.tile[x] * C::kTile, w.hq, w.b_coord);
+                    if (w.lo[x] >= w.hi[x] || !ok) continue;  // nothing is loaded for a tile that sees no key
+                    if (used[x] > 0) ok = warp_wait(bar(kFwdQEmpty + x), (used[x] - 1) & 1, abort_flag);
+                    if (ok) ptx::tma_load_tile_elect<C::kBoxes>(sbase + C::kOffQ + x * C::kOperandBytes, &tm_q, bar(kFwdQFull + x),
+                                                                w.q_base + w.tile[x] * C::kTile, w.hq, w.b_coord);
+                    ++used[x];
                 }
 #pragma unroll 1
-                for (int it = 0; it < n_iter; ++it) {
-                    const int s = it % C::kStages;
-                    const uint32_t wait_parity = ((it / C::kStages) & 1) ^ 1;
-                    const int kv_row = w.k_base + (w.t_begin + it) * C::kTile;
-                    if (!warp_wait(bar(kFwdKEmpty + s), wait_parity, abort_flag)) break;
-                    ptx::tma_load_tile_elect<C::kBoxes>(sbase + C::kOffK + s * C::kOperandBytes, &tm_k, bar(kFwdKFull + s), kv_row, w.kvh, w.b_coord);
-                    if (!warp_wait(bar(kFwdVEmpty + s), wait_parity, abort_flag)) break;
-                    ptx::tma_load_tile_elect<C::kBoxes>(sbase + C::kOffV + s * C::kOperandBytes, &tm_v, bar(kFwdVFull + s), kv_row, w.kvh, w.b_coord);
-                }
+                for (int it = 0; ok && it < w.n_iter; ++it) ok = ((n > 0 && it == 0) || load_k(it)) && load_v(it);
+                if (!ok) break;
+                g0 += w.n_iter;
+                more = next_tile(n, &w);
             }
         } else if (warp == 1) {
             // MMA issuer: the whole warp runs the role converged; the issue forms and the commits elect their
             // lane inside the asm.
             constexpr uint32_t kIdS = ptx::instr_desc_f16(kBf16, 128, 128, false, false);
             constexpr uint32_t kIdO = ptx::instr_desc_f16(kBf16, 128, D, false, true);
+            FwdWork w = first_tile();
+            uint32_t n = 0;
+            int g0 = 0, c[2] = {0, 0}, used[2] = {0, 0};  // ... and how often Q of either query tile was loaded
             // S of query tile x against the key tile of iteration `it`
             auto issue_s = [&](int x, int it) {
                 const uint32_t loQ = ptx::desc_lo_k_major(sbase + C::kOffQ + x * C::kOperandBytes);
-                const uint32_t loK = ptx::desc_lo_k_major(sbase + C::kOffK + (it % C::kStages) * C::kOperandBytes);
+                const uint32_t loK = ptx::desc_lo_k_major(sbase + C::kOffK + ((g0 + it) % C::kStages) * C::kOperandBytes);
                 const uint32_t dst = tmem + C::kColS + x * 128;
                 ptx::mma_ss<D / 16, ptx::KMajor, ptx::KMajor>(dst, loQ, loK, kIdS, 0);
                 ptx::tc_commit_elect(bar(kFwdSFull + x));
+                if (kPersist && it == w.hi[x] - 1) ptx::tc_commit_elect(bar(kFwdQEmpty + x));
             };
-            auto wait_k = [&](int it) { return warp_wait<false>(bar(kFwdKFull + it % C::kStages), (it / C::kStages) & 1, abort_flag); };
-            auto wait_v = [&](int it) { return warp_wait<false>(bar(kFwdVFull + it % C::kStages), (it / C::kStages) & 1, abort_flag); };
+            auto wait_k = [&](int it) { return warp_wait<false>(bar(kFwdKFull + (g0 + it) % C::kStages), ((g0 + it) / C::kStages) & 1, abort_flag); };
+            auto wait_v = [&](int it) { return warp_wait<false>(bar(kFwdVFull + (g0 + it) % C::kStages), ((g0 + it) / C::kStages) & 1, abort_flag); };
             // O of query tile x += P V of iteration `it`: on the first part of P as soon as it is there, then on the rest
             auto issue_pv = [&](int x, int it) {
-                const uint32_t loV = ptx::desc_lo_mn_major(sbase + C::kOffV + (it % C::kStages) * C::kOperandBytes, C::kBoxBytes);
+                const uint32_t loV = ptx::desc_lo_mn_major(sbase + C::kOffV + ((g0 + it) % C::kStages) * C::kOperandBytes, C::kBoxBytes);
                 const uint32_t p_cols = tmem + C::kColP + x * C::kPStride;
                 const uint32_t o_cols = tmem + C::kColO + x * D;
-                const uint32_t parity = (it - w.lo[x]) & 1;
+                const uint32_t parity = (c[x] + it - w.lo[x]) & 1;
                 const uint32_t accumulate = it > w.lo[x] ? 1u : 0u;
                 if (!warp_wait<false>(bar(kFwdPFirst + x), parity, abort_flag)) return false;
                 ptx::tc_fence_after();
@@ -402,24 +463,52 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 ptx::tc_commit_elect(bar(kFwdPvDone + x));
                 return true;
             };
-            bool ok = n_iter > 0;
+            // (own P) the scores in front of those of iteration `it` are in registers
+            auto wait_s_free = [&](int x, int it) {
+                const int before = c[x] + it - w.lo[x];
+                return before == 0 || warp_wait<false>(bar(kFwdSFree + x), (before - 1) & 1, abort_flag);
+            };
+            // Asks for the next tile, in front of the last P V of this one: late enough that tiles go to the CTAs in the order in
+            // which these become free, early enough that its K and V are there when this one's output is.  (Warp 2 has used
+            // the answer before.)
+            auto request = [&] {
+                if constexpr (kPersist) {
+                    if (lane == 0) {
+                        ptx::mbar_arrive_expect_tx(bar(kFwdAnswer), 16);
+                        ptx::request_block(answer, bar(kFwdAnswer));
+                    }
+                    __syncwarp();
+                }
+            };
+            bool ok = true;
+#pragma unroll 1
+            for (bool next = true; ok && next; ++n) {
+            const int n_iter = w.n_iter;
+            if (n_iter == 0) request();
 #pragma unroll
             for (int x = 0; x < 2; ++x) {
-                if (ok && w.lo[x] < w.hi[x]) ok = warp_wait<false>(bar(kFwdQFull + x), 0, abort_flag);
+                if (ok && w.lo[x] < w.hi[x]) ok = warp_wait<false>(bar(kFwdQFull + x), used[x]++ & 1, abort_flag);
             }
-            if (ok) ok = wait_k(0);
-            if (ok) {
+            if (ok && n_iter > 0) ok = wait_k(0);
+            if (ok && n_iter > 0) {
                 ptx::tc_fence_after();
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    if (w.active(x, 0)) issue_s(x, 0);
+                    if (ok && w.active(x, 0)) {
+                        if (C::kOwnP) {
+                            ok = wait_s_free(x, 0);
+                            ptx::tc_fence_after();
+                        }
+                        if (ok) issue_s(x, 0);
+                    }
                 }
-                ptx::tc_commit_elect(bar(kFwdKEmpty + 0));
+                ptx::tc_commit_elect(bar(kFwdKEmpty + g0 % C::kStages));
             }
             if constexpr (!C::kOwnP) {
 #pragma unroll 1
                 for (int it = 0; ok && it < n_iter; ++it) {
                     const bool more = it + 1 < n_iter;
+                    if (!more) request();
                     bool v_ready = false, k_ready = false;
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
@@ -441,20 +530,20 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                         }
                     }
                     if (!ok) break;
-                    if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + (it + 1) % C::kStages));
-                    ptx::tc_commit_elect(bar(kFwdVEmpty + it % C::kStages));
+                    if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + (g0 + it + 1) % C::kStages));
+                    ptx::tc_commit_elect(bar(kFwdVEmpty + (g0 + it) % C::kStages));
                 }
             } else {
                 // S(x, it+1) needs only "scores (x, it) in registers"; P V of tile B is issued one half
                 // iteration late, because the two softmax warpgroups settle half an iteration apart
 #pragma unroll 1
-                for (int it = 0; ok && it <= n_iter; ++it) {
+                for (int it = 0; ok && n_iter > 0 && it <= n_iter; ++it) {
                     const bool more = it + 1 < n_iter;
+                    if (it == n_iter - 1) request();
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
                         if (more && w.active(x, it + 1)) {
-                            // (its first key tile has no scores in front of it)
-                            if (w.active(x, it)) ok = warp_wait<false>(bar(kFwdSFree + x), (it - w.lo[x]) & 1, abort_flag);
+                            ok = wait_s_free(x, it + 1);
                             if (!(ok = ok && wait_k(it + 1))) break;
                             ptx::tc_fence_after();
                             issue_s(x, it + 1);
@@ -465,13 +554,47 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                         if (pv < n_iter && w.active(y, pv)) {
                             if (!(ok = wait_v(pv) && issue_pv(y, pv))) break;
                         }
-                        if (x == 0 && it > 0) ptx::tc_commit_elect(bar(kFwdVEmpty + (it - 1) % C::kStages));
+                        if (x == 0 && it > 0) ptx::tc_commit_elect(bar(kFwdVEmpty + (g0 + it - 1) % C::kStages));
                     }
                     if (!ok) break;
-                    if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + (it + 1) % C::kStages));
+                    if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + (g0 + it + 1) % C::kStages));
                 }
             }
-            if (ok) ptx::tc_commit_elect(bar(kFwdAllDone));
+            if (!ok) break;
+            if (n_iter > 0) ptx::tc_commit_elect(bar(kFwdAllDone));  // (waited for with one tile per CTA)
+            g0 += n_iter;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) c[x] += max(0, w.hi[x] - w.lo[x]);
+            next = next_tile(n, &w);
+            }
+        } else if (warp == 2 && kPersist) {
+            // which tile next
+#pragma unroll 1
+            for (uint32_t n = 0, answers = 0;; ++n) {  // the work of tile n + 1
+                const uint32_t buf = (n + 1) & 1;
+                FwdWork w;
+                bool ok;
+                while ((ok = warp_wait(bar(kFwdAnswer), answers & 1, abort_flag))) {
+                    ++answers;
+                    const int block = ptx::answered_block(answer);
+                    ptx::fence_proxy_async_smem();  // (it is written through the async proxy again)
+                    if (block >= 0) w = fwd_work<kMasked>(a, block);
+                    w.block = block;
+                    // (packed sequences: blocks without rows)
+                    if (block < 0 || min(w.tile[0], w.tile[1]) * C::kTile < w.slot_q) break;
+                    __syncwarp();
+                    if (lane == 0) {
+                        ptx::mbar_arrive_expect_tx(bar(kFwdAnswer), 16);
+                        ptx::request_block(answer, bar(kFwdAnswer));
+                    }
+                }
+                // (that of tile n - 1 has been read)
+                if (!ok || (n >= 1 && !warp_wait(bar(kFwdWorkEmpty + buf), ((n - 1) >> 1) & 1, abort_flag))) break;
+                if (lane == 0) store_work(work + 128 * buf, w);
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(bar(kFwdWorkFull + buf));
+                if (w.block < 0) break;
+            }
         }
         if (a.splits > 1) {  // (the softmax warps meet their peers around the merge)
             __syncwarp();
@@ -480,7 +603,6 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         }
     } else {
         ptx::setmaxnreg_inc<C::kRegsSoftmax>();
-        const FwdWork w = fwd_work<kMasked>(a);
         const uint32_t tmem = set_up_done();
         if (misaligned) {
             if (a.splits > 1) {
@@ -490,6 +612,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
         } else {
             const int x = (warp - 4) >> 2;      // which query tile
             const int i = threadIdx.x & 127;    // query row inside the tile == TMEM lane
+            FwdWork w = first_tile();
+            uint32_t n = 0;
+            int c0 = 0;  // steps of the tiles before
+            bool more = true;
+#pragma unroll 1
+            for (; more; ++n) {
             const int qt = x == 0 ? w.tile[0] : w.tile[1];
             const int n_steps = x == 0 ? w.hi[0] - w.lo[0] : w.hi[1] - w.lo[1];  // (selects, not indexing: no local array)
             const int k_begin = w.t_begin + (x == 0 ? w.lo[0] : w.lo[1]);
@@ -515,7 +643,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             bool ok = true;
 #pragma unroll 1
             for (int u = 0; u < n_steps; ++u) {
-                if (!(ok = warp_wait<false>(bar(kFwdSFull + x), u & 1, abort_flag))) break;
+                if (!(ok = warp_wait<false>(bar(kFwdSFull + x), (c0 + u) & 1, abort_flag))) break;
                 ptx::tc_fence_after();
                 const bool diagonal = kMasked && __any_sync(0xffffffffu, mask_from > 0 || mask_to < C::kTile - 1);
                 // ---- the whole score row of this tile goes to registers in one round trip
@@ -523,7 +651,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
 #pragma unroll
                 for (int c = 0; c < 4; ++c) ptx::tmem_ld32(s_cols + c * 32, r[c]);
                 // (asked ahead of its use: has P V of the previous key tile completed?)
-                const bool p_free = !C::kOwnP || u == 0 || ptx::mbar_test_wait(bar(kFwdPvDone + x), (u - 1) & 1);
+                const bool p_free = !C::kOwnP || u == 0 || ptx::mbar_test_wait(bar(kFwdPvDone + x), (c0 + u - 1) & 1);
                 ptx::tmem_ld_wait();
                 if (C::kOwnP) arrive(kFwdSFree);
                 if (kSoftcap) {
@@ -577,7 +705,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                     if (u > 0) {
                         // O carries the old reference: wait for P V of step u-1, then rescale these 32 rows (16
                         // columns at a time: the score row is still held in registers)
-                        if (!(ok = warp_wait<false>(bar(kFwdPvDone + x), (u - 1) & 1, abort_flag))) break;
+                        if (!(ok = warp_wait<false>(bar(kFwdPvDone + x), (c0 + u - 1) & 1, abort_flag))) break;
                         ptx::tc_fence_after();
 #pragma unroll 1
                         for (int c = 0; c < D / 16; ++c) {
@@ -595,7 +723,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 // has been read by now, where P has no columns of its own)
                 if (C::kOwnP) {
                     // P of the previous key tile must have been used before it is overwritten
-                    if (!__all_sync(0xffffffffu, p_free) && !(ok = warp_wait<false>(bar(kFwdPvDone + x), (u - 1) & 1, abort_flag))) break;
+                    if (!__all_sync(0xffffffffu, p_free) && !(ok = warp_wait<false>(bar(kFwdPvDone + x), (c0 + u - 1) & 1, abort_flag))) break;
                     ptx::tc_fence_after();
                 }
                 const float neg = m_ref == -INFINITY ? 0.0f : -m_ref * sl;
@@ -637,7 +765,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             const float inv = any_key ? 1.0f / l : 0.0f;
             // ln(sum exp(s*scale)) = (m_ref*scale_log2 + log2 l) * ln 2
             float* lse_dst = a.lse + int64_t(w.b_coord * a.heads_q + w.hq) * a.lse_rows + w.q_base + qi;
-            if (a.splits > 1) {
+            if (!kPersist && a.splits > 1) {
                 // This CTA's share of the keys: unnormalised O, fp32, and {m in log2 units, l} go to shared
                 // memory, over the K / V rings, for the merge below.
                 if (ok && w.n_iter > 0) ok = warp_wait(bar(kFwdAllDone), 0, abort_flag);
@@ -662,7 +790,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                     }
                 }
             } else {
-            if (ok && n_steps > 0) ok = warp_wait(bar(kFwdPvDone + x), (n_steps - 1) & 1, abort_flag);
+            if (ok && n_steps > 0) ok = warp_wait(bar(kFwdPvDone + x), (c0 + n_steps - 1) & 1, abort_flag);
             T* dst = reinterpret_cast<T*>(a.out) + w.b_coord * a.o_strides.batch + w.hq * a.o_strides.head +
                      int64_t(w.q_base + qi) * a.o_strides.row;
             if (ok && ((q_valid && n_steps == 0) || (!q_valid && qi < w.slot_q))) {
@@ -682,14 +810,19 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                     // through shared memory (the Q tile is dead: its last S completed before this O) and the copy
                     // engine: whole lines instead of 16 bytes of 32 rows per instruction, rows past the end clipped
                     const int w4 = warp & 3;
-                    const uint32_t stage = sbase + C::kOffQ + x * C::kOperandBytes + w4 * (C::kBoxes * 4096);
+                    const uint32_t stage = kPersist ? sbase + C::kOffOut + (x * 4 + w4) * 4096 : sbase + C::kOffQ + x * C::kOperandBytes + w4 * (C::kBoxes * 4096);
+                    const bool in_range = qt * C::kTile + w4 * 32 < w.slot_q;
                     const float scale_row = q_valid ? inv : 0.0f;  // (rows behind a used length hold zeros)
 #pragma unroll
                     for (int c = 0; c < D / 32; ++c) {
                         uint32_t r[32];
                         ptx::tmem_ld32(o_cols + c * 32, r);
                         ptx::tmem_ld_wait();
-                        const uint32_t row_addr = stage + (c >> 1) * 4096 + lane * 128;
+                        const uint32_t row_addr = stage + (kPersist ? 0 : c >> 1) * 4096 + lane * 128;
+                        if (kPersist && (c & 1) == 0) {  // (its 64 columns before have been read)
+                            if (lane == 0) ptx::bulk_wait_group_read<0>();
+                            __syncwarp();
+                        }
 #pragma unroll
                         for (int e = 0; e < 4; ++e) {
                             uint32_t o[4];
@@ -702,15 +835,25 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                             asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
                                          ::"r"(row_addr + (chunk << 4)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
                         }
+                        if (kPersist && (c & 1) == 1) {
+                            ptx::fence_proxy_async_smem();
+                            __syncwarp();
+                            if (lane == 0 && in_range) {
+                                ptx::tma_store_4d(&tm_o, stage, (c >> 1) * 64, qt * C::kTile + w4 * 32, w.hq, w.b);
+                                ptx::bulk_commit_group();
+                            }
+                        }
                     }
+                    if (!kPersist) {
                     ptx::fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0 && qt * C::kTile + w4 * 32 < w.slot_q) {
+                    if (lane == 0 && in_range) {
 #pragma unroll
                         for (int bx = 0; bx < C::kBoxes; ++bx)
                             ptx::tma_store_4d(&tm_o, stage + bx * 4096, bx * 64, qt * C::kTile + w4 * 32, w.hq, w.b);
                         ptx::bulk_commit_group();
                         ptx::bulk_wait_group_read<0>();
+                    }
                     }
                 } else {
 #pragma unroll
@@ -735,7 +878,12 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 }
             }
             }
-            if (a.splits > 1) {
+            if (kPersist) {
+                __syncwarp();
+                if (!ok) break;
+                c0 += max(0, n_steps);
+            }
+            if (!kPersist && a.splits > 1) {
                 // ---- merge of the cluster's shares: every CTA finishes 256 / splits of the w.pair's rows, reading
                 // the partial outputs of all peers through distributed shared memory
                 __syncwarp();
@@ -746,6 +894,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 __syncwarp();
                 ptx::cluster_sync();  // the peers read this CTA's shared memory until here
             }
+            more = next_tile(n, &w);
+            }
+            if (kPersist && lane == 0) ptx::bulk_wait_group_read<0>();  // (shared memory is not given back before)
         }
     }
 

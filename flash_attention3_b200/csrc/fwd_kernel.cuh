@@ -30,13 +30,16 @@
 // after: B=4, H=16, S=4096 full, D=64 567 and 823, D=128 930-990 and 1155-1170 (there the power limit holds the
 // clock near 1.6 GHz); B=2, Hq=32, Hkv=8, S=8192 causal, D=128 857 and 1063.
 //
+// With at least two pairs of query tiles per SM (kPersist) CTAs take over the pairs of CTAs that have not started, as in the
+// backward; the rule and what it measured stand beside the launch.
+//
 // When the pairs are too few to fill the GPU a cluster of 2, 4 or 8 CTAs shares the key tiles of a pair
 // (plan_fwd) and merges the partial outputs through distributed shared memory.
 //
 // Tensor-memory ledger: S_A [0,128)  S_B [128,256)  O_A [256,256+D)  O_B [256+D,256+2D); at D=64 also
 // P_A [384,448)  P_B [448,512).
 // Shared-memory ledger: Q_A, Q_B resident (2 x D*256), K and V rings of two stages (D=128) or three (D=64),
-// partial row statistics 2 KiB, mbarriers 256: 198,912 bytes at D=128, 133,376 at D=64.
+// partial row statistics 2 KiB, O of a pair taken over 32 KiB, mbarriers 288, work of a pair 256: 231,968 bytes at D=128, 166,432 at D=64.
 #pragma once
 
 #include <cuda.h>

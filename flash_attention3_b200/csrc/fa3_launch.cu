@@ -657,10 +657,11 @@ struct FwdLaunch {
 template <typename T, int D, bool kMasked, bool kSoftcap = false, bool kPersist = false>
 int launch_fwd_t(const FwdLaunch& L, cudaStream_t st) {
     auto kernel = fwd_kernel<T, D, kMasked, kSoftcap, kPersist>;
+    constexpr int kSmem = kPersist ? FwdCfg<D>::kSmemBytesPersist : FwdCfg<D>::kSmemBytes;
     static DeviceOnce configured;
     if (!configured.done()) {
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 FwdCfg<D>::kSmemBytes) != cudaSuccess) {
+                                 kSmem) != cudaSuccess) {
             return SHAOBO_FA3_STATUS_HIP_ERROR;
         }
         configured.mark();
@@ -668,7 +669,7 @@ int launch_fwd_t(const FwdLaunch& L, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(L.blocks));
     cfg.blockDim = dim3(FwdCfg<D>::kThreads);
-    cfg.dynamicSmemBytes = FwdCfg<D>::kSmemBytes;
+    cfg.dynamicSmemBytes = kSmem;
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // set-up overlaps the kernel in front

@@ -39,7 +39,8 @@
 // Tensor-memory ledger: S_A [0,128)  S_B [128,256)  O_A [256,256+D)  O_B [256+D,256+2D); at D=64 also
 // P_A [384,448)  P_B [448,512).
 // Shared-memory ledger: Q_A, Q_B resident (2 x D*256), K and V rings of two stages (D=128) or three (D=64),
-// partial row statistics 2 KiB, O of a pair taken over 32 KiB, mbarriers 288, work of a pair 256: 231,968 bytes at D=128, 166,432 at D=64.
+// partial row statistics 2 KiB, mbarriers 288, work of a pair 256: 199,200 bytes at D=128, 133,664 at D=64; with pairs taken over
+// 32 KiB more for their O: 232,448 and 166,912.
 #pragma once
 
 #include <cuda.h>
@@ -90,12 +91,13 @@ struct FwdCfg {
     static constexpr int kOffV = kOffK + kStages * kOperandBytes;
     static constexpr int kOffMerge = kOffK;                          // split: [2 tiles][128 rows][D] fp32 over the dead rings
     static constexpr int kOffStats = kOffV + kStages * kOperandBytes;  // split: [2 tiles][128 rows] {m, l}
-    static constexpr int kOffOut = kOffStats + 2 * 128 * 8;            // tiles taken over: [8 warps][32 rows][64 columns] of O
-    static constexpr int kOffBar = kOffOut + 8 * 4096;
+    static constexpr int kOffBar = kOffStats + 2 * 128 * 8;
     static constexpr int kOffWork = kOffBar + 288;                   // two buffers
+    static constexpr int kOffOut = kOffBar + 1024;                   // tiles taken over: [8 warps][32 rows][64 columns] of O
     static constexpr int kSmemBytes = kOffWork + 256;
+    static constexpr int kSmemBytesPersist = kOffOut + 8 * 4096;
     static_assert(kOffOut % 1024 == 0, "swizzled region");
-    static_assert(kSmemBytes <= 232448, "shared-memory ledger exceeds 227 KiB");
+    static_assert(kSmemBytesPersist <= 232448, "shared-memory ledger exceeds 227 KiB");
     static_assert(2 * 128 * D * 4 <= kOffStats - kOffMerge, "partial outputs do not fit over the rings");
     // P in columns of its own where they are free (D=64): the scores of the next key tile are then computed
     // while the exponentials of this one are, because the score columns are free once they are in registers

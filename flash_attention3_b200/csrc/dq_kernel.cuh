@@ -271,7 +271,7 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     delta = a.delta[stat_row];
                 }
             }
-            uint32_t ppk[32];  // what dP - delta is multiplied with, in 16 bits: P, or, capped, P (1 - t^2)
+            uint32_t ppk[kSoftcap ? 48 : 32];  // what dP - delta is multiplied with: P in 16 bits, or, capped, P (1 - t^2) in 24 (pack24)
             const uint64_t scale2 = ptx::f2_pack(a.scale_log2, a.scale_log2);
             const uint64_t post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
             const uint64_t neg2 = ptx::f2_pack(neg, neg), ndel2 = ptx::f2_pack(-delta, -delta);
@@ -296,6 +296,7 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     ptx::tmem_ld32(s_cols + c * 32, r);
                     ptx::tmem_ld_wait();
                     auto softmax_chunk = [&](auto small_tag) {
+                        float slope_p[4];
 #pragma unroll
                         for (int e = 0; e < 32; e += 2) {
                             const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
@@ -314,7 +315,13 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                                 p.x = (j + 0 >= mask_from && j + 0 <= mask_to) ? p.x : 0.0f;
                                 p.y = (j + 1 >= mask_from && j + 1 <= mask_to) ? p.y : 0.0f;
                             }
-                            ppk[c * 16 + e / 2] = ptx::Pack2<T>::pack(p.x, p.y);
+                            if constexpr (kSoftcap) {
+                                slope_p[e & 2] = p.x;
+                                slope_p[(e & 2) + 1] = p.y;
+                                if ((e & 2) != 0) ptx::pack24(slope_p, &ppk[c * 24 + e / 4 * 3]);
+                            } else {
+                                ppk[c * 16 + e / 2] = ptx::Pack2<T>::pack(p.x, p.y);
+                            }
                         }
                     };
                     if constexpr (kSoftcap) {
@@ -333,9 +340,13 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     ptx::tmem_ld32(dp_cols + c * 32, r);
                     ptx::tmem_ld_wait();
                     uint32_t o[16];
+                    float slope_p[4];
 #pragma unroll
                     for (int e = 0; e < 32; e += 2) {
-                        const float2 p = ptx::Pack2<T>::unpack(ppk[c * 16 + e / 2]);
+                        if constexpr (kSoftcap) {
+                            if ((e & 2) == 0) ptx::unpack24(&ppk[c * 24 + e / 4 * 3], slope_p);
+                        }
+                        const float2 p = kSoftcap ? make_float2(slope_p[e & 2], slope_p[(e & 2) + 1]) : ptx::Pack2<T>::unpack(ppk[c * 16 + e / 2]);
                         const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
                         const float2 ds = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, ndel2)));
                         o[e / 2] = ptx::Pack2<T>::pack(ds.x, ds.y);

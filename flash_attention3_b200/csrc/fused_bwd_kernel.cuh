@@ -426,7 +426,10 @@ struct StepWalk {
 // false turns the kernel into the four-GEMM dK/dV half of the split path.
 // kPersist: CTAs take over the tiles of CTAs that have not started (see above).
 // kSoftcap: softcapped scores (general form only).  dS then carries the slope 1 - t^2 of the cap, t the tanh: the second
-// softmax phase needs P only in that product, so P (1 - t^2) is what it is handed in registers, in P's place.
+// softmax phase needs P only in that product, so P (1 - t^2) is what it is handed in registers, in P's place.  In 24 bits: P itself
+// rounds to 16 almost exactly in a row that few keys dominate, and the product does not, nor does fp16 hold it where the
+// scores are far above the cap (S=8192, D=128, cap 15, scores of spread 40, fp16: dQ 9.8e-4 from exact with 16 bits, 3.1e-4 so;
+// 130 and 134 us, B=1, Hq=16, Hkv=8, S=4096, D=128, window 1024, cap 30).
 template <typename T, int D, bool kCausal, bool kWithDq, typename TOut, bool kSoftcap = false, bool kPersist = false>
 __global__ void __launch_bounds__(512, 1)
 fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -818,7 +821,8 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const uint64_t scale2 = ptx::f2_pack(a.scale_log2, a.scale_log2);
             const uint64_t post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
             const float small_score = kSoftcap ? ptx::kTanhPolyMax / fabsf(a.softcap_pre) : 0.0f;
-            uint32_t ppk[32];  // what dP - delta is multiplied with, in 16 bits: P, or P (1 - t^2)
+            // what dP - delta is multiplied with: P as it is handed to the MMA, in 16 bits, or P (1 - t^2), in 24 (pack24)
+            uint32_t ppk[kSoftcap ? 48 : 32];
             // one arrival per warp: every lane's accesses are ordered before it by the fence and the warp barrier
             auto arrive = [&](int which) {
                 ptx::tc_fence_before();
@@ -853,6 +857,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     uint32_t capped_p[16];  // P where ppk holds P (1 - t^2)
 #pragma unroll
                     for (int e = 0; e < 32; e += 4) {
+                        float slope_p[4];
                         const ptx::F4Pairs n4 = ptx::f2_ld_shared(negp + (c * 32 + e) * 4);
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
@@ -886,11 +891,13 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                             }
                             if constexpr (kSoftcap) {
                                 capped_p[el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
-                                ppk[c * 16 + el / 2] = ptx::Pack2<T>::pack(w2.x, w2.y);
+                                slope_p[2 * h] = w2.x;
+                                slope_p[2 * h + 1] = w2.y;
                             } else {
                                 ppk[c * 16 + el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
                             }
                         }
+                        if constexpr (kSoftcap) ptx::pack24(slope_p, &ppk[c * 24 + e / 4 * 3]);
                     }
                     // P chunk c -> columns [16c, 16c+16) of this half's S columns (already read)
                     if constexpr (kSoftcap) ptx::tmem_st16(s_cols + c * 16, capped_p);
@@ -936,9 +943,11 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                         for (int h = 0; h < 2; ++h) {
                             const ptx::F4Pairs d4 = ptx::f2_ld_shared(delp + (c * 32 + e + 4 * h) * 4);  // -delta
                             const int el = e + 4 * h;
+                            float slope_p[4];
+                            if constexpr (kSoftcap) ptx::unpack24(&ppk[c * 24 + el / 4 * 3], slope_p);
 #pragma unroll
                             for (int g = 0; g < 2; ++g) {
-                                const float2 p = ptx::Pack2<T>::unpack(ppk[c * 16 + el / 2 + g]);
+                                const float2 p = kSoftcap ? make_float2(slope_p[2 * g], slope_p[2 * g + 1]) : ptx::Pack2<T>::unpack(ppk[c * 16 + el / 2 + g]);
                                 const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[el + 2 * g]), __uint_as_float(r[el + 2 * g + 1]));
                                 const float2 ds = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, g == 0 ? d4.lo : d4.hi)));
                                 o[2 * h + g] = ptx::Pack2<T>::pack(ds.x, ds.y);

@@ -503,6 +503,24 @@ __device__ __forceinline__ bool all_small(const uint32_t* s, float limit) {
     return max_nan(top[0], top[1]) <= limit;
 }
 
+// Four fp32 values in three registers, the upper 24 bits of each (15 bits of significand, to within 2^-15 and without a bias: the
+// byte that is missing is taken to be like the one above it, which keeps 0, infinities and NaN as they are).
+__device__ __forceinline__ uint32_t byte_perm(uint32_t a, uint32_t b, uint32_t selector) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(selector));
+    return d;
+}
+__device__ __forceinline__ void pack24(const float* v, uint32_t* o) {
+    const uint32_t last = __float_as_uint(v[3]);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) o[i] = byte_perm(__float_as_uint(v[i]), last, 0x3215u + i);
+}
+__device__ __forceinline__ void unpack24(const uint32_t* o, float* v) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) v[i] = __uint_as_float(byte_perm(o[i], 0u, 0x3211u));
+    v[3] = __uint_as_float(byte_perm(byte_perm(o[0], o[1], 0x0400u), o[2], 0x4211u));
+}
+
 template <typename T>
 struct Pack2;
 template <>

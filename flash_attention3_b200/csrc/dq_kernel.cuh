@@ -77,6 +77,7 @@ struct DqCfg {
     static constexpr int kColS = 0;
     static constexpr int kColDP = 128;
     static constexpr int kColDQ = 256;
+    static constexpr int kTanhFmaPairs = 5;  // capped scores: as in the five-GEMM kernel
 };
 
 enum DqBar : int {
@@ -275,7 +276,7 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             const uint64_t scale2 = ptx::f2_pack(a.scale_log2, a.scale_log2);
             const uint64_t post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
             const uint64_t neg2 = ptx::f2_pack(neg, neg), ndel2 = ptx::f2_pack(-delta, -delta);
-            const float small_score = kSoftcap ? ptx::kTanhPolyMax / fabsf(a.softcap_pre) : 0.0f;
+            const uint64_t pre2 = ptx::f2_pack(a.softcap_pre * ptx::kTanhArg, a.softcap_pre * ptx::kTanhArg);
             auto arrive = [&](int which) {
                 ptx::tc_fence_before();
                 __syncwarp();
@@ -295,40 +296,32 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     uint32_t r[32];
                     ptx::tmem_ld32(s_cols + c * 32, r);
                     ptx::tmem_ld_wait();
-                    auto softmax_chunk = [&](auto small_tag) {
-                        float slope_p[4];
+                    float slope_p[4];
 #pragma unroll
-                        for (int e = 0; e < 32; e += 2) {
-                            const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
-                            uint64_t t2 = 0;
-                            if constexpr (kSoftcap) t2 = ptx::tanh_score<decltype(small_tag)::value>(s2, a.softcap_pre, small_score);
-                            float2 p = ptx::f2_unpack(kSoftcap ? ptx::f2_fma(t2, post2, neg2) : ptx::f2_fma(s2, scale2, neg2));
-                            p.x = ptx::ex2_approx(p.x);
-                            p.y = ptx::ex2_approx(p.y);
-                            if constexpr (kSoftcap) {
-                                const float2 tt = ptx::f2_unpack(t2);
-                                p = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y),
-                                                               ptx::f2_pack(fmaf(-tt.x, tt.x, 1.0f), fmaf(-tt.y, tt.y, 1.0f))));
-                            }
-                            if (diagonal) {
-                                const int j = c * 32 + e;
-                                p.x = (j + 0 >= mask_from && j + 0 <= mask_to) ? p.x : 0.0f;
-                                p.y = (j + 1 >= mask_from && j + 1 <= mask_to) ? p.y : 0.0f;
-                            }
-                            if constexpr (kSoftcap) {
-                                slope_p[e & 2] = p.x;
-                                slope_p[(e & 2) + 1] = p.y;
-                                if ((e & 2) != 0) ptx::pack24(slope_p, &ppk[c * 24 + e / 4 * 3]);
-                            } else {
-                                ppk[c * 16 + e / 2] = ptx::Pack2<T>::pack(p.x, p.y);
-                            }
+                    for (int e = 0; e < 32; e += 2) {
+                        const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
+                        uint64_t t2 = 0;
+                        if constexpr (kSoftcap) t2 = ptx::tanh_mixed<C::kTanhFmaPairs>(ptx::f2_mul(s2, pre2), e / 2);
+                        float2 p = ptx::f2_unpack(kSoftcap ? ptx::f2_fma(t2, post2, neg2) : ptx::f2_fma(s2, scale2, neg2));
+                        p.x = ptx::ex2_approx(p.x);
+                        p.y = ptx::ex2_approx(p.y);
+                        if constexpr (kSoftcap) {
+                            const float2 tt = ptx::f2_unpack(t2);
+                            p = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y),
+                                                           ptx::f2_pack(fmaf(-tt.x, tt.x, 1.0f), fmaf(-tt.y, tt.y, 1.0f))));
                         }
-                    };
-                    if constexpr (kSoftcap) {
-                        if (__all_sync(0xffffffffu, ptx::all_small<32>(r, small_score))) softmax_chunk(std::true_type{});
-                        else softmax_chunk(std::false_type{});
-                    } else {
-                        softmax_chunk(std::false_type{});
+                        if (diagonal) {
+                            const int j = c * 32 + e;
+                            p.x = (j + 0 >= mask_from && j + 0 <= mask_to) ? p.x : 0.0f;
+                            p.y = (j + 1 >= mask_from && j + 1 <= mask_to) ? p.y : 0.0f;
+                        }
+                        if constexpr (kSoftcap) {
+                            slope_p[e & 2] = p.x;
+                            slope_p[(e & 2) + 1] = p.y;
+                            if ((e & 2) != 0) ptx::pack24(slope_p, &ppk[c * 24 + e / 4 * 3]);
+                        } else {
+                            ppk[c * 16 + e / 2] = ptx::Pack2<T>::pack(p.x, p.y);
+                        }
                     }
                 }
                 arrive(kDqbSFree);

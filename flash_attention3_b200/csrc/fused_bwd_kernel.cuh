@@ -161,7 +161,7 @@ __host__ __device__ inline int remap_k_tile(int physical, int count, int mode, i
     return base + ((round & 1) == 0 ? slot : span - 1 - slot);
 }
 
-template <int D>
+template <int D, bool kSoftcap = false>
 struct FusedCfg {
     static constexpr int kTile = 128;
     static constexpr int kThreads = 512;
@@ -190,13 +190,18 @@ struct FusedCfg {
     static_assert(kSmemBytes <= 232448, "shared-memory ledger exceeds 227 KiB");
     static_assert(kOffStage % 1024 == 0 && kOffDS % 1024 == 0, "swizzled regions need 1 KiB alignment");
 
-    // setmaxnreg split per warpgroup (producer+MMA / softmax x2 / drain); sums to <= 512
-    static constexpr int kRegsControl = 96;
-    static constexpr int kRegsCompute = D == 128 ? 120 : 136;
-    static constexpr int kRegsDrain = D == 128 ? 176 : 136;
+    // setmaxnreg split per warpgroup (producer+MMA / softmax x2 / drain); sums to <= 512.  (Capped scores hold P (1 - t^2) in 48
+    // registers instead of P in 32.)
+    static constexpr int kRegsControl = kSoftcap && D == 128 ? 80 : 96;
+    static constexpr int kRegsCompute = (D == 128 ? 120 : 136) + (kSoftcap ? 8 : 0);
+    static constexpr int kRegsDrain = D == 128 ? 176 : kSoftcap ? 128 : 136;
     static constexpr int kRegsComputeNoDq = 160;  // without dQ the drain warpgroup idles at kRegsControl
     static_assert(kRegsControl + 2 * kRegsCompute + kRegsDrain <= 512, "register file over-committed");
     static_assert(2 * kRegsControl + 2 * kRegsComputeNoDq <= 512, "register file over-committed");
+
+    // Capped scores: of every 8 pairs of tanh, how many go to the FMA pipe (tanh_mixed).  us of the first gradients named there for 2,
+    // 3, 4, 5, 8 of 8: 144, 141, 140, 140, 147; of the last 352, 339, 335, 328, 340.
+    static constexpr int kTanhFmaPairs = 5;
 
     static constexpr int kTmemCols = 512;
     static constexpr int kColDK = 0;
@@ -429,13 +434,13 @@ struct StepWalk {
 // softmax phase needs P only in that product, so P (1 - t^2) is what it is handed in registers, in P's place.  In 24 bits: P itself
 // rounds to 16 almost exactly in a row that few keys dominate, and the product does not, nor does fp16 hold it where the
 // scores are far above the cap (S=8192, D=128, cap 15, scores of spread 40, fp16: dQ 9.8e-4 from exact with 16 bits, 3.1e-4 so;
-// 130 and 134 us, B=1, Hq=16, Hkv=8, S=4096, D=128, window 1024, cap 30).
+// 130 and 134 us, B=1, Hq=16, Hkv=8, S=4096, D=128, window 1024, cap 30, with the tanh as it was then).
 template <typename T, int D, bool kCausal, bool kWithDq, typename TOut, bool kSoftcap = false, bool kPersist = false>
 __global__ void __launch_bounds__(512, 1)
 fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                  const __grid_constant__ CUtensorMap tm_dqacc, const __grid_constant__ FusedArgs a) {
-    using C = FusedCfg<D>;
+    using C = FusedCfg<D, kSoftcap>;
     constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = ptx::smem_u32(smem);
@@ -807,7 +812,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         // ============================================ softmax / dS warpgroups
         if (!kWithDq) ptx::setmaxnreg_inc<C::kRegsComputeNoDq>();
         else if (C::kRegsCompute < 128) ptx::setmaxnreg_dec<C::kRegsCompute>();
-        else ptx::setmaxnreg_inc<C::kRegsCompute>();
+        else if (C::kRegsCompute > 128) ptx::setmaxnreg_inc<C::kRegsCompute>();
         set_up_done();
         const uint32_t tmem = flag_value(tmem_slot);
         FusedWork w = first_tile();
@@ -820,7 +825,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             const uint32_t stats = sbase + C::kOffStats + half * 256;  // this half's 64 queries
             const uint64_t scale2 = ptx::f2_pack(a.scale_log2, a.scale_log2);
             const uint64_t post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
-            const float small_score = kSoftcap ? ptx::kTanhPolyMax / fabsf(a.softcap_pre) : 0.0f;
+            const uint64_t pre2 = ptx::f2_pack(a.softcap_pre * ptx::kTanhArg, a.softcap_pre * ptx::kTanhArg);
             // what dP - delta is multiplied with: P as it is handed to the MMA, in 16 bits, or P (1 - t^2), in 24 (pack24)
             uint32_t ppk[kSoftcap ? 48 : 32];
             // one arrival per warp: every lane's accesses are ordered before it by the fence and the warp barrier
@@ -850,15 +855,15 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 // masked: element (key j, query i) survives iff mask_from <= i <= mask_to.
                 const bool diagonal = kCausal && tile_needs_mask(w.kt, qt, w.band);
                 int mask_from = 0, mask_to = 0;  // set only on masked tiles
-                // ---- P^T = exp2(S^T * scale_log2 + neg_i), masked as above.
-                // (two copies of the chunk code, so that unmasked tiles carry no per-element test)
-                auto softmax_chunk = [&](int c, const uint32_t* r, auto masked_tag, auto small_tag) {
+                // ---- P^T = exp2(S^T * scale_log2 + neg_i), masked as above: 32 scores from column `first` of this half on;
+                // p: their P, two in a register
+                // (two copies of the code, so that unmasked tiles carry no per-element test)
+                auto softmax_cols = [&](int first, const uint32_t* r, uint32_t* p, auto masked_tag) {
                     constexpr bool kMasked = decltype(masked_tag)::value;
-                    uint32_t capped_p[16];  // P where ppk holds P (1 - t^2)
 #pragma unroll
                     for (int e = 0; e < 32; e += 4) {
                         float slope_p[4];
-                        const ptx::F4Pairs n4 = ptx::f2_ld_shared(negp + (c * 32 + e) * 4);
+                        const ptx::F4Pairs n4 = ptx::f2_ld_shared(negp + (first + e) * 4);
 #pragma unroll
                         for (int h = 0; h < 2; ++h) {
                             const uint64_t neg2 = h == 0 ? n4.lo : n4.hi;
@@ -867,7 +872,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                             // capped score + (log2 r - m)
                             const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[el]), __uint_as_float(r[el + 1]));
                             uint64_t t2 = 0;
-                            if constexpr (kSoftcap) t2 = ptx::tanh_score<decltype(small_tag)::value>(s2, a.softcap_pre, small_score);
+                            if constexpr (kSoftcap) t2 = ptx::tanh_mixed<C::kTanhFmaPairs>(ptx::f2_mul(s2, pre2), el / 2);
                             // (exp2_poly for a part of these changed nothing: B=4,H=16,S=4096,D=64 791, 792, 795, 810 us for 0 to 3
                             // pairs of 8)
                             float2 p2 = ptx::f2_unpack(kSoftcap ? ptx::f2_fma(t2, post2, neg2) : ptx::f2_fma(s2, scale2, neg2));
@@ -880,7 +885,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                                                                 ptx::f2_pack(fmaf(-tt.x, tt.x, 1.0f), fmaf(-tt.y, tt.y, 1.0f))));
                             }
                             if (kMasked) {
-                                const int i = half * 64 + c * 32 + el;
+                                const int i = half * 64 + first + el;
                                 const bool sees0 = i + 0 >= mask_from && i + 0 <= mask_to, sees1 = i + 1 >= mask_from && i + 1 <= mask_to;
                                 p2.x = sees0 ? p2.x : 0.0f;
                                 p2.y = sees1 ? p2.y : 0.0f;
@@ -889,32 +894,24 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                                     w2.y = sees1 ? w2.y : 0.0f;
                                 }
                             }
+                            p[el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
                             if constexpr (kSoftcap) {
-                                capped_p[el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
                                 slope_p[2 * h] = w2.x;
                                 slope_p[2 * h + 1] = w2.y;
-                            } else {
-                                ppk[c * 16 + el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
                             }
                         }
-                        if constexpr (kSoftcap) ptx::pack24(slope_p, &ppk[c * 24 + e / 4 * 3]);
+                        if constexpr (kSoftcap) ptx::pack24(slope_p, &ppk[(first + e) / 4 * 3]);
                     }
-                    // P chunk c -> columns [16c, 16c+16) of this half's S columns (already read)
-                    if constexpr (kSoftcap) ptx::tmem_st16(s_cols + c * 16, capped_p);
-                    else ptx::tmem_st16(s_cols + c * 16, &ppk[c * 16]);
                 };
                 auto softmax_phase = [&](auto masked_tag) {
 #pragma unroll
                     for (int c = 0; c < 2; ++c) {
-                        uint32_t r[32];
+                        uint32_t r[32], capped_p[16];  // (capped_p: P where ppk holds P (1 - t^2))
+                        uint32_t* p = kSoftcap ? capped_p : &ppk[c * 16];
                         ptx::tmem_ld32(s_cols + c * 32, r);
                         ptx::tmem_ld_wait();
-                        if constexpr (kSoftcap) {
-                            if (__all_sync(0xffffffffu, ptx::all_small<32>(r, small_score))) softmax_chunk(c, r, masked_tag, std::true_type{});
-                            else softmax_chunk(c, r, masked_tag, std::false_type{});
-                        } else {
-                            softmax_chunk(c, r, masked_tag, std::false_type{});
-                        }
+                        softmax_cols(c * 32, r, p, masked_tag);
+                        ptx::tmem_st16(s_cols + c * 16, p);  // P chunk c -> columns [16c, 16c+16) of this half's S columns (already read)
                     }
                 };
                 if (diagonal) {
@@ -974,6 +971,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             }
             // ---- epilogue: the first warpgroup writes dK (scaled), the second dV
             if (!ok) break;
+            if constexpr (kSoftcap) w = load_work(work);  // (what only the epilogue needs is not held in registers before)
             const int w4 = warp & 3;  // which 32 rows of the tile
             const bool has_steps = w.n_steps > 0;
             const int64_t slab = int64_t(w.slab * 2 + half) * (C::kTile * D) + w4 * 32 * D;
@@ -1068,7 +1066,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             ptx::setmaxnreg_dec<C::kRegsControl>();
             set_up_done();
         } else {
-            ptx::setmaxnreg_inc<C::kRegsDrain>();
+            if (C::kRegsDrain > 128) ptx::setmaxnreg_inc<C::kRegsDrain>();
             set_up_done();
             const uint32_t tmem = flag_value(tmem_slot);
             FusedWork w = first_tile();

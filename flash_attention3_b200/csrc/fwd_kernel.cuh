@@ -112,6 +112,9 @@ struct FwdCfg {
     // Of every 8 pairs of exponentials, how many go to the FMA pipe (exp2_poly) instead of the special-function unit.
     // us per call of B=4, H=16, S=4096 full for 0, 1, 2, 3 of 8: D=64 348, 338, 355, 371; D=128 486, 492, 490, 500.
     static constexpr int kPolyPairs = D == 64 ? 1 : 0;
+    // ... and of every 8 pairs of tanh of capped scores (tanh_mixed): us of the forwards named there for 2, 4, 5, 8 of 8: 84.5, 81,
+    // 80, 87; 247, 227, 228, 259.  (6 of 8 spill at D=128.)
+    static constexpr int kTanhFmaPairs = 5;
     // setmaxnreg split: the kernel starts with 168 registers per thread (384 threads); the producer /
     // MMA warpgroup gives most of its share to the two softmax warpgroups, which hold a whole score
     // row (128 values) in registers
@@ -634,7 +637,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             const bool q_valid = qi < w.band.seqlen_q;
             float m_ref = -INFINITY;  // reference maximum (raw scores) the exponentials are taken against
             float l = 0.0f;           // sum of the exponentials, in units of exp2(m_ref * scale_log2)
-            const float sl = kSoftcap ? 1.0f : a.scale_log2;  // log2 units per unit of (transformed) score
+            const float sl = kSoftcap ? a.softcap_post : a.scale_log2;  // log2 units per unit of (transformed) score
             const uint64_t sl2 = ptx::f2_pack(sl, sl);
             // one arrival per warp: every lane's accesses are ordered before it by the fence and the warp barrier
             auto arrive = [&](int which) {
@@ -660,22 +663,17 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 ptx::tmem_ld_wait();
                 if (C::kOwnP) arrive(kFwdSFree);
                 if (kSoftcap) {
-                    // capped scores, already in log2 units: from here on they are used with a scale of 1
-                    const uint64_t post2 = ptx::f2_pack(a.softcap_post, a.softcap_post);
-                    const float small_score = ptx::kTanhPolyMax / fabsf(a.softcap_pre);
-                    auto cap_chunk = [&](uint32_t (&chunk)[32], auto small_tag) {
-#pragma unroll
-                        for (int e = 0; e < 32; e += 2) {
-                            const uint64_t s2 = ptx::f2_pack(__uint_as_float(chunk[e]), __uint_as_float(chunk[e + 1]));
-                            const float2 capped = ptx::f2_unpack(ptx::f2_mul(ptx::tanh_score<decltype(small_tag)::value>(s2, a.softcap_pre, small_score), post2));
-                            chunk[e] = __float_as_uint(capped.x);
-                            chunk[e + 1] = __float_as_uint(capped.y);
-                        }
-                    };
+                    // from here on the scores are the tanh, and their scale the cap
+                    const float pre = a.softcap_pre * ptx::kTanhArg;
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        if (__all_sync(0xffffffffu, ptx::all_small<32>(r[c], small_score))) cap_chunk(r[c], std::true_type{});
-                        else cap_chunk(r[c], std::false_type{});
+#pragma unroll
+                        for (int e = 0; e < 32; e += 2) {
+                            const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
+                            const float2 t = ptx::f2_unpack(ptx::tanh_mixed<C::kTanhFmaPairs>(ptx::f2_mul(s2, ptx::f2_pack(pre, pre)), e / 2));
+                            r[c][e] = __float_as_uint(t.x);
+                            r[c][e + 1] = __float_as_uint(t.y);
+                        }
                     }
                 }
                 if (diagonal) {
@@ -765,6 +763,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
                 mask_from -= C::kTile;
                 mask_to -= C::kTile;
             }
+            if constexpr (kSoftcap) w = load_work<FwdWork>(work);  // (what only the output needs is not held in registers before)
             // (m_ref, not l, says whether the row saw a key: exp2_poly leaves 2^-126 on a masked one)
             const bool any_key = q_valid && m_ref != -INFINITY;
             const float inv = any_key ? 1.0f / l : 0.0f;

@@ -459,48 +459,32 @@ __device__ __forceinline__ uint64_t tanh_pair(uint64_t x_arg2) {
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(ry) : "f"(d.y));
     return f2_fma(f2_pack(rx, ry), f2_pack(-2.0f, -2.0f), f2_pack(1.0f, 1.0f));
 }
-// tanh of two values of magnitude at most 1 on the FMA pipe alone: x p(x^2), p of degree 6 fitted for the smallest largest
-// relative error (5.0e-8); evaluated in fp32 the absolute error is at most 1.3e-7.  Eight packed operations, 16 cycles of the
-// FMA pipe for two values, where tanh_pair keeps the special-function unit busy for 32, which bounds the capped kernels: us,
-// B=1, Hq=16, Hkv=8, S=4096, D=128, window 1024, cap 30, forward 89.9 -> 78.6, gradients 153.6 -> 130.7 (the slope of the cap
-// taken from the tanh at once, and not from log2 of P later, included); B=4, H=16, S=2048, D=64 full, cap 50 263 -> 233 and
-// 399 -> 310.
-constexpr float kTanhPolyMax = 1.0f;
-__device__ __forceinline__ uint64_t tanh_poly(uint64_t x2) {
-    const uint64_t u2 = f2_mul(x2, x2);
-    uint64_t p2 = f2_pack(0x1.10e5d8p-10f, 0x1.10e5d8p-10f);
-    p2 = f2_fma(p2, u2, f2_pack(-0x1.968b6ep-8f, -0x1.968b6ep-8f));
-    p2 = f2_fma(p2, u2, f2_pack(0x1.4c6e58p-6f, 0x1.4c6e58p-6f));
-    p2 = f2_fma(p2, u2, f2_pack(-0x1.b5eb84p-5f, -0x1.b5eb84p-5f));
-    p2 = f2_fma(p2, u2, f2_pack(0x1.10e672p-3f, 0x1.10e672p-3f));
-    p2 = f2_fma(p2, u2, f2_pack(-0x1.55540ap-2f, -0x1.55540ap-2f));
-    p2 = f2_fma(p2, u2, f2_pack(0x1.fffffep-1f, 0x1.fffffep-1f));
-    return f2_mul(x2, p2);
+// The same on the FMA pipe but for one exponential per value: sign(x) (1 - z) / (1 + z), z = exp(-2|x|).  1 / (1 + z) by a
+// polynomial of degree 3 (relative error e up to 1.7e-3) and one step of third order, r + r (e + e^2).  Absolute error at most 1.9e-7.
+__device__ __forceinline__ uint64_t tanh_pair_fma(uint64_t x_arg2) {
+    const float2 x = f2_unpack(x_arg2);
+    const uint64_t one2 = f2_pack(1.0f, 1.0f), minus2 = f2_pack(-1.0f, -1.0f);
+    const uint64_t z2 = f2_pack(ex2_approx(-fabsf(x.x)), ex2_approx(-fabsf(x.y)));
+    uint64_t r2 = f2_pack(-0x1.c6527ep-3f, -0x1.c6527ep-3f);
+    r2 = f2_fma(r2, z2, f2_pack(0x1.54bde2p-1f, 0x1.54bde2p-1f));
+    r2 = f2_fma(r2, z2, f2_pack(-0x1.e2b7aep-1f, -0x1.e2b7aep-1f));
+    r2 = f2_fma(r2, z2, f2_pack(0x1.ff1cd6p-1f, 0x1.ff1cd6p-1f));
+    const uint64_t e2 = f2_fma(f2_fma(z2, minus2, minus2), r2, one2);  // 1 - (1 + z) r
+    r2 = f2_fma(r2, f2_fma(e2, e2, e2), r2);
+    const float2 t = f2_unpack(f2_mul(f2_fma(z2, minus2, one2), r2));
+    return f2_pack(copysignf(t.x, x.x), copysignf(t.y, x.y));
 }
-// tanh(s * pre) of two scores.  A score of magnitude at most `limit` (kTanhPolyMax / |pre|) takes the polynomial, any other,
-// a NaN too, the form above.  kSmall: the caller knows that both are small.  The form that a value takes depends on the
-// value alone, whatever the others of its tile are; where a warp's 32 columns hold some of either kind, both are evaluated.
-// (With four in ten scores above the cap, which a cap is not chosen for, the last of the shapes above takes 343 and 432 us.
-// Deciding for eight columns at a time there: 387 and 482, and 245 and 320 where all are small.)
-template <bool kSmall>
-__device__ __forceinline__ uint64_t tanh_score(uint64_t s2, float pre, float limit) {
-    const uint64_t small2 = tanh_poly(f2_mul(s2, f2_pack(pre, pre)));
-    if (kSmall) return small2;
-    const float2 s = f2_unpack(s2), small = f2_unpack(small2);
-    const float2 any = f2_unpack(tanh_pair(f2_mul(s2, f2_pack(pre * kTanhArg, pre * kTanhArg))));
-    return f2_pack(fabsf(s.x) <= limit ? small.x : any.x, fabsf(s.y) <= limit ? small.y : any.y);
-}
-// Whether all of a thread's kCount scores are small in that sense (false if one is NaN).
-template <int kCount>
-__device__ __forceinline__ bool all_small(const uint32_t* s, float limit) {
-    float top[2] = {0.0f, 0.0f};
-#pragma unroll
-    for (int e = 0; e < kCount; e += 4) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-            top[h] = max3_nan(top[h], fabsf(__uint_as_float(s[e + 2 * h])), fabsf(__uint_as_float(s[e + 2 * h + 1])));
-    }
-    return max_nan(top[0], top[1]) <= limit;
+// tanh of the `pair`-th pair of values of a thread: of every 8 pairs kFmaPairs take the second form.  The first keeps the
+// special-function unit busy for 32 cycles (the exponential of the softmax for 16 more), the second for 16 and the FMA pipe for
+// 20; a mix keeps both busy.  Which form a value takes depends on its place alone, and the time not on the scores.
+// us, all of the first form and so: B=1, Hq=16, Hkv=8, S=4096, D=128, window 1024, cap 30 forward 89.7 and 80.0, gradients 159 and 140,
+// reproducible 204 and 178; B=4, 16 x 2048 full, D=64, cap 50 262 and 228, 398 and 328, 684 and 570 (with P (1 - tanh^2) handed to the dS
+// phase instead of taken from log2 of P).  A polynomial on the FMA pipe alone where all of a warp's 32 x 32 scores are below
+// the cap, and both forms where some are not, measured 76, 134, 178 and 232, 311, 537 without such scores, but 114, 199, 240 and 334,
+// 491, 808 with one in a thousand above the cap, and 111, 171, 228 and 329, 432, 738 with four in ten.
+template <int kFmaPairs>
+__device__ __forceinline__ uint64_t tanh_mixed(uint64_t x_arg2, int pair) {
+    return (pair * kFmaPairs) % 8 + kFmaPairs >= 8 ? tanh_pair_fma(x_arg2) : tanh_pair(x_arg2);
 }
 
 // Four fp32 values in three registers, the upper 24 bits of each (15 bits of significand, to within 2^-15 and without a bias: the

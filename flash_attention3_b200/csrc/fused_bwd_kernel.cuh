@@ -336,6 +336,13 @@ __device__ __forceinline__ W load_work(uint32_t addr) {
     return w;
 }
 
+// A value that all lanes of a warp hold, in a form that tells the compiler so: what comes from shared memory might differ between them,
+// and loops and branches on it are compiled for that.  us, without and with it, on what the loops of the math warps and the
+// MMA warp test: forward, D=64, 11 x 2 heads x 4970 full 190 and 185.5, 4 x 8192 93.0 and 91.6, B=8, 32 x 512 35.9 and 35.2, D=128, B=8,
+// 32 x 300 causal 33.3 and 32.0; backward, D=64, 8 x 4096 causal 66.6 and 65.1, 4 x 16384 455 and 438, D=128, B=8, 32 x 300 79.3 and 78.0.
+// (All of the work handed over so: slower.)
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 template <bool kCausal>
 __device__ __forceinline__ FusedWork fused_work(const FusedArgs& a, int block) {
     FusedWork w;
@@ -624,7 +631,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             bool ok = true;
 #pragma unroll 1
             for (bool next = !misaligned; next; ++n) {
-                const int n_steps = w.n_steps;
+                const int n_steps = uniform(w.n_steps);
                 if (n_steps == 0) request();
                 if (n_steps > 0) {
                     ok = warp_wait<false>(bar(kKvFull), used & 1, abort_flag) && wait_q(g0);
@@ -839,6 +846,12 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             int g = 0;  // step, counted over all tiles
 #pragma unroll 1
             for (bool more = !misaligned; more; ++n) {
+            w.n_steps = uniform(w.n_steps);
+            w.kt = uniform(w.kt);
+            w.q_begin = uniform(w.q_begin);
+            w.steps_per_head = uniform(w.steps_per_head);
+            w.rotation = uniform(w.rotation);
+            w.q_tiles = uniform(w.q_tiles);
             StepWalk<kCausal> st(w);
 #pragma unroll 1
             for (int t = 0; t < w.n_steps; ++t, ++g, st.next(w)) {

@@ -626,8 +626,9 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             bool more = true;
 #pragma unroll 1
             for (; more; ++n) {
-            const int qt = x == 0 ? w.tile[0] : w.tile[1];
-            const int n_steps = x == 0 ? w.hi[0] - w.lo[0] : w.hi[1] - w.lo[1];  // (selects, not indexing: no local array)
+            // (selects, not indexing: no local array; uniform: see there)
+            const int qt = uniform(x == 0 ? w.tile[0] : w.tile[1]);
+            const int n_steps = uniform(x == 0 ? w.hi[0] - w.lo[0] : w.hi[1] - w.lo[1]);
             const int k_begin = w.t_begin + (x == 0 ? w.lo[0] : w.lo[1]);
             const uint32_t tl = tmem + (uint32_t((warp & 3) * 32) << 16);
             const uint32_t s_cols = tl + C::kColS + x * 128;

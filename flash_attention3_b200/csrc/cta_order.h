@@ -210,4 +210,20 @@ inline FwdPlan plan_fwd(const Band& band, long long bh_count, const FwdGangs& ga
     return best;
 }
 
+// Whether the CTAs of the forward take over pairs of query tiles of CTAs that have not started: from two pairs with rows per SM
+// on.  us per call, one CTA per pair and this: causal, 32 x 300 x B=8, D=128 38.6 and 32.0; 32 on 8 heads x 1024 x B=8, D=128 108.4 and 98,
+// D=64 88.4 and 87; full, 32 x 512 x B=8, D=64 41.6 and 35.2.  With fewer the longer code costs more than it gives: 256 pairs (16 x 2048 x
+// B=2, causal) D=128 42.3 and 41.2, D=64 35.6 and 38.3; 240 (80 x 700, D=64) 22.8 and 24.5; 160 (40 x 1000, D=128) 22.4 and 23.8.  (Long shapes
+// run under the power limit: the same within its spread.)
+// Packed (total_rows > 0): the grid is sized for the longest sequence, and most blocks may have no rows; a sequence fills half of its
+// last pair on average.  D=64, causal and full: 8 heads, one sequence of 1000 and 20 of 40 (192 pairs in 672 blocks) 16.6 and 18.1, 19.9 and
+// 23.0; 4 heads, 4096 and 15 of 100 (124 in 1024) 49.2 and 53.2, 54.3 and 58.5; 16 heads, 2048 and 20 of 128 (448 in 2688) 42.2 and 41.2, 51.0
+// and 58.0; 16 heads, 1024 and 50 of 30 (864 in 3264) 47.9 and 45.2, 48.7 and 47.8; 32 heads, 2048 and 20 of 128 (896 in 5376) 80.4 and 72.4,
+// 92.7 and 89.2.  Full attention, where the pairs of a sequence are equally long, needs more of them.
+inline bool fwd_takes_over(const Band& band, long long pairs, long long heads, int batch, long long total_rows, int sms) {
+    if (total_rows <= 0) return pairs >= 2LL * sms;
+    const long long with_rows = std::min(pairs, heads * (total_rows + kTileRows * (long long)batch) / (2 * kTileRows));
+    return 2 * with_rows >= (band_is_full(band) ? 7LL : 4LL) * sms;
+}
+
 }  // namespace fa3b200

@@ -691,12 +691,8 @@ int launch_fwd_d(const ShaoboFa3Params* p, const FwdLaunch& L) {
     if (p->softcap > 0.0f) {
         return p->head_dim_qk == 128 ? launch_fwd_t<T, 128, true, true>(L, st) : launch_fwd_t<T, 64, true, true>(L, st);
     }
-    // Twice as many pairs of query tiles as SMs: CTAs take over the tiles of those that have not started.  us per call, one CTA per
-    // pair and this: causal, 32 x 300 x B=8, D=128 39.1 and 33.4; 32 on 8 heads x 1024 x B=8, D=128 108.4 and 98, D=64 88.4 and 87;
-    // full, 32 x 512 x B=8, D=64 46.5 and 43; 16 x 2048 x B=4, D=128 149 and 144.  With fewer the longer code costs more than
-    // it gives: 256 pairs (16 x 2048 x B=2, causal) D=128 42.3 and 41.2, D=64 35.6 and 38.3; 240 (80 x 700, D=64) 22.8 and 24.5;
-    // 160 (40 x 1000, D=128) 22.4 and 23.8.  (Long shapes run under the power limit: the same within its spread.)
-    if (L.args.splits == 1 && L.blocks >= 2 * sm_count()) {
+    // (the line and both sides of it: cta_order.h)
+    if (L.args.splits == 1 && fwd_takes_over(L.args.band, L.blocks, p->num_heads_q, p->batch, is_varlen(p) ? p->total_q : 0, sm_count())) {
         if (p->head_dim_qk == 128) return masked ? launch_fwd_t<T, 128, true, false, true>(L, st) : launch_fwd_t<T, 128, false, false, true>(L, st);
         return masked ? launch_fwd_t<T, 64, true, false, true>(L, st) : launch_fwd_t<T, 64, false, false, true>(L, st);
     }

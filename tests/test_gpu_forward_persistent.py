@@ -41,14 +41,18 @@ def test_tiles_taken_over(b, hq, hkv, sq, sk, d, dtype, causal, layout, window, 
         assert torch.equal(again, out) and torch.equal(lse2, lse)
 
 
+PACKED = [(700, 700)] + [(5, 7), (130, 130), (1, 9), (257, 300), (64, 129)] * 5
+PACKED_HEADS = [8, 24]  # 8: too few pairs with rows, one per CTA; 24: taken over
+
+
+@pytest.mark.parametrize("heads", PACKED_HEADS)
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("causal", [False, True])
-def test_packed_tiles_taken_over(causal, d):
+def test_packed_tiles_taken_over(causal, d, heads):
     from flash_attention3_b200 import ops
     from tests.helpers import dev, host
     from tests.test_gpu_varlen import packed_problem
-    seqs = [(700, 700)] + [(5, 7), (130, 130), (1, 9), (257, 300), (64, 129)] * 5
-    packed, refs, cu_q, cu_k = packed_problem(seqs, 8, 4, d, "bf16", causal, (-1, -1), seed=17)
+    packed, refs, cu_q, cu_k = packed_problem(PACKED, heads, heads // 2, d, "bf16", causal, (-1, -1), seed=17)
     t = {n: dev(packed[n], "bf16") for n in ("q", "k", "v")}
     cu = [torch.from_numpy(c).cuda() for c in (cu_q, cu_k)]
     call = lambda: ops.fa3_fwd_varlen(t["q"], t["k"], t["v"], *cu, 700, 700, causal, sync=True)

@@ -1,0 +1,61 @@
+"""Where CTAs take over the work of CTAs that have not started (csrc/cta_order.h, host code compiled with g++)."""
+import ctypes
+import subprocess
+
+import pytest
+
+from tests.conftest import ROOT
+
+SRC = r'''
+#include "cta_order.h"
+using namespace fa3b200;
+extern "C" int forward(int longest, int causal, long long pairs, long long heads, int batch, long long rows) {
+    return fwd_takes_over(make_band(longest, longest, causal != 0, -1, -1), pairs, heads, batch, rows, 148);
+}
+'''
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    d = tmp_path_factory.mktemp("takeover")
+    (d / "t.cpp").write_text(SRC)
+    so = d / "libt.so"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", str(ROOT / "flash_attention3_b200/csrc"), str(d / "t.cpp"),
+                    "-o", str(so)], check=True)
+    lib = ctypes.CDLL(str(so))
+    lib.forward.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_longlong]
+    return lib
+
+
+def packed(lib, heads, lengths, causal):
+    pairs = (max(lengths) + 255) // 256 * len(lengths) * heads
+    return bool(lib.forward(max(lengths), causal, pairs, heads, len(lengths), sum(lengths)))
+
+
+@pytest.mark.parametrize("pairs,expected", [(295, False), (296, True), (1 << 31, True)])
+def test_forward_line(lib, pairs, expected):
+    assert bool(lib.forward(1024, 0, pairs, 8, 4, 0)) == bool(lib.forward(1024, 1, pairs, 8, 4, 0)) == expected
+
+
+@pytest.mark.parametrize("heads,lengths,full,causal", [
+    (8, [1000] + [40] * 20, False, False),     # 192 pairs with rows in 672 blocks
+    (4, [4096] + [100] * 15, False, False),    # 124 in 1024
+    (1, [4096] + [30] * 40, False, False),     # 56 in 656
+    (2, [8192] + [500] * 8, False, False),     # 96 in 576
+    (16, [2048] + [128] * 20, False, True),    # 448 in 2688
+    (32, [2048] + [128] * 20, True, True),     # 896 in 5376
+    (16, [1024] + [30] * 50, True, True),      # 864 in 3264
+    (16, [2048, 77, 1500, 300, 1024, 513, 129, 900, 1701], True, True),
+    (40, [1024, 1024], False, True),           # every block has rows
+    (36, [1024, 1024], False, False),
+])
+def test_forward_of_packed_sequences_counts_the_pairs_with_rows(lib, heads, lengths, full, causal):
+    assert packed(lib, heads, lengths, False) == full and packed(lib, heads, lengths, True) == causal
+
+
+def test_gpu_cases_reach_the_form_they_name(lib):
+    from tests.test_gpu_forward_persistent import CASES, PACKED, PACKED_HEADS
+    for b, hq, _, sq, _, _, _, causal, *_ in CASES:
+        assert lib.forward(sq, causal, (sq + 255) // 256 * b * hq, hq, b, 0), (b, hq, sq)
+    for causal in (False, True):
+        assert [packed(lib, heads, [q for q, _ in PACKED], causal) for heads in PACKED_HEADS] == [False, True]

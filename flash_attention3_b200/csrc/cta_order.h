@@ -210,6 +210,24 @@ inline FwdPlan plan_fwd(const Band& band, long long bh_count, const FwdGangs& ga
     return best;
 }
 
+// A CTA that takes over tiles has warps that wait for the next one from the start of a tile to its end (who works it out; a softmax
+// warpgroup whose query tile has fewer keys), and a wait gives up after 2e9 cycles.  A step takes 4000; longer tiles than this stay
+// with one per CTA, where no wait spans more than a step, and where the set-up saved is nothing beside them.
+constexpr long long kMostStepsTakenOver = 1 << 16;
+
+// Whether the CTAs of the dK/dV and five-GEMM kernels take over key tiles of CTAs that have not started: where there are more tiles than
+// SMs.  us per call, one CTA per tile and this:
+// full, 80 heads x 512, D=128 60.3 and 55.2; 32 x 512 x B=8, D=64 101 and 91; 16 x 1024 x B=8, D=64 144 and 139; causal, 40 x 512, D=128
+// 27.8 and 25.8; 16 x 1000 x B=4 91.5 and 85; 8 x 300 x B=32 84.3 and 78; D=64, 16 x 2048 x B=2 81.4 and 76; 8 x 4096 65.2 and 65.1; 176 tiles (1111
+// queries x 1300 keys) 46.4 and 46.6; reproducible gradients (dK/dV kernel), causal, 32 x 300 x B=8, D=128 108 and 93.6; 16 x 2048 x B=2 156 and
+// 154.  (Long shapes run under the power limit: the same within its spread.)  Packed, where blocks without rows are passed over by
+// the warp that works tiles out instead of starting: 9 x 4096, 16 heads, D=128 832 and 794; 16 heads, 2048 and 20 x 128, D=64 causal 116 and
+// 73; 1 head, 4096 and 40 x 30 (72 tiles in 1312 blocks), causal, D=64 55.9 and 54.8, reproducible 61.9 and 51.2, D=128 reproducible 74.8
+// and 64.5, but 77.3 and 84.1 when such calls follow one another (alone they take the same).
+inline bool bwd_takes_over(const Band& band, long long blocks, int group, int sms) {
+    return blocks > sms && (long long)group * tiles_of(band.seqlen_q) <= kMostStepsTakenOver;
+}
+
 // Whether the CTAs of the forward take over pairs of query tiles of CTAs that have not started: from two pairs with rows per SM
 // on.  us per call, one CTA per pair and this: causal, 32 x 300 x B=8, D=128 38.6 and 32.0; 32 on 8 heads x 1024 x B=8, D=128 108.4 and 98,
 // D=64 88.4 and 87; full, 32 x 512 x B=8, D=64 41.6 and 35.2.  With fewer the longer code costs more than it gives: 256 pairs (16 x 2048 x
@@ -221,6 +239,7 @@ inline FwdPlan plan_fwd(const Band& band, long long bh_count, const FwdGangs& ga
 // and 58.0; 16 heads, 1024 and 50 of 30 (864 in 3264) 47.9 and 45.2, 48.7 and 47.8; 32 heads, 2048 and 20 of 128 (896 in 5376) 80.4 and 72.4,
 // 92.7 and 89.2.  Full attention, where the pairs of a sequence are equally long, needs more of them.
 inline bool fwd_takes_over(const Band& band, long long pairs, long long heads, int batch, long long total_rows, int sms) {
+    if (tiles_of(band.seqlen_k) > kMostStepsTakenOver) return false;
     if (total_rows <= 0) return pairs >= 2LL * sms;
     const long long with_rows = std::min(pairs, heads * (total_rows + kTileRows * (long long)batch) / (2 * kTileRows));
     return 2 * with_rows >= (band_is_full(band) ? 7LL : 4LL) * sms;

@@ -372,15 +372,9 @@ int launch_fused_d(const ShaoboFa3Params* p, const CUtensorMap& mq, const CUtens
                    ? launch_fused_t<T, 128, true, kWithDq, TOut, true>(mq, mk, mv, mdo, mdq, args, blocks, st, pdl)
                    : launch_fused_t<T, 64, true, kWithDq, TOut, true>(mq, mk, mv, mdo, mdq, args, blocks, st, pdl);
     }
-    // More tiles than SMs: CTAs take over the tiles of those that have not started.  us per call, one CTA per tile and this:
-    // full, 80 heads x 512, D=128 60.3 and 55.2; 32 x 512 x B=8, D=64 101.6 and 94.9; 16 x 1024 x B=8, D=64 144 and 139; causal,
-    // 40 x 512, D=128 27.8 and 25.8; 16 x 1000 x B=4 86.9 and 83.4; 16 x 2048 x B=2 127.3 and 124.3; packed, 9 x 4096, 16 heads,
-    // D=128 832 and 794; 24 x 1024, D=64 135.8 and 133.7; reproducible gradients (dK/dV kernel), causal, 16 x 2048 x B=2, D=128
-    // 144.6 and 140.1; 32 x 300 x B=8 108 and 93.6; full, 16 x 2048 x B=4, D=64 341 and 333.  (Long shapes run under the power
-    // limit: the same within its spread.)  D=64 causal, 16 x 2048 x B=2 81.9 and 78.8; 32 x 700 x B=8 141 and 137.4; 176 tiles
-    // (1111 queries x 1300 keys) 46.4 and 46.6.
+    // (the line and both sides of it: cta_order.h)
     if constexpr (std::is_same<T, TOut>::value) {
-        if (args.chunk_steps == 0 && blocks > sm_count()) {
+        if (args.chunk_steps == 0 && bwd_takes_over(args.band, blocks, args.group, sm_count())) {
             if (p->head_dim_qk == 128) {
                 return banded ? launch_fused_t<T, 128, true, kWithDq, TOut, false, true>(mq, mk, mv, mdo, mdq, args, blocks, st, pdl)
                               : launch_fused_t<T, 128, false, kWithDq, TOut, false, true>(mq, mk, mv, mdo, mdq, args, blocks, st, pdl);

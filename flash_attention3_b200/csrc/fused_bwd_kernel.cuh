@@ -29,13 +29,13 @@
 // the second queries 64-127); warps 12-15 = dQ drain warpgroup.  Registers are
 // re-split with setmaxnreg (96 / 120 / 120 / 176 per thread at D=128).  All hand-offs go
 // through mbarriers; every wait is bounded and a time-out raises an error flag
-// instead of hanging.
+// instead of hanging.  (The longest that a correct run needs is that for the next tile, over a whole tile: kMostStepsTakenOver.)
 //
 // Tiles (kPersist): a CTA that is about to finish its tile asks for the block index of a CTA that has not started, warp 3
 // works out what that is and hands it to the other roles in shared memory, and the roles, rings and hand-offs run on: K, V, Q
 // and dO of the next tile are loaded and its first S is computed beside the epilogue, and the set-up (barriers, tensor memory,
 // cold instruction cache: 1300-2800 clk until the first loads, 3000-5000 until they have landed) is paid once.  Where every SM
-// has several tiles; the rule and what it measured stand beside the launch.  One warp works the tile out for all, in either
+// has several tiles; the rule and what it measured stand in cta_order.h.  One warp works the tile out for all, in either
 // form, because the index arithmetic inlined in five roles was 1400 clk of cold code in front of the first loads.
 //
 // Tensor-memory ledger (512 columns x 128 lanes x 32 bit):

@@ -31,7 +31,7 @@
 // clock near 1.6 GHz); B=2, Hq=32, Hkv=8, S=8192 causal, D=128 857 and 1063.
 //
 // With at least two pairs of query tiles per SM (kPersist) CTAs take over the pairs of CTAs that have not started, as in the
-// backward; the rule and what it measured stand beside the launch.
+// backward; the rule and what it measured stand in cta_order.h.
 //
 // When the pairs are too few to fill the GPU a cluster of 2, 4 or 8 CTAs shares the key tiles of a pair
 // (plan_fwd) and merges the partial outputs through distributed shared memory.

@@ -12,6 +12,7 @@ using namespace fa3b200;
 extern "C" int forward(int longest, int causal, long long pairs, long long heads, int batch, long long rows) {
     return fwd_takes_over(make_band(longest, longest, causal != 0, -1, -1), pairs, heads, batch, rows, 148);
 }
+extern "C" int backward(int sq, int sk, long long blocks, int group) { return bwd_takes_over(make_band(sq, sk, false, -1, -1), blocks, group, 148); }
 '''
 
 
@@ -24,6 +25,7 @@ def lib(tmp_path_factory):
                     "-o", str(so)], check=True)
     lib = ctypes.CDLL(str(so))
     lib.forward.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_longlong]
+    lib.backward.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
     return lib
 
 
@@ -53,9 +55,28 @@ def test_forward_of_packed_sequences_counts_the_pairs_with_rows(lib, heads, leng
     assert packed(lib, heads, lengths, False) == full and packed(lib, heads, lengths, True) == causal
 
 
+@pytest.mark.parametrize("blocks,expected", [(148, False), (149, True)])
+def test_backward_line(lib, blocks, expected):
+    assert bool(lib.backward(1024, 1024, blocks, 4)) == expected
+
+
+def test_no_wait_spans_a_tile_of_a_second(lib):
+    """Warps that wait from the start of a tile to its end give up after 2e9 cycles, about 500000 steps: 64 query heads on one key
+    head with a million queries, or as many keys."""
+    most = 1 << 16
+    assert 8 * 4000 * most > 2e9 >= 7 * 4000 * most  # with this much in hand
+    assert lib.backward(most * 128 // 64, 1 << 20, 8192, 64) and not lib.backward(most * 128 // 64 + 1, 1 << 20, 8192, 64)
+    assert not lib.backward(1 << 20, 1 << 20, 8192, 64)
+    assert lib.forward(most * 128, 0, 1 << 16, 1, 1, 0) and not lib.forward(most * 128 + 1, 0, 1 << 16, 1, 1, 0)
+    assert not lib.forward(most * 128 + 1, 1, 1 << 16, 1, 1, most * 128 + 1)
+
+
 def test_gpu_cases_reach_the_form_they_name(lib):
     from tests.test_gpu_forward_persistent import CASES, PACKED, PACKED_HEADS
     for b, hq, _, sq, _, _, _, causal, *_ in CASES:
         assert lib.forward(sq, causal, (sq + 255) // 256 * b * hq, hq, b, 0), (b, hq, sq)
+    from tests import test_gpu_persistent
+    for b, hq, hkv, sq, sk, *_ in test_gpu_persistent.CASES:
+        assert lib.backward(sq, sk, (sk + 127) // 128 * b * hkv, hq // hkv), (b, hkv, sk)
     for causal in (False, True):
         assert [packed(lib, heads, [q for q, _ in PACKED], causal) for heads in PACKED_HEADS] == [False, True]

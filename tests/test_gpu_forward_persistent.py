@@ -9,28 +9,28 @@ from oracle import golden
 
 pytestmark = pytest.mark.gpu
 
-# (b, hq, hkv, sq, sk, d, dtype, causal, layout, window, softcap)
+# (b, hq, hkv, sq, sk, d, dtype, causal, layout, window)
 CASES = [
-    (1, 300, 300, 128, 128, 64, "bf16", True, "bhsd", (-1, -1), 0.0),
-    (1, 300, 300, 128, 128, 128, "fp16", False, "bshd", (-1, -1), 0.0),
-    (1, 150, 150, 512, 512, 64, "fp16", True, "bshd", (-1, -1), 0.0),     # one and two steps, then three and four
-    (2, 80, 40, 512, 384, 128, "bf16", False, "bhsd", (-1, -1), 0.0),
-    (1, 100, 100, 700, 300, 64, "fp16", True, "bhsd", (-1, -1), 0.0),     # queries without keys
-    (1, 100, 50, 600, 900, 128, "bf16", True, "bshd", (200, -1), 0.0),
-    (1, 160, 160, 300, 300, 64, "bf16", True, "bhsd", (-1, -1), 0.0),
+    (1, 300, 300, 128, 128, 64, "bf16", True, "bhsd", (-1, -1)),
+    (1, 300, 300, 128, 128, 128, "fp16", False, "bshd", (-1, -1)),
+    (1, 150, 150, 512, 512, 64, "fp16", True, "bshd", (-1, -1)),     # one and two steps, then three and four
+    (2, 80, 40, 512, 384, 128, "bf16", False, "bhsd", (-1, -1)),
+    (1, 100, 100, 700, 300, 64, "fp16", True, "bhsd", (-1, -1)),     # queries without keys
+    (1, 100, 50, 600, 900, 128, "bf16", True, "bshd", (200, -1)),
+    (1, 160, 160, 300, 300, 64, "bf16", True, "bhsd", (-1, -1)),
 ]
 
 
-@pytest.mark.parametrize("b,hq,hkv,sq,sk,d,dtype,causal,layout,window,softcap", CASES)
-def test_tiles_taken_over(b, hq, hkv, sq, sk, d, dtype, causal, layout, window, softcap):
+@pytest.mark.parametrize("b,hq,hkv,sq,sk,d,dtype,causal,layout,window", CASES)
+def test_tiles_taken_over(b, hq, hkv, sq, sk, d, dtype, causal, layout, window):
     from flash_attention3_b200 import ops
     from tests.helpers import dev, host
     q, k, v, _ = golden.seeded_inputs(41 + sq, b, hq, hkv, sq, d, dtype, sk=sk)
     scale = 1.0 / float(np.sqrt(d))
-    ref = golden.backward(q, k, v, np.zeros_like(q), causal, scale, dtype, window, softcap)
+    ref = golden.backward(q, k, v, np.zeros_like(q), causal, scale, dtype, window)
     f = (lambda x: np.ascontiguousarray(x.transpose(0, 2, 1, 3))) if layout == "bshd" else (lambda x: x)
     t = [dev(f(x), dtype) for x in (q, k, v)]
-    call = lambda: ops.fa3_fwd(*t, causal, scale, layout=layout, window=window, softcap=softcap, sync=True)
+    call = lambda: ops.fa3_fwd(*t, causal, scale, layout=layout, window=window, sync=True)
     out, lse = call()
     assert golden.check_gradient(f(host(out)) if layout == "bshd" else host(out), ref["out"], dtype)["pass"]
     finite = np.isfinite(ref["lse"])

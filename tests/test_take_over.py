@@ -5,12 +5,16 @@ import subprocess
 import pytest
 
 from tests.conftest import ROOT
+from tests.test_split_plan import params, plan  # noqa: F401  (a fixture)
 
 SRC = r'''
 #include "cta_order.h"
 using namespace fa3b200;
 extern "C" int forward(int longest, int causal, long long pairs, long long heads, int batch, long long rows) {
     return fwd_takes_over(make_band(longest, longest, causal != 0, -1, -1), pairs, heads, batch, rows, 148);
+}
+extern "C" int clusters(int sq, int sk, int causal, int left, int right, long long heads) {
+    return plan_fwd(make_band(sq, sk, causal != 0, left, right), heads, FwdGangs{148, 74, 33, 15}, false).splits;
 }
 extern "C" int backward(int sq, int sk, long long blocks, int group) { return bwd_takes_over(make_band(sq, sk, false, -1, -1), blocks, group, 148); }
 '''
@@ -25,6 +29,7 @@ def lib(tmp_path_factory):
                     "-o", str(so)], check=True)
     lib = ctypes.CDLL(str(so))
     lib.forward.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_longlong, ctypes.c_int, ctypes.c_longlong]
+    lib.clusters.argtypes = [ctypes.c_int] * 5 + [ctypes.c_longlong]
     lib.backward.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_longlong, ctypes.c_int]
     return lib
 
@@ -71,12 +76,17 @@ def test_no_wait_spans_a_tile_of_a_second(lib):
     assert not lib.forward(most * 128 + 1, 1, 1 << 16, 1, 1, most * 128 + 1)
 
 
-def test_gpu_cases_reach_the_form_they_name(lib):
-    from tests.test_gpu_forward_persistent import CASES, PACKED, PACKED_HEADS
-    for b, hq, _, sq, _, _, _, causal, *_ in CASES:
+def test_gpu_cases_reach_the_form_they_name(lib, plan):
+    """Enough tiles, no clusters (forward), no split key tiles (backward)."""
+    from tests import test_gpu_forward_persistent as forward, test_gpu_persistent as backward
+    for b, hq, _, sq, sk, _, _, causal, _, window in forward.CASES:
         assert lib.forward(sq, causal, (sq + 255) // 256 * b * hq, hq, b, 0), (b, hq, sq)
-    from tests import test_gpu_persistent
-    for b, hq, hkv, sq, sk, *_ in test_gpu_persistent.CASES:
-        assert lib.backward(sq, sk, (sk + 127) // 128 * b * hkv, hq // hkv), (b, hkv, sk)
+        assert lib.clusters(sq, sk, causal, *window, b * hq) == 1
     for causal in (False, True):
-        assert [packed(lib, heads, [q for q, _ in PACKED], causal) for heads in PACKED_HEADS] == [False, True]
+        assert [packed(lib, heads, [q for q, _ in forward.PACKED], causal) for heads in forward.PACKED_HEADS] == [False, True]
+    for b, hq, hkv, sq, sk, d, dtype, causal, _, window in backward.CASES:
+        assert lib.backward(sq, sk, (sk + 127) // 128 * b * hkv, hq // hkv), (b, hkv, sk)
+        assert plan(params(b, hq, hkv, sq, d, dtype, causal, sk=sk, window_left=window[0], window_right=window[1]))[0] == 0
+    for b, hq, hkv, s, *_ in backward.USED:
+        assert lib.backward(s, s, (s + 127) // 128 * b * hkv, hq // hkv)
+        assert lib.forward(s, 1, (s + 255) // 256 * b * hq, hq, b, 0) and lib.clusters(s, s, 1, -1, -1, b * hq) == 1

@@ -371,24 +371,24 @@ dq_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                     ptx::tmem_ld32(tl + C::kColDQ + half * (D / 2) + c * 32, r);
                     ptx::tmem_ld_wait();
                     if (q_valid) {
-                    if (sizeof(TOut) == 4) {
-                        float4* d4 = reinterpret_cast<float4*>(dst + c * 32);
+                        if (sizeof(TOut) == 4) {
+                            float4* d4 = reinterpret_cast<float4*>(dst + c * 32);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            d4[e] = make_float4(__uint_as_float(r[4 * e]) * a.scale, __uint_as_float(r[4 * e + 1]) * a.scale,
-                                                __uint_as_float(r[4 * e + 2]) * a.scale, __uint_as_float(r[4 * e + 3]) * a.scale);
-                    } else {
-                        uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
+                            for (int e = 0; e < 8; ++e)
+                                d4[e] = make_float4(__uint_as_float(r[4 * e]) * a.scale, __uint_as_float(r[4 * e + 1]) * a.scale,
+                                                    __uint_as_float(r[4 * e + 2]) * a.scale, __uint_as_float(r[4 * e + 3]) * a.scale);
+                        } else {
+                            uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            uint4 o;
-                            o.x = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 0]) * a.scale, __uint_as_float(r[8 * e + 1]) * a.scale);
-                            o.y = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 2]) * a.scale, __uint_as_float(r[8 * e + 3]) * a.scale);
-                            o.z = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 4]) * a.scale, __uint_as_float(r[8 * e + 5]) * a.scale);
-                            o.w = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 6]) * a.scale, __uint_as_float(r[8 * e + 7]) * a.scale);
-                            d4[e] = o;
+                            for (int e = 0; e < 4; ++e) {
+                                uint4 o;
+                                o.x = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 0]) * a.scale, __uint_as_float(r[8 * e + 1]) * a.scale);
+                                o.y = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 2]) * a.scale, __uint_as_float(r[8 * e + 3]) * a.scale);
+                                o.z = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 4]) * a.scale, __uint_as_float(r[8 * e + 5]) * a.scale);
+                                o.w = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 6]) * a.scale, __uint_as_float(r[8 * e + 7]) * a.scale);
+                                d4[e] = o;
+                            }
                         }
-                    }
                     }
                     __syncwarp();  // reconverge before the next warp-wide load
                 }

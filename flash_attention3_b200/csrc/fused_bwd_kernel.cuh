@@ -846,231 +846,231 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
             int g = 0;  // step, counted over all tiles
 #pragma unroll 1
             for (bool more = !misaligned; more; ++n) {
-            w.n_steps = uniform(w.n_steps);
-            w.kt = uniform(w.kt);
-            w.q_begin = uniform(w.q_begin);
-            w.steps_per_head = uniform(w.steps_per_head);
-            w.rotation = uniform(w.rotation);
-            w.q_tiles = uniform(w.q_tiles);
-            StepWalk<kCausal> st(w);
+                w.n_steps = uniform(w.n_steps);
+                w.kt = uniform(w.kt);
+                w.q_begin = uniform(w.q_begin);
+                w.steps_per_head = uniform(w.steps_per_head);
+                w.rotation = uniform(w.rotation);
+                w.q_tiles = uniform(w.q_tiles);
+                StepWalk<kCausal> st(w);
 #pragma unroll 1
-            for (int t = 0; t < w.n_steps; ++t, ++g, st.next(w)) {
-                const bool traced = warp == 4 && n == 0 && t < 7;
-                if (traced && t == 3) TRACE(2, 0);
-                const int qt = st.qt;
-                const int buf = g & 1;
-                const uint32_t negp = stats + buf * 512;
-                const uint32_t delp = stats + 1024 + buf * 512;
-                if (!(ok = warp_wait2(bar(kStatsFull + buf), (g >> 1) & 1, bar(kSFull), g & 1, abort_flag))) break;
-                if (traced) TRACE(2, 4 + 8 * t + 1);
-                ptx::tc_fence_after();
-                // A tile that crosses an edge of the w.band or holds keys past the end of the sequence is
-                // masked: element (key j, query i) survives iff mask_from <= i <= mask_to.
-                const bool diagonal = kCausal && tile_needs_mask(w.kt, qt, w.band);
-                int mask_from = 0, mask_to = 0;  // set only on masked tiles
-                // ---- P^T = exp2(S^T * scale_log2 + neg_i), masked as above: 32 scores from column `first` of this half on;
-                // p: their P, two in a register
-                // (two copies of the code, so that unmasked tiles carry no per-element test)
-                auto softmax_cols = [&](int first, const uint32_t* r, uint32_t* p, auto masked_tag) {
-                    constexpr bool kMasked = decltype(masked_tag)::value;
+                for (int t = 0; t < w.n_steps; ++t, ++g, st.next(w)) {
+                    const bool traced = warp == 4 && n == 0 && t < 7;
+                    if (traced && t == 3) TRACE(2, 0);
+                    const int qt = st.qt;
+                    const int buf = g & 1;
+                    const uint32_t negp = stats + buf * 512;
+                    const uint32_t delp = stats + 1024 + buf * 512;
+                    if (!(ok = warp_wait2(bar(kStatsFull + buf), (g >> 1) & 1, bar(kSFull), g & 1, abort_flag))) break;
+                    if (traced) TRACE(2, 4 + 8 * t + 1);
+                    ptx::tc_fence_after();
+                    // A tile that crosses an edge of the band or holds keys past the end of the sequence is
+                    // masked: element (key j, query i) survives iff mask_from <= i <= mask_to.
+                    const bool diagonal = kCausal && tile_needs_mask(w.kt, qt, w.band);
+                    int mask_from = 0, mask_to = 0;  // set only on masked tiles
+                    // ---- P^T = exp2(S^T * scale_log2 + neg_i), masked as above: 32 scores from column `first` of this half on;
+                    // p: their P, two in a register
+                    // (two copies of the code, so that unmasked tiles carry no per-element test)
+                    auto softmax_cols = [&](int first, const uint32_t* r, uint32_t* p, auto masked_tag) {
+                        constexpr bool kMasked = decltype(masked_tag)::value;
 #pragma unroll
-                    for (int e = 0; e < 32; e += 4) {
-                        float slope_p[4];
-                        const ptx::F4Pairs n4 = ptx::f2_ld_shared(negp + (first + e) * 4);
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const uint64_t neg2 = h == 0 ? n4.lo : n4.hi;
-                            const int el = e + 2 * h;
-                            // score in log2 units, relative to the row's reference: s * scale*log2e + (log2 r - m), or the
-                            // capped score + (log2 r - m)
-                            const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[el]), __uint_as_float(r[el + 1]));
-                            uint64_t t2 = 0;
-                            if constexpr (kSoftcap) t2 = ptx::tanh_mixed<C::kTanhFmaPairs>(ptx::f2_mul(s2, pre2), el / 2);
-                            // (exp2_poly for a part of these changed nothing: B=4,H=16,S=4096,D=64 791, 792, 795, 810 us for 0 to 3
-                            // pairs of 8)
-                            float2 p2 = ptx::f2_unpack(kSoftcap ? ptx::f2_fma(t2, post2, neg2) : ptx::f2_fma(s2, scale2, neg2));
-                            p2.x = ptx::ex2_approx(p2.x);
-                            p2.y = ptx::ex2_approx(p2.y);
-                            float2 w2;
-                            if constexpr (kSoftcap) {
-                                const float2 tt = ptx::f2_unpack(t2);
-                                w2 = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p2.x, p2.y),
-                                                                ptx::f2_pack(fmaf(-tt.x, tt.x, 1.0f), fmaf(-tt.y, tt.y, 1.0f))));
-                            }
-                            if (kMasked) {
-                                const int i = half * 64 + first + el;
-                                const bool sees0 = i + 0 >= mask_from && i + 0 <= mask_to, sees1 = i + 1 >= mask_from && i + 1 <= mask_to;
-                                p2.x = sees0 ? p2.x : 0.0f;
-                                p2.y = sees1 ? p2.y : 0.0f;
-                                if constexpr (kSoftcap) {
-                                    w2.x = sees0 ? w2.x : 0.0f;
-                                    w2.y = sees1 ? w2.y : 0.0f;
-                                }
-                            }
-                            p[el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
-                            if constexpr (kSoftcap) {
-                                slope_p[2 * h] = w2.x;
-                                slope_p[2 * h + 1] = w2.y;
-                            }
-                        }
-                        if constexpr (kSoftcap) ptx::pack24(slope_p, &ppk[(first + e) / 4 * 3]);
-                    }
-                };
-                auto softmax_phase = [&](auto masked_tag) {
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) {
-                        uint32_t r[32], capped_p[16];  // (capped_p: P where ppk holds P (1 - t^2))
-                        uint32_t* p = kSoftcap ? capped_p : &ppk[c * 16];
-                        ptx::tmem_ld32(s_cols + c * 32, r);
-                        ptx::tmem_ld_wait();
-                        softmax_cols(c * 32, r, p, masked_tag);
-                        ptx::tmem_st16(s_cols + c * 16, p);  // P chunk c -> columns [16c, 16c+16) of this half's S columns (already read)
-                    }
-                };
-                if (diagonal) {
-                    query_range_of_key(w.kt * C::kTile + j, qt * C::kTile, w.band, &mask_from, &mask_to);
-                    softmax_phase(std::true_type{});
-                } else {
-                    softmax_phase(std::false_type{});
-                }
-                if (traced) TRACE(2, 4 + 8 * t + 2);
-                ptx::tmem_st_wait();
-                arrive(kPReady);
-                if (traced) TRACE(2, 4 + 8 * t + 3);
-                // ---- dS^T = P^T * (dP^T - delta_i), stored [key][query] in the 128-byte swizzle
-                if (!(ok = warp_wait(bar(kDpFull), g & 1, abort_flag))) break;
-                if (traced) TRACE(2, 4 + 8 * t + 4);
-                // (the dS buffer is free: dP was issued behind dK and dQ of the step before, the readers of its dS,
-                // and the barrier just passed completes only when every MMA issued before it has)
-                if (traced) TRACE(2, 4 + 8 * t + 5);
-                ptx::tc_fence_after();
-                const uint32_t ds_row = sbase + C::kOffDS + half * C::kBoxBytes + j * 128;
-                auto ds_chunk = [&](int c, const uint32_t* r) {
-#pragma unroll
-                    for (int e = 0; e < 32; e += 8) {
-                        uint32_t o[4];
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            const ptx::F4Pairs d4 = ptx::f2_ld_shared(delp + (c * 32 + e + 4 * h) * 4);  // -delta
-                            const int el = e + 4 * h;
+                        for (int e = 0; e < 32; e += 4) {
                             float slope_p[4];
-                            if constexpr (kSoftcap) ptx::unpack24(&ppk[c * 24 + el / 4 * 3], slope_p);
+                            const ptx::F4Pairs n4 = ptx::f2_ld_shared(negp + (first + e) * 4);
 #pragma unroll
-                            for (int g = 0; g < 2; ++g) {
-                                const float2 p = kSoftcap ? make_float2(slope_p[2 * g], slope_p[2 * g + 1]) : ptx::Pack2<T>::unpack(ppk[c * 16 + el / 2 + g]);
-                                const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[el + 2 * g]), __uint_as_float(r[el + 2 * g + 1]));
-                                const float2 ds = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, g == 0 ? d4.lo : d4.hi)));
-                                o[2 * h + g] = ptx::Pack2<T>::pack(ds.x, ds.y);
-                            }
-                        }
-                        const int chunk = c * 4 + e / 8;  // 16-byte chunk inside this half's box
-                        const uint32_t addr = ds_row + ((chunk ^ (j & 7)) << 4);
-                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(o[0]),
-                                     "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-                    }
-                };
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    uint32_t r[32];
-                    ptx::tmem_ld32(dp_cols + c * 32, r);
-                    ptx::tmem_ld_wait();
-                    ds_chunk(c, r);
-                }
-                if (traced) TRACE(2, 4 + 8 * t + 6);
-                ptx::fence_proxy_async_smem();
-                arrive(kDsReady);
-                if (lane == 0) ptx::mbar_arrive(bar(kStatsEmpty + buf));
-                if (traced) TRACE(2, 4 + 8 * t + 7);
-            }
-            // ---- epilogue: the first warpgroup writes dK (scaled), the second dV
-            if (!ok) break;
-            if constexpr (kSoftcap) w = load_work(work);  // (what only the epilogue needs is not held in registers before)
-            const int w4 = warp & 3;  // which 32 rows of the tile
-            const bool has_steps = w.n_steps > 0;
-            const int64_t slab = int64_t(w.slab * 2 + half) * (C::kTile * D) + w4 * 32 * D;
-            const int rows = w.slot_k - (w.kt * C::kTile + w4 * 32);
-            // (rows between the used length and the end of the slot hold exact zeros)
-            TOut* out = reinterpret_cast<TOut*>(half == 0 ? a.dk : a.dv) + w.b_coord * a.kv_strides.batch +
-                        w.kvh * a.kv_strides.head + int64_t(w.k_base + w.kt * C::kTile + w4 * 32) * a.kv_strides.row;
-            more = next_tile(n, &w);  // (while the last MMAs of this one run)
-            if (has_steps && !(ok = warp_wait(bar(kDkvFull), used & 1, abort_flag))) break;
-            if (warp == 4 && n == 0) TRACE(2, 60);
-            if (has_steps) {
-                // Every MMA of the tile has completed.  Each warp stages its 32 key rows in shared memory and stores them again in
-                // whole lines: over the dead Q / dO / dS^T buffers, 512 contiguous bytes (or two rows) per instruction, or, where
-                // the next tile's Q and dO are being loaded, over its own rows of dS^T, 128 bytes of each row at a time.
-                // (Stores through the copy engine queue behind the drain's last reduce-adds, about 2700 clk at D=128; a thread
-                // storing its own row straight from registers writes 16 bytes per line and instruction.)
-                ++used;
-                ptx::tc_fence_after();
-                const float mul = half == 0 ? a.scale : 1.0f;
-                const uint32_t col0 = tl + (half == 0 ? C::kColDK : C::kColDV);
-                // rows of element type O at dst, `pitch` elements apart, of which the first `rows_here` are written
-                auto store_rows = [&](auto tag, void* dst_rows, int64_t pitch, int rows_here) {
-                    using O = decltype(tag);
-                    constexpr int kPass = kPersist ? 128 : D * int(sizeof(O));  // bytes of a row
-                    constexpr int kCols = kPass / int(sizeof(O));
-                    constexpr int kChunks = kPass / 16;
-                    constexpr int kPerLoad = 32 * int(sizeof(O)) / 16;  // 16-byte chunks of 32 columns
-                    constexpr int kRowsAtOnce = 32 / kChunks;
-                    const uint32_t scratch = sbase + (kPersist ? C::kOffDS + half * C::kBoxBytes + w4 * 32 * kPass
-                                                               : C::kOffQ + (half * 4 + w4) * 32 * kPass);
-                    const int sub = lane / kChunks, ch = lane % kChunks;
-                    O* dst = static_cast<O*>(dst_rows) + ch * (16 / int(sizeof(O)));
-#pragma unroll 1
-                    for (int col = 0; col < D; col += kCols) {
-#pragma unroll
-                        for (int c = 0; c < kCols / 32; ++c) {
-                            uint32_t r[32];
-                            ptx::tmem_ld32(col0 + col + c * 32, r);
-                            ptx::tmem_ld_wait();
-#pragma unroll
-                            for (int e = 0; e < kPerLoad; ++e) {
-                                uint32_t o[4];
-#pragma unroll
-                                for (int h = 0; h < 4; ++h) {
-                                    if constexpr (sizeof(O) == 4) {
-                                        o[h] = __float_as_uint(__uint_as_float(r[4 * e + h]) * mul);
-                                    } else {
-                                        o[h] = ptx::Pack2<O>::pack(__uint_as_float(r[8 * e + 2 * h]) * mul, __uint_as_float(r[8 * e + 2 * h + 1]) * mul);
+                            for (int h = 0; h < 2; ++h) {
+                                const uint64_t neg2 = h == 0 ? n4.lo : n4.hi;
+                                const int el = e + 2 * h;
+                                // score in log2 units, relative to the row's reference: s * scale*log2e + (log2 r - m), or the
+                                // capped score + (log2 r - m)
+                                const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[el]), __uint_as_float(r[el + 1]));
+                                uint64_t t2 = 0;
+                                if constexpr (kSoftcap) t2 = ptx::tanh_mixed<C::kTanhFmaPairs>(ptx::f2_mul(s2, pre2), el / 2);
+                                // (exp2_poly for a part of these changed nothing: B=4,H=16,S=4096,D=64 791, 792, 795, 810 us for 0 to 3
+                                // pairs of 8)
+                                float2 p2 = ptx::f2_unpack(kSoftcap ? ptx::f2_fma(t2, post2, neg2) : ptx::f2_fma(s2, scale2, neg2));
+                                p2.x = ptx::ex2_approx(p2.x);
+                                p2.y = ptx::ex2_approx(p2.y);
+                                float2 w2;
+                                if constexpr (kSoftcap) {
+                                    const float2 tt = ptx::f2_unpack(t2);
+                                    w2 = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p2.x, p2.y),
+                                                                    ptx::f2_pack(fmaf(-tt.x, tt.x, 1.0f), fmaf(-tt.y, tt.y, 1.0f))));
+                                }
+                                if (kMasked) {
+                                    const int i = half * 64 + first + el;
+                                    const bool sees0 = i + 0 >= mask_from && i + 0 <= mask_to, sees1 = i + 1 >= mask_from && i + 1 <= mask_to;
+                                    p2.x = sees0 ? p2.x : 0.0f;
+                                    p2.y = sees1 ? p2.y : 0.0f;
+                                    if constexpr (kSoftcap) {
+                                        w2.x = sees0 ? w2.x : 0.0f;
+                                        w2.y = sees1 ? w2.y : 0.0f;
                                     }
                                 }
-                                const int chunk = (c * kPerLoad + e) ^ (lane & 7);  // (spread over the banks)
-                                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
-                                             ::"r"(scratch + lane * kPass + chunk * 16), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+                                p[el / 2] = ptx::Pack2<T>::pack(p2.x, p2.y);
+                                if constexpr (kSoftcap) {
+                                    slope_p[2 * h] = w2.x;
+                                    slope_p[2 * h + 1] = w2.y;
+                                }
                             }
+                            if constexpr (kSoftcap) ptx::pack24(slope_p, &ppk[(first + e) / 4 * 3]);
                         }
-                        __syncwarp();
-#pragma unroll 8
-                        for (int row = sub; row < 32; row += kRowsAtOnce) {
-                            uint4 v;
-                            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                                         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                                         : "r"(scratch + row * kPass + ((ch ^ (row & 7)) << 4)) : "memory");
-                            if (row < rows_here) *reinterpret_cast<uint4*>(dst + row * pitch + col) = v;
-                        }
-                        __syncwarp();
-                    }
-                };
-                if (kWithDq && a.chunk_steps > 0) {
-                    // a share of a split tile: the partial sums go to this CTA's slabs (slab 2x: dK, 2x+1: dV).  fp32, but
-                    // fp16 for fp16 inputs where the tiles are fewer than the SMs: the bytes written, not the arithmetic,
-                    // bound this epilogue.  (With as many tiles as SMs, fp16 slabs had taken dK and dV, whose sums stay in
-                    // tensor memory when their tile is not split, 1.16 and 1.23 times as far from the exact values.)
-                    if (!kBf16 && a.slabs_f16) store_rows(__half{}, static_cast<__half*>(a.dkv_slabs) + slab, D, 32);
-                    else store_rows(float{}, static_cast<float*>(a.dkv_slabs) + slab, D, 32);
-                } else {
-                    store_rows(TOut{}, out, a.kv_strides.row, rows);
-                }
-            } else if (a.chunk_steps == 0) {
-                // nobody attends to these keys (possible with a left-bounded window), but dK / dV still owe zeros
-                if (lane < rows) {
-                    uint4* d4 = reinterpret_cast<uint4*>(out + lane * a.kv_strides.row);
+                    };
+                    auto softmax_phase = [&](auto masked_tag) {
 #pragma unroll
-                    for (int e = 0; e < int(D * sizeof(TOut) / 16); ++e) d4[e] = make_uint4(0u, 0u, 0u, 0u);
+                        for (int c = 0; c < 2; ++c) {
+                            uint32_t r[32], capped_p[16];  // (capped_p: P where ppk holds P (1 - t^2))
+                            uint32_t* p = kSoftcap ? capped_p : &ppk[c * 16];
+                            ptx::tmem_ld32(s_cols + c * 32, r);
+                            ptx::tmem_ld_wait();
+                            softmax_cols(c * 32, r, p, masked_tag);
+                            ptx::tmem_st16(s_cols + c * 16, p);  // P chunk c -> columns [16c, 16c+16) of this half's S columns (already read)
+                        }
+                    };
+                    if (diagonal) {
+                        query_range_of_key(w.kt * C::kTile + j, qt * C::kTile, w.band, &mask_from, &mask_to);
+                        softmax_phase(std::true_type{});
+                    } else {
+                        softmax_phase(std::false_type{});
+                    }
+                    if (traced) TRACE(2, 4 + 8 * t + 2);
+                    ptx::tmem_st_wait();
+                    arrive(kPReady);
+                    if (traced) TRACE(2, 4 + 8 * t + 3);
+                    // ---- dS^T = P^T * (dP^T - delta_i), stored [key][query] in the 128-byte swizzle
+                    if (!(ok = warp_wait(bar(kDpFull), g & 1, abort_flag))) break;
+                    if (traced) TRACE(2, 4 + 8 * t + 4);
+                    // (the dS buffer is free: dP was issued behind dK and dQ of the step before, the readers of its dS,
+                    // and the barrier just passed completes only when every MMA issued before it has)
+                    if (traced) TRACE(2, 4 + 8 * t + 5);
+                    ptx::tc_fence_after();
+                    const uint32_t ds_row = sbase + C::kOffDS + half * C::kBoxBytes + j * 128;
+                    auto ds_chunk = [&](int c, const uint32_t* r) {
+#pragma unroll
+                        for (int e = 0; e < 32; e += 8) {
+                            uint32_t o[4];
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) {
+                                const ptx::F4Pairs d4 = ptx::f2_ld_shared(delp + (c * 32 + e + 4 * h) * 4);  // -delta
+                                const int el = e + 4 * h;
+                                float slope_p[4];
+                                if constexpr (kSoftcap) ptx::unpack24(&ppk[c * 24 + el / 4 * 3], slope_p);
+#pragma unroll
+                                for (int g = 0; g < 2; ++g) {
+                                    const float2 p = kSoftcap ? make_float2(slope_p[2 * g], slope_p[2 * g + 1]) : ptx::Pack2<T>::unpack(ppk[c * 16 + el / 2 + g]);
+                                    const uint64_t dp2 = ptx::f2_pack(__uint_as_float(r[el + 2 * g]), __uint_as_float(r[el + 2 * g + 1]));
+                                    const float2 ds = ptx::f2_unpack(ptx::f2_mul(ptx::f2_pack(p.x, p.y), ptx::f2_add(dp2, g == 0 ? d4.lo : d4.hi)));
+                                    o[2 * h + g] = ptx::Pack2<T>::pack(ds.x, ds.y);
+                                }
+                            }
+                            const int chunk = c * 4 + e / 8;  // 16-byte chunk inside this half's box
+                            const uint32_t addr = ds_row + ((chunk ^ (j & 7)) << 4);
+                            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(o[0]),
+                                         "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+                        }
+                    };
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        uint32_t r[32];
+                        ptx::tmem_ld32(dp_cols + c * 32, r);
+                        ptx::tmem_ld_wait();
+                        ds_chunk(c, r);
+                    }
+                    if (traced) TRACE(2, 4 + 8 * t + 6);
+                    ptx::fence_proxy_async_smem();
+                    arrive(kDsReady);
+                    if (lane == 0) ptx::mbar_arrive(bar(kStatsEmpty + buf));
+                    if (traced) TRACE(2, 4 + 8 * t + 7);
                 }
-            }
-            if (warp == 4 && n == 0) TRACE(2, 61);
+                // ---- epilogue: the first warpgroup writes dK (scaled), the second dV
+                if (!ok) break;
+                if constexpr (kSoftcap) w = load_work(work);  // (what only the epilogue needs is not held in registers before)
+                const int w4 = warp & 3;  // which 32 rows of the tile
+                const bool has_steps = w.n_steps > 0;
+                const int64_t slab = int64_t(w.slab * 2 + half) * (C::kTile * D) + w4 * 32 * D;
+                const int rows = w.slot_k - (w.kt * C::kTile + w4 * 32);
+                // (rows between the used length and the end of the slot hold exact zeros)
+                TOut* out = reinterpret_cast<TOut*>(half == 0 ? a.dk : a.dv) + w.b_coord * a.kv_strides.batch +
+                            w.kvh * a.kv_strides.head + int64_t(w.k_base + w.kt * C::kTile + w4 * 32) * a.kv_strides.row;
+                more = next_tile(n, &w);  // (while the last MMAs of this one run)
+                if (has_steps && !(ok = warp_wait(bar(kDkvFull), used & 1, abort_flag))) break;
+                if (warp == 4 && n == 0) TRACE(2, 60);
+                if (has_steps) {
+                    // Every MMA of the tile has completed.  Each warp stages its 32 key rows in shared memory and stores them again in
+                    // whole lines: over the dead Q / dO / dS^T buffers, 512 contiguous bytes (or two rows) per instruction, or, where
+                    // the next tile's Q and dO are being loaded, over its own rows of dS^T, 128 bytes of each row at a time.
+                    // (Stores through the copy engine queue behind the drain's last reduce-adds, about 2700 clk at D=128; a thread
+                    // storing its own row straight from registers writes 16 bytes per line and instruction.)
+                    ++used;
+                    ptx::tc_fence_after();
+                    const float mul = half == 0 ? a.scale : 1.0f;
+                    const uint32_t col0 = tl + (half == 0 ? C::kColDK : C::kColDV);
+                    // rows of element type O at dst, `pitch` elements apart, of which the first `rows_here` are written
+                    auto store_rows = [&](auto tag, void* dst_rows, int64_t pitch, int rows_here) {
+                        using O = decltype(tag);
+                        constexpr int kPass = kPersist ? 128 : D * int(sizeof(O));  // bytes of a row
+                        constexpr int kCols = kPass / int(sizeof(O));
+                        constexpr int kChunks = kPass / 16;
+                        constexpr int kPerLoad = 32 * int(sizeof(O)) / 16;  // 16-byte chunks of 32 columns
+                        constexpr int kRowsAtOnce = 32 / kChunks;
+                        const uint32_t scratch = sbase + (kPersist ? C::kOffDS + half * C::kBoxBytes + w4 * 32 * kPass
+                                                                   : C::kOffQ + (half * 4 + w4) * 32 * kPass);
+                        const int sub = lane / kChunks, ch = lane % kChunks;
+                        O* dst = static_cast<O*>(dst_rows) + ch * (16 / int(sizeof(O)));
+#pragma unroll 1
+                        for (int col = 0; col < D; col += kCols) {
+#pragma unroll
+                            for (int c = 0; c < kCols / 32; ++c) {
+                                uint32_t r[32];
+                                ptx::tmem_ld32(col0 + col + c * 32, r);
+                                ptx::tmem_ld_wait();
+#pragma unroll
+                                for (int e = 0; e < kPerLoad; ++e) {
+                                    uint32_t o[4];
+#pragma unroll
+                                    for (int h = 0; h < 4; ++h) {
+                                        if constexpr (sizeof(O) == 4) {
+                                            o[h] = __float_as_uint(__uint_as_float(r[4 * e + h]) * mul);
+                                        } else {
+                                            o[h] = ptx::Pack2<O>::pack(__uint_as_float(r[8 * e + 2 * h]) * mul, __uint_as_float(r[8 * e + 2 * h + 1]) * mul);
+                                        }
+                                    }
+                                    const int chunk = (c * kPerLoad + e) ^ (lane & 7);  // (spread over the banks)
+                                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                                                 ::"r"(scratch + lane * kPass + chunk * 16), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+                                }
+                            }
+                            __syncwarp();
+#pragma unroll 8
+                            for (int row = sub; row < 32; row += kRowsAtOnce) {
+                                uint4 v;
+                                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                                             : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                                             : "r"(scratch + row * kPass + ((ch ^ (row & 7)) << 4)) : "memory");
+                                if (row < rows_here) *reinterpret_cast<uint4*>(dst + row * pitch + col) = v;
+                            }
+                            __syncwarp();
+                        }
+                    };
+                    if (kWithDq && a.chunk_steps > 0) {
+                        // a share of a split tile: the partial sums go to this CTA's slabs (slab 2x: dK, 2x+1: dV).  fp32, but
+                        // fp16 for fp16 inputs where the tiles are fewer than the SMs: the bytes written, not the arithmetic,
+                        // bound this epilogue.  (With as many tiles as SMs, fp16 slabs had taken dK and dV, whose sums stay in
+                        // tensor memory when their tile is not split, 1.16 and 1.23 times as far from the exact values.)
+                        if (!kBf16 && a.slabs_f16) store_rows(__half{}, static_cast<__half*>(a.dkv_slabs) + slab, D, 32);
+                        else store_rows(float{}, static_cast<float*>(a.dkv_slabs) + slab, D, 32);
+                    } else {
+                        store_rows(TOut{}, out, a.kv_strides.row, rows);
+                    }
+                } else if (a.chunk_steps == 0) {
+                    // nobody attends to these keys (possible with a left-bounded window), but dK / dV still owe zeros
+                    if (lane < rows) {
+                        uint4* d4 = reinterpret_cast<uint4*>(out + lane * a.kv_strides.row);
+#pragma unroll
+                        for (int e = 0; e < int(D * sizeof(TOut) / 16); ++e) d4[e] = make_uint4(0u, 0u, 0u, 0u);
+                    }
+                }
+                if (warp == 4 && n == 0) TRACE(2, 61);
             }
         }
     } else {
@@ -1095,56 +1095,56 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 int g = 0;
 #pragma unroll 1
                 for (bool more = !misaligned; more; ++n) {
-                StepWalk<kCausal> st(w);
+                    StepWalk<kCausal> st(w);
 #pragma unroll 1
-                for (int t = 0; t < w.n_steps; ++t, ++g, st.next(w)) {
-                    const bool traced = warp == 12 && n == 0 && t < 12;
-                    const int q_row = st.qt * C::kTile + qd * 32;  // row inside the head
-                    const int q_head = w.b_coord * a.heads_q + st.hq;
-                    if (!(ok = warp_wait(bar(kDqFull), g & 1, abort_flag))) break;
-                    if (traced) TRACE(3, 4 + 4 * t + 0);
-                    ptx::tc_fence_after();
-                    // pull the whole dQ tile row into registers and hand the columns back at once
-                    uint32_t r[D / 32][32];
+                    for (int t = 0; t < w.n_steps; ++t, ++g, st.next(w)) {
+                        const bool traced = warp == 12 && n == 0 && t < 12;
+                        const int q_row = st.qt * C::kTile + qd * 32;  // row inside the head
+                        const int q_head = w.b_coord * a.heads_q + st.hq;
+                        if (!(ok = warp_wait(bar(kDqFull), g & 1, abort_flag))) break;
+                        if (traced) TRACE(3, 4 + 4 * t + 0);
+                        ptx::tc_fence_after();
+                        // pull the whole dQ tile row into registers and hand the columns back at once
+                        uint32_t r[D / 32][32];
 #pragma unroll
-                    for (int c = 0; c < D / 32; ++c) ptx::tmem_ld32(tl + C::kColDQ + c * 32, r[c]);
-                    ptx::tmem_ld_wait();
-                    ptx::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(bar(kDqEmpty));
-                    if (traced) TRACE(3, 4 + 4 * t + 1);
-#pragma unroll
-                    for (int hf = 0; hf < D / 64; ++hf) {
-                        if (pending) {
-                            if (lane == 0) ptx::bulk_wait_group_read<0>();
-                            __syncwarp();
-                        }
-#pragma unroll
-                        for (int bx = 0; bx < 2; ++bx) {
-                            const uint32_t row_addr = stage + bx * C::kStageBoxBytes + lane * 128;
-#pragma unroll
-                            for (int c = 0; c < 8; ++c) {
-                                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
-                                             ::"r"(row_addr + ((c ^ (lane & 7)) << 4)), "r"(r[hf * 2 + bx][4 * c]),
-                                               "r"(r[hf * 2 + bx][4 * c + 1]), "r"(r[hf * 2 + bx][4 * c + 2]),
-                                               "r"(r[hf * 2 + bx][4 * c + 3])
-                                             : "memory");
-                            }
-                        }
-                        ptx::fence_proxy_async_smem();
+                        for (int c = 0; c < D / 32; ++c) ptx::tmem_ld32(tl + C::kColDQ + c * 32, r[c]);
+                        ptx::tmem_ld_wait();
+                        ptx::tc_fence_before();
                         __syncwarp();
-                        // accumulator map: [batch*head][row][D]; rows past the sequence end are dropped
-                        if (lane == 0 && q_row < w.band.seqlen_q) {
-                            ptx::tma_reduce_add_3d(&tm_dqacc, stage, hf * 64, w.q_base + q_row, q_head);
-                            ptx::tma_reduce_add_3d(&tm_dqacc, stage + C::kStageBoxBytes, hf * 64 + 32, w.q_base + q_row, q_head);
-                            ptx::bulk_commit_group();
+                        if (lane == 0) ptx::mbar_arrive(bar(kDqEmpty));
+                        if (traced) TRACE(3, 4 + 4 * t + 1);
+#pragma unroll
+                        for (int hf = 0; hf < D / 64; ++hf) {
+                            if (pending) {
+                                if (lane == 0) ptx::bulk_wait_group_read<0>();
+                                __syncwarp();
+                            }
+#pragma unroll
+                            for (int bx = 0; bx < 2; ++bx) {
+                                const uint32_t row_addr = stage + bx * C::kStageBoxBytes + lane * 128;
+#pragma unroll
+                                for (int c = 0; c < 8; ++c) {
+                                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                                                 ::"r"(row_addr + ((c ^ (lane & 7)) << 4)), "r"(r[hf * 2 + bx][4 * c]),
+                                                   "r"(r[hf * 2 + bx][4 * c + 1]), "r"(r[hf * 2 + bx][4 * c + 2]),
+                                                   "r"(r[hf * 2 + bx][4 * c + 3])
+                                                 : "memory");
+                                }
+                            }
+                            ptx::fence_proxy_async_smem();
+                            __syncwarp();
+                            // accumulator map: [batch*head][row][D]; rows past the sequence end are dropped
+                            if (lane == 0 && q_row < w.band.seqlen_q) {
+                                ptx::tma_reduce_add_3d(&tm_dqacc, stage, hf * 64, w.q_base + q_row, q_head);
+                                ptx::tma_reduce_add_3d(&tm_dqacc, stage + C::kStageBoxBytes, hf * 64 + 32, w.q_base + q_row, q_head);
+                                ptx::bulk_commit_group();
+                            }
+                            pending = true;
                         }
-                        pending = true;
+                        if (traced) TRACE(3, 4 + 4 * t + 2);
                     }
-                    if (traced) TRACE(3, 4 + 4 * t + 2);
-                }
-                if (!ok) break;
-                more = next_tile(n, &w);
+                    if (!ok) break;
+                    more = next_tile(n, &w);
                 }
                 if (lane == 0) ptx::bulk_wait_group<0>();
                 if (warp == 12) TRACE(3, 59);

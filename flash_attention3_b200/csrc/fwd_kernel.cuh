@@ -491,89 +491,89 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             bool ok = true;
 #pragma unroll 1
             for (bool next = true; ok && next; ++n) {
-            const int n_iter = w.n_iter;
-            if (n_iter == 0) request();
-#pragma unroll
-            for (int x = 0; x < 2; ++x) {
-                if (ok && w.lo[x] < w.hi[x]) ok = warp_wait<false>(bar(kFwdQFull + x), used[x]++ & 1, abort_flag);
-            }
-            if (ok && n_iter > 0) ok = wait_k(0);
-            if (ok && n_iter > 0) {
-                ptx::tc_fence_after();
+                const int n_iter = w.n_iter;
+                if (n_iter == 0) request();
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    if (ok && w.active(x, 0)) {
-                        if (C::kOwnP) {
-                            ok = wait_s_free(x, 0);
-                            ptx::tc_fence_after();
-                        }
-                        if (ok) issue_s(x, 0);
-                    }
+                    if (ok && w.lo[x] < w.hi[x]) ok = warp_wait<false>(bar(kFwdQFull + x), used[x]++ & 1, abort_flag);
                 }
-                ptx::tc_commit_elect(bar(kFwdKEmpty + g0 % C::kStages));
-            }
-            if constexpr (!C::kOwnP) {
-#pragma unroll 1
-                for (int it = 0; ok && it < n_iter; ++it) {
-                    const bool more = it + 1 < n_iter;
-                    if (!more) request();
-                    bool v_ready = false, k_ready = false;
+                if (ok && n_iter > 0) ok = wait_k(0);
+                if (ok && n_iter > 0) {
+                    ptx::tc_fence_after();
 #pragma unroll
                     for (int x = 0; x < 2; ++x) {
-                        if (w.active(x, it)) {
-                            if (!v_ready) {
-                                if (!(ok = wait_v(it))) break;
-                                v_ready = true;
-                            }
-                            if (!(ok = issue_pv(x, it))) break;
-                        }
-                        // S of the next key tile goes over P of this one: it follows P V in the pipe
-                        if (more && w.active(x, it + 1)) {
-                            if (!k_ready) {
-                                if (!(ok = wait_k(it + 1))) break;
-                                k_ready = true;
+                        if (ok && w.active(x, 0)) {
+                            if (C::kOwnP) {
+                                ok = wait_s_free(x, 0);
                                 ptx::tc_fence_after();
                             }
-                            issue_s(x, it + 1);
+                            if (ok) issue_s(x, 0);
                         }
                     }
-                    if (!ok) break;
-                    if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + (g0 + it + 1) % C::kStages));
-                    ptx::tc_commit_elect(bar(kFwdVEmpty + (g0 + it) % C::kStages));
+                    ptx::tc_commit_elect(bar(kFwdKEmpty + g0 % C::kStages));
                 }
-            } else {
-                // S(x, it+1) needs only "scores (x, it) in registers"; P V of tile B is issued one half
-                // iteration late, because the two softmax warpgroups settle half an iteration apart
+                if constexpr (!C::kOwnP) {
 #pragma unroll 1
-                for (int it = 0; ok && n_iter > 0 && it <= n_iter; ++it) {
-                    const bool more = it + 1 < n_iter;
-                    if (it == n_iter - 1) request();
+                    for (int it = 0; ok && it < n_iter; ++it) {
+                        const bool more = it + 1 < n_iter;
+                        if (!more) request();
+                        bool v_ready = false, k_ready = false;
 #pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        if (more && w.active(x, it + 1)) {
-                            ok = wait_s_free(x, it + 1);
-                            if (!(ok = ok && wait_k(it + 1))) break;
-                            ptx::tc_fence_after();
-                            issue_s(x, it + 1);
+                        for (int x = 0; x < 2; ++x) {
+                            if (w.active(x, it)) {
+                                if (!v_ready) {
+                                    if (!(ok = wait_v(it))) break;
+                                    v_ready = true;
+                                }
+                                if (!(ok = issue_pv(x, it))) break;
+                            }
+                            // S of the next key tile goes over P of this one: it follows P V in the pipe
+                            if (more && w.active(x, it + 1)) {
+                                if (!k_ready) {
+                                    if (!(ok = wait_k(it + 1))) break;
+                                    k_ready = true;
+                                    ptx::tc_fence_after();
+                                }
+                                issue_s(x, it + 1);
+                            }
                         }
-                        // x = 0: P V of tile B, previous iteration; x = 1: P V of tile A, this iteration
-                        const int pv = it - (x == 0 ? 1 : 0);
-                        const int y = x ^ 1;
-                        if (pv < n_iter && w.active(y, pv)) {
-                            if (!(ok = wait_v(pv) && issue_pv(y, pv))) break;
-                        }
-                        if (x == 0 && it > 0) ptx::tc_commit_elect(bar(kFwdVEmpty + (g0 + it - 1) % C::kStages));
+                        if (!ok) break;
+                        if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + (g0 + it + 1) % C::kStages));
+                        ptx::tc_commit_elect(bar(kFwdVEmpty + (g0 + it) % C::kStages));
                     }
-                    if (!ok) break;
-                    if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + (g0 + it + 1) % C::kStages));
-                }
-            }
-            if (!ok) break;
-            if (n_iter > 0) ptx::tc_commit_elect(bar(kFwdAllDone));  // (waited for with one tile per CTA)
-            g0 += n_iter;
+                } else {
+                    // S(x, it+1) needs only "scores (x, it) in registers"; P V of tile B is issued one half
+                    // iteration late, because the two softmax warpgroups settle half an iteration apart
+#pragma unroll 1
+                    for (int it = 0; ok && n_iter > 0 && it <= n_iter; ++it) {
+                        const bool more = it + 1 < n_iter;
+                        if (it == n_iter - 1) request();
 #pragma unroll
-            for (int x = 0; x < 2; ++x) c[x] += max(0, w.hi[x] - w.lo[x]);
-            next = next_tile(n, &w);
+                        for (int x = 0; x < 2; ++x) {
+                            if (more && w.active(x, it + 1)) {
+                                ok = wait_s_free(x, it + 1);
+                                if (!(ok = ok && wait_k(it + 1))) break;
+                                ptx::tc_fence_after();
+                                issue_s(x, it + 1);
+                            }
+                            // x = 0: P V of tile B, previous iteration; x = 1: P V of tile A, this iteration
+                            const int pv = it - (x == 0 ? 1 : 0);
+                            const int y = x ^ 1;
+                            if (pv < n_iter && w.active(y, pv)) {
+                                if (!(ok = wait_v(pv) && issue_pv(y, pv))) break;
+                            }
+                            if (x == 0 && it > 0) ptx::tc_commit_elect(bar(kFwdVEmpty + (g0 + it - 1) % C::kStages));
+                        }
+                        if (!ok) break;
+                        if (more) ptx::tc_commit_elect(bar(kFwdKEmpty + (g0 + it + 1) % C::kStages));
+                    }
+                }
+                if (!ok) break;
+                if (n_iter > 0) ptx::tc_commit_elect(bar(kFwdAllDone));  // (waited for with one tile per CTA)
+                g0 += n_iter;
+#pragma unroll
+                for (int x = 0; x < 2; ++x) c[x] += max(0, w.hi[x] - w.lo[x]);
+                next = next_tile(n, &w);
             }
         } else if (warp == 2 && kPersist) {
             // which tile next
@@ -626,280 +626,280 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
             bool more = true;
 #pragma unroll 1
             for (; more; ++n) {
-            // (selects, not indexing: no local array; uniform: see there)
-            const int qt = uniform(x == 0 ? w.tile[0] : w.tile[1]);
-            const int n_steps = uniform(x == 0 ? w.hi[0] - w.lo[0] : w.hi[1] - w.lo[1]);
-            const int k_begin = w.t_begin + (x == 0 ? w.lo[0] : w.lo[1]);
-            const uint32_t tl = tmem + (uint32_t((warp & 3) * 32) << 16);
-            const uint32_t s_cols = tl + C::kColS + x * 128;
-            const uint32_t p_cols = tl + C::kColP + x * C::kPStride;
-            const uint32_t o_cols = tl + C::kColO + x * D;
-            const int qi = qt * C::kTile + i;  // query row inside the head
-            const bool q_valid = qi < w.band.seqlen_q;
-            float m_ref = -INFINITY;  // reference maximum (raw scores) the exponentials are taken against
-            float l = 0.0f;           // sum of the exponentials, in units of exp2(m_ref * scale_log2)
-            const float sl = kSoftcap ? a.softcap_post : a.scale_log2;  // log2 units per unit of (transformed) score
-            const uint64_t sl2 = ptx::f2_pack(sl, sl);
-            // one arrival per warp: every lane's accesses are ordered before it by the fence and the warp barrier
-            auto arrive = [&](int which) {
-                ptx::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(bar(which + x));
-            };
-            // key j of key tile k_begin + u survives for query i iff mask_from <= j <= mask_to
-            int mask_from = 0, mask_to = 0;
-            if (kMasked) key_range_of_query(qi, k_begin * C::kTile, w.band, &mask_from, &mask_to);
-            bool ok = true;
+                // (selects, not indexing: no local array; uniform: see there)
+                const int qt = uniform(x == 0 ? w.tile[0] : w.tile[1]);
+                const int n_steps = uniform(x == 0 ? w.hi[0] - w.lo[0] : w.hi[1] - w.lo[1]);
+                const int k_begin = w.t_begin + (x == 0 ? w.lo[0] : w.lo[1]);
+                const uint32_t tl = tmem + (uint32_t((warp & 3) * 32) << 16);
+                const uint32_t s_cols = tl + C::kColS + x * 128;
+                const uint32_t p_cols = tl + C::kColP + x * C::kPStride;
+                const uint32_t o_cols = tl + C::kColO + x * D;
+                const int qi = qt * C::kTile + i;  // query row inside the head
+                const bool q_valid = qi < w.band.seqlen_q;
+                float m_ref = -INFINITY;  // reference maximum (raw scores) the exponentials are taken against
+                float l = 0.0f;           // sum of the exponentials, in units of exp2(m_ref * scale_log2)
+                const float sl = kSoftcap ? a.softcap_post : a.scale_log2;  // log2 units per unit of (transformed) score
+                const uint64_t sl2 = ptx::f2_pack(sl, sl);
+                // one arrival per warp: every lane's accesses are ordered before it by the fence and the warp barrier
+                auto arrive = [&](int which) {
+                    ptx::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(bar(which + x));
+                };
+                // key j of key tile k_begin + u survives for query i iff mask_from <= j <= mask_to
+                int mask_from = 0, mask_to = 0;
+                if (kMasked) key_range_of_query(qi, k_begin * C::kTile, w.band, &mask_from, &mask_to);
+                bool ok = true;
 #pragma unroll 1
-            for (int u = 0; u < n_steps; ++u) {
-                if (!(ok = warp_wait<false>(bar(kFwdSFull + x), (c0 + u) & 1, abort_flag))) break;
-                ptx::tc_fence_after();
-                const bool diagonal = kMasked && __any_sync(0xffffffffu, mask_from > 0 || mask_to < C::kTile - 1);
-                // ---- the whole score row of this tile goes to registers in one round trip
-                uint32_t r[4][32];
+                for (int u = 0; u < n_steps; ++u) {
+                    if (!(ok = warp_wait<false>(bar(kFwdSFull + x), (c0 + u) & 1, abort_flag))) break;
+                    ptx::tc_fence_after();
+                    const bool diagonal = kMasked && __any_sync(0xffffffffu, mask_from > 0 || mask_to < C::kTile - 1);
+                    // ---- the whole score row of this tile goes to registers in one round trip
+                    uint32_t r[4][32];
 #pragma unroll
-                for (int c = 0; c < 4; ++c) ptx::tmem_ld32(s_cols + c * 32, r[c]);
-                // (asked ahead of its use: has P V of the previous key tile completed?)
-                const bool p_free = !C::kOwnP || u == 0 || ptx::mbar_test_wait(bar(kFwdPvDone + x), (c0 + u - 1) & 1);
-                ptx::tmem_ld_wait();
-                if (C::kOwnP) arrive(kFwdSFree);
-                if (kSoftcap) {
-                    // from here on the scores are the tanh, and their scale the cap
-                    const float pre = a.softcap_pre * ptx::kTanhArg;
+                    for (int c = 0; c < 4; ++c) ptx::tmem_ld32(s_cols + c * 32, r[c]);
+                    // (asked ahead of its use: has P V of the previous key tile completed?)
+                    const bool p_free = !C::kOwnP || u == 0 || ptx::mbar_test_wait(bar(kFwdPvDone + x), (c0 + u - 1) & 1);
+                    ptx::tmem_ld_wait();
+                    if (C::kOwnP) arrive(kFwdSFree);
+                    if (kSoftcap) {
+                        // from here on the scores are the tanh, and their scale the cap
+                        const float pre = a.softcap_pre * ptx::kTanhArg;
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+#pragma unroll
+                            for (int e = 0; e < 32; e += 2) {
+                                const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
+                                const float2 t = ptx::f2_unpack(ptx::tanh_mixed<C::kTanhFmaPairs>(ptx::f2_mul(s2, ptx::f2_pack(pre, pre)), e / 2));
+                                r[c][e] = __float_as_uint(t.x);
+                                r[c][e + 1] = __float_as_uint(t.y);
+                            }
+                        }
+                    }
+                    if (diagonal) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) {
+                                const int j = c * 32 + e;
+                                if (j < mask_from || j > mask_to) r[c][e] = 0xff800000u;  // -inf
+                            }
+                        }
+                    }
+                    // four chains of three-input maxima; a NaN among the visible scores makes the maximum NaN
+                    float mx[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) mx[c] = ptx::max_nan(__uint_as_float(r[c][0]), __uint_as_float(r[c][1]));
+#pragma unroll
+                    for (int e = 2; e < 32; e += 2) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) mx[c] = ptx::max3_nan(mx[c], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
+                    }
+                    const float mt = ptx::max_nan(ptx::max3_nan(mx[0], mx[1], mx[2]), mx[3]);
+                    // ---- move the reference maximum only when it is more than 2^8 too small (or NaN)
+                    const bool move = m_ref == -INFINITY ? mt != -INFINITY : !((mt - m_ref) * sl <= C::kRescaleThreshold);
+                    if (__any_sync(0xffffffffu, move)) {
+                        // exp2(-inf) = 0 on the first move
+                        const float alpha = move ? ptx::ex2_approx((m_ref - mt) * sl) : 1.0f;
+                        if (move) m_ref = mt;
+                        // a NaN or +inf score makes l, and by it O and the log-sum-exp, NaN (mt - mt): not every exponential
+                        // of such a row would be NaN (exp2_poly)
+                        l = fmaf(l, alpha, move ? mt - mt : 0.0f);
+                        if (u > 0) {
+                            // O carries the old reference: wait for P V of step u-1, then rescale these 32 rows (16
+                            // columns at a time: the score row is still held in registers)
+                            if (!(ok = warp_wait<false>(bar(kFwdPvDone + x), (c0 + u - 1) & 1, abort_flag))) break;
+                            ptx::tc_fence_after();
+#pragma unroll 1
+                            for (int c = 0; c < D / 16; ++c) {
+                                uint32_t acc[16];
+                                ptx::tmem_ld16(o_cols + c * 16, acc);
+                                ptx::tmem_ld_wait();
+#pragma unroll
+                                for (int e = 0; e < 16; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
+                                ptx::tmem_st16(o_cols + c * 16, acc);
+                            }
+                            ptx::tmem_st_wait();
+                        }
+                    }
+                    // ---- P = exp2((S - m_ref) * scale_log2), written as 16-bit pairs (over S, every column of which
+                    // has been read by now, where P has no columns of its own)
+                    if (C::kOwnP) {
+                        // P of the previous key tile must have been used before it is overwritten
+                        if (!__all_sync(0xffffffffu, p_free) && !(ok = warp_wait<false>(bar(kFwdPvDone + x), (c0 + u - 1) & 1, abort_flag))) break;
+                        ptx::tc_fence_after();
+                    }
+                    const float neg = m_ref == -INFINITY ? 0.0f : -m_ref * sl;
+                    const uint64_t neg2 = ptx::f2_pack(neg, neg);
+                    uint64_t sum2[2] = {0, 0};
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
+                        uint32_t o[16];
 #pragma unroll
                         for (int e = 0; e < 32; e += 2) {
-                            const uint64_t s2 = ptx::f2_pack(__uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
-                            const float2 t = ptx::f2_unpack(ptx::tanh_mixed<C::kTanhFmaPairs>(ptx::f2_mul(s2, ptx::f2_pack(pre, pre)), e / 2));
-                            r[c][e] = __float_as_uint(t.x);
-                            r[c][e + 1] = __float_as_uint(t.y);
+                            const uint64_t x2 = ptx::f2_fma(ptx::f2_pack(__uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1])), sl2, neg2);
+                            float2 pr;
+                            // (the pairs that take the polynomial are spread evenly over the row)
+                            if (((e / 2) * C::kPolyPairs) % 8 + C::kPolyPairs >= 8 && C::kPolyPairs > 0) {
+                                pr = ptx::exp2_poly(x2);
+                            } else {
+                                pr = ptx::f2_unpack(x2);
+                                pr.x = ptx::ex2_approx(pr.x);
+                                pr.y = ptx::ex2_approx(pr.y);
+                            }
+                            sum2[(e / 2) & 1] = ptx::f2_add(sum2[(e / 2) & 1], ptx::f2_pack(pr.x, pr.y));
+                            o[e / 2] = ptx::Pack2<T>::pack(pr.x, pr.y);
+                        }
+                        ptx::tmem_st16(p_cols + c * 16, o);
+                        if (c == 1) {
+                            ptx::tmem_st_wait();
+                            arrive(kFwdPFirst);
                         }
                     }
+                    ptx::tmem_st_wait();
+                    arrive(kFwdPReady);
+                    const float2 sum = ptx::f2_unpack(ptx::f2_add(sum2[0], sum2[1]));
+                    l += sum.x + sum.y;
+                    mask_from -= C::kTile;
+                    mask_to -= C::kTile;
                 }
-                if (diagonal) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) {
-                            const int j = c * 32 + e;
-                            if (j < mask_from || j > mask_to) r[c][e] = 0xff800000u;  // -inf
-                        }
-                    }
-                }
-                // four chains of three-input maxima; a NaN among the visible scores makes the maximum NaN
-                float mx[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) mx[c] = ptx::max_nan(__uint_as_float(r[c][0]), __uint_as_float(r[c][1]));
-#pragma unroll
-                for (int e = 2; e < 32; e += 2) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) mx[c] = ptx::max3_nan(mx[c], __uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1]));
-                }
-                const float mt = ptx::max_nan(ptx::max3_nan(mx[0], mx[1], mx[2]), mx[3]);
-                // ---- move the reference maximum only when it is more than 2^8 too small (or NaN)
-                const bool move = m_ref == -INFINITY ? mt != -INFINITY : !((mt - m_ref) * sl <= C::kRescaleThreshold);
-                if (__any_sync(0xffffffffu, move)) {
-                    // exp2(-inf) = 0 on the first move
-                    const float alpha = move ? ptx::ex2_approx((m_ref - mt) * sl) : 1.0f;
-                    if (move) m_ref = mt;
-                    // a NaN or +inf score makes l, and by it O and the log-sum-exp, NaN (mt - mt): not every exponential
-                    // of such a row would be NaN (exp2_poly)
-                    l = fmaf(l, alpha, move ? mt - mt : 0.0f);
-                    if (u > 0) {
-                        // O carries the old reference: wait for P V of step u-1, then rescale these 32 rows (16
-                        // columns at a time: the score row is still held in registers)
-                        if (!(ok = warp_wait<false>(bar(kFwdPvDone + x), (c0 + u - 1) & 1, abort_flag))) break;
-                        ptx::tc_fence_after();
-#pragma unroll 1
-                        for (int c = 0; c < D / 16; ++c) {
-                            uint32_t acc[16];
-                            ptx::tmem_ld16(o_cols + c * 16, acc);
-                            ptx::tmem_ld_wait();
-#pragma unroll
-                            for (int e = 0; e < 16; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
-                            ptx::tmem_st16(o_cols + c * 16, acc);
-                        }
-                        ptx::tmem_st_wait();
-                    }
-                }
-                // ---- P = exp2((S - m_ref) * scale_log2), written as 16-bit pairs (over S, every column of which
-                // has been read by now, where P has no columns of its own)
-                if (C::kOwnP) {
-                    // P of the previous key tile must have been used before it is overwritten
-                    if (!__all_sync(0xffffffffu, p_free) && !(ok = warp_wait<false>(bar(kFwdPvDone + x), (c0 + u - 1) & 1, abort_flag))) break;
+                if constexpr (kSoftcap) w = load_work<FwdWork>(work);  // (what only the output needs is not held in registers before)
+                // (m_ref, not l, says whether the row saw a key: exp2_poly leaves 2^-126 on a masked one)
+                const bool any_key = q_valid && m_ref != -INFINITY;
+                const float inv = any_key ? 1.0f / l : 0.0f;
+                // ln(sum exp(s*scale)) = (m_ref*scale_log2 + log2 l) * ln 2
+                float* lse_dst = a.lse + int64_t(w.b_coord * a.heads_q + w.hq) * a.lse_rows + w.q_base + qi;
+                if (!kPersist && a.splits > 1) {
+                    // This CTA's share of the keys: unnormalised O, fp32, and {m in log2 units, l} go to shared
+                    // memory, over the K / V rings, for the merge below.
+                    if (ok && w.n_iter > 0) ok = warp_wait(bar(kFwdAllDone), 0, abort_flag);
                     ptx::tc_fence_after();
-                }
-                const float neg = m_ref == -INFINITY ? 0.0f : -m_ref * sl;
-                const uint64_t neg2 = ptx::f2_pack(neg, neg);
-                uint64_t sum2[2] = {0, 0};
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    uint32_t o[16];
-#pragma unroll
-                    for (int e = 0; e < 32; e += 2) {
-                        const uint64_t x2 = ptx::f2_fma(ptx::f2_pack(__uint_as_float(r[c][e]), __uint_as_float(r[c][e + 1])), sl2, neg2);
-                        float2 pr;
-                        // (the pairs that take the polynomial are spread evenly over the row)
-                        if (((e / 2) * C::kPolyPairs) % 8 + C::kPolyPairs >= 8 && C::kPolyPairs > 0) {
-                            pr = ptx::exp2_poly(x2);
-                        } else {
-                            pr = ptx::f2_unpack(x2);
-                            pr.x = ptx::ex2_approx(pr.x);
-                            pr.y = ptx::ex2_approx(pr.y);
-                        }
-                        sum2[(e / 2) & 1] = ptx::f2_add(sum2[(e / 2) & 1], ptx::f2_pack(pr.x, pr.y));
-                        o[e / 2] = ptx::Pack2<T>::pack(pr.x, pr.y);
-                    }
-                    ptx::tmem_st16(p_cols + c * 16, o);
-                    if (c == 1) {
-                        ptx::tmem_st_wait();
-                        arrive(kFwdPFirst);
-                    }
-                }
-                ptx::tmem_st_wait();
-                arrive(kFwdPReady);
-                const float2 sum = ptx::f2_unpack(ptx::f2_add(sum2[0], sum2[1]));
-                l += sum.x + sum.y;
-                mask_from -= C::kTile;
-                mask_to -= C::kTile;
-            }
-            if constexpr (kSoftcap) w = load_work<FwdWork>(work);  // (what only the output needs is not held in registers before)
-            // (m_ref, not l, says whether the row saw a key: exp2_poly leaves 2^-126 on a masked one)
-            const bool any_key = q_valid && m_ref != -INFINITY;
-            const float inv = any_key ? 1.0f / l : 0.0f;
-            // ln(sum exp(s*scale)) = (m_ref*scale_log2 + log2 l) * ln 2
-            float* lse_dst = a.lse + int64_t(w.b_coord * a.heads_q + w.hq) * a.lse_rows + w.q_base + qi;
-            if (!kPersist && a.splits > 1) {
-                // This CTA's share of the keys: unnormalised O, fp32, and {m in log2 units, l} go to shared
-                // memory, over the K / V rings, for the merge below.
-                if (ok && w.n_iter > 0) ok = warp_wait(bar(kFwdAllDone), 0, abort_flag);
-                ptx::tc_fence_after();
-                *reinterpret_cast<float2*>(smem + C::kOffStats + (x * 128 + i) * 8) =
-                    make_float2(any_key ? m_ref * sl : -INFINITY, any_key ? l : 0.0f);
-                const uint32_t row_addr = sbase + C::kOffMerge + (x * 128 + i) * (D * 4);
+                    *reinterpret_cast<float2*>(smem + C::kOffStats + (x * 128 + i) * 8) =
+                        make_float2(any_key ? m_ref * sl : -INFINITY, any_key ? l : 0.0f);
+                    const uint32_t row_addr = sbase + C::kOffMerge + (x * 128 + i) * (D * 4);
 #pragma unroll 1
-                for (int c = 0; c < D / 32; ++c) {
-                    uint32_t r[32];
-                    if (n_steps > 0) {
-                        ptx::tmem_ld32(o_cols + c * 32, r);
-                        ptx::tmem_ld_wait();
-                    }
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const int chunk = (c * 8 + e) ^ (i & 7);  // (rows are 256 or 512 bytes apart: spread over the banks)
-                        const bool keep = n_steps > 0 && any_key;
-                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
-                                     ::"r"(row_addr + chunk * 16), "r"(keep ? r[4 * e] : 0u), "r"(keep ? r[4 * e + 1] : 0u),
-                                       "r"(keep ? r[4 * e + 2] : 0u), "r"(keep ? r[4 * e + 3] : 0u) : "memory");
-                    }
-                }
-            } else {
-            if (ok && n_steps > 0) ok = warp_wait(bar(kFwdPvDone + x), (c0 + n_steps - 1) & 1, abort_flag);
-            T* dst = reinterpret_cast<T*>(a.out) + w.b_coord * a.o_strides.batch + w.hq * a.o_strides.head +
-                     int64_t(w.q_base + qi) * a.o_strides.row;
-            if (ok && ((q_valid && n_steps == 0) || (!q_valid && qi < w.slot_q))) {
-                // no visible key at all, or a row behind the used length: O = 0, lse = -inf
-                uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-                for (int e = 0; e < D / 8; ++e) d4[e] = make_uint4(0u, 0u, 0u, 0u);
-                *lse_dst = -INFINITY;
-            }
-            __syncwarp();
-            if (ok && n_steps > 0) {
-                // (tensor-memory loads are warp-wide: every lane runs them, only the stores of query rows
-                // past the end of the sequence are skipped)
-                ptx::tc_fence_after();
-                if (q_valid) *lse_dst = any_key ? (m_ref * sl + __log2f(l)) * 0.69314718055994531f : -INFINITY;
-                if (a.staged_store) {
-                    // through shared memory (the Q tile is dead: its last S completed before this O) and the copy
-                    // engine: whole lines instead of 16 bytes of 32 rows per instruction, rows past the end clipped
-                    const int w4 = warp & 3;
-                    const uint32_t stage = kPersist ? sbase + C::kOffOut + (x * 4 + w4) * 4096 : sbase + C::kOffQ + x * C::kOperandBytes + w4 * (C::kBoxes * 4096);
-                    const bool in_range = qt * C::kTile + w4 * 32 < w.slot_q;
-                    const float scale_row = q_valid ? inv : 0.0f;  // (rows behind a used length hold zeros)
-#pragma unroll
                     for (int c = 0; c < D / 32; ++c) {
                         uint32_t r[32];
-                        ptx::tmem_ld32(o_cols + c * 32, r);
-                        ptx::tmem_ld_wait();
-                        const uint32_t row_addr = stage + (kPersist ? 0 : c >> 1) * 4096 + lane * 128;
-                        if (kPersist && (c & 1) == 0) {  // (its 64 columns before have been read)
-                            if (lane == 0) ptx::bulk_wait_group_read<0>();
-                            __syncwarp();
+                        if (n_steps > 0) {
+                            ptx::tmem_ld32(o_cols + c * 32, r);
+                            ptx::tmem_ld_wait();
                         }
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            uint32_t o[4];
-#pragma unroll
-                            for (int h = 0; h < 4; ++h) {
-                                const float lo = __uint_as_float(r[8 * e + 2 * h]) * scale_row, hi = __uint_as_float(r[8 * e + 2 * h + 1]) * scale_row;
-                                o[h] = scale_row != 0.0f ? ptx::Pack2<T>::pack(lo, hi) : 0u;
-                            }
-                            const int chunk = ((c & 1) * 4 + e) ^ (lane & 7);
+                        for (int e = 0; e < 8; ++e) {
+                            const int chunk = (c * 8 + e) ^ (i & 7);  // (rows are 256 or 512 bytes apart: spread over the banks)
+                            const bool keep = n_steps > 0 && any_key;
                             asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
-                                         ::"r"(row_addr + (chunk << 4)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+                                         ::"r"(row_addr + chunk * 16), "r"(keep ? r[4 * e] : 0u), "r"(keep ? r[4 * e + 1] : 0u),
+                                           "r"(keep ? r[4 * e + 2] : 0u), "r"(keep ? r[4 * e + 3] : 0u) : "memory");
                         }
-                        if (kPersist && (c & 1) == 1) {
-                            ptx::fence_proxy_async_smem();
-                            __syncwarp();
-                            if (lane == 0 && in_range) {
-                                ptx::tma_store_4d(&tm_o, stage, (c >> 1) * 64, qt * C::kTile + w4 * 32, w.hq, w.b);
-                                ptx::bulk_commit_group();
-                            }
-                        }
-                    }
-                    if (!kPersist) {
-                    ptx::fence_proxy_async_smem();
-                    __syncwarp();
-                    if (lane == 0 && in_range) {
-#pragma unroll
-                        for (int bx = 0; bx < C::kBoxes; ++bx)
-                            ptx::tma_store_4d(&tm_o, stage + bx * 4096, bx * 64, qt * C::kTile + w4 * 32, w.hq, w.b);
-                        ptx::bulk_commit_group();
-                        ptx::bulk_wait_group_read<0>();
-                    }
                     }
                 } else {
+                    if (ok && n_steps > 0) ok = warp_wait(bar(kFwdPvDone + x), (c0 + n_steps - 1) & 1, abort_flag);
+                    T* dst = reinterpret_cast<T*>(a.out) + w.b_coord * a.o_strides.batch + w.hq * a.o_strides.head +
+                             int64_t(w.q_base + qi) * a.o_strides.row;
+                    if (ok && ((q_valid && n_steps == 0) || (!q_valid && qi < w.slot_q))) {
+                        // no visible key at all, or a row behind the used length: O = 0, lse = -inf
+                        uint4* d4 = reinterpret_cast<uint4*>(dst);
 #pragma unroll
-                for (int c = 0; c < D / 32; ++c) {
-                    uint32_t r[32];
-                    ptx::tmem_ld32(o_cols + c * 32, r);
-                    ptx::tmem_ld_wait();
-                    if (q_valid) {
-                        uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
+                        for (int e = 0; e < D / 8; ++e) d4[e] = make_uint4(0u, 0u, 0u, 0u);
+                        *lse_dst = -INFINITY;
+                    }
+                    __syncwarp();
+                    if (ok && n_steps > 0) {
+                        // (tensor-memory loads are warp-wide: every lane runs them, only the stores of query rows
+                        // past the end of the sequence are skipped)
+                        ptx::tc_fence_after();
+                        if (q_valid) *lse_dst = any_key ? (m_ref * sl + __log2f(l)) * 0.69314718055994531f : -INFINITY;
+                        if (a.staged_store) {
+                            // through shared memory (the Q tile is dead: its last S completed before this O) and the copy
+                            // engine: whole lines instead of 16 bytes of 32 rows per instruction, rows past the end clipped
+                            const int w4 = warp & 3;
+                            const uint32_t stage = kPersist ? sbase + C::kOffOut + (x * 4 + w4) * 4096 : sbase + C::kOffQ + x * C::kOperandBytes + w4 * (C::kBoxes * 4096);
+                            const bool in_range = qt * C::kTile + w4 * 32 < w.slot_q;
+                            const float scale_row = q_valid ? inv : 0.0f;  // (rows behind a used length hold zeros)
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            uint4 o;
-                            o.x = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 0]) * inv, __uint_as_float(r[8 * e + 1]) * inv);
-                            o.y = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 2]) * inv, __uint_as_float(r[8 * e + 3]) * inv);
-                            o.z = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 4]) * inv, __uint_as_float(r[8 * e + 5]) * inv);
-                            o.w = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 6]) * inv, __uint_as_float(r[8 * e + 7]) * inv);
-                            d4[e] = o;
+                            for (int c = 0; c < D / 32; ++c) {
+                                uint32_t r[32];
+                                ptx::tmem_ld32(o_cols + c * 32, r);
+                                ptx::tmem_ld_wait();
+                                const uint32_t row_addr = stage + (kPersist ? 0 : c >> 1) * 4096 + lane * 128;
+                                if (kPersist && (c & 1) == 0) {  // (its 64 columns before have been read)
+                                    if (lane == 0) ptx::bulk_wait_group_read<0>();
+                                    __syncwarp();
+                                }
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    uint32_t o[4];
+#pragma unroll
+                                    for (int h = 0; h < 4; ++h) {
+                                        const float lo = __uint_as_float(r[8 * e + 2 * h]) * scale_row, hi = __uint_as_float(r[8 * e + 2 * h + 1]) * scale_row;
+                                        o[h] = scale_row != 0.0f ? ptx::Pack2<T>::pack(lo, hi) : 0u;
+                                    }
+                                    const int chunk = ((c & 1) * 4 + e) ^ (lane & 7);
+                                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                                                 ::"r"(row_addr + (chunk << 4)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+                                }
+                                if (kPersist && (c & 1) == 1) {
+                                    ptx::fence_proxy_async_smem();
+                                    __syncwarp();
+                                    if (lane == 0 && in_range) {
+                                        ptx::tma_store_4d(&tm_o, stage, (c >> 1) * 64, qt * C::kTile + w4 * 32, w.hq, w.b);
+                                        ptx::bulk_commit_group();
+                                    }
+                                }
+                            }
+                            if (!kPersist) {
+                                ptx::fence_proxy_async_smem();
+                                __syncwarp();
+                                if (lane == 0 && in_range) {
+#pragma unroll
+                                    for (int bx = 0; bx < C::kBoxes; ++bx)
+                                        ptx::tma_store_4d(&tm_o, stage + bx * 4096, bx * 64, qt * C::kTile + w4 * 32, w.hq, w.b);
+                                    ptx::bulk_commit_group();
+                                    ptx::bulk_wait_group_read<0>();
+                                }
+                            }
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < D / 32; ++c) {
+                                uint32_t r[32];
+                                ptx::tmem_ld32(o_cols + c * 32, r);
+                                ptx::tmem_ld_wait();
+                                if (q_valid) {
+                                    uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
+#pragma unroll
+                                    for (int e = 0; e < 4; ++e) {
+                                        uint4 o;
+                                        o.x = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 0]) * inv, __uint_as_float(r[8 * e + 1]) * inv);
+                                        o.y = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 2]) * inv, __uint_as_float(r[8 * e + 3]) * inv);
+                                        o.z = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 4]) * inv, __uint_as_float(r[8 * e + 5]) * inv);
+                                        o.w = ptx::Pack2<T>::pack(__uint_as_float(r[8 * e + 6]) * inv, __uint_as_float(r[8 * e + 7]) * inv);
+                                        d4[e] = o;
+                                    }
+                                }
+                                __syncwarp();  // reconverge before the next warp-wide load
+                            }
                         }
                     }
-                    __syncwarp();  // reconverge before the next warp-wide load
                 }
+                if (kPersist) {
+                    __syncwarp();
+                    if (!ok) break;
+                    c0 += max(0, n_steps);
                 }
-            }
-            }
-            if (kPersist) {
-                __syncwarp();
-                if (!ok) break;
-                c0 += max(0, n_steps);
-            }
-            if (!kPersist && a.splits > 1) {
-                // ---- merge of the cluster's shares: every CTA finishes 256 / splits of the w.pair's rows, reading
-                // the partial outputs of all peers through distributed shared memory
-                __syncwarp();
-                ptx::cluster_sync();
-                if (a.splits == 2) fwd_merge<T, D, 2>(a, w, sbase);
-                else if (a.splits == 4) fwd_merge<T, D, 4>(a, w, sbase);
-                else fwd_merge<T, D, 8>(a, w, sbase);
-                __syncwarp();
-                ptx::cluster_sync();  // the peers read this CTA's shared memory until here
-            }
-            more = next_tile(n, &w);
+                if (!kPersist && a.splits > 1) {
+                    // ---- merge of the cluster's shares: every CTA finishes 256 / splits of the pair's rows, reading
+                    // the partial outputs of all peers through distributed shared memory
+                    __syncwarp();
+                    ptx::cluster_sync();
+                    if (a.splits == 2) fwd_merge<T, D, 2>(a, w, sbase);
+                    else if (a.splits == 4) fwd_merge<T, D, 4>(a, w, sbase);
+                    else fwd_merge<T, D, 8>(a, w, sbase);
+                    __syncwarp();
+                    ptx::cluster_sync();  // the peers read this CTA's shared memory until here
+                }
+                more = next_tile(n, &w);
             }
             if (kPersist && lane == 0) ptx::bulk_wait_group_read<0>();  // (shared memory is not given back before)
         }

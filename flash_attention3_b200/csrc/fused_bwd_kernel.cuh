@@ -97,9 +97,11 @@ __device__ __forceinline__ long long trace_globaltimer() {
 }
 #define TRACE(role, ev) do { if ((threadIdx.x & 31) == 0 && blockIdx.x < kTraceCtas && (ev) < kTraceEvents) g_trace[blockIdx.x][role][ev] = clock64(); } while (0)
 #define TRACE_GT(role, ev) do { if ((threadIdx.x & 31) == 0 && blockIdx.x < kTraceCtas) g_trace[blockIdx.x][role][ev] = trace_globaltimer(); } while (0)
+#define TRACE_VALUE(role, ev, v) do { if ((threadIdx.x & 31) == 0 && blockIdx.x < kTraceCtas) g_trace[blockIdx.x][role][ev] = (v); } while (0)
 #else
 #define TRACE(role, ev) do {} while (0)
 #define TRACE_GT(role, ev) do {} while (0)
+#define TRACE_VALUE(role, ev, v) do {} while (0)
 #endif
 
 struct FusedArgs {
@@ -713,6 +715,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                 g0 += n_steps;
                 next = next_tile(n, &w);
             }
+            TRACE_VALUE(1, 63, n);  // tiles of this CTA (every other stamp but the drain's last and the CTA's end is of the first)
         } else if (warp == 2) {
             // ============================================== row statistics
             // One warp fetches the statistics of the next step's 128 query rows while the math warps work and
@@ -942,7 +945,6 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                     if (traced) TRACE(2, 4 + 8 * t + 4);
                     // (the dS buffer is free: dP was issued behind dK and dQ of the step before, the readers of its dS,
                     // and the barrier just passed completes only when every MMA issued before it has)
-                    if (traced) TRACE(2, 4 + 8 * t + 5);
                     ptx::tc_fence_after();
                     const uint32_t ds_row = sbase + C::kOffDS + half * C::kBoxBytes + j * 128;
                     auto ds_chunk = [&](int c, const uint32_t* r) {

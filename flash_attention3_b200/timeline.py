@@ -8,7 +8,8 @@ GEMM kernel then stamps clock64() at the hand-offs of every role of every CTA (s
 MMA group, both softmax phases, the drain, the epilogue) and the two row-wise kernels stamp their
 first start and last end with %globaltimer.  This module runs three warm-up calls and one stamped
 call (L2 flushed before each, as in bench.py) and prints medians / minima / maxima over the CTAs.
-The stamps cost a few hundred cycles per CTA: read the split of the time, not the total.
+The stamps cost a few hundred cycles per CTA: read the split of the time, not the total.  Where CTAs take over tiles of CTAs that
+have not started, the stamps are those of a CTA's first tile, but for the lines that say otherwise.
 """
 from __future__ import annotations
 
@@ -99,7 +100,8 @@ def main():
     print(f"== {label}: call {e0.elapsed_time(e1)*1e3:.1f} us (CUDA events)")
     lib.shaobo_fa3_b200_trace_read(buf.ctypes.data, rw.ctypes.data)
     ctas = [c for c in range(N) if buf[c, 0, 0] != 0]
-    print("CTAs traced:", len(ctas))
+    tiles = sorted(int(buf[c, 1, 63]) for c in ctas)
+    print(f"CTAs traced: {len(ctas)}, tiles per CTA: {tiles[0]} to {tiles[-1]}, together {sum(tiles)}")
     gt0 = min(buf[c, 0, 1] for c in ctas)
     gt_end = max(buf[c, 0, 62] for c in ctas)
     print(f"fused kernel: first CTA start .. last CTA end = {(gt_end-gt0)/1e3:.2f} us (globaltimer)")
@@ -138,12 +140,9 @@ def main():
     stat("softmax: first dP seen", [rel(c, 2, 4 + 4) for c in ctas])
     stat("softmax: first dS written", [rel(c, 2, 4 + 6) for c in ctas])
     stat("drain: first dQ seen", [rel(c, 3, 4 + 0) for c in ctas])
-    print("-- top of step 3, softmax warp 4 (first warpgroup: row statistics bookkeeping)")
+    print("-- top of step 3, softmax warp 4")
     stat("dS(2) handed over -> loop top", [diff(c, 2, 0, 2, 4 + 8 * 2 + 7) for c in ctas])
-    stat("tile coordinates of the step", [diff(c, 2, 1, 2, 0) for c in ctas])
-    stat("statistics published", [diff(c, 2, 2, 2, 1) for c in ctas])
-    stat("next statistics requested", [diff(c, 2, 3, 2, 2) for c in ctas])
-    stat("statistics barrier passed", [diff(c, 2, 4 + 8 * 3 + 0, 2, 3) for c in ctas])
+    stat("loop top -> statistics and S there", [diff(c, 2, 4 + 8 * 3 + 1, 2, 0) for c in ctas])
     print("-- per step (clk), softmax warp 4")
     for t in range(0, 6):
         tb = 4 + 8 * t
@@ -152,13 +151,11 @@ def main():
         print(f" step {t}")
         if t > 0:
             stat("  period (dS written(t) - dS written(t-1))", [diff(c, 2, tb + 6, 2, tb - 8 + 6) for c in ctas])
-            stat("  wait: stats", [diff(c, 2, tb + 0, 2, tb - 8 + 7) for c in ctas])
-        stat("  wait: S full after stats", [diff(c, 2, tb + 1, 2, tb + 0) for c in ctas])
+            stat("  dS handed over -> statistics and S there", [diff(c, 2, tb + 1, 2, tb - 8 + 7) for c in ctas])
         stat("  phase A (ld, exp2, P store issued)", [diff(c, 2, tb + 2, 2, tb + 1) for c in ctas])
         stat("  P store wait + arrive", [diff(c, 2, tb + 3, 2, tb + 2) for c in ctas])
         stat("  wait: dP full", [diff(c, 2, tb + 4, 2, tb + 3) for c in ctas])
-        stat("  wait: dS buffer free", [diff(c, 2, tb + 5, 2, tb + 4) for c in ctas])
-        stat("  phase B (ld, dS, smem store)", [diff(c, 2, tb + 6, 2, tb + 5) for c in ctas])
+        stat("  phase B (ld, dS, smem store)", [diff(c, 2, tb + 6, 2, tb + 4) for c in ctas])
     print("-- per step (clk), MMA warp")
     for t in range(0, 6):
         tb = 8 + 8 * t
@@ -184,8 +181,8 @@ def main():
     stat("MMA warp: last commit issued (from CTA start)", [rel(c, 1, 62) for c in ctas])
     stat("softmax: all MMAs done (dK/dV complete), from CTA start", [rel(c, 2, 60) for c in ctas])
     stat("softmax: epilogue (dK/dV written) duration", [diff(c, 2, 61, 2, 60) for c in ctas])
-    stat("drain: all reduce-adds complete, from CTA start", [rel(c, 3, 59) for c in ctas])
-    stat("CTA end (after teardown), from CTA start", [rel(c, 0, 63) for c in ctas])
+    stat("drain: all reduce-adds complete (all tiles), from CTA start", [rel(c, 3, 59) for c in ctas])
+    stat("CTA end (all tiles, after teardown), from CTA start", [rel(c, 0, 63) for c in ctas])
     nsteps = []
     for c in ctas:
         n = 0

@@ -218,7 +218,7 @@ constexpr long long kMostStepsTakenOver = 1 << 16;
 // Whether the CTAs of the dK/dV and five-GEMM kernels take over key tiles of CTAs that have not started: where there are more tiles than
 // SMs.  us per call, one CTA per tile and this:
 // full, 80 heads x 512, D=128 60.3 and 55.2; 32 x 512 x B=8, D=64 101 and 91; 16 x 1024 x B=8, D=64 144 and 139; causal, 40 x 512, D=128
-// 27.8 and 25.8; 16 x 1000 x B=4 91.5 and 85; 8 x 300 x B=32 84.3 and 78; D=64, 16 x 2048 x B=2 81.4 and 76; 8 x 4096 65.2 and 65.1; 176 tiles (1111
+// 27.8 and 25.8; 16 x 1000 x B=4 91.5 and 85; 32 x 300 x B=8 84.3 and 78; D=64, 16 x 2048 x B=2 81.4 and 76; 8 x 4096 65.2 and 65.1; 176 tiles (1111
 // queries x 1300 keys) 46.4 and 46.6; reproducible gradients (dK/dV kernel), causal, 32 x 300 x B=8, D=128 108 and 93.6; 16 x 2048 x B=2 156 and
 // 154.  (Long shapes run under the power limit: the same within its spread.)  Packed, where blocks without rows are passed over by
 // the warp that works tiles out instead of starting: 9 x 4096, 16 heads, D=128 832 and 794; 16 heads, 2048 and 20 x 128, D=64 causal 116 and

@@ -450,6 +450,7 @@ fused_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
                  const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                  const __grid_constant__ CUtensorMap tm_dqacc, const __grid_constant__ FusedArgs a) {
     using C = FusedCfg<D, kSoftcap>;
+    static_assert(!kSoftcap || !kPersist, "with capped scores the epilogue reads the work of the first tile again");
     constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = ptx::smem_u32(smem);

@@ -113,7 +113,7 @@ struct FwdCfg {
     // us per call of B=4, H=16, S=4096 full for 0, 1, 2, 3 of 8: D=64 348, 338, 355, 371; D=128 486, 492, 490, 500.
     static constexpr int kPolyPairs = D == 64 ? 1 : 0;
     // ... and of every 8 pairs of tanh of capped scores (tanh_mixed): us of the forwards named there for 2, 4, 5, 8 of 8: 84.5, 81,
-    // 80, 87; 247, 227, 228, 259.  (6 of 8 spill at D=128.)
+    // 80, 87; 247, 227, 228, 259 (before the loop was compiled as uniform: 78.5 and 222 now).  6 of 8 spill at D=128.
     static constexpr int kTanhFmaPairs = 5;
     // setmaxnreg split: the kernel starts with 168 registers per thread (384 threads); the producer /
     // MMA warpgroup gives most of its share to the two softmax warpgroups, which hold a whole score
@@ -299,6 +299,7 @@ fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUt
            const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o,
            const __grid_constant__ FwdArgs a) {
     using C = FwdCfg<D>;
+    static_assert(!kSoftcap || !kPersist, "with capped scores the output reads the work of the first tile again");
     constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t sbase = ptx::smem_u32(smem);

@@ -477,8 +477,8 @@ __device__ __forceinline__ uint64_t tanh_pair_fma(uint64_t x_arg2) {
 // tanh of the `pair`-th pair of values of a thread: of every 8 pairs kFmaPairs take the second form.  The first keeps the
 // special-function unit busy for 32 cycles (the exponential of the softmax for 16 more), the second for 16 and the FMA pipe for
 // 20; a mix keeps both busy.  Which form a value takes depends on its place alone, and the time not on the scores.
-// us, all of the first form and so: B=1, Hq=16, Hkv=8, S=4096, D=128, window 1024, cap 30 forward 89.7 and 80.0, gradients 159 and 140,
-// reproducible 204 and 178; B=4, 16 x 2048 full, D=64, cap 50 262 and 228, 398 and 328, 684 and 570 (with P (1 - tanh^2) handed to the dS
+// us, all of the first form and so: B=1, Hq=16, Hkv=8, S=4096, D=128, window 1024, cap 30 forward 89.8 and 78.5, gradients 157 and 138,
+// reproducible 204 and 177; B=4, 16 x 2048 full, D=64, cap 50 262 and 222, 397 and 327, 684 and 569 (with P (1 - tanh^2) handed to the dS
 // phase instead of taken from log2 of P).  A polynomial on the FMA pipe alone where all of a warp's 32 x 32 scores are below
 // the cap, and both forms where some are not, measured 76, 134, 178 and 232, 311, 537 without such scores, but 114, 199, 240 and 334,
 // 491, 808 with one in a thousand above the cap, and 111, 171, 228 and 329, 432, 738 with four in ten.

@@ -129,3 +129,65 @@ def test_streams_and_graphs(d, causal):
     torch.cuda.synchronize()
     for got in (*results, replayed):
         assert all(torch.equal(a, b) for a, b in zip(got, alone))
+
+
+# (rows of the slot, rows used) of queries and keys
+USED_PACKED = [((384, 0), (384, 384)), ((130, 130), (260, 200)), ((5, 5), (7, 0)), ((256, 100), (128, 128)), ((300, 300), (300, 150)),
+               ((64, 64), (500, 333)), ((384, 384), (384, 77)), ((130, 1), (260, 260)), ((5, 0), (7, 7)), ((256, 256), (128, 100)),
+               ((300, 17), (300, 300)), ((64, 60), (500, 64))]
+USED_PACKED_HEADS = (24, 12)
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_used_lengths_of_packed_sequences(d):
+    """The same with the entries' slots laid end to end (C ABI)."""
+    import ctypes
+    from flash_attention3_b200 import capi
+    from oracle import golden
+    from tests.helpers import dev, host, poison
+    (hq, hkv), scale, lib = USED_PACKED_HEADS, 1.0 / float(np.sqrt(d)), capi.load()
+    slots = [np.concatenate([[0], np.cumsum([e[i][0] for e in USED_PACKED])]).astype(np.int32) for i in (0, 1)]
+    total_q, total_k = int(slots[0][-1]), int(slots[1][-1])
+    q, k, v, do = (x[0] for x in golden.seeded_inputs(77, 1, hq, hkv, total_q, d, "bf16", sk=total_k))
+    rows_first = lambda x: dev(np.ascontiguousarray(x.transpose(1, 0, 2)), "bf16")
+    tq, tk, tv, tdo = (rows_first(x) for x in (q, k, v, do))
+    ints = lambda x: torch.tensor(np.asarray(x), dtype=torch.int32, device="cuda")
+    cu, used = [ints(s) for s in slots], [ints([e[i][1] for e in USED_PACKED]) for i in (0, 1)]
+    longest = [max(e[i][0] for e in USED_PACKED) for i in (0, 1)]
+    params = capi.new_params(batch=len(USED_PACKED), num_heads_q=hq, num_heads_kv=hkv, head_dim_qk=d, head_dim_v=d, causal=1,
+                             dtype=capi.DTYPE_BF16, cu_seqlens_q=cu[0].data_ptr(), cu_seqlens_k=cu[1].data_ptr(), total_q=total_q,
+                             total_k=total_k, seqlen_q=longest[0], seqlen_k=longest[1], max_seqlen_q=longest[0],
+                             max_seqlen_k=longest[1], seqused_q=used[0].data_ptr(), seqused_k=used[1].data_ptr(), sync_after_launch=1)
+    vp = lambda t: ctypes.c_void_p(t.data_ptr())
+    out, lse = poison(tq.shape, tq.dtype), poison((hq, total_q), torch.float32)
+    assert lib.shaobo_fa3_b200_fwd(vp(tq), vp(tk), vp(tv), vp(out), vp(lse), ctypes.byref(params)) == capi.STATUS_SUCCESS
+    results = []
+    for deterministic in (0, 1):
+        params.deterministic = deterministic
+        need = lib.shaobo_fa3_bwd_v2_workspace_bytes(ctypes.byref(params))
+        workspace = torch.full((need,), 0xFF, dtype=torch.uint8, device="cuda")
+        params.workspace, params.workspace_bytes = workspace.data_ptr(), need
+        grads, delta = [poison(t.shape, t.dtype) for t in (tq, tk, tv)], poison(lse.shape, torch.float32)
+        torch.cuda.synchronize()
+        assert lib.shaobo_fa3_bwd_v2(vp(tdo), vp(tq), vp(tk), vp(tv), vp(out), vp(lse), *map(vp, grads), vp(delta),
+                                     ctypes.byref(params)) == capi.STATUS_SUCCESS
+        torch.cuda.synchronize()
+        assert lib.shaobo_fa3_b200_device_error(1) == 0
+        results.append([host(g).transpose(1, 0, 2) for g in grads])
+    out, lse = host(out).transpose(1, 0, 2), host(lse)
+    for i, ((slot_q, uq), (slot_k, uk)) in enumerate(USED_PACKED):
+        q0, k0 = slots[0][i], slots[1][i]
+        assert (out[:, q0 + uq:q0 + slot_q] == 0).all() and np.isneginf(lse[:, q0 + uq:q0 + slot_q]).all(), (i, "forward")
+        ref = None if uq == 0 or uk == 0 else golden.backward(q[None, :, q0:q0 + uq], k[None, :, k0:k0 + uk], v[None, :, k0:k0 + uk],
+                                                              do[None, :, q0:q0 + uq], True, scale, "bf16")
+        if ref is None:
+            assert (out[:, q0:q0 + slot_q] == 0).all() and np.isneginf(lse[:, q0:q0 + slot_q]).all(), i
+        else:
+            assert golden.check_gradient(out[None, :, q0:q0 + uq], ref["out"], "bf16")["pass"], (i, "out")
+        for grads in results:
+            for name, g, first, n, slot in zip(("dq", "dk", "dv"), grads, (q0, k0, k0), (uq, uk, uk), (slot_q, slot_k, slot_k)):
+                assert (g[:, first + n:first + slot] == 0).all(), (i, name, "behind")
+                if ref is None:
+                    assert (g[:, first:first + slot] == 0).all(), (i, name)
+                else:
+                    assert golden.check_gradient(g[None, :, first:first + n], ref[name], "bf16")["pass"], (i, name)

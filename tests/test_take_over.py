@@ -90,3 +90,7 @@ def test_gpu_cases_reach_the_form_they_name(lib, plan):
     for b, hq, hkv, s, *_ in backward.USED:
         assert lib.backward(s, s, (s + 127) // 128 * b * hkv, hq // hkv)
         assert lib.forward(s, 1, (s + 255) // 256 * b * hq, hq, b, 0) and lib.clusters(s, s, 1, -1, -1, b * hq) == 1
+    heads, heads_kv = backward.USED_PACKED_HEADS
+    assert packed(lib, heads, [slot for (slot, _), _ in backward.USED_PACKED], True)
+    longest = max(slot for _, (slot, _) in backward.USED_PACKED)
+    assert lib.backward(384, longest, (longest + 127) // 128 * len(backward.USED_PACKED) * heads_kv, heads // heads_kv)
